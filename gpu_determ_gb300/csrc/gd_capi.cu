@@ -262,6 +262,7 @@ static void destroy_context(Context &c)
     gd_cmatrix_destroy(c.cmatrix);
     c.cmatrix = nullptr;
     pair_tc_free(c);
+    orbit_free(c);
     cudaFree(c.d_cmap);
     cudaFree(c.d_nodes);
     cudaFree(c.d_b);
@@ -369,6 +370,7 @@ static int create_context(Context &c, const gd_grid_spec &spec, int device)
     cudaFree(a_dense);
     if (rc) return rc;
     if ((rc = build_row_groups(c))) return rc;
+    if ((rc = orbit_build(c))) return rc;
     // scatter updates: distinct sign patterns of g whose target lies in the sphere
     int64_t sc = 0;
     for (int sx = 0; sx < d.sx; sx++)

@@ -1,5 +1,8 @@
 // gd_gain.cu -- gain term of the hard-sphere collision integral (sm_103a).
 //
+// Serves the lattices that the orbit kernel (gd_orbit.cu) has no tables for:
+// more than 1024 orbits of in-sphere nodes, or rows past a CTA's shared memory.
+//
 // The reference sums, for each output node i, over partners i1 and
 // post-collision offsets n (collision_integral.cu:75-188, host loop :637-648):
 //   I_i = sum_{i1} sum_n w(|i - i1|, n) P(i + i1, n),
@@ -310,6 +313,7 @@ int gain_bounds_device(Context &c, int nchunks, const int **out)
 
 int run_gain(Context &c, const float *f, int ncells, int ld, float *gain, cudaStream_t st)
 {
+    if (c.orbit) return run_orbit(c, f, ncells, ld, gain, st);
     const Dims &d = c.d;
     int cb = 0, nblk = 0, nchunks = 0;
     size_t smem = 0;

@@ -14,6 +14,7 @@
 namespace gd {
 
 struct PairTc;
+struct OrbitGain;
 
 // Lattice sizes derived from a grid spec.  The "class box" of a parity
 // class is the set of offsets v with 0 <= v_a < n_a and v_a of one parity per
@@ -98,6 +99,7 @@ struct Context {
     int64_t pair_products = 0, contraction_terms = 0, scatter_terms = 0;
     int gain_path = GD_GAIN_PAIR;    // gain algorithm for gd_collision / gd_step
     gd_cmatrix *cmatrix = nullptr;   // collision matrices when gain_path is a GD_GAIN_CMATRIX_*
+    OrbitGain *orbit = nullptr;      // tables of the orbit gain kernel (null: the grid runs gain_pair_kernel)
     PairTc *pair_tc = nullptr;       // per-D weight table when gain_path is GD_GAIN_PAIR_TC
     int gain_cb = 32;                // cells per lane row of the gain kernel (fixed per grid)
     bool gain_cmap_smem = true;      // its box -> compact map in shared memory (else through L1)
@@ -191,6 +193,19 @@ int gain_bounds_device(Context &c, int nchunks, const int **out);
 // gain[node][c] = sum over chunks of part[chunk][node][c], in chunk order
 int reduce_gain_partials(Context &c, const float *part, int nchunks, int cells_pad, int ncells, int ld,
                          float *gain, cudaStream_t st);
+
+// FP32 gain with all eight reflections of a pair sum at once (gd_orbit.cu):
+// tables (built with the context), chunk count and bounds, buffer sizes, and
+// the launch into a caller-provided buffer (packed f, then chunk partials)
+int orbit_build(Context &c);
+void orbit_free(Context &c);
+int orbit_chunks(const Context &c, int ncells);
+void orbit_chunk_bounds(const Context &c, int nchunks, int *bounds);
+size_t orbit_pack_bytes(const Context &c, int ncells);
+size_t orbit_part_bytes(const Context &c, int ncells, int nchunks);
+int launch_orbit(Context &c, const float *f, int ncells, int ld, float *gain, void *buf, int nchunks,
+                 const int *d_bounds, cudaStream_t st);
+int run_orbit(Context &c, const float *f, int ncells, int ld, float *gain, cudaStream_t st);
 
 // pair-product gain with the contraction on the tensor cores (gd_pair_tc.cu)
 int pair_tc_build(Context &c);

@@ -77,6 +77,19 @@ int scratch_address(int dev, void **out)
     return GD_OK;
 }
 
+// The array's address and, in its header, the chunk bounds of this call.
+int noalloc_bounds(Context &c, int nchunks, void (*fill)(const Context &, int, int *), cudaStream_t st, void **base)
+{
+    int rc = scratch_address(c.device, base);
+    if (rc) return rc;
+    ChunkBounds b{};
+    b.n = nchunks;
+    fill(c, nchunks, b.v);
+    write_bounds_kernel<<<1, kMaxChunks + 1, 0, st>>>(b, static_cast<int *>(*base));
+    GD_CUDA(cudaGetLastError());
+    return GD_OK;
+}
+
 }  // namespace
 }  // namespace gd
 
@@ -92,12 +105,14 @@ extern "C" int gd_gain_noalloc(gd_ctx *ctx, const float *f, int ncells, int ld, 
     if (prev != c.device && cudaSetDevice(c.device) != cudaSuccess)
         return set_error(GD_ERR_CUDA, "cudaSetDevice failed");
     int rc = GD_OK;
+    void *base = nullptr;
     do {
+        cudaStream_t st = (cudaStream_t)stream;
+        const size_t room = kNoAllocScratchBytes - kHeaderBytes;
         int cb = 0, nblk = 0, want = 0;
         size_t smem = 0;
         if ((rc = gain_launch_shape(c, ncells, &cb, &smem, &nblk, &want))) break;
         const size_t per_chunk = (size_t)c.d.n_pnt * nblk * cb * sizeof(float);
-        const size_t room = kNoAllocScratchBytes - kHeaderBytes;
         const int fit = (int)std::min<size_t>(room / per_chunk, kMaxChunks);
         if (fit < 1) {
             const size_t max_cells = room / ((size_t)c.d.n_pnt * sizeof(float)) / cb * cb;
@@ -108,21 +123,21 @@ extern "C" int gd_gain_noalloc(gd_ctx *ctx, const float *f, int ncells, int ld, 
                                " cells on this grid) -- split the batch or use gd_collision");
             break;
         }
-        const int nchunks = std::min(want, fit);
-        void *base = nullptr;
-        if ((rc = scratch_address(c.device, &base))) break;
-        int *d_bounds = static_cast<int *>(base);
-        float *part = reinterpret_cast<float *>(static_cast<unsigned char *>(base) + kHeaderBytes);
-        ChunkBounds b{};
-        b.n = nchunks;
-        gain_chunk_bounds(c, nchunks, b.v);
-        cudaStream_t st = (cudaStream_t)stream;
-        write_bounds_kernel<<<1, kMaxChunks + 1, 0, st>>>(b, d_bounds);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) {
-            rc = cuda_error(e, "write_bounds_kernel");
+        if (c.orbit) {
+            // the packed f and the partial sums of as many chunks as fit (one
+            // chunk writes the gain itself, and its packed f fits wherever one
+            // chunk's partial sums do)
+            int nchunks = std::min(orbit_chunks(c, ncells), kMaxChunks);
+            while (nchunks > 1 && orbit_pack_bytes(c, ncells) + orbit_part_bytes(c, ncells, nchunks) > room) nchunks--;
+            if ((rc = noalloc_bounds(c, nchunks, orbit_chunk_bounds, st, &base))) break;
+            rc = launch_orbit(c, f, ncells, ld, gain, static_cast<unsigned char *>(base) + kHeaderBytes, nchunks,
+                              static_cast<const int *>(base), st);
             break;
         }
+        const int nchunks = std::min(want, fit);
+        if ((rc = noalloc_bounds(c, nchunks, gain_chunk_bounds, st, &base))) break;
+        float *part = reinterpret_cast<float *>(static_cast<unsigned char *>(base) + kHeaderBytes);
+        const int *d_bounds = static_cast<const int *>(base);
         rc = launch_gain_pair(c, f, ncells, ld, gain, part, nchunks, d_bounds, cb, smem, st);
     } while (0);
     if (prev >= 0 && prev != c.device) cudaSetDevice(prev);
