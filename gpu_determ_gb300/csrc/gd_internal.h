@@ -56,6 +56,20 @@ struct Scratch {
     size_t bytes = 0;
 };
 
+// Tables of the orbit gain kernel (gd_orbit.cu): the warps' streams of work, per
+// low-octant pair sum, and the node of each row 8 o + e (orbit o of the
+// lattice's reflections, bit a of e: upper half of axis a).
+struct OrbitGain {
+    int cpt = 8, nslot = 0, norb = 0, pcap = 0, mcap = 0, nsteps = 0;
+    size_t smem = 0;
+    std::vector<int> cuts;            // steps between which the walk may be cut (no D continues)
+    std::vector<double> cost_prefix;  // work before each cut
+    int *row_node = nullptr;          // [n_pnt]
+    uint4 *stream = nullptr;
+    int *start = nullptr;  // [step][warp] first chunk
+    std::map<int, int *> bounds_dev;
+};
+
 // Floats of a context's reduction buffer (block maxima of nu', then dt).
 constexpr int kReduceFloats = 2048;
 

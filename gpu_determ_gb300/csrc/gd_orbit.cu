@@ -21,11 +21,15 @@
 //    is read back or written in between, and no two warps share one, so every
 //    sum has a fixed order and results are bitwise reproducible.
 //
-// A CTA takes one tile of CPT cells and one chunk of the steps; a step is as
-// many D as fit the P and C buffers, so that the two barriers of a step are
-// paid for ~1e4 cycles of work.  Contraction works on blocks of four rows of
-// neighbouring |g|, whose shells overlap: one P row is read for four rows
-// (1.2 times the terms, a third of the shared-memory reads).
+// A CTA takes one tile of CPT cells and one chunk of the steps.  f of the tile,
+// the P rows and the C rows of a step sit in shared memory.  A step is as many D
+// as fit these rows, or a part of one D's offsets (by shell |n|, its C rows then
+// accumulate over the parts).  Contraction works on blocks of four rows of
+// neighbouring |g|, whose shells overlap: one P row is read for four rows (1.2
+// times the terms, a third of the shared-memory reads).  What a warp has to do
+// is one linear stream of 512-byte chunks (products, contraction entries,
+// targets, step by step), copied ahead into a ring of shared memory with
+// cp.async, so that no table read waits for L2.
 //
 // Bound: shared-memory and L1 wavefronts (products, contraction and outputs
 // all read one row per operation).  It replaces gain_pair_kernel (gd_gain.cu)
@@ -46,27 +50,46 @@ namespace {
 
 constexpr int kOWarps = 16;
 constexpr int kOThreads = 32 * kOWarps;
-constexpr int kORows = 4;              // rows of a contraction block
-constexpr int kOStage = 1024;          // bytes of a warp's staged target list
-constexpr uint32_t kNoPair = 0xffffffffu;
+constexpr int kORows = 4;            // rows of a contraction block
+constexpr int kOChunk = 512;         // bytes of a stream chunk: one 16-byte copy per lane
+constexpr int kORing = 4 * kOChunk;  // a warp's ring
+constexpr int kOQuads = 6;           // contraction quads (80 bytes) per chunk
+constexpr int kOProd = 31;           // products per warp and step (one chunk, after its header)
+constexpr uint32_t kNoPair = 0xffff7fffu;
 
 struct OrbitArgs {
-    const float *ft;       // [tile][row][CPT]
-    const uint4 *prod;     // per P row up to four pairs t1 | t2 << 16 (kNoPair: none); bit 15 of the
-                           // low half of word a: axis a of D is its own mirror
-    const int4 *steps;     // {first product, products, 0, 0}
-    const int4 *work;      // [step][warp] {first block, end block, first quad of the target list, quads}
-    const int4 *blocks;    // {first entry, entry quads, C byte offset, 0}
-    const uint4 *ent_off;  // P byte offsets of four entries
-    const float4 *ent_w;   // the four rows' weights of one entry
-    const uint2 *targets;  // per (step, warp): a count per slot (bytes, in quads), then 16-bit entries row << 3 | e
-    const int *bounds;     // [chunks + 1] step bounds
+    const float *ft;      // [tile][row][CPT]
+    const uint4 *stream;  // per warp: the chunks of every step
+    const int *start;     // [step][warp] first chunk
+    const int *bounds;    // [chunks + 1] step bounds
     const int *row_node;
-    float *part;           // [chunk][row][cells_pad], or null: write gain
+    float *part;          // [chunk][row][cells_pad], or null: write gain
     float *gain;
     int norb, ns, cells_pad, ncells, ld;
-    int kcap, mcap;
+    int pcap, mcap;
 };
+
+// Two FP32 operations per instruction where a lane holds two cells.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
+{
+    float2 d;
+    asm("{\n\t.reg .b64 x, y, z, w;\n\t"
+        "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+        "fma.rn.f32x2 w, x, y, z;\n\tmov.b64 {%0, %1}, w;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b)
+{
+    float2 d;
+    asm("{\n\t.reg .b64 x, y, w;\n\t"
+        "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+        "add.rn.f32x2 w, x, y;\n\tmov.b64 {%0, %1}, w;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
 
 template <int CPT>
 struct Vec;
@@ -74,143 +97,247 @@ template <>
 struct Vec<8> {
     using T = float2;
     static __device__ __forceinline__ T zero() { return make_float2(0.f, 0.f); }
-    static __device__ __forceinline__ T fma(T a, T b, T c) { return make_float2(__fmaf_rn(a.x, b.x, c.x), __fmaf_rn(a.y, b.y, c.y)); }
-    static __device__ __forceinline__ T fma(float w, T b, T c) { return make_float2(__fmaf_rn(w, b.x, c.x), __fmaf_rn(w, b.y, c.y)); }
-    static __device__ __forceinline__ T add(T a, T b) { return make_float2(a.x + b.x, a.y + b.y); }
+    static __device__ __forceinline__ T mac(T a, T b, T c) { return fma2(a, b, c); }
+    static __device__ __forceinline__ T mac(float w, T b, T c)
+    {
+        return make_float2(__fmaf_rn(w, b.x, c.x), __fmaf_rn(w, b.y, c.y));
+    }
+    static __device__ __forceinline__ T add(T a, T b) { return add2(a, b); }
 };
 template <>
 struct Vec<4> {
     using T = float;
     static __device__ __forceinline__ T zero() { return 0.f; }
-    static __device__ __forceinline__ T fma(T a, T b, T c) { return __fmaf_rn(a, b, c); }
-    static __device__ __forceinline__ T add(T a, T b) { return a + b; }
+    static __device__ __forceinline__ T mac(T a, T b, T c) { return __fmaf_rn(a, b, c); }
+    static __device__ __forceinline__ T add(T a, T b) { return __fadd_rn(a, b); }
 };
+
+template <typename T>
+__device__ __forceinline__ T lds(uint32_t addr);
+template <>
+__device__ __forceinline__ float lds<float>(uint32_t addr)
+{
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+    return v;
+}
+template <>
+__device__ __forceinline__ float2 lds<float2>(uint32_t addr)
+{
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
+    return v;
+}
+template <>
+__device__ __forceinline__ float4 lds<float4>(uint32_t addr)
+{
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
+    return v;
+}
+template <>
+__device__ __forceinline__ uint2 lds<uint2>(uint32_t addr)
+{
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
+    return v;
+}
+template <>
+__device__ __forceinline__ uint4 lds<uint4>(uint32_t addr)
+{
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ void sts(uint32_t addr, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
+__device__ __forceinline__ void sts(uint32_t addr, float2 v)
+{
+    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(v.x), "f"(v.y) : "memory");
+}
 
 template <int CPT, int NSLOT>
 __global__ void __launch_bounds__(kOThreads, 1) orbit_gain_kernel(const __grid_constant__ OrbitArgs a)
 {
     using V = Vec<CPT>;
     using T = typename V::T;
-    constexpr uint32_t kRow = 32 * sizeof(T);        // bytes of a P or C row
-    constexpr int kEntryShift = CPT == 8 ? 5 : 4;    // (row << 3 | e) -> bytes: e selects CPT cells
+    constexpr uint32_t kRow = 32 * sizeof(T);      // bytes of a P or C row
+    constexpr int kShift = CPT == 8 ? 5 : 4;       // (row << 3 | e) -> bytes: e selects CPT cells
     extern __shared__ __align__(1024) unsigned char smem[];
-    unsigned char *P = smem;
-    unsigned char *C = smem + (size_t)a.kcap * kRow;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned char *stage = C + (size_t)(a.mcap + 1) * kRow + warp * kOStage;
     const uint32_t lb = lane * (uint32_t)sizeof(T);  // r * (CPT cells) + cell, in bytes
     const int r = lane >> 2;
-    const unsigned char *ft = reinterpret_cast<const unsigned char *>(a.ft + (size_t)blockIdx.x * a.ns * CPT);
-    T acc[NSLOT];
-#pragma unroll
-    for (int j = 0; j < NSLOT; j++) acc[j] = V::zero();
-    if (warp == 0) *reinterpret_cast<T *>(C + (size_t)a.mcap * kRow + lb) = V::zero();  // padding targets read this row
+    // rings, f, P and C
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(smem) + warp * kORing;
+    const uint32_t F = (uint32_t)__cvta_generic_to_shared(smem) + kOWarps * kORing;
+    const uint32_t P = F + (uint32_t)a.ns * CPT * 4, C = P + (uint32_t)a.pcap * kRow;
 
     const int s0 = a.bounds[blockIdx.y], s1 = a.bounds[blockIdx.y + 1];
-    // targets of the step whose list is staged: C rows into this warp's outputs
-    auto gather = [&]() {
-        const unsigned char *pos = stage + NSLOT;
-#pragma unroll
-        for (int j4 = 0; j4 < NSLOT; j4 += 4) {
-            const uint32_t cw = *reinterpret_cast<const uint32_t *>(stage + j4);
-            if (cw == 0) continue;
-#pragma unroll
-            for (int jj = 0; jj < 4; jj++) {
-                const int n = (cw >> (8 * jj)) & 255;
-                T s = V::zero();
-#pragma unroll 1
-                for (int q = 0; q < n; q++, pos += 8) {
-                    const uint2 v = *reinterpret_cast<const uint2 *>(pos);
-                    constexpr uint32_t m = 0xffffu << kEntryShift;
-                    const uint32_t o0 = ((v.x << kEntryShift) & m) ^ lb, o1 = ((v.x >> (16 - kEntryShift)) & m) ^ lb;
-                    const uint32_t o2 = ((v.y << kEntryShift) & m) ^ lb, o3 = ((v.y >> (16 - kEntryShift)) & m) ^ lb;
-                    const T c0 = *reinterpret_cast<const T *>(C + o0), c1 = *reinterpret_cast<const T *>(C + o1);
-                    const T c2 = *reinterpret_cast<const T *>(C + o2), c3 = *reinterpret_cast<const T *>(C + o3);
-                    s = V::add(s, V::add(V::add(c0, c1), V::add(c2, c3)));
-                }
-                acc[j4 + jj] = V::add(acc[j4 + jj], s);
-            }
+    if (s0 < s1) {
+        // the ring: chunk c sits at (c % 4) chunks; three chunks are in flight
+        const uint4 *src = a.stream + (size_t)__ldg(a.start + s0 * kOWarps + warp) * (kOChunk / 16) + lane;
+        uint32_t head = 0;  // bytes consumed so far
+        auto fetch = [&](uint32_t at) {
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ring + (at & (kORing - 1)) + lane * 16), "l"(src)
+                         : "memory");
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            src += kOChunk / 16;
+        };
+        for (int k = 0; k < 3; k++) fetch(k * kOChunk);
+        // the next chunk has landed: its address; the chunk before it is done with
+        auto next = [&]() -> uint32_t {
+            __syncwarp();
+            fetch(head + 3 * kOChunk);
+            asm volatile("cp.async.wait_group 3;" ::: "memory");
+            __syncwarp();
+            const uint32_t at = ring + (head & (kORing - 1));
+            head += kOChunk;
+            return at;
+        };
+        const float4 *ft = reinterpret_cast<const float4 *>(a.ft + (size_t)blockIdx.x * a.ns * CPT);
+        for (int i = threadIdx.x; i < a.ns * CPT / 4; i += kOThreads) {
+            const float4 v = __ldg(ft + i);
+            asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(F + i * 16), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+                         : "memory");
         }
-    };
+        if (warp == 0) sts(C + a.mcap * kRow + lb, V::zero());  // padding targets read this row
+        T acc[NSLOT];
+#pragma unroll
+        for (int j = 0; j < NSLOT; j++) acc[j] = V::zero();
+        __syncthreads();
 
-    for (int st = s0; st < s1; st++) {
-        if (st > s0) gather();
-        // products
-        const int4 hd = __ldg(a.steps + st);
-        for (int k = warp; k < hd.y; k += kOWarps) {
-            const uint4 d = __ldg(a.prod + hd.x + k);
-            const uint32_t w[4] = {d.x, d.y, d.z, d.w};
-            T x[4], y[4];
+        // C rows of a step into this warp's outputs: per slot a count of quads,
+        // then 16-bit entries row << 3 | e; the list may wrap around the ring
+        auto gather = [&](int nchunks) {
+            if (nchunks == 0) return;
+            uint32_t pos = next() - ring;
+            if (nchunks == 2) {  // the second chunk too, the first still in use
+                asm volatile("cp.async.wait_group 2;" ::: "memory");
+                __syncwarp();
+            }
+            uint32_t cpos = pos;
+            pos += NSLOT;
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                x[q] = y[q] = V::zero();
-                if ((int)w[q] >= 0) {
-                    constexpr uint32_t m = 0x7fffu << kEntryShift;
-                    const uint32_t o1 = ((w[q] << kEntryShift) & m) ^ lb;
-                    const uint32_t o2 = ((w[q] >> (16 - kEntryShift)) & m) ^ lb;
-                    x[q] = __ldg(reinterpret_cast<const T *>(ft + o1));
-                    y[q] = __ldg(reinterpret_cast<const T *>(ft + o2));
+            for (int j4 = 0; j4 < NSLOT; j4 += 8, cpos += 8) {
+                const uint2 cw2 = lds<uint2>(ring + cpos);
+#pragma unroll
+                for (int jj = 0; jj < 8; jj++) {
+                    const uint32_t cw = jj < 4 ? cw2.x : cw2.y;
+                    const int n = (cw >> (8 * (jj & 3))) & 255;
+                    T s = V::zero();
+#pragma unroll 1
+                    for (int q = 0; q < n; q++, pos += 8) {
+                        const uint2 v = lds<uint2>(ring + (pos & (kORing - 1)));
+                        constexpr uint32_t m = 0xffffu << kShift;
+                        const T c0 = lds<T>(C + (((v.x << kShift) & m) ^ lb)), c1 = lds<T>(C + (((v.x >> (16 - kShift)) & m) ^ lb));
+                        const T c2 = lds<T>(C + (((v.y << kShift) & m) ^ lb)), c3 = lds<T>(C + (((v.y >> (16 - kShift)) & m) ^ lb));
+                        s = V::add(s, V::add(V::add(c0, c1), V::add(c2, c3)));
+                    }
+                    acc[j4 + jj] = V::add(acc[j4 + jj], s);
                 }
             }
-            T p = V::fma(x[0], y[0], V::fma(x[1], y[1], V::zero()));
-            p = V::add(p, V::fma(x[2], y[2], V::fma(x[3], y[3], V::zero())));
-            // a reflection of an axis on which D is its own mirror repeats D
-            const uint32_t self = ((w[0] >> 15) & 1u) | ((w[1] >> 14) & 2u) | ((w[2] >> 13) & 4u);
-            if (self & (uint32_t)r) p = V::zero();
-            *reinterpret_cast<T *>(P + (size_t)k * kRow + lb) = p;
-        }
-        __syncthreads();
-        // contraction
-        const int4 wk = __ldg(a.work + st * kOWarps + warp);
-        for (int i = lane; i < wk.w; i += 32)
-            reinterpret_cast<uint2 *>(stage)[i] = __ldg(a.targets + wk.z + i);
-        for (int b = wk.x; b < wk.y; b++) {
-            const int4 h = __ldg(a.blocks + b);
-            T c0 = V::zero(), c1 = V::zero(), c2 = V::zero(), c3 = V::zero();
-            const uint4 *po = a.ent_off + (h.x >> 2);
-            const float4 *pw = a.ent_w + h.x;
-#pragma unroll 2
-            for (int g = 0; g < h.y; g++, po++, pw += 4) {
-                const uint4 o = __ldg(po);
-                const float4 w0 = __ldg(pw), w1 = __ldg(pw + 1), w2 = __ldg(pw + 2), w3 = __ldg(pw + 3);
-                const T p0 = *reinterpret_cast<const T *>(P + o.x + lb), p1 = *reinterpret_cast<const T *>(P + o.y + lb);
-                const T p2 = *reinterpret_cast<const T *>(P + o.z + lb), p3 = *reinterpret_cast<const T *>(P + o.w + lb);
-#define GD_MAC(wv, pv)           \
-    c0 = V::fma((wv).x, pv, c0); \
-    c1 = V::fma((wv).y, pv, c1); \
-    c2 = V::fma((wv).z, pv, c2); \
-    c3 = V::fma((wv).w, pv, c3)
-                GD_MAC(w0, p0);
-                GD_MAC(w1, p1);
-                GD_MAC(w2, p2);
-                GD_MAC(w3, p3);
-#undef GD_MAC
+            if (nchunks == 2) {
+                __syncwarp();
+                fetch(head + 3 * kOChunk);
+                head += kOChunk;
             }
-            unsigned char *cr = C + h.z + lb;
-            *reinterpret_cast<T *>(cr) = c0;
-            *reinterpret_cast<T *>(cr + kRow) = c1;
-            *reinterpret_cast<T *>(cr + 2 * kRow) = c2;
-            *reinterpret_cast<T *>(cr + 3 * kRow) = c3;
-        }
-        __syncthreads();
-    }
-    if (s1 > s0) gather();
-    // lane (r, cells): output row 8 o + r
-    const int cell = blockIdx.x * CPT + (lane & 3) * (CPT / 4);
+        };
+
+        int tgt_chunks = 0;
+        for (int st = s0; st < s1; st++) {
+            gather(tgt_chunks);
+            // products: this warp's rows warp, warp + 16, ...
+            uint32_t at = next();
+            const uint4 hd = lds<uint4>(at);  // products, contraction quads, target chunks
+            uint32_t prow = P + warp * kRow + lb;
+#pragma unroll 1
+            for (uint32_t k = 0; k < hd.x; k++, prow += kOWarps * kRow) {
+                at += 16;
+                const uint4 d = lds<uint4>(at);
+                const uint32_t w[4] = {d.x, d.y, d.z, d.w};
+                T x[4], y[4];
 #pragma unroll
-    for (int j = 0; j < NSLOT; j++) {
-        const int o = warp + j * kOWarps;
-        if (o >= a.norb) continue;
-        const int row = 8 * o + r;
-        if (a.part) {
-            *reinterpret_cast<T *>(a.part + ((size_t)blockIdx.y * a.ns + row) * a.cells_pad + cell) = acc[j];
-        } else {
-            float *g = a.gain + (size_t)__ldg(a.row_node + row) * a.ld + cell;
-            const float *v = reinterpret_cast<const float *>(&acc[j]);
-#pragma unroll
-            for (int q = 0; q < CPT / 4; q++)
-                if (cell + q < a.ncells) g[q] = v[q];
+                for (int q = 0; q < 4; q++) {
+                    x[q] = y[q] = V::zero();
+                    if ((int)w[q] >= 0) {
+                        constexpr uint32_t m = 0x7fffu << kShift;
+                        x[q] = lds<T>(F + (((w[q] << kShift) & m) ^ lb));
+                        y[q] = lds<T>(F + (((w[q] >> (16 - kShift)) & m) ^ lb));
+                    }
+                }
+                T p = V::mac(x[0], y[0], V::mac(x[1], y[1], V::zero()));
+                p = V::add(p, V::mac(x[2], y[2], V::mac(x[3], y[3], V::zero())));
+                // a reflection of an axis on which D is its own mirror repeats D
+                const uint32_t self = ((w[0] >> 15) & 1u) | ((w[1] >> 14) & 2u) | ((w[2] >> 13) & 4u);
+                if (self & (uint32_t)r) p = V::zero();
+                sts(prow, p);
+            }
+            __syncthreads();
+            // contraction: per quad four entries {P offset; the block's four weights};
+            // bit 0 of the first offset: last quad of its block, bit 1: the block's
+            // sums continue those of an earlier part; the C row in the second's top bits
+            T c0 = V::zero(), c1 = V::zero(), c2 = V::zero(), c3 = V::zero();
+            for (uint32_t left = hd.y; left > 0;) {
+                uint32_t e = next();
+                const uint32_t n = min(left, (uint32_t)kOQuads);
+                left -= n;
+#pragma unroll 1
+                for (uint32_t q = 0; q < n; q++, e += 80) {
+                    const uint4 o = lds<uint4>(e);
+                    const float4 w0 = lds<float4>(e + 16), w1 = lds<float4>(e + 32), w2 = lds<float4>(e + 48),
+                                 w3 = lds<float4>(e + 64);
+                    const T p0 = lds<T>(P + (o.x & ~3u) + lb), p1 = lds<T>(P + (o.y & 0x3ffffu) + lb);
+                    const T p2 = lds<T>(P + o.z + lb), p3 = lds<T>(P + o.w + lb);
+                    const uint32_t cr = C + (o.y >> 18) * kRow + lb;
+                    if (o.x & 2u) {
+                        c0 = lds<T>(cr);
+                        c1 = lds<T>(cr + kRow);
+                        c2 = lds<T>(cr + 2 * kRow);
+                        c3 = lds<T>(cr + 3 * kRow);
+                    }
+#define GD_MAC(wv, pv)           \
+    c0 = V::mac((wv).x, pv, c0); \
+    c1 = V::mac((wv).y, pv, c1); \
+    c2 = V::mac((wv).z, pv, c2); \
+    c3 = V::mac((wv).w, pv, c3)
+                    GD_MAC(w0, p0);
+                    GD_MAC(w1, p1);
+                    GD_MAC(w2, p2);
+                    GD_MAC(w3, p3);
+#undef GD_MAC
+                    if (o.x & 1u) {
+                        sts(cr, c0);
+                        sts(cr + kRow, c1);
+                        sts(cr + 2 * kRow, c2);
+                        sts(cr + 3 * kRow, c3);
+                        c0 = c1 = c2 = c3 = V::zero();
+                    }
+                }
+            }
+            tgt_chunks = (int)hd.z;
+            __syncthreads();
         }
+        gather(tgt_chunks);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");  // the copies ahead of the last chunk
+        // lane (r, cells): output row 8 o + r
+        const int cell = blockIdx.x * CPT + (lane & 3) * (CPT / 4);
+#pragma unroll
+        for (int j = 0; j < NSLOT; j++) {
+            const int o = warp + j * kOWarps;
+            if (o >= a.norb) continue;
+            const int row = 8 * o + r;
+            if (a.part) {
+                *reinterpret_cast<T *>(a.part + ((size_t)blockIdx.y * a.ns + row) * a.cells_pad + cell) = acc[j];
+            } else {
+                float *g = a.gain + (size_t)__ldg(a.row_node + row) * a.ld + cell;
+                const float *v = reinterpret_cast<const float *>(&acc[j]);
+#pragma unroll
+                for (int q = 0; q < CPT / 4; q++)
+                    if (cell + q < a.ncells) g[q] = v[q];
+            }
+        }
+    } else if (a.part) {  // an empty chunk (more chunks than work): zero partial sums
+        for (int t = threadIdx.x; t < a.ns * CPT; t += kOThreads)
+            a.part[((size_t)blockIdx.y * a.ns + t / CPT) * a.cells_pad + blockIdx.x * CPT + t % CPT] = 0.f;
     }
 }
 
@@ -252,46 +379,12 @@ __global__ void orbit_reduce_kernel(const float *__restrict__ part, int nchunks,
 // One D of the low octant with anything to do.
 struct DItem {
     int K = 0, nblk = 0;
-    std::vector<uint4> prod;
-    std::vector<int> blk_n;                    // entries per block, padded to four
-    std::vector<uint32_t> off;                 // P row per entry
+    std::vector<uint4> prod;                   // by shell |n|
+    std::vector<int> blk_n;                    // entries per block
+    std::vector<uint32_t> off;                 // P row per entry, ascending within a block
     std::vector<float4> w;
     std::vector<std::pair<int, int>> targets;  // (output row 8 o + e, C row), by output row
 };
-
-}  // namespace
-
-struct OrbitGain {
-    int cpt = 8, nslot = 0, norb = 0, kcap = 0, mcap = 0, nsteps = 0;
-    size_t smem = 0;
-    std::vector<double> cost_prefix;  // [nsteps + 1]
-    int *row_node = nullptr;
-    uint4 *prod = nullptr;
-    int4 *steps = nullptr, *work = nullptr, *blocks = nullptr;
-    uint4 *ent_off = nullptr;
-    float4 *ent_w = nullptr;
-    uint2 *targets = nullptr;
-    std::map<int, int *> bounds_dev;
-};
-
-void orbit_free(Context &c)
-{
-    OrbitGain *g = c.orbit;
-    if (!g) return;
-    cudaFree(g->row_node);
-    cudaFree(g->prod);
-    cudaFree(g->steps);
-    cudaFree(g->work);
-    cudaFree(g->blocks);
-    cudaFree(g->ent_off);
-    cudaFree(g->ent_w);
-    cudaFree(g->targets);
-    for (auto &kv : g->bounds_dev) cudaFree(kv.second);
-    delete g;
-    c.orbit = nullptr;
-}
-
-namespace {
 
 template <typename T>
 int upload(T **dst, const std::vector<T> &src)
@@ -312,7 +405,8 @@ OrbitKernel orbit_kernel(int cpt, int need, int *nslot)
     };
     static const Inst inst[] = {{8, 8, orbit_gain_kernel<8, 8>},   {8, 16, orbit_gain_kernel<8, 16>},
                                 {8, 24, orbit_gain_kernel<8, 24>}, {8, 32, orbit_gain_kernel<8, 32>},
-                                {4, 48, orbit_gain_kernel<4, 48>}, {4, 64, orbit_gain_kernel<4, 64>}};
+                                {4, 48, orbit_gain_kernel<4, 48>}, {4, 56, orbit_gain_kernel<4, 56>},
+                                {4, 64, orbit_gain_kernel<4, 64>}};
     for (const Inst &i : inst)
         if (i.cpt == cpt && i.nslot >= need) {
             *nslot = i.nslot;
@@ -322,6 +416,18 @@ OrbitKernel orbit_kernel(int cpt, int need, int *nslot)
 }
 
 }  // namespace
+
+void orbit_free(Context &c)
+{
+    OrbitGain *g = c.orbit;
+    if (!g) return;
+    cudaFree(g->row_node);
+    cudaFree(g->stream);
+    cudaFree(g->start);
+    for (auto &kv : g->bounds_dev) cudaFree(kv.second);
+    delete g;
+    c.orbit = nullptr;
+}
 
 // Tables of the orbit kernel; leaves c.orbit null (the pair kernel of
 // gd_gain.cu then serves the grid) when the lattice has no reflection symmetry
@@ -369,12 +475,15 @@ int orbit_build(Context &c)
         std::vector<std::array<float, kORows>> w4(d.nclass);
         std::vector<int> touched;
         std::vector<char> mark(d.nclass, 0);
+        std::vector<double> n2;
+        std::vector<int> by;
         for (int Did = t0; Did < d.nxyz; Did += nt) {
             const int D[3] = {Did / d.nyz, (Did / d.nz) % d.ny, Did % d.nz};
             DItem &it = items[Did];
             const uint32_t self = (D[0] == d.nx - 1 ? 1u : 0u) | (D[1] == d.ny - 1 ? 2u : 0u) | (D[2] == d.nz - 1 ? 4u : 0u);
             cls.clear();
             want.clear();
+            n2.clear();
             for (int x2 = 0; x2 <= D[0] >> 1; x2++)
                 for (int y2 = 0; y2 <= D[1] >> 1; y2++)
                     for (int z2 = 0; z2 <= D[2] >> 1; z2++) {
@@ -394,13 +503,15 @@ int orbit_build(Context &c)
                             if (t1 >= 0 && t2 >= 0) pw[np++] = (uint32_t)t1 | (uint32_t)t2 << 16;
                         }
                         have = np;
-                        while (np < 4) pw[np++] = kNoPair & ~0x8000u;
+                        while (np < 4) pw[np++] = kNoPair;
                         const int k = (x2 * d.hy + y2) * d.hz + z2;
                         if (have) {
                             for (int q = 0; q < 3; q++)
                                 if ((self >> q) & 1u) pw[q] |= 0x8000u;
-                            prow[k] = it.K++;
+                            it.K++;
                             cls.push_back(k);
+                            n2.push_back((double)(d.du * n[0]) * (d.du * n[0]) + (double)(d.dv * n[1]) * (d.dv * n[1]) +
+                                         (double)(d.dw * n[2]) * (d.dw * n[2]));
                             it.prod.push_back(make_uint4(pw[0], pw[1], pw[2], pw[3]));
                         }
                         const int grp = gid[(n[0] * d.ny + n[1]) * d.nz + n[2]];
@@ -415,6 +526,15 @@ int orbit_build(Context &c)
                         }
                     }
             if (it.K && !want.empty()) {
+                by.resize(it.K);
+                for (int k = 0; k < it.K; k++) by[k] = k;
+                std::stable_sort(by.begin(), by.end(), [&](int x, int y) { return n2[x] < n2[y]; });
+                std::vector<uint4> sorted(it.K);
+                for (int k = 0; k < it.K; k++) {
+                    sorted[k] = it.prod[by[k]];
+                    prow[cls[by[k]]] = k;
+                }
+                it.prod.swap(sorted);
                 std::sort(want.begin(), want.end(), [&](int x, int y) { return g2[x] != g2[y] ? g2[x] < g2[y] : x < y; });
                 for (size_t k = 0; k < want.size(); k++) crow[want[k]] = (int)k;
                 it.nblk = ((int)want.size() + kORows - 1) / kORows;
@@ -441,12 +561,7 @@ int orbit_build(Context &c)
                         it.off.push_back((uint32_t)pr);
                         it.w.push_back(make_float4(w4[pr][0], w4[pr][1], w4[pr][2], w4[pr][3]));
                     }
-                    int n = (int)touched.size();
-                    for (; n & 3; n++) {  // padding repeats a row of the block with weight 0
-                        it.off.push_back((uint32_t)touched[0]);
-                        it.w.push_back(make_float4(0.f, 0.f, 0.f, 0.f));
-                    }
-                    it.blk_n.push_back(n);
+                    it.blk_n.push_back((int)touched.size());
                 }
                 for (auto &t : it.targets) t.second = crow[t.second];
                 std::sort(it.targets.begin(), it.targets.end());
@@ -463,157 +578,219 @@ int orbit_build(Context &c)
         build_items(0, nt);
         for (auto &t : th) t.join();
     }
-    int kmax = 0, mmax = 0;
+    int mmax = 0;
+    int64_t ktotal = 0;
     for (const DItem &it : items) {
-        kmax = std::max(kmax, it.K);
+        ktotal += it.K;
         mmax = std::max(mmax, it.nblk * kORows);
     }
-    if (!kmax || !mmax) return GD_OK;
+    if (!ktotal || !mmax) return GD_OK;
 
     // tile width: eight cells where their outputs and rows fit, else four
     int max_smem = 0;
     GD_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c.device));
     const int slots = (norb + kOWarps - 1) / kOWarps;
-    int cpt = 0, nslot = 0, cap = 0;
+    int cpt = 0, nslot = 0, pcap = 0, mcap = 0;
     for (int w : {8, 4}) {
         if (!orbit_kernel(w, slots, &nslot)) continue;
-        cap = (max_smem - kOWarps * kOStage) / (32 * 4 * (w / 4)) - 1;  // P and C rows
-        if (cap >= kmax + mmax) {
+        const int rows = (max_smem - kOWarps * kORing - d.n_pnt * w * 4) / (32 * w) - 1;  // P and C rows
+        mcap = std::min(8184, std::max(mmax, rows * 2 / 5 / kORows * kORows));
+        pcap = std::min(kOWarps * kOProd, rows - mcap);
+        if (pcap >= 64) {
             cpt = w;
             break;
         }
     }
     if (!cpt) return GD_OK;
-    const int mcap = std::min({8188, std::max(mmax, cap * 3 / 10 / kORows * kORows), (cap - kmax) / kORows * kORows});
-    const int kcap = cap - mcap;
     // a small lattice still gets ~96 steps, so that few cells spread over the SMs
-    int64_t ktotal = 0;
-    for (const DItem &it : items) ktotal += it.K;
-    const int kstep = std::min(kcap, std::max<int>(kmax, (int)(ktotal / 96)));
-    const uint32_t row_bytes = 32u * 4u * (uint32_t)(cpt / 4);
+    const int kstep = std::min(pcap, std::max(32, (int)(ktotal / 96)));
+    const uint32_t row_bytes = 32u * (uint32_t)cpt;
 
-    // steps: consecutive D while their rows and target lists fit
-    std::vector<uint4> prod;
-    std::vector<int4> steps, work, blocks;
-    std::vector<uint32_t> ent_off;
-    std::vector<float4> ent_w;
-    std::vector<uint2> targets;
     OrbitGain *og = new OrbitGain;
+    og->cuts.push_back(0);
     og->cost_prefix.push_back(0.0);
-    const int max_quads = (kOStage - nslot) / 8;
-    std::vector<int> cur;
+    double cost = 0.0;
+    std::vector<std::vector<uint4>> ws(kOWarps);  // the warps' streams
+    std::vector<std::vector<int>> start(kOWarps);
+    auto pad_chunk = [](std::vector<uint4> &v) {
+        while (v.size() % (kOChunk / 16)) v.push_back(make_uint4(0, 0, 0, 0));
+    };
     std::vector<std::vector<uint16_t>> tl(norb);
+    const int max_quads = (2 * kOChunk - nslot) / 8;
     auto list_quads = [&](int warp) {
         int q = 0;
         for (int o = warp; o < norb; o += kOWarps) q += ((int)tl[o].size() + 3) / 4;
         return q;
     };
-    auto close_step = [&]() {
-        // the blocks go to the warps largest first, each to the least loaded
+    // a step: rows [k0, k1) of each of its D, all of their C rows; the target
+    // lists in tl (empty before a D's last part)
+    struct Part {
+        int item, k0, k1;
+    };
+    auto emit = [&](const std::vector<Part> &parts, bool last) {
         struct Blk {
-            int cost, item, b, e0, row;
+            int n, item, b, e0, crow, k0, kbase;
+            bool cont;
         };
         std::vector<Blk> bl;
-        int krow = 0, mrow = 0;
-        const int p0 = (int)prod.size();
-        std::vector<int> kbase(cur.size());
-        double cost = 0.0;
-        for (size_t i = 0; i < cur.size(); i++) {
-            const DItem &it = items[cur[i]];
-            kbase[i] = krow;
-            prod.insert(prod.end(), it.prod.begin(), it.prod.end());
+        std::vector<const uint4 *> prod;
+        int mrow = 0;
+        double entries = 0.0, targets = 0.0;
+        for (const Part &pt : parts) {
+            const DItem &it = items[pt.item];
+            const int kbase = (int)prod.size();
+            for (int k = pt.k0; k < pt.k1; k++) prod.push_back(&it.prod[k]);
             int e0 = 0;
-            for (int b = 0; b < it.nblk; b++) {
-                bl.push_back(Blk{it.blk_n[b] * 3 + 30, (int)i, b, e0, mrow + b * kORows});
-                e0 += it.blk_n[b];
+            for (int b = 0; b < it.nblk; e0 += it.blk_n[b++]) {
+                const auto lo = it.off.begin() + e0, hi = lo + it.blk_n[b];
+                const int f0 = (int)(std::lower_bound(lo, hi, (uint32_t)pt.k0) - lo),
+                          f1 = (int)(std::lower_bound(lo, hi, (uint32_t)pt.k1) - lo);
+                // a block starts in the first part that has entries of it, or
+                // in the first part when no part has (its C rows are zero)
+                if (f0 == f1 && !(pt.k0 == 0 && it.blk_n[b] == 0)) continue;
+                bl.push_back(Blk{f1 - f0, pt.item, b, e0 + f0, mrow + b * kORows, pt.k0, kbase, f0 > 0});
+                entries += f1 - f0;
             }
-            cost += 9.0 * it.K + 4.0 * e0 + 2.5 * (double)it.targets.size();
-            krow += it.K;
             mrow += it.nblk * kORows;
         }
-        std::stable_sort(bl.begin(), bl.end(), [](const Blk &x, const Blk &y) { return x.cost > y.cost; });
+        // the blocks go to the warps largest first, each to the least loaded
+        std::stable_sort(bl.begin(), bl.end(), [](const Blk &x, const Blk &y) { return x.n > y.n; });
         std::vector<std::vector<const Blk *>> mine(kOWarps);
         std::vector<int> load(kOWarps, 0);
         for (const Blk &b : bl) {
             const int w = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-            load[w] += b.cost;
+            load[w] += b.n + 6;
             mine[w].push_back(&b);
         }
-        steps.push_back(make_int4(p0, krow, 0, 0));
         for (int w = 0; w < kOWarps; w++) {
-            const int b0 = (int)blocks.size(), q0 = (int)targets.size();
+            std::vector<uint4> &v = ws[w];
+            start[w].push_back((int)(v.size() / (kOChunk / 16)));
+            const size_t h = v.size();
+            v.push_back(make_uint4(0, 0, 0, 0));
+            uint32_t np = 0, nq = 0;
+            for (size_t k = w; k < prod.size(); k += kOWarps, np++) v.push_back(*prod[k]);
+            pad_chunk(v);
             for (const Blk *b : mine[w]) {
-                const DItem &it = items[cur[b->item]];
-                const int n = it.blk_n[b->b];
-                blocks.push_back(make_int4((int)ent_w.size(), n / 4, (int)((uint32_t)b->row * row_bytes), 0));
-                for (int e = 0; e < n; e++) {
-                    ent_off.push_back((it.off[b->e0 + e] + (uint32_t)kbase[b->item]) * row_bytes);
-                    ent_w.push_back(it.w[b->e0 + e]);
+                const DItem &it = items[b->item];
+                const int quads = std::max(1, (b->n + 3) / 4);
+                for (int q = 0; q < quads; q++, nq++) {
+                    if (nq && nq % kOQuads == 0) pad_chunk(v);
+                    uint32_t off[4];
+                    float4 wt[4];
+                    for (int z = 0; z < 4; z++) {
+                        const int e = 4 * q + z;
+                        // padding repeats a row of the block with weight 0
+                        const int row = b->n ? (int)it.off[b->e0 + std::min(e, b->n - 1)] - b->k0 : 0;
+                        off[z] = (uint32_t)(row + b->kbase) * row_bytes;
+                        wt[z] = e < b->n ? it.w[b->e0 + e] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
+                    off[0] |= (q == quads - 1 ? 1u : 0u) | (q == 0 && b->cont ? 2u : 0u);
+                    off[1] |= (uint32_t)b->crow << 18;
+                    v.push_back(make_uint4(off[0], off[1], off[2], off[3]));
+                    for (int z = 0; z < 4; z++) {
+                        uint4 u;
+                        std::memcpy(&u, &wt[z], 16);
+                        v.push_back(u);
+                    }
                 }
             }
-            std::vector<uint8_t> cnt(nslot, 0);
-            std::vector<uint16_t> ent;
+            pad_chunk(v);
+            uint32_t tc = 0;
+            std::vector<uint8_t> list(nslot, 0);
             for (int j = 0, o = w; o < norb; j++, o += kOWarps) {
-                cnt[j] = (uint8_t)((tl[o].size() + 3) / 4);
-                ent.insert(ent.end(), tl[o].begin(), tl[o].end());
-                while (ent.size() & 3) ent.push_back((uint16_t)(mcap << 3));  // the zero row
+                list[j] = (uint8_t)((tl[o].size() + 3) / 4);
+                targets += (double)tl[o].size();
+                for (size_t t = 0; t < (size_t)list[j] * 4; t++) {
+                    const uint16_t e = t < tl[o].size() ? tl[o][t] : (uint16_t)(mcap << 3);  // the zero row
+                    list.push_back((uint8_t)(e & 255));
+                    list.push_back((uint8_t)(e >> 8));
+                }
             }
-            const size_t quads = (size_t)nslot / 8 + ent.size() / 4;
-            targets.resize(q0 + quads);
-            std::memcpy(&targets[q0], cnt.data(), nslot);
-            if (!ent.empty()) std::memcpy(&targets[q0 + nslot / 8], ent.data(), ent.size() * 2);
-            work.push_back(make_int4(b0, (int)blocks.size(), q0, (int)quads));
+            if ((int)list.size() > nslot) {
+                list.resize((list.size() + 15) / 16 * 16, 0);
+                const size_t at = v.size();
+                v.resize(at + list.size() / 16);
+                std::memcpy(&v[at], list.data(), list.size());
+                pad_chunk(v);
+                tc = (uint32_t)((v.size() - at) / (kOChunk / 16));
+            }
+            v[h] = make_uint4(np, nq, tc, 0);
         }
-        og->cost_prefix.push_back(og->cost_prefix.back() + cost);
+        cost += 600.0 + 15.0 * (double)prod.size() + 3.5 * entries + 8.0 * (double)bl.size() + 2.3 * targets;
+        og->nsteps++;
+        if (last) {
+            og->cuts.push_back(og->nsteps);
+            og->cost_prefix.push_back(cost);
+        }
         for (auto &t : tl) t.clear();
-        cur.clear();
     };
+    std::vector<Part> cur;
     int krow = 0, mrow = 0;
+    auto close = [&]() {
+        if (!cur.empty()) emit(cur, true);
+        cur.clear();
+        krow = mrow = 0;
+    };
+    auto add_targets = [&](const DItem &it) {
+        for (const auto &t : it.targets) tl[t.first >> 3].push_back((uint16_t)((mrow + t.second) << 3 | (t.first & 7)));
+        bool fits = true;
+        for (int w = 0; fits && w < kOWarps; w++) fits = list_quads(w) <= max_quads;
+        for (const auto &t : it.targets) fits = fits && tl[t.first >> 3].size() <= 1020;
+        if (!fits)
+            for (const auto &t : it.targets) tl[t.first >> 3].pop_back();
+        return fits;
+    };
     for (int Did = 0; Did < d.nxyz; Did++) {
         const DItem &it = items[Did];
         if (!it.nblk) continue;
-        for (int pass = 0; pass < 2; pass++) {
-            bool fits = krow + it.K <= kstep && mrow + it.nblk * kORows <= mcap;
-            if (fits) {
-                for (const auto &t : it.targets) tl[t.first >> 3].push_back((uint16_t)((mrow + t.second) << 3 | (t.first & 7)));
-                for (int w = 0; fits && w < kOWarps; w++) fits = list_quads(w) <= max_quads;
-                for (const auto &t : it.targets) fits = fits && tl[t.first >> 3].size() <= 1020;
-                if (!fits)
-                    for (const auto &t : it.targets) tl[t.first >> 3].pop_back();
+        if (it.K > kstep) {  // parts of its own
+            close();
+            const int parts = (it.K + kstep - 1) / kstep;
+            for (int p = 0; p < parts; p++) {
+                if (p == parts - 1 && !add_targets(it)) {
+                    delete og;
+                    return GD_OK;
+                }
+                emit({Part{Did, (int)((int64_t)it.K * p / parts), (int)((int64_t)it.K * (p + 1) / parts)}}, p == parts - 1);
             }
-            if (fits) {
+            continue;
+        }
+        for (int pass = 0; pass < 2; pass++) {
+            if (krow + it.K <= kstep && mrow + it.nblk * kORows <= mcap && add_targets(it)) {
                 krow += it.K;
                 mrow += it.nblk * kORows;
-                cur.push_back(Did);
+                cur.push_back(Part{Did, 0, it.K});
                 break;
             }
             if (cur.empty()) {  // a single D that does not fit
                 delete og;
                 return GD_OK;
             }
-            close_step();
-            krow = mrow = 0;
+            close();
         }
     }
-    if (!cur.empty()) close_step();
+    close();
     og->cpt = cpt;
     og->nslot = nslot;
     og->norb = norb;
-    og->kcap = kcap;
+    og->pcap = pcap;
     og->mcap = mcap;
-    og->nsteps = (int)steps.size();
-    og->smem = (size_t)(kcap + mcap + 1) * row_bytes + kOWarps * kOStage;
-    std::vector<uint4> off4(ent_off.size() / 4);
-    if (!off4.empty()) std::memcpy(off4.data(), ent_off.data(), ent_off.size() * 4);
+    og->smem = (size_t)kOWarps * kORing + (size_t)d.n_pnt * cpt * 4 + (size_t)(pcap + mcap + 1) * row_bytes;
+    // one buffer: warp after warp, each followed by the chunks that the last
+    // steps fetch ahead
+    std::vector<uint4> stream;
+    std::vector<int> st((size_t)og->nsteps * kOWarps);
+    for (int w = 0; w < kOWarps; w++) {
+        const int base = (int)(stream.size() / (kOChunk / 16));
+        for (int k = 0; k < og->nsteps; k++) st[(size_t)k * kOWarps + w] = base + start[w][k];
+        stream.insert(stream.end(), ws[w].begin(), ws[w].end());
+        stream.resize(stream.size() + 4 * (kOChunk / 16), make_uint4(0, 0, 0, 0));
+        std::vector<uint4>().swap(ws[w]);
+    }
     c.orbit = og;
     int rc = upload(&og->row_node, row_node);
-    if (!rc) rc = upload(&og->prod, prod);
-    if (!rc) rc = upload(&og->steps, steps);
-    if (!rc) rc = upload(&og->work, work);
-    if (!rc) rc = upload(&og->blocks, blocks);
-    if (!rc) rc = upload(&og->ent_off, off4);
-    if (!rc) rc = upload(&og->ent_w, ent_w);
-    if (!rc) rc = upload(&og->targets, targets);
+    if (!rc) rc = upload(&og->stream, stream);
+    if (!rc) rc = upload(&og->start, st);
     return rc;  // the caller destroys the context on failure
 }
 
@@ -623,10 +800,11 @@ int orbit_chunks(const Context &c, int ncells)
 {
     const OrbitGain &g = *c.orbit;
     const int tiles = (ncells + g.cpt - 1) / g.cpt, sms = std::max(1, c.sm_count);
-    const int lo = std::min(g.nsteps, std::max(1, (std::max(1, c.gain_waves) * sms + tiles - 1) / tiles));
+    const int most = (int)g.cuts.size() - 1;
+    const int lo = std::min(most, std::max(1, (std::max(1, c.gain_waves) * sms + tiles - 1) / tiles));
     int best = lo;
     double best_fill = 0.0;
-    for (int k = lo; k <= std::min(g.nsteps, lo + 8); k++) {
+    for (int k = lo; k <= std::min(most, lo + 8); k++) {
         const int64_t ctas = (int64_t)tiles * k;
         const double fill = (double)ctas / (double)((ctas + sms - 1) / sms * sms) - 0.002 * (k - lo);
         if (fill > best_fill + 1e-9) {
@@ -651,16 +829,19 @@ size_t orbit_part_bytes(const Context &c, int ncells, int nchunks)
 
 void orbit_chunk_bounds(const Context &c, int nchunks, int *bounds)
 {
-    const std::vector<double> &pre = c.orbit->cost_prefix;
-    const int n = c.orbit->nsteps;
+    const OrbitGain &g = *c.orbit;
+    const std::vector<double> &pre = g.cost_prefix;
+    const int n = (int)g.cuts.size() - 1;
+    int at = 0;
     bounds[0] = 0;
     for (int k = 1; k < nchunks; k++) {
         const double want = pre[n] * k / nchunks;
         int b = (int)(std::lower_bound(pre.begin(), pre.end(), want) - pre.begin());
         if (b > 0 && want - pre[b - 1] < pre[b] - want) b--;
-        bounds[k] = std::min(n, std::max(bounds[k - 1], b));
+        at = std::min(n, std::max(at, b));
+        bounds[k] = g.cuts[at];
     }
-    bounds[nchunks] = n;
+    bounds[nchunks] = g.nsteps;
 }
 
 int launch_orbit(Context &c, const float *f, int ncells, int ld, float *gain, void *buf, int nchunks,
@@ -676,8 +857,8 @@ int launch_orbit(Context &c, const float *f, int ncells, int ld, float *gain, vo
     orbit_pack_kernel<<<dim3((cells_pad + 31) / 32, d.n_pnt / 8), dim3(32, 8), 0, st>>>(
         f, ld, ncells, d.n_pnt, g.cpt, g.row_node, ft, cells_pad);
     GD_CUDA(cudaGetLastError());
-    const OrbitArgs a{ft,        g.prod,     g.steps, g.work, g.blocks, g.ent_off, g.ent_w, g.targets, d_bounds,
-                      g.row_node, part,      gain,    g.norb, d.n_pnt,  cells_pad, ncells,  ld,        g.kcap, g.mcap};
+    const OrbitArgs a{ft,     g.stream, g.start,   d_bounds, g.row_node, part,  gain,
+                      g.norb, d.n_pnt,  cells_pad, ncells,   ld,         g.pcap, g.mcap};
     int nslot = 0;
     OrbitKernel kern = orbit_kernel(g.cpt, g.nslot, &nslot);
     GD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
