@@ -67,6 +67,8 @@ struct OrbitGain {
     int *row_node = nullptr;          // [n_pnt]
     uint4 *stream = nullptr;
     int *start = nullptr;  // [step][warp] first chunk
+    int opad = 0;               // orbits padded to the loss kernel's tile
+    float *bx = nullptr;        // [8][o'][opad] loss matrices folded by the reflections' characters
     std::map<int, int *> bounds_dev;
 };
 
@@ -212,6 +214,7 @@ int reduce_gain_partials(Context &c, const float *part, int nchunks, int cells_p
 // tables (built with the context), chunk count and bounds, buffer sizes, and
 // the launch into a caller-provided buffer (packed f, then chunk partials)
 int orbit_build(Context &c);
+int fold_loss_build(Context &c);  // its loss matrices (gd_loss.cu)
 void orbit_free(Context &c);
 int orbit_chunks(const Context &c, int ncells);
 void orbit_chunk_bounds(const Context &c, int nchunks, int *bounds);

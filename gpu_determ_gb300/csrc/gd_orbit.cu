@@ -424,6 +424,7 @@ void orbit_free(Context &c)
     cudaFree(g->row_node);
     cudaFree(g->stream);
     cudaFree(g->start);
+    cudaFree(g->bx);
     for (auto &kv : g->bounds_dev) cudaFree(kv.second);
     delete g;
     c.orbit = nullptr;
@@ -791,6 +792,7 @@ int orbit_build(Context &c)
     int rc = upload(&og->row_node, row_node);
     if (!rc) rc = upload(&og->stream, stream);
     if (!rc) rc = upload(&og->start, st);
+    if (!rc) rc = fold_loss_build(c);
     return rc;  // the caller destroys the context on failure
 }
 

@@ -65,3 +65,33 @@ def test_orbit_gain_of_a_cell_does_not_depend_on_its_neighbours(cuda, gdlib, nc)
     assert bool(torch.isfinite(out[:, 0]).all())
     if nc > 1:
         assert not bool(torch.isfinite(out[:, 1]).all()) and not bool(torch.isfinite(out[:, 2]).all())
+
+
+# 1, 4, 105 and 512 orbits (the tiles are 32 orbits by 8 or 32 cells, steps of 16
+# orbits); cells around the tile width and, in the last, enough for the wide tile
+@pytest.mark.parametrize("dims,R,nc,ld", [((2, 2, 2), 16.5, 1, 1), ((4, 4, 4), 16.5, 8, 9), ((12, 12, 12), 4.8, 33, 33),
+                                          ((12, 10, 8), 4.2, 9, 12), ((16, 16, 16), 16.5, 31, 31),
+                                          ((16, 16, 16), 16.5, 321, 324)])
+def test_folded_loss_matches_oracle(cuda, gdlib, dims, R, nc, ld):
+    """The loss with f and b folded by the lattice's reflections.  Each
+    character's sum takes chains of 16 products (16 roundings of 6e-8 at most),
+    compensated sums of them, three roundings in the fold and one at the end:
+    1.3e-6 of the largest frequency among a node's mirrors if all roundings add
+    up, and those frequencies differ by a factor below 4; independent roundings
+    stay near the root of that count, 3e-7 in relative L2."""
+    torch = cuda
+    spec = gdlib.GridSpec(*dims, R=R)
+    ctx = gdlib.Context(spec)
+    f = inputs.mixtures(spec.fill(), nc, seed=nc)
+    ft = torch.full((ctx.n_pnt, ld), float("nan"), dtype=torch.float32, device="cuda")
+    ft[:, :nc] = torch.from_numpy(f).cuda()
+    out = [torch.full_like(ft, -1.0) for _ in range(2)]
+    for o in out:
+        ctx.collision(ft, nc, ld, o, None)
+    torch.cuda.synchronize()
+    assert torch.equal(out[0], out[1]) and bool((out[0][:, nc:] == -1.0).all())
+    got = out[0][:, :nc].cpu().numpy().astype(np.float64)
+    o = Oracle(*dims, R=R)
+    ref = o.loss_f64(o.to_box(f))
+    assert np.max(np.abs(got - ref) / ref) <= 5e-6
+    assert np.linalg.norm(got - ref) <= 3e-7 * np.linalg.norm(ref)
