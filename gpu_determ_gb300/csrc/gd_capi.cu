@@ -267,6 +267,9 @@ static void destroy_context(Context &c)
     cudaFree(c.d_nodes);
     cudaFree(c.d_b);
     cudaFree(c.d_phi);
+    cudaFree(c.d_lines);
+    cudaFree(c.d_line_xy);
+    cudaFree(c.d_zpow);
     cudaFree(c.d_list_off);
     cudaFree(c.d_list);
     cudaFree(c.d_grp_row_off);
@@ -359,6 +362,32 @@ static int create_context(Context &c, const gd_grid_spec &spec, int device)
     GD_CUDA(cudaMemcpy(c.d_cmap, cmap16.data(), sizeof(int16_t) * d.nxyz, cudaMemcpyHostToDevice));
     GD_CUDA(cudaMemcpy(c.d_nodes, nodes.data(), sizeof(uint32_t) * d.n_pnt, cudaMemcpyHostToDevice));
     GD_CUDA(cudaMemcpy(c.d_phi, phi.data(), sizeof(double) * 5 * d.n_pnt, cudaMemcpyHostToDevice));
+
+    {
+        std::vector<int4> lines;
+        std::vector<double2> xy;
+        std::vector<double2> zpow(2 * d.nz);
+        for (int p = 0; p < d.n_pnt; p++) {
+            // a line's nodes have consecutive z (the sphere is convex)
+            if (p == 0 || c.ui[p] != c.ui[p - 1] || c.vi[p] != c.vi[p - 1] || c.wi[p] != c.wi[p - 1] + 1) {
+                lines.push_back(make_int4(p, p, c.wi[p], 0));
+                xy.push_back(make_double2(c.u[c.ui[p]], c.v[c.vi[p]]));
+            }
+            lines.back().y = p + 1;
+        }
+        for (int k = 0; k < d.nz; k++) {
+            const double z = c.w[k], z2 = z * z;
+            zpow[2 * k] = make_double2(z, z2);
+            zpow[2 * k + 1] = make_double2(z2 * z, z2 * z2);
+        }
+        c.nlines = (int)lines.size();
+        GD_CUDA(cudaMalloc(&c.d_lines, sizeof(int4) * lines.size()));
+        GD_CUDA(cudaMalloc(&c.d_line_xy, sizeof(double2) * xy.size()));
+        GD_CUDA(cudaMalloc(&c.d_zpow, sizeof(double2) * zpow.size()));
+        GD_CUDA(cudaMemcpy(c.d_lines, lines.data(), sizeof(int4) * lines.size(), cudaMemcpyHostToDevice));
+        GD_CUDA(cudaMemcpy(c.d_line_xy, xy.data(), sizeof(double2) * xy.size(), cudaMemcpyHostToDevice));
+        GD_CUDA(cudaMemcpy(c.d_zpow, zpow.data(), sizeof(double2) * zpow.size(), cudaMemcpyHostToDevice));
+    }
 
     if ((rc = gain_plan_cells(c))) return rc;
     // analytic weights: dense FP64-built table (transient), compacted to rows

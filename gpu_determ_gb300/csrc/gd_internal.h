@@ -88,6 +88,12 @@ struct Context {
     uint32_t *d_nodes = nullptr;  // [n_pnt] packed box coords x | y << 10 | z << 20
     float *d_b = nullptr;         // [nxyz] loss kernel by |g|
     double *d_phi = nullptr;      // [5][n_pnt] basis 1, xi_x, xi_y, xi_z, xi^2 (FP64)
+    // the nodes as lines along z (consecutive nodes of one (x, y)): {first node,
+    // end node, z index of the first, 0}, (x, y), and (z, z^2), (z^3, z^4) per z index
+    int nlines = 0;
+    int4 *d_lines = nullptr;
+    double2 *d_line_xy = nullptr;
+    double2 *d_zpow = nullptr;
     int *d_list_off = nullptr;    // [nxyz + 1] weight-row offsets by |g| box index
     WEntry *d_list = nullptr;     // nonzero weights, rows in box order of |g|
     int64_t n_entries = 0;

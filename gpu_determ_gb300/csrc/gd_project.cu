@@ -6,9 +6,20 @@
 //   A_kl = sum_i f_i nu_i phi_k phi_l,  B_k = sum_i (I_i - f_i nu_i) phi_k,
 //   A X = B,  nu'_i = nu_i (1 + X.phi_i),  Q_i = I_i - f_i nu'_i,
 // after which sum_i Q_i phi_k = 0 (mass, momentum, energy) up to FP64 rounding.
-// Lane = cell; warps split the nodes; the per-warp FP64 partial sums are
-// combined across warps in warp order, so the sums are reproducible.
+// A warp takes LC cells times 32 / LC lines.  The nodes of one (x, y) form a line along z, and the sums over a
+// line need only powers of z: 11 FP64 accumulators per node (z^0..z^4 of f nu,
+// z^0..z^2 of I - f nu and of f) that enter the 25 sums once per line, 18 FP64
+// operations per node and cell instead of 46; the second pass likewise takes
+// two fused operations for 1 + X.phi instead of five.  A cluster of CTAs shares
+// the lines of LC cells, and LC is smaller for few cells, so that they still
+// spread over the chip; partial sums are combined lane group by lane group,
+// warp by warp, then CTA by CTA, in fixed order, so the sums are reproducible.
+// Bound: the FP64 pipe (its rate is 1/64 of the FP32 rate and a hardware float to
+// double conversion takes a slot of it, so to_double does that in integers).
+// 20^3: 4096 cells 1.54 -> 0.88 ms (the FP64 pipe 76 % busy where SMs have work; a
+// cluster of eight leaves some without), 256 cells 1.6 -> 0.105, one cell 1.6 -> 0.06.
 #include "gd_internal.h"
+#include "gd_tc.cuh"
 
 #include <algorithm>
 #include <cfloat>
@@ -18,12 +29,16 @@ namespace {
 
 constexpr int kWarps = 8;
 constexpr int kSums = 25;  // 5 B, 15 A (upper triangle), 5 moments
+constexpr size_t kProjSmem = (size_t)(kWarps + 1) * kSums * 32 * sizeof(double);  // the warps' sums, the CTA's
 
 struct ProjArgs {
     Dims d;
     const float *f, *nu, *gain;
     int ld, ncells;
-    const double *phi;  // [5][n_pnt]
+    int nlines;
+    const int4 *lines;      // {first node, end node, z index of the first, 0}
+    const double2 *line_xy;
+    const double2 *zpow;    // (z, z^2), (z^3, z^4) per z index
     float *nu_corr;
     double *q;
     double *x;
@@ -34,128 +49,241 @@ struct ProjArgs {
     unsigned int *status;  // [0] flags (1 non-finite sums, 2 singular system), [1] first cell
 };
 
-// Gaussian elimination with partial pivoting on a symmetric 5x5 system.
-__device__ bool solve5(double A[5][5], double b[5], double x[5])
+// Gaussian elimination with partial pivoting on a symmetric 5x5 system, all
+// indices static (rows swapped by selection).
+__device__ __forceinline__ bool solve5(double A[5][5], double b[5], double x[5])
 {
+#pragma unroll
     for (int k = 0; k < 5; k++) {
         int piv = k;
         double best = fabs(A[k][k]);
+#pragma unroll
         for (int r = k + 1; r < 5; r++)
             if (fabs(A[r][k]) > best) {
                 best = fabs(A[r][k]);
                 piv = r;
             }
-        if (!(best > 0.0)) {
-            for (int t = 0; t < 5; t++) x[t] = 0.;
-            return false;
-        }
-        if (piv != k) {
-            for (int t = 0; t < 5; t++) {
-                const double tmp = A[k][t];
-                A[k][t] = A[piv][t];
-                A[piv][t] = tmp;
+        if (!(best > 0.0)) return false;
+#pragma unroll
+        for (int r = k + 1; r < 5; r++) {
+            const bool p = piv == r;
+#pragma unroll
+            for (int t = k; t < 5; t++) {
+                const double u = A[k][t], v = A[r][t];
+                A[k][t] = p ? v : u;
+                A[r][t] = p ? u : v;
             }
-            const double tb = b[k];
-            b[k] = b[piv];
-            b[piv] = tb;
+            const double u = b[k], v = b[r];
+            b[k] = p ? v : u;
+            b[r] = p ? u : v;
         }
+#pragma unroll
         for (int r = k + 1; r < 5; r++) {
             const double m = A[r][k] / A[k][k];
+#pragma unroll
             for (int t = k; t < 5; t++) A[r][t] -= m * A[k][t];
             b[r] -= m * b[k];
         }
     }
+#pragma unroll
     for (int k = 4; k >= 0; k--) {
         double s = b[k];
+#pragma unroll
         for (int t = k + 1; t < 5; t++) s -= A[k][t] * x[t];
         x[k] = s / A[k][k];
     }
     return true;
 }
 
-__global__ void __launch_bounds__(kWarps * 32) project_kernel(ProjArgs a)
+// A double in another CTA's shared memory (same offset), rank `rank`.
+__device__ __forceinline__ double peer_load(const double *p, uint32_t rank)
 {
-    __shared__ double red[kSums][32];
+    double v;
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(tc::mapa_cluster(tc::smem_u32(p), rank)) : "memory");
+    return v;
+}
+
+// (double)v, by moving the bits where v is a normal number.
+__device__ __forceinline__ double to_double(float v)
+{
+    const uint32_t u = __float_as_uint(v);
+    if (((u >> 23) & 255u) - 1u < 254u)
+        return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(u << 29));
+    return (double)v;
+}
+
+template <bool M5, int LC>
+__global__ void __launch_bounds__(kWarps * 32) project_kernel(const __grid_constant__ ProjArgs a, int cs)
+{
+    extern __shared__ __align__(16) double red[];  // [kWarps][kSums][32], then the CTA's sums [kSums][32]
     __shared__ double xs[5][32];
+    double *mine = red + kWarps * kSums * 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int cell = blockIdx.x * 32 + lane;
+    const int rank = (int)blockIdx.x % cs;
+    constexpr int G = 32 / LC;  // lines side by side in a warp
+    const int col = lane % LC;
+    const int cell = (int)blockIdx.x / cs * LC + col;
     const bool live = cell < a.ncells;
-    const int n = a.d.n_pnt;
+    const int first = (rank * kWarps + warp) * G + lane / LC, step = cs * kWarps * G;
     double s[kSums];
 #pragma unroll
     for (int k = 0; k < kSums; k++) s[k] = 0.;
     if (live) {
-        for (int i = warp; i < n; i += kWarps) {
-            const size_t o = (size_t)i * a.ld + cell;
-            const double fv = a.f[o], nv = a.nu[o], gv = a.gain[o];
-            const double ph[5] = {1.0, a.phi[n + i], a.phi[2 * n + i], a.phi[3 * n + i], a.phi[4 * n + i]};
-            const double fn = fv * nv, r = gv - fn;
+        for (int l = first; l < a.nlines; l += step) {
+            const int4 ln = __ldg(a.lines + l);
+            double S0 = 0., S1 = 0., S2 = 0., S3 = 0., S4 = 0., R0 = 0., R1 = 0., R2 = 0., M0 = 0., M1 = 0., M2 = 0.;
+            const double2 *zp = a.zpow + 2 * ln.z;
+            size_t o = (size_t)ln.x * a.ld + cell;
+#pragma unroll 4
+            for (int i = ln.x; i < ln.y; i++, zp += 2, o += a.ld) {
+                const double fv = to_double(a.f[o]), nv = to_double(a.nu[o]), gv = to_double(a.gain[o]);
+                const double z = zp[0].x, z2 = zp[0].y;
+                const double fn = fv * nv, r = gv - fn;
+                R0 += r;
+                R1 += r * z;
+                R2 += r * z2;
+                S0 += fn;
+                S1 += fn * z;
+                S2 += fn * z2;
+                S3 += fn * zp[1].x;
+                S4 += fn * zp[1].y;
+                M0 += fv;
+                if (M5) {
+                    M1 += fv * z;
+                    M2 += fv * z2;
+                }
+            }
+            const double2 xy = __ldg(a.line_xy + l);
+            const double x = xy.x, y = xy.y, rho = x * x + y * y;
+            const double E0 = rho * S0 + S2, E1 = rho * S1 + S3, E2 = rho * (E0 + S2) + S4, xS = x * S0, yS = y * S0;
+            s[0] += R0;
+            s[1] += x * R0;
+            s[2] += y * R0;
+            s[3] += R1;
+            s[4] += rho * R0 + R2;
+            s[5] += S0;
+            s[6] += xS;
+            s[7] += yS;
+            s[8] += S1;
+            s[9] += E0;
+            s[10] += x * xS;
+            s[11] += x * yS;
+            s[12] += x * S1;
+            s[13] += x * E0;
+            s[14] += y * yS;
+            s[15] += y * S1;
+            s[16] += y * E0;
+            s[17] += S2;
+            s[18] += E1;
+            s[19] += E2;
+            s[20] += M0;
+            if (M5) {
+                s[21] += x * M0;
+                s[22] += y * M0;
+                s[23] += M1;
+                s[24] += rho * M0 + M2;
+            }
+        }
+    }
+    // combine the lane groups' partial sums, the warps' in warp order, then the
+    // CTAs' in rank order
 #pragma unroll
-            for (int k = 0; k < 5; k++) s[k] += r * ph[k];
+    for (int k = 0; k < kSums; k++) {
+#pragma unroll
+        for (int w = LC; w < 32; w *= 2) s[k] += __shfl_xor_sync(0xffffffffu, s[k], w);
+        red[((size_t)warp * kSums + k) * 32 + lane] = s[k];
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < kSums * 32; t += kWarps * 32) {
+        double v = red[t];
+        for (int w = 1; w < kWarps; w++) v += red[(size_t)w * kSums * 32 + t];
+        mine[t] = v;
+    }
+    if (cs > 1) tc::cluster_sync();
+    else __syncthreads();
+    if (rank == 0) {
+        if (cs > 1) {
+            for (int t = threadIdx.x; t < kSums * 32; t += kWarps * 32) {
+                double v = mine[t];
+                for (int k = 1; k < cs; k++) v += peer_load(mine + t, (uint32_t)k);
+                red[t] = v;
+            }
+            __syncthreads();
+        }
+        if (warp == 0) {
+            const double *all = cs > 1 ? red : mine;
+            double tot[kSums];
+#pragma unroll
+            for (int k = 0; k < kSums; k++) tot[k] = all[k * 32 + lane];
+            double A[5][5], B[5], X[5];
             int t = 5;
+#pragma unroll
+            for (int k = 0; k < 5; k++) B[k] = tot[k];
 #pragma unroll
             for (int k = 0; k < 5; k++)
 #pragma unroll
-                for (int l = k; l < 5; l++) s[t++] += fn * ph[k] * ph[l];
+                for (int l = k; l < 5; l++) {
+                    A[k][l] = tot[t];
+                    A[l][k] = tot[t];
+                    t++;
+                }
+            bool finite = true;
 #pragma unroll
-            for (int k = 0; k < 5; k++) s[20 + k] += fv * ph[k];
+            for (int k = 0; k < kSums; k++) finite = finite && isfinite(tot[k]);
+            const bool solved = finite && solve5(A, B, X);
+            if (!solved) {
+#pragma unroll
+                for (int k = 0; k < 5; k++) X[k] = 0.;
+                // recorded for gd_ctx_check: the flags OR together, the smallest
+                // failing cell wins, so the record does not depend on scheduling
+                if (live && lane < LC && a.status && (!finite || tot[20] != 0.0)) {  // an empty cell has nothing to correct
+                    atomicOr(a.status, finite ? 2u : 1u);
+                    atomicMin(a.status + 1, (unsigned int)cell);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 5; k++) xs[k][lane] = X[k];
+            if (live && lane < LC) {
+                if (a.x)
+#pragma unroll
+                    for (int k = 0; k < 5; k++) a.x[(size_t)cell * 5 + k] = X[k];
+                if (M5 && a.m5)
+#pragma unroll
+                    for (int k = 0; k < 5; k++) a.m5[(size_t)cell * 5 + k] = tot[20 + k] * (double)a.d.d3v;
+            }
         }
     }
-    // combine the warps' partial sums in warp order
-    for (int w = 0; w < kWarps; w++) {
-        if (warp == w)
+    double X[5];
+    if (cs > 1) {
+        tc::cluster_sync();
 #pragma unroll
-            for (int k = 0; k < kSums; k++) red[k][lane] = (w == 0 ? 0. : red[k][lane]) + s[k];
+        for (int k = 0; k < 5; k++) X[k] = peer_load(&xs[k][lane], 0);
+        // rank 0's shared memory stays until every CTA has read it
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    } else {
         __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 5; k++) X[k] = xs[k][lane];
     }
-    if (warp == 0) {
-        double tot[kSums];
-#pragma unroll
-        for (int k = 0; k < kSums; k++) tot[k] = red[k][lane];
-        double A[5][5], B[5], X[5];
-        int t = 5;
-        for (int k = 0; k < 5; k++) B[k] = tot[k];
-        for (int k = 0; k < 5; k++)
-            for (int l = k; l < 5; l++) {
-                A[k][l] = tot[t];
-                A[l][k] = tot[t];
-                t++;
-            }
-        bool finite = true;
-#pragma unroll
-        for (int k = 0; k < kSums; k++) finite = finite && isfinite(tot[k]);
-        const bool solved = finite && solve5(A, B, X);
-        if (!solved) {
-            for (int k = 0; k < 5; k++) X[k] = 0.;
-            // recorded for gd_ctx_check: the flags OR together, the smallest
-            // failing cell wins, so the record does not depend on scheduling
-            if (live && a.status && (!finite || tot[20] != 0.0)) {  // an empty cell has nothing to correct
-                atomicOr(a.status, finite ? 2u : 1u);
-                atomicMin(a.status + 1, (unsigned int)cell);
+    if (live) {
+        for (int l = first; l < a.nlines; l += step) {
+            const int4 ln = __ldg(a.lines + l);
+            const double2 xy = __ldg(a.line_xy + l);
+            const double c0 = 1. + X[0] + X[1] * xy.x + X[2] * xy.y + X[4] * (xy.x * xy.x + xy.y * xy.y);
+            const double2 *zp = a.zpow + 2 * ln.z;
+            size_t o = (size_t)ln.x * a.ld + cell;
+#pragma unroll 4
+            for (int i = ln.x; i < ln.y; i++, zp += 2, o += a.ld) {
+                const double fv = to_double(a.f[o]), nv = to_double(a.nu[o]), gv = to_double(a.gain[o]);
+                const double nc = nv * (c0 + X[3] * zp->x + X[4] * zp->y);
+                const double qv = gv - fv * nc;
+                if (a.nu_corr) a.nu_corr[o] = (float)nc;
+                if (a.q) a.q[o] = qv;
+                if (a.update) a.f_out[o] = (float)(fv + (double)a.dt * qv);
             }
         }
-        for (int k = 0; k < 5; k++) xs[k][lane] = X[k];
-        if (live) {
-            if (a.x)
-                for (int k = 0; k < 5; k++) a.x[(size_t)cell * 5 + k] = X[k];
-            if (a.m5)
-                for (int k = 0; k < 5; k++) a.m5[(size_t)cell * 5 + k] = tot[20 + k] * (double)a.d.d3v;
-        }
     }
-    __syncthreads();
-    if (!live) return;
-    const double X0 = xs[0][lane], X1 = xs[1][lane], X2 = xs[2][lane], X3 = xs[3][lane], X4 = xs[4][lane];
-    for (int i = warp; i < n; i += kWarps) {
-        const size_t o = (size_t)i * a.ld + cell;
-        const double fv = a.f[o], nv = a.nu[o], gv = a.gain[o];
-        const double scale = 1. + X0 + X1 * a.phi[n + i] + X2 * a.phi[2 * n + i] +
-                             X3 * a.phi[3 * n + i] + X4 * a.phi[4 * n + i];
-        const double nc = nv * scale;
-        const double qv = gv - fv * nc;
-        if (a.nu_corr) a.nu_corr[o] = (float)nc;
-        if (a.q) a.q[o] = qv;
-        if (a.update) a.f_out[o] = (float)(fv + (double)a.dt * qv);
-    }
+    if (cs > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // Per-block maximum of nu' (non-negative); a second launch with one block
@@ -282,9 +410,33 @@ int run_project(Context &c, const float *f, const float *nu, const float *gain, 
                 float *nu_corr, double *q, double *x, int fixed_dt_mode, float dt, float *f_out,
                 double *m5, cudaStream_t st)
 {
-    ProjArgs a{c.d, f, nu, gain, ld, ncells, c.d_phi, nu_corr, q, x, fixed_dt_mode ? 1 : 0, dt, f_out, m5,
-               c.d_status};
-    project_kernel<<<(ncells + 31) / 32, kWarps * 32, 0, st>>>(a);
+    const ProjArgs a{c.d,   f, nu, gain, ld,                     ncells, c.nlines, c.d_lines, c.d_line_xy, c.d_zpow, nu_corr,
+                     q,     x, fixed_dt_mode ? 1 : 0, dt, f_out, m5,     c.d_status};
+    // cells per warp: 32, or eight or one when a cluster per 32 cells leaves
+    // SMs idle (20^3: 600 cells 0.230 ms with 32, 0.256 with 8; 256 cells 0.132
+    // and 0.105; one cell 0.132, 0.062 and 0.060 with 1)
+    const int lc = ncells > 512 ? 32 : ncells > 8 ? 8 : 1;
+    // CTAs per lc cells: about six CTAs per SM, so that the last wave costs little
+    const int blocks = (ncells + lc - 1) / lc;
+    int cs = 1;
+    while (cs < 8 && blocks * cs < 6 * c.sm_count) cs *= 2;
+    auto kern = lc == 32 ? (m5 ? project_kernel<true, 32> : project_kernel<false, 32>)
+                : lc == 8 ? (m5 ? project_kernel<true, 8> : project_kernel<false, 8>)
+                          : (m5 ? project_kernel<true, 1> : project_kernel<false, 1>);
+    GD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProjSmem));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(blocks * cs));
+    cfg.blockDim = dim3(kWarps * 32);
+    cfg.dynamicSmemBytes = kProjSmem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)cs;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    GD_CUDA(cudaLaunchKernelEx(&cfg, kern, a, cs));
     GD_CUDA(cudaGetLastError());
     return GD_OK;
 }
