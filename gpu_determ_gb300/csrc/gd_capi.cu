@@ -661,7 +661,11 @@ int gd_ctx_check(gd_ctx *ctx, gd_stream stream)
         GD_CUDA(cudaMemcpyAsync(c.d_status, clear, sizeof(clear), cudaMemcpyHostToDevice, st));
         GD_CUDA(cudaStreamSynchronize(st));
     }
-    bool cm_timeout = false, pt_timeout = false;
+    bool cm_timeout = false, pt_timeout = false, orbit_timeout = false;
+    if (c.orbit) {
+        const int rc = gd::orbit_take_timeout(c, st, &orbit_timeout);
+        if (rc) return rc;
+    }
     if (c.cmatrix) {
         const int rc = gd::cmatrix_take_timeout(c.cmatrix, st, &cm_timeout);
         if (rc) return rc;
@@ -673,11 +677,12 @@ int gd_ctx_check(gd_ctx *ctx, gd_stream stream)
     std::string msg;
     if (cm_timeout) msg += "collision-matrix kernel: a pipeline wait timed out";
     if (pt_timeout) msg += std::string(msg.empty() ? "" : "; ") + "pair tensor-core gain kernel: a pipeline wait timed out";
+    if (orbit_timeout) msg += std::string(msg.empty() ? "" : "; ") + "FP32 gain kernel: a pipeline wait timed out";
     if (h[0])
         msg += std::string(msg.empty() ? "" : "; ") +
                (h[0] & 1u ? "non-finite distribution, frequency or gain" : "singular conservation system") +
                " in the projection (first affected cell " + std::to_string(h[1]) + ")";
-    if (cm_timeout || pt_timeout) return set_error(GD_ERR_CUDA, msg);
+    if (cm_timeout || pt_timeout || orbit_timeout) return set_error(GD_ERR_CUDA, msg);
     if (h[0]) return set_error(GD_ERR_SINGULAR, msg);
     return GD_OK;
 }

@@ -61,12 +61,14 @@ struct Scratch {
 // lattice's reflections, bit a of e: upper half of axis a).
 struct OrbitGain {
     int cpt = 8, nslot = 0, norb = 0, pcap = 0, mcap = 0, nsteps = 0;
-    size_t smem = 0;
+    uint32_t p_at = 0, zero_at = 0;  // shared-memory offsets of the P rows and of the zero C row
+    size_t smem = 0, stream_bytes = 0;
     std::vector<int> cuts;            // steps between which the walk may be cut (no D continues)
     std::vector<double> cost_prefix;  // work before each cut
     int *row_node = nullptr;          // [n_pnt]
     uint4 *stream = nullptr;
-    int *start = nullptr;  // [step][warp] first chunk
+    int *start = nullptr;  // [step][warp] position in the stream, in 16-byte units
+    int *err = nullptr;    // set by the kernel when a copy of the stream is not seen to land
     int opad = 0;               // orbits padded to the loss kernel's tile
     float *bx = nullptr;        // [8][o'][opad] loss matrices folded by the reflections' characters
     std::map<int, int *> bounds_dev;
@@ -229,6 +231,8 @@ size_t orbit_part_bytes(const Context &c, int ncells, int nchunks);
 int launch_orbit(Context &c, const float *f, int ncells, int ld, float *gain, void *buf, int nchunks,
                  const int *d_bounds, cudaStream_t st);
 int run_orbit(Context &c, const float *f, int ncells, int ld, float *gain, cudaStream_t st);
+// reads (synchronising st) and clears its pipeline time-out record
+int orbit_take_timeout(Context &c, cudaStream_t st, bool *timed_out);
 
 // pair-product gain with the contraction on the tensor cores (gd_pair_tc.cu)
 int pair_tc_build(Context &c);

@@ -16,8 +16,9 @@
 //    it and weights of absent products are not in the tables (20^3, R = 4.8:
 //    3.0e6 products, 2.4e6 group rows and 4.1e7 weight terms per cell; the class
 //    boxes hold 9.3e6, 3.9e6 and 1.4e8).
-//  - The outputs stay in registers for a whole chunk of the walk: warp w owns
-//    the orbits w, w + 16, ..., and reads each C row once per target.  No output
+//  - The outputs stay in registers for a whole chunk of the walk: a warp
+//    owns groups of four neighbouring orbits and reads each C row once per
+//    target.  No output
 //    is read back or written in between, and no two warps share one, so every
 //    sum has a fixed order and results are bitwise reproducible.
 //
@@ -27,17 +28,24 @@
 // accumulate over the parts).  Contraction works on blocks of four rows of
 // neighbouring |g|, whose shells overlap: one P row is read for four rows (1.2
 // times the terms, a third of the shared-memory reads).  What a warp has to do
-// is one linear stream of 512-byte chunks (products, contraction entries,
-// targets, step by step), copied ahead into a ring of shared memory with
-// cp.async, so that no table read waits for L2.
+// is one linear stream of 512-byte chunks (products, contraction blocks,
+// targets, step by step), copied ahead into a ring of shared memory by bulk
+// copies, so that no table read waits for L2 or takes load slots.  The tables
+// hold shared-memory offsets ready for use: an access costs one logic operation
+// and the load.
 //
-// Bound: shared-memory and L1 wavefronts (products, contraction and outputs
-// all read one row per operation).  It replaces gain_pair_kernel (gd_gain.cu)
-// on every lattice whose rows fit: 12^3 (R = 4.8), 1501 cells 20.3 -> 2.1 ms;
-// 16^3 (whole box), 256 cells 22.6 -> 5.8 ms; 20^3 (R = 4.8), one cell 10.5 ->
-// 0.30 ms; its error against FP64 is half as large (two-level sums: targets of
-// a step, then steps).
+// Bound: shared-memory wavefronts of the three phases (all read one row per
+// operation, the outputs' phase at the rate of the load unit) for 60 % of the
+// time, the rest the warps' own control flow, some 400 instructions per warp and
+// step.  It replaces gain_pair_kernel (gd_gain.cu) on every lattice whose rows
+// fit: 12^3 (R = 4.8), 1501 cells 20.3 -> 1.30 ms; 16^3 (whole box), 256 cells
+// 22.6 -> 3.82 ms; 20^3 (R = 4.8), one cell 10.5 -> 0.18 ms, 4096 cells 67.5 ms;
+// its error against FP64 is half as large (two-level sums: targets of a step,
+// then steps).  Measured and not better: 8, 12, 20 or 24 warps; groups of eight
+// slots with one target a round (73.4 ms at 20^3); chunk-free dense streams (78 ms:
+// a check per record costs more than the padding).
 #include "gd_internal.h"
+#include "gd_tc.cuh"
 
 #include <algorithm>
 #include <array>
@@ -50,23 +58,26 @@ namespace {
 
 constexpr int kOWarps = 16;
 constexpr int kOThreads = 32 * kOWarps;
-constexpr int kORows = 4;            // rows of a contraction block
-constexpr int kOChunk = 512;         // bytes of a stream chunk: one 16-byte copy per lane
-constexpr int kORing = 4 * kOChunk;  // a warp's ring
-constexpr int kOQuads = 6;           // contraction quads (80 bytes) per chunk
-constexpr int kOProd = 31;           // products per warp and step (one chunk, after its header)
-constexpr uint32_t kNoPair = 0xffff7fffu;
+constexpr int kORows = 4;                        // rows of a contraction block
+constexpr uint32_t kOChunk = 512;                // bytes of a stream chunk
+constexpr uint32_t kORing = 4 * kOChunk;         // a warp's ring: three chunks in flight
+constexpr uint32_t kOBars = kOWarps * kORing;    // offset of the rings' barriers
+constexpr uint32_t kOF = kOBars + 1024;          // offset of f
+constexpr uint32_t kOQuad = 80;                  // bytes of a contraction quad
+constexpr int kOSlots = 4;                       // output slots gathered side by side
+constexpr int kOGroup = 16;                      // rounds (two targets per slot, 32 bytes) of a group in a step: at most a chunk
 
 struct OrbitArgs {
-    const float *ft;      // [tile][row][CPT]
-    const uint4 *stream;  // per warp: the chunks of every step
-    const int *start;     // [step][warp] first chunk
-    const int *bounds;    // [chunks + 1] step bounds
+    const float *ft;              // [tile][row][CPT]
+    const unsigned char *stream;  // per warp: the chunks of every step
+    const int *start;             // [step][warp] first chunk
+    const int *bounds;            // [chunks + 1] step bounds
     const int *row_node;
-    float *part;          // [chunk][row][cells_pad], or null: write gain
+    float *part;                  // [chunk][row][cells_pad], or null: write gain
     float *gain;
+    int *err;                     // set to 1 when a copy is not seen to land
     int norb, ns, cells_pad, ncells, ld;
-    int pcap, mcap;
+    uint32_t p_at, zero_at;       // shared-memory offsets of the P rows and of the zero C row
 };
 
 // Two FP32 operations per instruction where a lane holds two cells.
@@ -103,6 +114,7 @@ struct Vec<8> {
         return make_float2(__fmaf_rn(w, b.x, c.x), __fmaf_rn(w, b.y, c.y));
     }
     static __device__ __forceinline__ T add(T a, T b) { return add2(a, b); }
+    static __device__ __forceinline__ T mul(T a, T b) { return make_float2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y)); }
 };
 template <>
 struct Vec<4> {
@@ -110,6 +122,7 @@ struct Vec<4> {
     static __device__ __forceinline__ T zero() { return 0.f; }
     static __device__ __forceinline__ T mac(T a, T b, T c) { return __fmaf_rn(a, b, c); }
     static __device__ __forceinline__ T add(T a, T b) { return __fadd_rn(a, b); }
+    static __device__ __forceinline__ T mul(T a, T b) { return __fmul_rn(a, b); }
 };
 
 template <typename T>
@@ -136,17 +149,17 @@ __device__ __forceinline__ float4 lds<float4>(uint32_t addr)
     return v;
 }
 template <>
-__device__ __forceinline__ uint2 lds<uint2>(uint32_t addr)
-{
-    uint2 v;
-    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
-    return v;
-}
-template <>
 __device__ __forceinline__ uint4 lds<uint4>(uint32_t addr)
 {
     uint4 v;
     asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+    return v;
+}
+template <>
+__device__ __forceinline__ uint32_t lds<uint32_t>(uint32_t addr)
+{
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
     return v;
 }
 __device__ __forceinline__ void sts(uint32_t addr, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
@@ -160,175 +173,235 @@ __global__ void __launch_bounds__(kOThreads, 1) orbit_gain_kernel(const __grid_c
 {
     using V = Vec<CPT>;
     using T = typename V::T;
-    constexpr uint32_t kRow = 32 * sizeof(T);      // bytes of a P or C row
-    constexpr int kShift = CPT == 8 ? 5 : 4;       // (row << 3 | e) -> bytes: e selects CPT cells
+    constexpr uint32_t kRow = 32 * sizeof(T);  // bytes of a P or C row
+    // rings, their barriers, f (and eight zero rows), P and C
     extern __shared__ __align__(1024) unsigned char smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t lb = lane * (uint32_t)sizeof(T);  // r * (CPT cells) + cell, in bytes
     const int r = lane >> 2;
-    // rings, f, P and C
-    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(smem) + warp * kORing;
-    const uint32_t F = (uint32_t)__cvta_generic_to_shared(smem) + kOWarps * kORing;
-    const uint32_t P = F + (uint32_t)a.ns * CPT * 4, C = P + (uint32_t)a.pcap * kRow;
+    const uint32_t sm = (uint32_t)__cvta_generic_to_shared(smem), slb = sm + lb;
 
     const int s0 = a.bounds[blockIdx.y], s1 = a.bounds[blockIdx.y + 1];
     if (s0 < s1) {
-        // the ring: chunk c sits at (c % 4) chunks; three chunks are in flight
-        const uint4 *src = a.stream + (size_t)__ldg(a.start + s0 * kOWarps + warp) * (kOChunk / 16) + lane;
-        uint32_t head = 0;  // bytes consumed so far
-        auto fetch = [&](uint32_t at) {
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ring + (at & (kORing - 1)) + lane * 16), "l"(src)
-                         : "memory");
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            src += kOChunk / 16;
-        };
-        for (int k = 0; k < 3; k++) fetch(k * kOChunk);
-        // the next chunk has landed: its address; the chunk before it is done with
-        auto next = [&]() -> uint32_t {
-            __syncwarp();
-            fetch(head + 3 * kOChunk);
-            asm volatile("cp.async.wait_group 3;" ::: "memory");
-            __syncwarp();
-            const uint32_t at = ring + (head & (kORing - 1));
-            head += kOChunk;
-            return at;
-        };
-        const float4 *ft = reinterpret_cast<const float4 *>(a.ft + (size_t)blockIdx.x * a.ns * CPT);
-        for (int i = threadIdx.x; i < a.ns * CPT / 4; i += kOThreads) {
-            const float4 v = __ldg(ft + i);
-            asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(F + i * 16), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
-                         : "memory");
+        const uint32_t ring = sm + warp * kORing, bar = sm + kOBars + warp * 32;
+        if (lane == 0) {
+            for (int k = 0; k < 4; k++) tc::mbar_init(bar + 8 * k, 1);
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
-        if (warp == 0) sts(C + a.mcap * kRow + lb, V::zero());  // padding targets read this row
+        __syncwarp();
+        // the ring: chunk c sits at (c % 4) chunks
+        const uint32_t first = (uint32_t)__ldg(a.start + s0 * kOWarps + warp) * 16u;
+        const unsigned char *src = a.stream + (first & ~(kOChunk - 1));
+        uint32_t issued = 0, taken = 0;
+        uint32_t at = 0, room = 0;  // the stream's position, and the bytes to its chunk's end
+        bool ok = true;
+        auto fetch = [&]() {
+            if (lane == 0) {
+                const uint32_t b = bar + 8 * (issued & 3);
+                tc::mbar_expect_tx(b, kOChunk);
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                 ring + (issued & 3) * kOChunk),
+                             "l"(src), "r"(kOChunk), "r"(b)
+                             : "memory");
+            }
+            src += kOChunk;
+            issued++;
+        };
+        // `bytes` of the stream at `at`, moving to the next chunk when this one has
+        // less left: it has landed, the one before it is done with and its place
+        // takes the third chunk ahead
+        auto need = [&](uint32_t bytes) -> bool {
+            if (room < bytes) {
+                __syncwarp();
+                fetch();
+                ok = __all_sync(0xffffffffu, tc::mbar_wait(bar + 8 * (taken & 3), (taken >> 2) & 1, a.err)) && ok;
+                at = ring + (taken & 3) * kOChunk;
+                taken++;
+                room = kOChunk;
+            }
+            return ok;
+        };
+        auto skip = [&](uint32_t bytes) {
+            at += bytes;
+            room -= bytes;
+        };
+        for (int k = 0; k < 3; k++) fetch();
+        const float4 *ft = reinterpret_cast<const float4 *>(a.ft + (size_t)blockIdx.x * a.ns * CPT);
+        for (int i = threadIdx.x; i < (a.ns + 8) * CPT / 4; i += kOThreads)
+            *reinterpret_cast<float4 *>(smem + kOF + i * 16) = i < a.ns * CPT / 4 ? __ldg(ft + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (warp == 0) sts(slb + a.zero_at, V::zero());  // padding targets read this row
+        need(1);
+        skip(first & (kOChunk - 1));
         T acc[NSLOT];
 #pragma unroll
         for (int j = 0; j < NSLOT; j++) acc[j] = V::zero();
         __syncthreads();
 
-        // C rows of a step into this warp's outputs: per slot a count of quads,
-        // then 16-bit entries row << 3 | e; the list may wrap around the ring
-        auto gather = [&](int nchunks) {
-            if (nchunks == 0) return;
-            uint32_t pos = next() - ring;
-            if (nchunks == 2) {  // the second chunk too, the first still in use
-                asm volatile("cp.async.wait_group 2;" ::: "memory");
-                __syncwarp();
-            }
-            uint32_t cpos = pos;
-            pos += NSLOT;
+        // C rows of a step into this warp's outputs: a count of rounds per group of
+        // four slots, then the rounds: two offsets (of row and octant, the lane's
+        // own by exclusive or) for each of the four, so that eight independent
+        // loads are in flight
+        auto gather = [&]() {
+            constexpr uint32_t kCounts = (NSLOT / kOSlots + 15) & ~15;
+            if (!need(kCounts)) return;
+            uint32_t cw[(NSLOT / kOSlots + 3) / 4];
 #pragma unroll
-            for (int j4 = 0; j4 < NSLOT; j4 += 8, cpos += 8) {
-                const uint2 cw2 = lds<uint2>(ring + cpos);
+            for (int k = 0; k < (NSLOT / kOSlots + 3) / 4; k++) cw[k] = lds<uint32_t>(at + 4 * k);
+            skip(kCounts);
 #pragma unroll
-                for (int jj = 0; jj < 8; jj++) {
-                    const uint32_t cw = jj < 4 ? cw2.x : cw2.y;
-                    const int n = (cw >> (8 * (jj & 3))) & 255;
-                    T s = V::zero();
+            for (int g = 0; g < NSLOT / kOSlots; g++) {
+                const int n = (cw[g / 4] >> (8 * (g & 3))) & 255;
+                if (n == 0) continue;
+                if (!need(32 * n)) return;
+                room -= 32 * n;
+                T s0 = V::zero(), s1 = V::zero(), s2 = V::zero(), s3 = V::zero();
+                uint4 u = lds<uint4>(at), v = lds<uint4>(at + 16);
 #pragma unroll 1
-                    for (int q = 0; q < n; q++, pos += 8) {
-                        const uint2 v = lds<uint2>(ring + (pos & (kORing - 1)));
-                        constexpr uint32_t m = 0xffffu << kShift;
-                        const T c0 = lds<T>(C + (((v.x << kShift) & m) ^ lb)), c1 = lds<T>(C + (((v.x >> (16 - kShift)) & m) ^ lb));
-                        const T c2 = lds<T>(C + (((v.y << kShift) & m) ^ lb)), c3 = lds<T>(C + (((v.y >> (16 - kShift)) & m) ^ lb));
-                        s = V::add(s, V::add(V::add(c0, c1), V::add(c2, c3)));
-                    }
-                    acc[j4 + jj] = V::add(acc[j4 + jj], s);
+                for (int q = 0; q < n; q++) {
+                    const T a0 = lds<T>(sm + (u.x ^ lb)), b0 = lds<T>(sm + (u.y ^ lb)), a1 = lds<T>(sm + (u.z ^ lb)),
+                            b1 = lds<T>(sm + (u.w ^ lb)), a2 = lds<T>(sm + (v.x ^ lb)), b2 = lds<T>(sm + (v.y ^ lb)),
+                            a3 = lds<T>(sm + (v.z ^ lb)), b3 = lds<T>(sm + (v.w ^ lb));
+                    at += q + 1 < n ? 32 : 0;
+                    u = lds<uint4>(at);  // the next round's (after the last: its own again)
+                    v = lds<uint4>(at + 16);
+                    s0 = V::add(s0, V::add(a0, b0));
+                    s1 = V::add(s1, V::add(a1, b1));
+                    s2 = V::add(s2, V::add(a2, b2));
+                    s3 = V::add(s3, V::add(a3, b3));
                 }
-            }
-            if (nchunks == 2) {
-                __syncwarp();
-                fetch(head + 3 * kOChunk);
-                head += kOChunk;
+                at += 32;
+                acc[4 * g] = V::add(acc[4 * g], s0);
+                acc[4 * g + 1] = V::add(acc[4 * g + 1], s1);
+                acc[4 * g + 2] = V::add(acc[4 * g + 2], s2);
+                acc[4 * g + 3] = V::add(acc[4 * g + 3], s3);
             }
         };
 
-        int tgt_chunks = 0;
+        bool targets = false;
         for (int st = s0; st < s1; st++) {
-            gather(tgt_chunks);
-            // products: this warp's rows warp, warp + 16, ...
-            uint32_t at = next();
-            const uint4 hd = lds<uint4>(at);  // products, contraction quads, target chunks
-            uint32_t prow = P + warp * kRow + lb;
-#pragma unroll 1
-            for (uint32_t k = 0; k < hd.x; k++, prow += kOWarps * kRow) {
-                at += 16;
-                const uint4 d = lds<uint4>(at);
-                const uint32_t w[4] = {d.x, d.y, d.z, d.w};
-                T x[4], y[4];
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    x[q] = y[q] = V::zero();
-                    if ((int)w[q] >= 0) {
-                        constexpr uint32_t m = 0x7fffu << kShift;
-                        x[q] = lds<T>(F + (((w[q] << kShift) & m) ^ lb));
-                        y[q] = lds<T>(F + (((w[q] >> (16 - kShift)) & m) ^ lb));
-                    }
-                }
-                T p = V::mac(x[0], y[0], V::mac(x[1], y[1], V::zero()));
-                p = V::add(p, V::mac(x[2], y[2], V::mac(x[3], y[3], V::zero())));
-                // a reflection of an axis on which D is its own mirror repeats D
-                const uint32_t self = ((w[0] >> 15) & 1u) | ((w[1] >> 14) & 2u) | ((w[2] >> 13) & 4u);
-                if (self & (uint32_t)r) p = V::zero();
-                sts(prow, p);
+            if (targets) gather();
+            // products: rows of four pairs, then rows of at most two; a missing pair
+            // reads the zero rows; low bits of the first offset: the axes on which
+            // D is its own mirror, whose reflections repeat D
+            uint4 hd = make_uint4(0, 0, 0, 0);  // rows of four, rows of two, first row of two, blocks (bit 31: targets)
+            if (need(16)) {
+                hd = lds<uint4>(at);
+                skip(16);
             }
-            __syncthreads();
-            // contraction: per quad four entries {P offset; the block's four weights};
-            // bit 0 of the first offset: last quad of its block, bit 1: the block's
-            // sums continue those of an earlier part; the C row in the second's top bits
-            T c0 = V::zero(), c1 = V::zero(), c2 = V::zero(), c3 = V::zero();
-            for (uint32_t left = hd.y; left > 0;) {
-                uint32_t e = next();
-                const uint32_t n = min(left, (uint32_t)kOQuads);
+            uint32_t prow = slb + a.p_at + warp * kRow;
+            for (uint32_t left = hd.x; left > 0;) {
+                if (!need(32)) break;
+                const uint32_t n = min(left, room / 32);
                 left -= n;
+                room -= 32 * n;
 #pragma unroll 1
-                for (uint32_t q = 0; q < n; q++, e += 80) {
-                    const uint4 o = lds<uint4>(e);
-                    const float4 w0 = lds<float4>(e + 16), w1 = lds<float4>(e + 32), w2 = lds<float4>(e + 48),
-                                 w3 = lds<float4>(e + 64);
-                    const T p0 = lds<T>(P + (o.x & ~3u) + lb), p1 = lds<T>(P + (o.y & 0x3ffffu) + lb);
-                    const T p2 = lds<T>(P + o.z + lb), p3 = lds<T>(P + o.w + lb);
-                    const uint32_t cr = C + (o.y >> 18) * kRow + lb;
-                    if (o.x & 2u) {
-                        c0 = lds<T>(cr);
-                        c1 = lds<T>(cr + kRow);
-                        c2 = lds<T>(cr + 2 * kRow);
-                        c3 = lds<T>(cr + 3 * kRow);
+                for (uint32_t k = 0; k < n; k++, prow += kOWarps * kRow, at += 32) {
+                    const uint4 u = lds<uint4>(at), w = lds<uint4>(at + 16);
+                    const uint32_t self = u.x & 7u;
+                    const T x0 = lds<T>(sm + ((u.x & ~7u) ^ lb)), y0 = lds<T>(sm + (u.y ^ lb)), x1 = lds<T>(sm + (u.z ^ lb)),
+                            y1 = lds<T>(sm + (u.w ^ lb)), x2 = lds<T>(sm + (w.x ^ lb)), y2 = lds<T>(sm + (w.y ^ lb)),
+                            x3 = lds<T>(sm + (w.z ^ lb)), y3 = lds<T>(sm + (w.w ^ lb));
+                    T p = V::add(V::mac(x0, y0, V::mul(x1, y1)), V::mac(x2, y2, V::mul(x3, y3)));
+                    if (self && (self & (uint32_t)r)) p = V::zero();
+                    sts(prow, p);
+                }
+            }
+            prow = slb + a.p_at + (hd.z + warp) * kRow;
+            for (uint32_t left = hd.y; ok && left > 0;) {
+                if (!need(16)) break;
+                const uint32_t n = min(left, room / 16);
+                left -= n;
+                room -= 16 * n;
+#pragma unroll 1
+                for (uint32_t k = 0; k < n; k += 2, prow += 2 * kOWarps * kRow, at += 32) {
+                    // two rows at a time (the second past the last: not stored)
+                    const uint4 u = lds<uint4>(at), w = lds<uint4>(k + 1 < n ? at + 16 : at);
+                    const T x0 = lds<T>(sm + ((u.x & ~7u) ^ lb)), y0 = lds<T>(sm + (u.y ^ lb)), x1 = lds<T>(sm + (u.z ^ lb)),
+                            y1 = lds<T>(sm + (u.w ^ lb)), x2 = lds<T>(sm + ((w.x & ~7u) ^ lb)), y2 = lds<T>(sm + (w.y ^ lb)),
+                            x3 = lds<T>(sm + (w.z ^ lb)), y3 = lds<T>(sm + (w.w ^ lb));
+                    T p = V::mac(x0, y0, V::mul(x1, y1)), p2 = V::mac(x2, y2, V::mul(x3, y3));
+                    if ((u.x | w.x) & 7u) {
+                        if (u.x & (uint32_t)r) p = V::zero();
+                        if (w.x & (uint32_t)r) p2 = V::zero();
                     }
+                    sts(prow, p);
+                    if (k + 1 < n) sts(prow + kOWarps * kRow, p2);
+                }
+                if (n & 1) {
+                    at -= 16;
+                    prow -= kOWarps * kRow;
+                }
+            }
+            if (__syncthreads_or(!ok)) {
+                ok = false;
+                break;
+            }
+            // contraction: blocks {quads, C offset, 1: its sums continue those of an
+            // earlier part}, each quad four entries {P offset; the four rows' weights}
+            for (uint32_t b = hd.w & 0x7fffffffu; b > 0; b--) {
+                if (!need(16)) break;
+                const uint4 h = lds<uint4>(at);
+                skip(16);
+                const uint32_t cr = slb + h.y;
+                T c0 = V::zero(), c1 = V::zero(), c2 = V::zero(), c3 = V::zero();
+                if (h.z) {
+                    c0 = lds<T>(cr);
+                    c1 = lds<T>(cr + kRow);
+                    c2 = lds<T>(cr + 2 * kRow);
+                    c3 = lds<T>(cr + 3 * kRow);
+                }
+                for (uint32_t left = h.x; left > 0;) {
+                    if (!need(kOQuad)) break;
+                    const uint32_t n = min(left, room / kOQuad);
+                    left -= n;
+                    room -= kOQuad * n;
+                    uint4 o = lds<uint4>(at);
+#pragma unroll 1
+                    for (uint32_t q = 0; q < n; q++) {
+                        const float4 w0 = lds<float4>(at + 16), w1 = lds<float4>(at + 32), w2 = lds<float4>(at + 48),
+                                     w3 = lds<float4>(at + 64);
+                        const T p0 = lds<T>(o.x + slb), p1 = lds<T>(o.y + slb), p2 = lds<T>(o.z + slb), p3 = lds<T>(o.w + slb);
+                        at += q + 1 < n ? kOQuad : 0;
+                        o = lds<uint4>(at);  // the next quad's (after the last: its own again)
 #define GD_MAC(wv, pv)           \
     c0 = V::mac((wv).x, pv, c0); \
     c1 = V::mac((wv).y, pv, c1); \
     c2 = V::mac((wv).z, pv, c2); \
     c3 = V::mac((wv).w, pv, c3)
-                    GD_MAC(w0, p0);
-                    GD_MAC(w1, p1);
-                    GD_MAC(w2, p2);
-                    GD_MAC(w3, p3);
+                        GD_MAC(w0, p0);
+                        GD_MAC(w1, p1);
+                        GD_MAC(w2, p2);
+                        GD_MAC(w3, p3);
 #undef GD_MAC
-                    if (o.x & 1u) {
-                        sts(cr, c0);
-                        sts(cr + kRow, c1);
-                        sts(cr + 2 * kRow, c2);
-                        sts(cr + 3 * kRow, c3);
-                        c0 = c1 = c2 = c3 = V::zero();
                     }
+                    at += kOQuad;
                 }
+                if (!ok) break;
+                sts(cr, c0);
+                sts(cr + kRow, c1);
+                sts(cr + 2 * kRow, c2);
+                sts(cr + 3 * kRow, c3);
             }
-            tgt_chunks = (int)hd.z;
-            __syncthreads();
+            targets = (hd.w >> 31) != 0;
+            if (__syncthreads_or(!ok)) {
+                ok = false;
+                break;
+            }
         }
-        gather(tgt_chunks);
-        asm volatile("cp.async.wait_group 0;" ::: "memory");  // the copies ahead of the last chunk
+        if (ok && targets) gather();
+        // the copies in flight land before the CTA leaves
+        for (; taken != issued; taken++) tc::mbar_wait(bar + 8 * (taken & 3), (taken >> 2) & 1, a.err);
+        if (!ok) return;  // recorded in err
         // lane (r, cells): output row 8 o + r
         const int cell = blockIdx.x * CPT + (lane & 3) * (CPT / 4);
 #pragma unroll
         for (int j = 0; j < NSLOT; j++) {
-            const int o = warp + j * kOWarps;
+            const int o = (j / kOSlots * kOWarps + warp) * kOSlots + j % kOSlots;
             if (o >= a.norb) continue;
-            const int row = 8 * o + r;
             if (a.part) {
-                *reinterpret_cast<T *>(a.part + ((size_t)blockIdx.y * a.ns + row) * a.cells_pad + cell) = acc[j];
+                *reinterpret_cast<T *>(a.part + ((size_t)blockIdx.y * a.ns + 8 * o + r) * a.cells_pad + cell) = acc[j];
             } else {
-                float *g = a.gain + (size_t)__ldg(a.row_node + row) * a.ld + cell;
+                float *g = a.gain + (size_t)__ldg(a.row_node + 8 * o + r) * a.ld + cell;
                 const float *v = reinterpret_cast<const float *>(&acc[j]);
 #pragma unroll
                 for (int q = 0; q < CPT / 4; q++)
@@ -379,7 +452,8 @@ __global__ void orbit_reduce_kernel(const float *__restrict__ part, int nchunks,
 // One D of the low octant with anything to do.
 struct DItem {
     int K = 0, nblk = 0;
-    std::vector<uint4> prod;                   // by shell |n|
+    std::vector<std::array<int16_t, 9>> prod;  // by shell |n|: four pairs of rows (-1: none), their count
+    uint32_t self = 0;                         // axes on which D is its own mirror
     std::vector<int> blk_n;                    // entries per block
     std::vector<uint32_t> off;                 // P row per entry, ascending within a block
     std::vector<float4> w;
@@ -425,6 +499,7 @@ void orbit_free(Context &c)
     cudaFree(g->stream);
     cudaFree(g->start);
     cudaFree(g->bx);
+    cudaFree(g->err);
     for (auto &kv : g->bounds_dev) cudaFree(kv.second);
     delete g;
     c.orbit = nullptr;
@@ -440,8 +515,17 @@ int orbit_build(Context &c)
     // box, so each low-octant node has its seven mirrors
     std::vector<int> row_of(d.nxyz, -1), row_node;
     int norb = 0;
-    for (int m = 0; m < d.n_pnt; m++) {
-        if (c.ui[m] >= d.hx || c.vi[m] >= d.hy || c.wi[m] >= d.hz) continue;
+    // orbits in blocks of 2 x 2 x 2: the four slots a warp gathers side by side
+    // are then mostly of one block, with much the same number of targets in a D
+    std::vector<int> low;
+    for (int m = 0; m < d.n_pnt; m++)
+        if (c.ui[m] < d.hx && c.vi[m] < d.hy && c.wi[m] < d.hz) low.push_back(m);
+    auto block_key = [&](int m) {
+        const int x = c.ui[m], y = c.vi[m], z = c.wi[m];
+        return (((x >> 1) * 32 + (y >> 1)) * 32 + (z >> 1)) * 8 + (x & 1) * 4 + (y & 1) * 2 + (z & 1);
+    };
+    std::stable_sort(low.begin(), low.end(), [&](int p, int q) { return block_key(p) < block_key(q); });
+    for (int m : low) {
         for (int e = 0; e < 8; e++) {
             const int x = e & 1 ? d.nx - 1 - c.ui[m] : c.ui[m], y = e & 2 ? d.ny - 1 - c.vi[m] : c.vi[m],
                       z = e & 4 ? d.nz - 1 - c.wi[m] : c.wi[m];
@@ -481,7 +565,7 @@ int orbit_build(Context &c)
         for (int Did = t0; Did < d.nxyz; Did += nt) {
             const int D[3] = {Did / d.nyz, (Did / d.nz) % d.ny, Did % d.nz};
             DItem &it = items[Did];
-            const uint32_t self = (D[0] == d.nx - 1 ? 1u : 0u) | (D[1] == d.ny - 1 ? 2u : 0u) | (D[2] == d.nz - 1 ? 4u : 0u);
+            it.self = (D[0] == d.nx - 1 ? 1u : 0u) | (D[1] == d.ny - 1 ? 2u : 0u) | (D[2] == d.nz - 1 ? 4u : 0u);
             cls.clear();
             want.clear();
             n2.clear();
@@ -497,23 +581,23 @@ int orbit_build(Context &c)
                         }
                         // the four sign patterns l / l1: (+++), (+--), (++-), (+-+)
                         static const int pat[4] = {7, 1, 3, 5};
-                        uint32_t pw[4], have = 0;
-                        int np = 0;
+                        std::array<int16_t, 9> pw;
+                        pw.fill(-1);
+                        int have = 0;
                         for (int q = 0; q < 4; q++) {
                             const int t1 = at[pat[q]], t2 = at[7 - pat[q]];
-                            if (t1 >= 0 && t2 >= 0) pw[np++] = (uint32_t)t1 | (uint32_t)t2 << 16;
+                            if (t1 < 0 || t2 < 0) continue;
+                            pw[2 * have] = (int16_t)t1;
+                            pw[2 * have++ + 1] = (int16_t)t2;
                         }
-                        have = np;
-                        while (np < 4) pw[np++] = kNoPair;
+                        pw[8] = (int16_t)have;
                         const int k = (x2 * d.hy + y2) * d.hz + z2;
                         if (have) {
-                            for (int q = 0; q < 3; q++)
-                                if ((self >> q) & 1u) pw[q] |= 0x8000u;
                             it.K++;
                             cls.push_back(k);
                             n2.push_back((double)(d.du * n[0]) * (d.du * n[0]) + (double)(d.dv * n[1]) * (d.dv * n[1]) +
                                          (double)(d.dw * n[2]) * (d.dw * n[2]));
-                            it.prod.push_back(make_uint4(pw[0], pw[1], pw[2], pw[3]));
+                            it.prod.push_back(pw);
                         }
                         const int grp = gid[(n[0] * d.ny + n[1]) * d.nz + n[2]];
                         for (int s = 0; s < 8; s++) {
@@ -530,7 +614,7 @@ int orbit_build(Context &c)
                 by.resize(it.K);
                 for (int k = 0; k < it.K; k++) by[k] = k;
                 std::stable_sort(by.begin(), by.end(), [&](int x, int y) { return n2[x] < n2[y]; });
-                std::vector<uint4> sorted(it.K);
+                std::vector<std::array<int16_t, 9>> sorted(it.K);
                 for (int k = 0; k < it.K; k++) {
                     sorted[k] = it.prod[by[k]];
                     prow[cls[by[k]]] = k;
@@ -590,13 +674,14 @@ int orbit_build(Context &c)
     // tile width: eight cells where their outputs and rows fit, else four
     int max_smem = 0;
     GD_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c.device));
-    const int slots = (norb + kOWarps - 1) / kOWarps;
+    const int slots = (norb + kOWarps * kOSlots - 1) / (kOWarps * kOSlots) * kOSlots;
+    auto orbit_of = [](int w, int j) { return (j / kOSlots * kOWarps + w) * kOSlots + j % kOSlots; };
     int cpt = 0, nslot = 0, pcap = 0, mcap = 0;
     for (int w : {8, 4}) {
         if (!orbit_kernel(w, slots, &nslot)) continue;
-        const int rows = (max_smem - kOWarps * kORing - d.n_pnt * w * 4) / (32 * w) - 1;  // P and C rows
-        mcap = std::min(8184, std::max(mmax, rows * 2 / 5 / kORows * kORows));
-        pcap = std::min(kOWarps * kOProd, rows - mcap);
+        const int rows = (max_smem - (int)kOF - (d.n_pnt + 8) * w * 4) / (32 * w) - 1;  // P and C rows
+        mcap = std::max(mmax, rows * 2 / 5 / kORows * kORows);
+        pcap = rows - mcap;
         if (pcap >= 64) {
             cpt = w;
             break;
@@ -611,18 +696,19 @@ int orbit_build(Context &c)
     og->cuts.push_back(0);
     og->cost_prefix.push_back(0.0);
     double cost = 0.0;
+    // shared-memory offsets, held in the tables
+    const uint32_t f_row = 4u * (uint32_t)cpt, p_at = kOF + ((uint32_t)d.n_pnt + 8u) * f_row, c_at = p_at + (uint32_t)pcap * row_bytes;
+    const uint32_t zero_at = c_at + (uint32_t)mcap * row_bytes, zero_f = kOF + (uint32_t)d.n_pnt * f_row;
     std::vector<std::vector<uint4>> ws(kOWarps);  // the warps' streams
     std::vector<std::vector<int>> start(kOWarps);
     auto pad_chunk = [](std::vector<uint4> &v) {
         while (v.size() % (kOChunk / 16)) v.push_back(make_uint4(0, 0, 0, 0));
     };
-    std::vector<std::vector<uint16_t>> tl(norb);
-    const int max_quads = (2 * kOChunk - nslot) / 8;
-    auto list_quads = [&](int warp) {
-        int q = 0;
-        for (int o = warp; o < norb; o += kOWarps) q += ((int)tl[o].size() + 3) / 4;
-        return q;
+    auto need = [&](std::vector<uint4> &v, uint32_t bytes) {  // a record does not cross a chunk's end
+        const uint32_t used = (uint32_t)(v.size() % (kOChunk / 16)) * 16u;
+        if (used && kOChunk - used < bytes) pad_chunk(v);
     };
+    std::vector<std::vector<uint16_t>> tl(norb);  // per orbit: C row << 3 | octant
     // a step: rows [k0, k1) of each of its D, all of their C rows; the target
     // lists in tl (empty before a D's last part)
     struct Part {
@@ -634,13 +720,19 @@ int orbit_build(Context &c)
             bool cont;
         };
         std::vector<Blk> bl;
-        std::vector<const uint4 *> prod;
+        struct Row {
+            const std::array<int16_t, 9> *pairs;
+            uint32_t self;
+            int at;  // its P row
+        };
+        std::vector<Row> prod;
         int mrow = 0;
-        double entries = 0.0, targets = 0.0;
+        size_t targets = 0;
+        for (const auto &t : tl) targets += t.size();
         for (const Part &pt : parts) {
             const DItem &it = items[pt.item];
             const int kbase = (int)prod.size();
-            for (int k = pt.k0; k < pt.k1; k++) prod.push_back(&it.prod[k]);
+            for (int k = pt.k0; k < pt.k1; k++) prod.push_back(Row{&it.prod[k], it.self, 0});
             int e0 = 0;
             for (int b = 0; b < it.nblk; e0 += it.blk_n[b++]) {
                 const auto lo = it.off.begin() + e0, hi = lo + it.blk_n[b];
@@ -650,10 +742,17 @@ int orbit_build(Context &c)
                 // in the first part when no part has (its C rows are zero)
                 if (f0 == f1 && !(pt.k0 == 0 && it.blk_n[b] == 0)) continue;
                 bl.push_back(Blk{f1 - f0, pt.item, b, e0 + f0, mrow + b * kORows, pt.k0, kbase, f0 > 0});
-                entries += f1 - f0;
             }
             mrow += it.nblk * kORows;
         }
+        // P rows: those of three or four pairs first
+        int na = 0, nb = 0;
+        for (Row &rw : prod)
+            if ((*rw.pairs)[8] > 2) rw.at = na++;
+        for (Row &rw : prod)
+            if ((*rw.pairs)[8] <= 2) rw.at = na + nb++;
+        std::vector<const Row *> by_row(prod.size());
+        for (const Row &rw : prod) by_row[rw.at] = &rw;
         // the blocks go to the warps largest first, each to the least loaded
         std::stable_sort(bl.begin(), bl.end(), [](const Blk &x, const Blk &y) { return x.n > y.n; });
         std::vector<std::vector<const Blk *>> mine(kOWarps);
@@ -665,28 +764,40 @@ int orbit_build(Context &c)
         }
         for (int w = 0; w < kOWarps; w++) {
             std::vector<uint4> &v = ws[w];
-            start[w].push_back((int)(v.size() / (kOChunk / 16)));
+            need(v, 16);
+            start[w].push_back((int)v.size());
             const size_t h = v.size();
             v.push_back(make_uint4(0, 0, 0, 0));
-            uint32_t np = 0, nq = 0;
-            for (size_t k = w; k < prod.size(); k += kOWarps, np++) v.push_back(*prod[k]);
-            pad_chunk(v);
+            uint4 hd = make_uint4(0, 0, (uint32_t)na, (uint32_t)mine[w].size());
+            for (int half = 0; half < 2; half++) {
+                uint32_t &count = half ? hd.y : hd.x;
+                for (int k = (half ? na : 0) + w; k < (half ? na + nb : na); k += kOWarps, count++) {
+                    uint32_t off[8];
+                    for (int q = 0; q < 8; q++) {
+                        const int t = (*by_row[k]->pairs)[q];
+                        off[q] = t < 0 ? zero_f : kOF + (uint32_t)t * f_row;
+                    }
+                    off[0] |= by_row[k]->self;
+                    need(v, half ? 16 : 32);
+                    v.push_back(make_uint4(off[0], off[1], off[2], off[3]));
+                    if (!half) v.push_back(make_uint4(off[4], off[5], off[6], off[7]));
+                }
+            }
             for (const Blk *b : mine[w]) {
                 const DItem &it = items[b->item];
-                const int quads = std::max(1, (b->n + 3) / 4);
-                for (int q = 0; q < quads; q++, nq++) {
-                    if (nq && nq % kOQuads == 0) pad_chunk(v);
+                const int quads = (b->n + 3) / 4;
+                need(v, 16);
+                v.push_back(make_uint4((uint32_t)quads, c_at + (uint32_t)b->crow * row_bytes, b->cont ? 1u : 0u, 0));
+                for (int q = 0; q < quads; q++) {
                     uint32_t off[4];
                     float4 wt[4];
                     for (int z = 0; z < 4; z++) {
-                        const int e = 4 * q + z;
                         // padding repeats a row of the block with weight 0
-                        const int row = b->n ? (int)it.off[b->e0 + std::min(e, b->n - 1)] - b->k0 : 0;
-                        off[z] = (uint32_t)(row + b->kbase) * row_bytes;
+                        const int e = 4 * q + z, e1 = std::min(e, b->n - 1);
+                        off[z] = p_at + (uint32_t)prod[it.off[b->e0 + e1] - b->k0 + b->kbase].at * row_bytes;
                         wt[z] = e < b->n ? it.w[b->e0 + e] : make_float4(0.f, 0.f, 0.f, 0.f);
                     }
-                    off[0] |= (q == quads - 1 ? 1u : 0u) | (q == 0 && b->cont ? 2u : 0u);
-                    off[1] |= (uint32_t)b->crow << 18;
+                    need(v, kOQuad);
                     v.push_back(make_uint4(off[0], off[1], off[2], off[3]));
                     for (int z = 0; z < 4; z++) {
                         uint4 u;
@@ -695,29 +806,35 @@ int orbit_build(Context &c)
                     }
                 }
             }
-            pad_chunk(v);
-            uint32_t tc = 0;
-            std::vector<uint8_t> list(nslot, 0);
-            for (int j = 0, o = w; o < norb; j++, o += kOWarps) {
-                list[j] = (uint8_t)((tl[o].size() + 3) / 4);
-                targets += (double)tl[o].size();
-                for (size_t t = 0; t < (size_t)list[j] * 4; t++) {
-                    const uint16_t e = t < tl[o].size() ? tl[o][t] : (uint16_t)(mcap << 3);  // the zero row
-                    list.push_back((uint8_t)(e & 255));
-                    list.push_back((uint8_t)(e >> 8));
+            std::vector<uint8_t> counts((nslot / kOSlots + 15) / 16 * 16, 0);
+            for (int j = 0; j < nslot; j++)
+                if (const int o = orbit_of(w, j); o < norb)
+                    counts[j / kOSlots] = std::max(counts[j / kOSlots], (uint8_t)((tl[o].size() + 1) / 2));
+            if (*std::max_element(counts.begin(), counts.end())) {
+                hd.w |= 0x80000000u;
+                need(v, (uint32_t)counts.size());
+                v.resize(v.size() + counts.size() / 16);
+                std::memcpy(&v[v.size() - counts.size() / 16], counts.data(), counts.size());
+                for (int g = 0; g < nslot / kOSlots; g++) {
+                    need(v, 32u * counts[g]);
+                    for (size_t q = 0; q < counts[g]; q++) {
+                        uint32_t off[2 * kOSlots];
+                        for (int z = 0; z < 2 * kOSlots; z++) {
+                            const int o = orbit_of(w, g * kOSlots + z / 2);
+                            const size_t t = 2 * q + z % 2;
+                            off[z] = o < norb && t < tl[o].size() ? c_at + (uint32_t)(tl[o][t] >> 3) * row_bytes + (tl[o][t] & 7u) * f_row
+                                                                  : zero_at;
+                        }
+                        v.push_back(make_uint4(off[0], off[1], off[2], off[3]));
+                        v.push_back(make_uint4(off[4], off[5], off[6], off[7]));
+                    }
                 }
             }
-            if ((int)list.size() > nslot) {
-                list.resize((list.size() + 15) / 16 * 16, 0);
-                const size_t at = v.size();
-                v.resize(at + list.size() / 16);
-                std::memcpy(&v[at], list.data(), list.size());
-                pad_chunk(v);
-                tc = (uint32_t)((v.size() - at) / (kOChunk / 16));
-            }
-            v[h] = make_uint4(np, nq, tc, 0);
+            v[h] = hd;
         }
-        cost += 600.0 + 15.0 * (double)prod.size() + 3.5 * entries + 8.0 * (double)bl.size() + 2.3 * targets;
+        // instructions of the busiest warp: the kernel is bound by issue
+        const double most = (double)*std::max_element(load.begin(), load.end());
+        cost += 400.0 + 3.1 * (double)prod.size() + 15.0 * most + 0.34 * (double)targets;
         og->nsteps++;
         if (last) {
             og->cuts.push_back(og->nsteps);
@@ -735,63 +852,84 @@ int orbit_build(Context &c)
     auto add_targets = [&](const DItem &it) {
         for (const auto &t : it.targets) tl[t.first >> 3].push_back((uint16_t)((mrow + t.second) << 3 | (t.first & 7)));
         bool fits = true;
-        for (int w = 0; fits && w < kOWarps; w++) fits = list_quads(w) <= max_quads;
-        for (const auto &t : it.targets) fits = fits && tl[t.first >> 3].size() <= 1020;
+        for (const auto &t : it.targets) fits = fits && (int)tl[t.first >> 3].size() <= 2 * kOGroup;
         if (!fits)
             for (const auto &t : it.targets) tl[t.first >> 3].pop_back();
         return fits;
     };
+    // D past the P rows run in parts of their own; the others, largest first,
+    // are packed into steps with the largest that still fit, so that a step's
+    // barriers and per-slot work are paid for as much work as its rows hold
+    std::vector<int> rest;
     for (int Did = 0; Did < d.nxyz; Did++) {
         const DItem &it = items[Did];
         if (!it.nblk) continue;
-        if (it.K > kstep) {  // parts of its own
-            close();
-            const int parts = (it.K + kstep - 1) / kstep;
-            for (int p = 0; p < parts; p++) {
-                if (p == parts - 1 && !add_targets(it)) {
-                    delete og;
-                    return GD_OK;
-                }
-                emit({Part{Did, (int)((int64_t)it.K * p / parts), (int)((int64_t)it.K * (p + 1) / parts)}}, p == parts - 1);
-            }
+        if (it.K <= kstep) {
+            rest.push_back(Did);
             continue;
         }
-        for (int pass = 0; pass < 2; pass++) {
+        const int parts = (it.K + kstep - 1) / kstep;
+        for (int p = 0; p < parts; p++) {
+            if (p == parts - 1 && !add_targets(it)) {
+                delete og;
+                return GD_OK;
+            }
+            emit({Part{Did, (int)((int64_t)it.K * p / parts), (int)((int64_t)it.K * (p + 1) / parts)}}, p == parts - 1);
+        }
+    }
+    std::stable_sort(rest.begin(), rest.end(), [&](int x, int y) { return items[x].K > items[y].K; });
+    while (!rest.empty()) {
+        std::vector<int> left;
+        for (int Did : rest) {
+            const DItem &it = items[Did];
             if (krow + it.K <= kstep && mrow + it.nblk * kORows <= mcap && add_targets(it)) {
                 krow += it.K;
                 mrow += it.nblk * kORows;
                 cur.push_back(Part{Did, 0, it.K});
-                break;
+            } else {
+                left.push_back(Did);
             }
-            if (cur.empty()) {  // a single D that does not fit
-                delete og;
-                return GD_OK;
-            }
-            close();
         }
+        if (cur.empty()) {  // a single D that does not fit
+            delete og;
+            return GD_OK;
+        }
+        close();
+        rest.swap(left);
     }
-    close();
     og->cpt = cpt;
     og->nslot = nslot;
     og->norb = norb;
     og->pcap = pcap;
     og->mcap = mcap;
-    og->smem = (size_t)kOWarps * kORing + (size_t)d.n_pnt * cpt * 4 + (size_t)(pcap + mcap + 1) * row_bytes;
-    // one buffer: warp after warp, each followed by the chunks that the last
-    // steps fetch ahead
+    og->p_at = p_at;
+    og->zero_at = zero_at;
+    og->smem = (size_t)zero_at + row_bytes;
+    // one buffer: warp after warp, each followed by the chunks that its last
+    // steps copy ahead
     std::vector<uint4> stream;
     std::vector<int> st((size_t)og->nsteps * kOWarps);
+    size_t total = 0;
+    for (const auto &v : ws) total += v.size() + 5 * (kOChunk / 16);
+    if (total * 16 >= (size_t)1 << 32) {  // positions are 32-bit
+        delete og;
+        return GD_OK;
+    }
+    stream.reserve(total);
     for (int w = 0; w < kOWarps; w++) {
-        const int base = (int)(stream.size() / (kOChunk / 16));
+        const int base = (int)stream.size();
         for (int k = 0; k < og->nsteps; k++) st[(size_t)k * kOWarps + w] = base + start[w][k];
+        pad_chunk(ws[w]);
         stream.insert(stream.end(), ws[w].begin(), ws[w].end());
         stream.resize(stream.size() + 4 * (kOChunk / 16), make_uint4(0, 0, 0, 0));
         std::vector<uint4>().swap(ws[w]);
     }
+    og->stream_bytes = stream.size() * 16;
     c.orbit = og;
     int rc = upload(&og->row_node, row_node);
     if (!rc) rc = upload(&og->stream, stream);
     if (!rc) rc = upload(&og->start, st);
+    if (!rc) rc = upload(&og->err, std::vector<int>(1, 0));
     if (!rc) rc = fold_loss_build(c);
     return rc;  // the caller destroys the context on failure
 }
@@ -859,8 +997,8 @@ int launch_orbit(Context &c, const float *f, int ncells, int ld, float *gain, vo
     orbit_pack_kernel<<<dim3((cells_pad + 31) / 32, d.n_pnt / 8), dim3(32, 8), 0, st>>>(
         f, ld, ncells, d.n_pnt, g.cpt, g.row_node, ft, cells_pad);
     GD_CUDA(cudaGetLastError());
-    const OrbitArgs a{ft,     g.stream, g.start,   d_bounds, g.row_node, part,  gain,
-                      g.norb, d.n_pnt,  cells_pad, ncells,   ld,         g.pcap, g.mcap};
+    const OrbitArgs a{ft,      reinterpret_cast<const unsigned char *>(g.stream), g.start, d_bounds, g.row_node, part, gain, g.err, g.norb,
+                      d.n_pnt, cells_pad, ncells, ld, g.p_at, g.zero_at};
     int nslot = 0;
     OrbitKernel kern = orbit_kernel(g.cpt, g.nslot, &nslot);
     GD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
@@ -895,6 +1033,19 @@ int run_orbit(Context &c, const float *f, int ncells, int ld, float *gain, cudaS
     int rc = ensure_scratch(c, orbit_pack_bytes(c, ncells) + orbit_part_bytes(c, ncells, nchunks));
     if (rc) return rc;
     return launch_orbit(c, f, ncells, ld, gain, c.scratch.ptr, nchunks, it->second, st);
+}
+
+int orbit_take_timeout(Context &c, cudaStream_t st, bool *timed_out)
+{
+    int flag = 0;
+    GD_CUDA(cudaMemcpyAsync(&flag, c.orbit->err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    GD_CUDA(cudaStreamSynchronize(st));
+    *timed_out = flag != 0;
+    if (flag) {
+        GD_CUDA(cudaMemsetAsync(c.orbit->err, 0, sizeof(int), st));
+        GD_CUDA(cudaStreamSynchronize(st));
+    }
+    return GD_OK;
 }
 
 }  // namespace gd
