@@ -21,7 +21,7 @@ device->host after every step; `accuracy` compares the step's projected Q with
 the FP32 pair kernel's on the same cells, per cell, and (from the CPU-baseline
 leg, where the oracle runs) with the oracle's FP64 path on the first cells;
 `roofline` covers the plain gain kernel (tensor pipe for the collision
-matrices, measured FP32 FMA peak for the SIMT pair kernels); `cpu_baseline`
+matrices, measured FP32 FMA peak for the pair-product kernels); `cpu_baseline`
 times the oracle's OpenMP FP32 host path on a bounded sample.  Under torchrun each rank runs its own batch (weak scaling, no
 collective on the data path) and the time is the maximum over ranks.
 """
@@ -377,6 +377,9 @@ def run_ours(args):
              "bf16": "bf16 (FP32 accumulate)",
              "bf16x3": "bf16x3 (hi/lo split, FP32 accumulate, at most 256 products per tensor-core accumulation)"
              }[args.gain]
+    if fp32_gain(args.gain, ctx):
+        dtype = "f32 gain" + ("" if args.gain == "pair" else
+                              "; bf16x3 loss (hi/lo split, FP32 accumulate, at most 256 products per accumulation)")
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None,
@@ -430,14 +433,23 @@ def run_ours(args):
         dist.destroy_process_group()
 
 
+def fp32_gain(name, ctx):
+    """Whether the FP32 kernel that does all reflections of a pair sum at once
+    computes this path's gain: every lattice of this workload but, for BF16x3,
+    those small enough that their matrices are faster (then they are built)."""
+    return name in ("pair", "pair_tc") or (name == "bf16x3" and ctx._info()["cmatrix_tiles"] == 0)
+
+
 def path_launches(name, ctx):
     """Kernel launches of the loss and of the gain on a gain path: the FP32
     loss kernel, or on the tensor-core paths the BF16 conversion of f and one
-    tensor-core GEMM; the FP32 gain kernel and its chunk reduction, the
-    pair tensor-core kernel between its scale and conversion kernels, or the
-    conversion of f and the collision-matrix kernel."""
+    tensor-core GEMM; the packing of f, the FP32 gain kernel and its chunk
+    reduction (on the tensor-core paths that it serves after the cells'
+    scales), or the conversion of f and the collision-matrix kernel."""
     if name == "pair":
-        return 1, 2
+        return 1, 3
+    if fp32_gain(name, ctx):
+        return 2, 4
     if name == "pair_tc":
         return 2, 3
     return 2, 2
@@ -566,16 +578,16 @@ def time_gain(ctx, f0, nc, stream, flush, reps):
 def gain_roofline(name, ctx, f0, nc, stream, flush, peak, reps):
     """Throughput of the gain launch against its bounding pipe: the BF16
     tensor peak for the collision-matrix kernel (FLOP of the tiles issued),
-    the measured FP32 FMA peak for the SIMT pair-product kernels (algorithmic
+    the measured FP32 FMA peak for the pair-product kernel (algorithmic
     FLOP of the pair-product formulation)."""
     g_avg = time_gain(ctx, f0, nc, stream, flush, reps)
     traffic, traffic_src = None, None
-    if name in ("pair", "pair_tc"):
+    if fp32_gain(name, ctx):
         inf = ctx.info
         flop = nc * (7 * inf["pair_products"] + 2 * inf["contraction_terms"] + inf["scatter_terms"])
-        kernel = "gain_pair_kernel (+ chunk reduction)" if name == "pair" else \
-            "pair_tc_kernel (tcgen05 contraction, + chunk reduction)"
-        work = "7 FLOP per pair product + 2 per nonzero-weight term + 1 per scatter update"
+        kernel = "orbit_gain_kernel (+ packing of f, chunk reduction)"
+        work = "7 FLOP per pair product + 2 per nonzero-weight term + 1 per scatter update, over the class boxes " \
+            "(the kernel leaves out what lies outside the sphere: at 20^3 two thirds of them)"
         bound, pk, src = "fp32", peak["fp32"], peak["fma_source"]
     else:
         # stored tiles: the nonzero 256 x 64 tiles of each G_i's block upper
@@ -601,7 +613,7 @@ def gain_roofline(name, ctx, f0, nc, stream, flush, peak, reps):
     out = {"bound": bound, "kernel": kernel, "achieved": ach, "peak": pk, "unit": "TFLOP/s",
            "frac": ach / pk, "peak_source": src, "work": work,
            "flop_per_launch": flop, "traffic": traffic, "traffic_source": traffic_src, "launch_ms": g_avg * 1000.0}
-    if name not in ("pair", "pair_tc"):
+    if not fp32_gain(name, ctx):
         # the dense bilinear form's count, 2 n^3 + 2 n^2 FLOP per cell: what the
         # launch computes without exploiting the symmetry of G_i and its zero tiles
         n = ctx.n_pnt

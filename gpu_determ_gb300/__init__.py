@@ -263,7 +263,8 @@ class Context:
 
     def set_gain_path(self, path: int):
         """GAIN_PAIR (FP32 pair-product kernel), GAIN_CMATRIX_BF16, GAIN_CMATRIX_BF16X3 or
-        GAIN_PAIR_TC (pair products with the weight contraction on the tensor cores)."""
+        GAIN_PAIR_TC (pair products with the weight contraction on the tensor cores).  The
+        FP32 kernel computes the last two's gain as well wherever it is faster."""
         _check(lib().gd_ctx_set_gain_path(self._h, int(path)))
 
     # tables -----------------------------------------------------------------
@@ -526,7 +527,8 @@ class Batch:
         """BATCH_STREAMS (per-group steps on forked streams),
         BATCH_FUSED_PAIR_TC (every group's gain in one persistent launch of the
         pair-product kernel) or BATCH_FUSED_CMATRIX (every group's gain in one
-        launch of the collision-matrix kernel)."""
+        launch of the collision-matrix kernel); groups whose gain the FP32 kernel
+        computes launch that instead."""
         _check(lib().gd_batch_set_mode(self._h, int(mode)))
 
     def check(self):

@@ -70,21 +70,23 @@ int enqueue_steps(gd_batch *b)
     return GD_OK;
 }
 
-// The fused modes: every group's loss, then ONE launch of the gain for all
-// groups (GD_BATCH_FUSED_PAIR_TC: the persistent pair-product kernel with its
-// contraction on the tensor cores; GD_BATCH_FUSED_CMATRIX: the collision-
-// matrix kernel over every grid's nodes), then every group's projection and
-// relaxation, all on the batch stream.  Each group's results equal gd_step on
-// its context's gain path bit for bit (the same per-unit work: integer sums
-// on the pair path, the same CTA pairs on the matrix path).
+// The fused modes: every group's loss and, where the FP32 gain kernel serves
+// its path (orbit_serves), its gain, which fills the chip by itself; then ONE
+// launch of the gain for the remaining groups (GD_BATCH_FUSED_PAIR_TC: the
+// persistent pair-product kernel with its contraction on the tensor cores;
+// GD_BATCH_FUSED_CMATRIX: the collision-matrix kernel over every grid's nodes),
+// then every group's projection and relaxation, all on the batch stream.  Each
+// group's results equal gd_step on its context's gain path bit for bit (the same
+// per-unit work: integer sums on the pair path, the same CTA pairs on the matrix
+// path).
 int enqueue_fused(gd_batch *b)
 {
     using namespace gd;
     const size_t ng = b->groups.size();
     std::vector<float *> nu(ng), gain(ng);
     std::vector<double *> q(ng);
-    std::vector<PtJob> jobs(ng);
-    std::vector<CmJob> cjobs(ng);
+    std::vector<PtJob> jobs;
+    std::vector<CmJob> cjobs;
     for (size_t k = 0; k < ng; k++) {
         const gd_batch::Group &g = b->groups[k];
         Context &c = g.ctx->c;
@@ -93,11 +95,18 @@ int enqueue_fused(gd_batch *b)
         int rc = step_buffers(c, g.ld, b->main, &nu[k], &gain[k], &q[k]);
         if (!rc) rc = run_loss_path(c, g.f, g.ncells, g.ld, nu[k], b->main);
         if (rc) return rc;
-        jobs[k] = PtJob{&c, g.f, g.ncells, g.ld, gain[k]};
-        cjobs[k] = CmJob{c.cmatrix, g.f, g.ncells, g.ld, gain[k]};
+        if (orbit_serves(c, c.gain_path)) {
+            rc = run_gain_path(c, g.f, g.ncells, g.ld, gain[k], b->main);
+            if (rc) return rc;
+        } else if (b->mode == GD_BATCH_FUSED_CMATRIX) {
+            cjobs.push_back(CmJob{c.cmatrix, g.f, g.ncells, g.ld, gain[k]});
+        } else {
+            jobs.push_back(PtJob{&c, g.f, g.ncells, g.ld, gain[k]});
+        }
     }
-    int rc = b->mode == GD_BATCH_FUSED_CMATRIX ? launch_cmatrix(cjobs.data(), (int)ng, b->main)
-                                               : launch_pair_tc(jobs.data(), (int)ng, b->main);
+    int rc = GD_OK;
+    if (!cjobs.empty()) rc = launch_cmatrix(cjobs.data(), (int)cjobs.size(), b->main);
+    if (!jobs.empty()) rc = launch_pair_tc(jobs.data(), (int)jobs.size(), b->main);
     if (rc) return rc;
     for (size_t k = 0; k < ng; k++) {
         const gd_batch::Group &g = b->groups[k];

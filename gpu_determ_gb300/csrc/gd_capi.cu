@@ -504,7 +504,8 @@ int gd_ctx_set_gain_path(gd_ctx *ctx, int path)
         if (rc) return rc;
     } else if (path != GD_GAIN_PAIR) {
         const int mode = path == GD_GAIN_CMATRIX_BF16 ? GD_CMATRIX_BF16 : GD_CMATRIX_BF16X3;
-        int rc = gd_cmatrix_create(ctx, mode, &c.cmatrix);
+        int rc = gd::orbit_serves(c, path) ? gd::cmatrix_create_loss_only(ctx, &c.cmatrix)
+                                           : gd_cmatrix_create(ctx, mode, &c.cmatrix);
         if (rc) return rc;
     }
     c.gain_path = path;

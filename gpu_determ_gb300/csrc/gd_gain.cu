@@ -313,7 +313,7 @@ int gain_bounds_device(Context &c, int nchunks, const int **out)
 
 int run_gain(Context &c, const float *f, int ncells, int ld, float *gain, cudaStream_t st)
 {
-    if (c.orbit) return run_orbit(c, f, ncells, ld, gain, st);
+    if (c.orbit) return run_orbit(c, f, ncells, ld, gain, false, st);
     const Dims &d = c.d;
     int cb = 0, nblk = 0, nchunks = 0;
     size_t smem = 0;

@@ -229,8 +229,9 @@ void orbit_chunk_bounds(const Context &c, int nchunks, int *bounds);
 size_t orbit_pack_bytes(const Context &c, int ncells);
 size_t orbit_part_bytes(const Context &c, int ncells, int nchunks);
 int launch_orbit(Context &c, const float *f, int ncells, int ld, float *gain, void *buf, int nchunks,
-                 const int *d_bounds, cudaStream_t st);
-int run_orbit(Context &c, const float *f, int ncells, int ld, float *gain, cudaStream_t st);
+                 const int *d_bounds, float2 *scale, cudaStream_t st);
+int run_orbit(Context &c, const float *f, int ncells, int ld, float *gain, bool guard, cudaStream_t st);
+bool orbit_serves(const Context &c, int path);  // whether run_orbit computes this path's gain
 // reads (synchronising st) and clears its pipeline time-out record
 int orbit_take_timeout(Context &c, cudaStream_t st, bool *timed_out);
 

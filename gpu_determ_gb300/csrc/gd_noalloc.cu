@@ -131,7 +131,7 @@ extern "C" int gd_gain_noalloc(gd_ctx *ctx, const float *f, int ncells, int ld, 
             while (nchunks > 1 && orbit_pack_bytes(c, ncells) + orbit_part_bytes(c, ncells, nchunks) > room) nchunks--;
             if ((rc = noalloc_bounds(c, nchunks, orbit_chunk_bounds, st, &base))) break;
             rc = launch_orbit(c, f, ncells, ld, gain, static_cast<unsigned char *>(base) + kHeaderBytes, nchunks,
-                              static_cast<const int *>(base), st);
+                              static_cast<const int *>(base), nullptr, st);
             break;
         }
         const int nchunks = std::min(want, fit);

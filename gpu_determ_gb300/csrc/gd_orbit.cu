@@ -64,6 +64,8 @@ constexpr uint32_t kORing = 4 * kOChunk;         // a warp's ring: three chunks 
 constexpr uint32_t kOBars = kOWarps * kORing;    // offset of the rings' barriers
 constexpr uint32_t kOF = kOBars + 1024;          // offset of f
 constexpr uint32_t kOQuad = 80;                  // bytes of a contraction quad
+constexpr int kOMatrixNodes = 512;               // BF16x3 matrices stay below this (orbit_serves)
+constexpr int kOSlice = 65536;                   // cells of one launch of the guarded gain: n_pnt of them stay below 2^31
 constexpr int kOSlots = 4;                       // output slots gathered side by side
 constexpr int kOGroup = 16;                      // rounds (two targets per slot, 32 bytes) of a group in a step: at most a chunk
 
@@ -75,6 +77,7 @@ struct OrbitArgs {
     const int *row_node;
     float *part;                  // [chunk][row][cells_pad], or null: write gain
     float *gain;
+    const float2 *scale;          // [cells_pad] power-of-two factors of f and back, or null
     int *err;                     // set to 1 when a copy is not seen to land
     int norb, ns, cells_pad, ncells, ld;
     uint32_t p_at, zero_at;       // shared-memory offsets of the P rows and of the zero C row
@@ -101,6 +104,9 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b)
         : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
     return d;
 }
+
+// A gain of f 2^-k back to that of f (two factors: 4^k may exceed FP32's range).
+__device__ __forceinline__ float unscale(float v, float s) { return __fmul_rn(__fmul_rn(v, s), s); }
 
 template <int CPT>
 struct Vec;
@@ -405,7 +411,7 @@ __global__ void __launch_bounds__(kOThreads, 1) orbit_gain_kernel(const __grid_c
                 const float *v = reinterpret_cast<const float *>(&acc[j]);
 #pragma unroll
                 for (int q = 0; q < CPT / 4; q++)
-                    if (cell + q < a.ncells) g[q] = v[q];
+                    if (cell + q < a.ncells) g[q] = a.scale ? unscale(v[q], a.scale[cell + q].y) : v[q];
             }
         }
     } else if (a.part) {  // an empty chunk (more chunks than work): zero partial sums
@@ -414,21 +420,49 @@ __global__ void __launch_bounds__(kOThreads, 1) orbit_gain_kernel(const __grid_c
     }
 }
 
+// scale[cell] = {2^-k, 2^k} for max|f| of the cell in [2^k, 2^(k+1)) where that
+// is beyond 2^+-40 (products could leave FP32's range), {1, 1} for the others,
+// {1, NaN} for a cell with a non-finite f.  Block = 32 cells x 32 node strides: 16 MB of
+// loads in flight at 4096 cells.
+__global__ void __launch_bounds__(1024) orbit_scale_kernel(const float *__restrict__ f, int ld, int ncells, int ns,
+                                                           float2 *__restrict__ scale, int cells_pad)
+{
+    __shared__ unsigned red[32][32];
+    const int x = threadIdx.x, y = threadIdx.y, cell = blockIdx.x * 32 + x;
+    unsigned m = 0;  // bit patterns of |f| order like the values, infinity and NaN above all
+    if (cell < ncells)
+#pragma unroll 8
+        for (int p = y; p < ns; p += 32) m = max(m, __float_as_uint(__ldg(f + (size_t)p * ld + cell)) & 0x7fffffffu);
+    red[y][x] = m;
+    __syncthreads();
+    if (y == 0 && cell < cells_pad) {
+        for (int k = 1; k < 32; k++) m = max(m, red[k][x]);
+        const int e = (int)(m >> 23);  // 0: zero or subnormal, 255: not finite
+        int k = e == 0 ? -126 : min(126, e - 127);
+        if (m == 0 || abs(k) <= 40) k = 0;
+        scale[cell] = e == 255 ? make_float2(1.f, __int_as_float(0x7fc00000))
+                               : make_float2(__int_as_float((127 - k) << 23), __int_as_float((127 + k) << 23));
+    }
+}
+
 // ft[tile][row][CPT] from f[node][cell]: the packed rows the product loads
 // read; cells past ncells are zero.  Block = 32 cells x 8 rows.
 __global__ void orbit_pack_kernel(const float *__restrict__ f, int ld, int ncells, int ns, int cpt,
-                                  const int *__restrict__ row_node, float *__restrict__ ft, int cells_pad)
+                                  const int *__restrict__ row_node, const float2 *__restrict__ scale,
+                                  float *__restrict__ ft, int cells_pad)
 {
     const int cell = blockIdx.x * 32 + threadIdx.x, row = blockIdx.y * 8 + threadIdx.y;
     if (row >= ns || cell >= cells_pad) return;
-    const float v = cell < ncells ? f[(size_t)__ldg(row_node + row) * ld + cell] : 0.f;
+    float v = cell < ncells ? f[(size_t)__ldg(row_node + row) * ld + cell] : 0.f;
+    if (scale) v = __fmul_rn(v, scale[cell].x);
     ft[((size_t)(cell / cpt) * ns + row) * cpt + cell % cpt] = v;
 }
 
 // gain[node][cell] = sum over the chunks: each of the block's eight y rows adds
 // a contiguous eighth of the chunks in order, and the eight are added in order.
 __global__ void orbit_reduce_kernel(const float *__restrict__ part, int nchunks, int ns, int cells_pad, int ncells,
-                                    int ld, const int *__restrict__ row_node, float *__restrict__ gain)
+                                    int ld, const int *__restrict__ row_node, const float2 *__restrict__ scale,
+                                    float *__restrict__ gain)
 {
     __shared__ float red[8][32];
     const int x = threadIdx.x, y = threadIdx.y;
@@ -445,7 +479,7 @@ __global__ void orbit_reduce_kernel(const float *__restrict__ part, int nchunks,
     __syncthreads();
     if (y == 0 && o < total) {
         for (int k = 1; k < 8; k++) s += red[k][x];
-        gain[(size_t)__ldg(row_node + row) * ld + cell] = s;
+        gain[(size_t)__ldg(row_node + row) * ld + cell] = scale ? unscale(s, scale[cell].y) : s;
     }
 }
 
@@ -984,21 +1018,28 @@ void orbit_chunk_bounds(const Context &c, int nchunks, int *bounds)
     bounds[nchunks] = g.nsteps;
 }
 
+// buf holds orbit_pack_bytes + orbit_part_bytes; scale is null or one entry per
+// cell of the padded tiles.
 int launch_orbit(Context &c, const float *f, int ncells, int ld, float *gain, void *buf, int nchunks,
-                 const int *d_bounds, cudaStream_t st)
+                 const int *d_bounds, float2 *scale, cudaStream_t st)
 {
     OrbitGain &g = *c.orbit;
     const Dims &d = c.d;
     const int tiles = (ncells + g.cpt - 1) / g.cpt, cells_pad = tiles * g.cpt;
-    if ((int64_t)d.n_pnt * std::max(ld, cells_pad) >= ((int64_t)1 << 31))
+    if ((int64_t)d.n_pnt * (scale ? cells_pad : std::max(ld, cells_pad)) >= ((int64_t)1 << 31))
         return set_error(GD_ERR_UNSUPPORTED, "pair gain: n_pnt * ld must stay below 2^31");
     float *ft = static_cast<float *>(buf);
     float *part = nchunks > 1 ? ft + (size_t)cells_pad * d.n_pnt : nullptr;
+    if (scale) {
+        orbit_scale_kernel<<<(cells_pad + 31) / 32, dim3(32, 32), 0, st>>>(f, ld, ncells, d.n_pnt, scale, cells_pad);
+        GD_CUDA(cudaGetLastError());
+    }
     orbit_pack_kernel<<<dim3((cells_pad + 31) / 32, d.n_pnt / 8), dim3(32, 8), 0, st>>>(
-        f, ld, ncells, d.n_pnt, g.cpt, g.row_node, ft, cells_pad);
+        f, ld, ncells, d.n_pnt, g.cpt, g.row_node, scale, ft, cells_pad);
     GD_CUDA(cudaGetLastError());
-    const OrbitArgs a{ft,      reinterpret_cast<const unsigned char *>(g.stream), g.start, d_bounds, g.row_node, part, gain, g.err, g.norb,
-                      d.n_pnt, cells_pad, ncells, ld, g.p_at, g.zero_at};
+    const OrbitArgs a{ft,    reinterpret_cast<const unsigned char *>(g.stream),
+                      g.start, d_bounds, g.row_node, part, gain, scale, g.err, g.norb, d.n_pnt, cells_pad, ncells, ld,
+                      g.p_at, g.zero_at};
     int nslot = 0;
     OrbitKernel kern = orbit_kernel(g.cpt, g.nslot, &nslot);
     GD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
@@ -1007,16 +1048,42 @@ int launch_orbit(Context &c, const float *f, int ncells, int ld, float *gain, vo
     if (part) {
         const int64_t outs = (int64_t)d.n_pnt * ncells;
         orbit_reduce_kernel<<<(unsigned)((outs + 31) / 32), dim3(32, 8), 0, st>>>(part, nchunks, d.n_pnt, cells_pad, ncells,
-                                                                                 ld, g.row_node, gain);
+                                                                                 ld, g.row_node, scale, gain);
         GD_CUDA(cudaGetLastError());
     }
     return GD_OK;
 }
 
-int run_orbit(Context &c, const float *f, int ncells, int ld, float *gain, cudaStream_t st)
+// The tensor-core gain paths whose gain this kernel computes: it is the faster
+// one, with a smaller error against FP64, on all but the smallest lattices.
+// Measured against the BF16x3 matrices (ms; R = 4.8, 4096 cells unless said): 12^3
+// 3.57 / 5.35 (one cell 0.03 / 0.28), 16^3 (1024 cells) 4.1 / 9.5, 20^3 67 / 208,
+// 24^3 (512 cells) 35 / 107, 8^3 whole box (512 nodes) 1.16 / 1.38; 10^3 (480 nodes)
+// 1.42 / 1.37 and 8^3 (208 nodes) 0.57 / 0.35, where the matrices stay.  Against
+// pair_tc_kernel it wins wherever it exists: 4^3 0.06 / 0.49, 8^3 0.57 / 5.5, 24^3
+// (512 cells) 35 / 168.
+bool orbit_serves(const Context &c, int path)
+{
+    return c.orbit && (path == GD_GAIN_PAIR_TC || (path == GD_GAIN_CMATRIX_BF16X3 && c.d.n_pnt >= kOMatrixNodes));
+}
+
+// With guard a cell whose f is so large or small that products would leave FP32's
+// range is scaled by a power of two (orbit_scale_kernel), and a cell with a
+// non-finite f gets NaN for all its outputs; other cells' bits are the same.
+int run_orbit(Context &c, const float *f, int ncells, int ld, float *gain, bool guard, cudaStream_t st)
 {
     OrbitGain &g = *c.orbit;
-    const int nchunks = orbit_chunks(c, ncells);
+    if (guard && ncells > kOSlice) {
+        // the BF16x3 path has no limit on n_pnt * ld: slices of cells
+        for (int at = 0; at < ncells; at += kOSlice) {
+            const int rc = run_orbit(c, f + at, std::min(kOSlice, ncells - at), ld, gain + at, guard, st);
+            if (rc) return rc;
+        }
+        return GD_OK;
+    }
+    int nchunks = orbit_chunks(c, ncells);
+    // the partial sums are bounded at 16 GiB
+    while (nchunks > 1 && orbit_part_bytes(c, ncells, nchunks) > ((size_t)16 << 30)) nchunks--;
     auto it = g.bounds_dev.find(nchunks);
     if (it == g.bounds_dev.end()) {
         std::vector<int> b(nchunks + 1);
@@ -1030,9 +1097,12 @@ int run_orbit(Context &c, const float *f, int ncells, int ld, float *gain, cudaS
         }
         it = g.bounds_dev.emplace(nchunks, dev).first;
     }
-    int rc = ensure_scratch(c, orbit_pack_bytes(c, ncells) + orbit_part_bytes(c, ncells, nchunks));
+    const size_t bytes = orbit_pack_bytes(c, ncells) + orbit_part_bytes(c, ncells, nchunks);
+    const int cells_pad = (ncells + g.cpt - 1) / g.cpt * g.cpt;
+    int rc = ensure_scratch(c, bytes + (guard ? sizeof(float2) * cells_pad : 0));
     if (rc) return rc;
-    return launch_orbit(c, f, ncells, ld, gain, c.scratch.ptr, nchunks, it->second, st);
+    float2 *scale = guard ? reinterpret_cast<float2 *>(static_cast<char *>(c.scratch.ptr) + bytes) : nullptr;
+    return launch_orbit(c, f, ncells, ld, gain, c.scratch.ptr, nchunks, it->second, scale, st);
 }
 
 int orbit_take_timeout(Context &c, cudaStream_t st, bool *timed_out)

@@ -61,7 +61,7 @@ typedef struct {
     int64_t pair_products;     /* (s, n) pair products formed per cell-eval */
     int64_t contraction_terms; /* nonzero-weight x pair-product terms per cell-eval */
     int64_t scatter_terms;     /* (s, g, sign) output updates per cell-eval */
-    int64_t cmatrix_tiles;     /* stored 256 x 64 tiles of the collision matrices (0 without) */
+    int64_t cmatrix_tiles;     /* stored 256 x 64 tiles of the collision matrices (0 without, see gd_ctx_set_gain_path) */
     int64_t cmatrix_slices;    /* 256 x 16 slices with a nonzero entry over every node's matrix: the MMA
                                   K steps one cell tile issues in GD_CMATRIX_BF16X3 mode */
     int64_t cmatrix_node_tiles; /* tiles over every node's matrix (a node uses the stored tiles of its
@@ -124,10 +124,9 @@ int gd_correction_basis(gd_ctx *ctx, float *basis, gd_stream stream);
 /* ---- collision operator ------------------------------------------------ */
 /* Loss frequency nu[i][c] = sum_j b(|i-j|) f[j][c] and gain I[i][c] over the
  * in-sphere nodes (either output may be NULL), on the context's gain path:
- * GD_GAIN_PAIR computes both in FP32 (SIMT kernels); the tensor-core paths
- * (collision matrices, GD_GAIN_PAIR_TC) compute the gain on the tensor cores
- * and, when ld is a multiple of 4, the loss as one BF16x3 GEMM (see
- * gd_ctx_set_gain_path).  Replaces the
+ * GD_GAIN_PAIR computes both in FP32 (SIMT kernels); the other paths compute
+ * the gain as gd_ctx_set_gain_path says and, when ld is a multiple of 4, the
+ * loss as one BF16x3 GEMM on the tensor cores.  Replaces the
  * loss and gain stages of evolve_colisions (collision_integral.h:11-17,
  * collision_integral.cu:32-188, 587-648). */
 int gd_collision(gd_ctx *ctx, const float *f, int ncells, int ld, float *nu, float *gain,
@@ -217,12 +216,16 @@ int gd_cmatrix_set_chain(gd_cmatrix *cm, int tiles);
 int gd_cmatrix_check(gd_cmatrix *cm, gd_stream stream);
 /* Gain algorithm used by gd_collision and gd_step for this context:
  * GD_GAIN_PAIR (default, FP32 pair-product kernel), GD_GAIN_CMATRIX_BF16 or
- * GD_GAIN_CMATRIX_BF16X3 (builds the context's collision matrices), or
+ * GD_GAIN_CMATRIX_BF16X3 (the context's collision matrices), or
  * GD_GAIN_PAIR_TC (the pair-product formulation with its weight contraction on
  * the tensor cores, pair products and weights split into BF16 hi + lo, each
  * cell's outputs summed in 64-bit fixed point scaled by a bound on its gain;
  * builds a per-class-box weight table of a few GB at 24^3 instead of n^3
  * matrices, so it serves the grids whose collision matrices do not fit).
+ * Where the FP32 kernel is faster, and its error no larger, it computes the gain
+ * of GD_GAIN_CMATRIX_BF16X3 (lattices of 512 nodes or more; the matrices are then
+ * not built) and of GD_GAIN_PAIR_TC too: every lattice whose half-box rows fit
+ * its shared memory, up to 24^3 with R = 4.8.
  * The two pair paths need n_pnt * ld < 2^31 (GD_ERR_UNSUPPORTED otherwise). */
 enum { GD_GAIN_PAIR = 0, GD_GAIN_CMATRIX_BF16 = 1, GD_GAIN_CMATRIX_BF16X3 = 2, GD_GAIN_PAIR_TC = 3 };
 int gd_ctx_set_gain_path(gd_ctx *ctx, int path);
@@ -279,7 +282,8 @@ int gd_batch_step(gd_batch *b, int use_graph, gd_stream stream);
  * distinct contexts whose gain path is GD_GAIN_PAIR_TC) in one persistent
  * launch of the pair-product kernel that walks a device list of (grid,
  * 128-cell tile, s-chunk) units, each group's loss, projection and
- * relaxation around it on the batch stream; results equal gd_step on each
+ * relaxation around it on the batch stream (groups whose gain the FP32 kernel
+ * computes, see gd_ctx_set_gain_path, launch that instead); results equal gd_step on each
  * group's context bit for bit.  A pipeline time-out of the fused launch is
  * recorded on the first group's context.  GD_BATCH_FUSED_CMATRIX: the same
  * with the gains of all groups (at most 4, on distinct contexts whose gain

@@ -95,3 +95,37 @@ def test_folded_loss_matches_oracle(cuda, gdlib, dims, R, nc, ld):
     ref = o.loss_f64(o.to_box(f))
     assert np.max(np.abs(got - ref) / ref) <= 5e-6
     assert np.linalg.norm(got - ref) <= 3e-7 * np.linalg.norm(ref)
+
+
+# lattices whose gain the FP32 kernel computes on the tensor-core paths too; up
+# to 1216 cells of eight (tiles x 152) run in chunks of the walk, then in one
+@pytest.mark.parametrize("dims,R,nc,ld", [((8, 8, 8), 16.5, 1216, 1216), ((12, 10, 8), 4.2, 7, 9),
+                                          ((12, 12, 12), 4.8, 65, 67), ((22, 22, 22), 4.8, 3, 3)])
+def test_orbit_gain_serves_the_tensor_core_paths(cuda, gdlib, dims, R, nc, ld):
+    """The FP32 path's gain bit for bit; a cell with a non-finite f gets NaN
+    alone; a cell scaled by 2^+-50, whose products would leave FP32's range,
+    gets the exactly scaled gain, rounded once."""
+    torch = cuda
+    spec = gdlib.GridSpec(*dims, R=R)
+    ctx = gdlib.Context(spec)
+    f = torch.full((ctx.n_pnt, ld), float("nan"), dtype=torch.float32, device="cuda")
+    # no product of f itself is subnormal
+    f[:, :nc] = torch.from_numpy(np.maximum(inputs.dirichlet_mixtures(spec.fill(), nc, seed=5), 1e-12)).cuda()
+    ref = torch.full_like(f, -1.0)
+    ctx.collision(f, nc, ld, None, ref)
+    g = f.clone()
+    g[3, 1] = float("inf")
+    g[:, 2] *= 2.0 ** -50
+    g[:, 0] *= 2.0 ** 50
+    paths = [gdlib.GAIN_PAIR_TC] + ([gdlib.GAIN_CMATRIX_BF16X3] if ctx.n_pnt >= 512 else [])
+    for path in paths:
+        ctx.set_gain_path(path)
+        out = [torch.full_like(f, -1.0) for _ in range(2)]
+        for x, o in zip((f, g), out):
+            ctx.collision(x, nc, ld, None, o)
+        ctx.check()
+        assert torch.equal(out[0], ref)
+        assert torch.equal(out[1][:, 3:], ref[:, 3:]) and bool(torch.isnan(out[1][:, 1]).all())
+        r = ref.cpu().numpy().astype(np.float64)
+        assert np.array_equal(out[1][:, 0].cpu().numpy(), np.ldexp(r[:, 0], 100).astype(np.float32))
+        assert np.array_equal(out[1][:, 2].cpu().numpy(), np.ldexp(r[:, 2], -100).astype(np.float32))
