@@ -597,18 +597,16 @@ def gain_roofline(name, ctx, f0, nc, stream, flush, peak, reps):
         tiles = inf["cmatrix_tiles"]  # stored (one matrix per orbit of the lattice's reflections)
         # issued over every node; one BF16 pass issues whole tiles (4 K steps each)
         slices = inf["cmatrix_slices"] if name == "bf16x3" else 4 * inf["cmatrix_node_tiles"]
-        flop = 2.0 * ((nc + 127) // 128 * 128) * 256 * 16 * slices * (3 if name == "bf16x3" else 1)
+        flop = 2.0 * ((nc + 31) // 32 * 32) * 256 * 16 * slices * (3 if name == "bf16x3" else 1)
         kernel, work = "cmatrix_gain_kernel (tcgen05)", \
             "MACs x 2 of the 128x256x16 MMA K steps issued (nonzero slices of the stored tiles of the block upper triangle of each symmetric G_i; x3 for bf16x3)"
         bound, pk, src = "tensor", peak["bf16"], peak["bf16_source"]
-        # DRAM bytes per launch: every node's matrix tiles stream through about
-        # once (a representative's tiles once per reflection: the launch runs
-        # reflection-major).  An ncu capture of the BF16x3 kernel (CTA pairs) on
-        # 14^3 / 4096 cells read and wrote 7.806 GB for 5.820 GB of tiles the
-        # nodes stream (ratio 1.341); scaled here by the 20^3 launch's tiles.
-        g_bytes = inf["cmatrix_node_tiles"] * 256 * 64 * 2 * (2 if name == "bf16x3" else 1)
-        traffic = 1.341 * g_bytes
-        traffic_src = "ncu dram__bytes_read+write of a 14^3/4096-cell launch, scaled by the matrix tile bytes the nodes stream"
+        # DRAM bytes per launch: the matrices once per group of cell tiles and the
+        # rows of f about once.  An ncu capture of the one-pass kernel (CTA pairs)
+        # on 14^3 / 4096 cells read and wrote 7.213 GB for 1.192e13 FLOP issued;
+        # scaled here by the FLOP.
+        traffic = 7.213e9 / 1.192e13 * flop / (3 if name == "bf16x3" else 1) * (2 if name == "bf16x3" else 1)
+        traffic_src = "ncu dram__bytes_read+write of a 14^3/4096-cell one-pass launch, scaled by the FLOP issued"
     ach = flop / g_avg / 1e12
     out = {"bound": bound, "kernel": kernel, "achieved": ach, "peak": pk, "unit": "TFLOP/s",
            "frac": ach / pk, "peak_source": src, "work": work,

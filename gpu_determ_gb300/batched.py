@@ -12,7 +12,7 @@ launch the autotuner picks on its own cells; one gd_batch holds all groups,
 and each step (collision, FP64 projection, Courant relaxation per grid) is
 one CUDA graph launch after the first two.  With --fused, every grid's gain
 runs in ONE launch per step: the collision-matrix kernel over all grids'
-(cell tile, node) pairs (cmatrix), or the persistent pair-product kernel over
+(cell tile, representative node) pairs (cmatrix), or the persistent pair-product kernel over
 all grids' (cell tile, s-chunk) units (pair_tc).  Reported: cells*steps/s over the
 timed steps (CUDA events on the launching stream), per-grid moment drift
 between the first and last step, the autotuner's choices.

@@ -12,12 +12,18 @@
 // matrix order, and only for one node per orbit of the lattice's reflections
 // (node R(i) uses G_i with f reflected by R).
 //
-// Contraction: for output node i and 128 cells c,
-//   D[c][b] = sum_a F[c][a] G_i[a][b]   (tcgen05.mma, BF16 x BF16 -> FP32 in TMEM)
-//   I[i][c] = sum_b D[c][b] f[b][c]      (epilogue, FP32)
-// One CTA per (128-cell tile, i), by default two CTAs per cluster running each
-// MMA as a CTA pair (M = 256 cells); one launch may serve several grids.  Warp 0 issues TMA loads of F (cells x
-// 64 a) and of G_i (256 b x 64 a, or this CTA's half of it) into a ring of
+// Contraction: for a representative i and 128 rows r = (R, c), 16 cells c under
+// each of the eight reflections R, with F[r] = f[c] o R,
+//   D[r][b] = sum_a F[r][a] G_i[a][b]   (tcgen05.mma, BF16 x BF16 -> FP32 in TMEM)
+//   I[R(i)][c] = sum_b D[r][b] F[r][b]  (epilogue, FP32)
+// One CTA per (16-cell tile, i), by default two CTAs per cluster running each
+// MMA as a CTA pair (M = 256 rows, 32 cells); one launch may serve several grids.
+// All of a representative's nodes in one tile of rows: its matrix is read once
+// for them instead of once per reflection, and a batch is padded to 32 cells
+// instead of 256 (20^3, R = 4.8, one pass, against 128 cells of one node per CTA:
+// 777 cells 23.3 -> 17.7 ms, one cell 5.4 -> 0.8, 4096 cells 92.8 -> 90.0, which
+// is the tensor pipe's rate; BF16x3, 64 cells 11.3 -> 3.4).
+// Warp 0 issues TMA loads of F (rows x 64 a) and of G_i (256 b x 64 a, or this CTA's half of it) into a ring of
 // shared-memory stages (128-byte swizzle); warp 1 issues the MMAs (N = 256,
 // K = 16) into one of two TMEM accumulators, or relays its CTA's landed
 // stages to the pair's issuing CTA; warps 2..9 read the finished accumulator
@@ -40,7 +46,8 @@
 namespace gd {
 namespace {
 
-constexpr int BM = 128;  // cells per tile (MMA M, TMEM lanes)
+constexpr int BM = 128;  // rows per tile (MMA M, TMEM lanes): 16 cells under 8 reflections
+constexpr int BC = BM / 8;  // cells per tile
 constexpr int BN = 256;  // b per accumulator tile (MMA N, TMEM columns)
 constexpr int BK = 64;   // a per stage (128 bytes of BF16: one swizzle row)
 constexpr int kSlices = BK / 16;  // MMA K steps per tile, skipped one by one when all zero
@@ -97,27 +104,29 @@ __device__ __forceinline__ int stage_len(const uint32_t *tiles, int j, int cnt, 
 constexpr int kDefaultChainBf16x3 = 4;
 constexpr int kChainUnlimited = 1 << 30;
 constexpr int kLossChunk = 256;
+// Bytes of the rows (BF16 and FP32) of a group of cell tiles: half of L2 (20^3,
+// 4096 cells, one pass: 90.0 ms; 90.8 with 32 MB, 92.2 with 100 MB).
+constexpr int64_t kGroupBytes = (int64_t)64 << 20;
 
 struct CmParams {
     int ns;       // in-sphere nodes
     int ns_k;     // padded node count (multiple of BK)
     int ncells, ld;
-    const float *f;  // [8][ns_k][ldf] FP32 distribution in matrix order, per reflection (epilogue)
-    int ldf;
+    const float *f;  // [cell tile][ns_k][BM] FP32 rows in matrix order (epilogue)
     float *gain;     // [ns][ld]
     int *err;        // set to 1 when a wait times out
     const int *node_off;     // [orbits + 1] each orbit representative's range of stored tiles
     const uint32_t *tiles;   // stored tiles (mask << 28 | n << 16 | k), n-major then k per representative
-    const int *orbit;        // [ns] node -> representative's slot << 3 | reflection
-    const int *order;        // [ns] the nodes in launch order (reflection-major)
+    const int *nodes;        // [orbits][8] node R(representative)
     int m_tiles;             // cell tiles, padded to whole clusters
     int chain;               // most stored tiles summed in one tensor-memory accumulation (even)
 };
 
 // One launch serves up to kCmMaxGrids velocity grids (each with its own
-// matrices, f and gain): blockIdx.y in [ystart[j], ystart[j + 1]) is node
-// blockIdx.y - ystart[j] (in launch order) of grid j, blockIdx.x its cell
-// tile (CTAs past the grid's m_tiles leave at once, pairs together).
+// matrices, f and gain): blockIdx.y in [ystart[j], ystart[j + 1]) is the
+// representative blockIdx.y - ystart[j] of grid j, blockIdx.x + gridDim.x *
+// blockIdx.z the cell tile (CTAs past the grid's m_tiles leave at once, pairs
+// together).
 constexpr int kCmMaxGrids = 4;
 struct CmLaunch {
     CmParams g[kCmMaxGrids];
@@ -141,10 +150,9 @@ __host__ __device__ __forceinline__ int k_end(int n, int num_k)
 
 // NPASS = 1: D = F_hi G_hi.  NPASS = 3: D = F_hi G_hi + F_hi G_lo + F_lo G_hi.
 // CL = 2: a CTA pair (cluster of two) holding adjacent cell tiles of the same
-// node runs each tile as one pair MMA (tcgen05 cta_group::2, M = 256 cells):
-// each CTA loads its own F tile and half of the G tile (BN / 2 rows), the even
-// CTA issues the MMAs, and each CTA's tensor memory receives its own cells'
-// rows.  A CTA then brings 32 KB per tile into its shared memory instead of
+// representative runs each tile as one pair MMA (tcgen05 cta_group::2, M = 256
+// rows): each CTA loads its own F tile and half of the G tile (BN / 2 rows), the
+// even CTA issues the MMAs, and each CTA's tensor memory receives its own rows.  A CTA then brings 32 KB per tile into its shared memory instead of
 // 48 KB, and a G tile crosses L2 once per pair.
 template <int NPASS, int CL, bool MULTI>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -159,7 +167,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     const CmParams &p = L.g[MULTI ? gj : 0];
     // cell tiles past this grid's extent (m_tiles is a multiple of CL, so the
     // two CTAs of a pair leave together, before any barrier)
-    if ((int)blockIdx.x >= p.m_tiles) return;
+    const int m_tile = blockIdx.x + gridDim.x * blockIdx.z;
+    if (m_tile >= p.m_tiles) return;
     const int mj = MULTI ? gj : 0;
     const CUtensorMap &tmFh = maps.fh[mj], &tmFl = maps.fl[mj], &tmGh = maps.gh[mj], &tmGl = maps.gl[mj];
     constexpr int NPARTS = NPASS == 1 ? 1 : 2;
@@ -215,12 +224,11 @@ __global__ void __launch_bounds__(kThreads, 1)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_base_holder;
 
-    // one CTA per (cell tile, node); a pair holds adjacent cell tiles of one node.
-    // Node i = R(i0) for the representative i0 of its orbit under the lattice's
-    // reflections: G_i[a][b] = G_i0[R a][R b], so I_i(f) = I_i0(f o R), and the
-    // CTA contracts i0's stored tiles with the copy of f reflected by R.
-    const int m_tile = blockIdx.x, node = __ldg(p.order + (blockIdx.y - (MULTI ? L.ystart[gj] : 0)));
-    const int ob = __ldg(p.orbit + node), rep = ob >> 3, refl = ob & 7;
+    // one CTA per (cell tile, representative i0); a pair holds adjacent cell tiles.
+    // A node i = R(i0) of its orbit under the lattice's reflections has
+    // G_i[a][b] = G_i0[R a][R b], so I_i(f) = I_i0(f o R): the rows (R, cell) of
+    // the tile, the cells' f reflected by R, give all eight nodes.
+    const int rep = blockIdx.y - (MULTI ? L.ystart[gj] : 0);
     const int l0 = __ldg(p.node_off + rep), cnt = __ldg(p.node_off + rep + 1) - l0;
 
     if (warp == 0) {
@@ -241,14 +249,14 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const uint32_t fb = smem_u32(&full_bar[s]);
                 mbar_expect_tx(fb, (uint32_t)len * kTileSlot);
                 for (int t = 0; t < len; t++) {
-                    // F: this CTA's cells; G: stored tile l0 + j + t ([slot][BN rows][BK]),
+                    // F: this CTA's rows (16 cells of each reflected copy); G: stored tile l0 + j + t ([slot][BN rows][BK]),
                     // this CTA's BN / CL rows of it
                     const int k = (int)tile_k(__ldg(tl + j + t));
                     unsigned char *ts = st + (size_t)t * kTileSlot;
-                    tma_load_3d(smem_u32(ts), &tmFh, k * BK, m_tile * BM, refl, fb);
+                    tma_load_3d(smem_u32(ts), &tmFh, k * BK, m_tile * BC, 0, fb);
                     tma_load_3d(smem_u32(ts + kTileA), &tmGh, 0, (int)crank * (BN / CL), l0 + j + t, fb);
                     if (NPARTS == 2) {
-                        tma_load_3d(smem_u32(ts + kTileA + kTileBc), &tmFl, k * BK, m_tile * BM, refl, fb);
+                        tma_load_3d(smem_u32(ts + kTileA + kTileBc), &tmFl, k * BK, m_tile * BC, 0, fb);
                         tma_load_3d(smem_u32(ts + 2 * kTileA + kTileBc), &tmGl, 0, (int)crank * (BN / CL),
                                     l0 + j + t, fb);
                     }
@@ -364,23 +372,23 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int row = quad * 32 + lane;
         int grp = 0;
         bool failed = false;
-        const int cell = m_tile * BM + row;
+        const int cell = m_tile * BC + (row & (BC - 1));
         const bool live = cell < p.ncells;
-        // the gain of this cell (this half's columns): each accumulation's
+        // the gain of this row (this half's columns): each accumulation's
         // 128 products D[c][b] f_b are summed in four interleaved partials,
         // and the accumulations' sums are added with compensated (Kahan)
         // summation, so the rounding of one long FP32 chain of thousands of
         // terms does not limit the result
         float sum = 0.f, comp = 0.f;
-        // f[b][cell] for this warp's 128 b of a group; rows b >= ns of G are
+        // F[row][b] for this warp's 128 b of a group; rows b >= ns of G are
         // zero, so T[b] = 0 there and clamping b keeps every load in bounds
         // without a branch.  A group's values are requested as soon as the
         // previous group is folded, so they arrive while its MMAs run.
-        const float *fcell = p.f + (size_t)refl * p.ns_k * p.ldf + (live ? cell : 0);
+        const float *frow = p.f + (size_t)m_tile * p.ns_k * BM + row;
         float fv[BN / 2];
         auto load_f = [&](int b0) {
 #pragma unroll
-            for (int q = 0; q < BN / 2; q++) fv[q] = __ldg(fcell + (size_t)min(b0 + q, p.ns - 1) * p.ldf);
+            for (int q = 0; q < BN / 2; q++) fv[q] = __ldg(frow + (size_t)min(b0 + q, p.ns - 1) * BM);
         };
         int j = 0;
         int n = cnt > 0 ? (int)tile_n(__ldg(p.tiles + l0)) : 0;
@@ -433,11 +441,12 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (live && n_next >= 0 && n_next != n) load_f(n_next * BN + half * (BN / 2));
             n = n_next;
         }
-        // the two column halves of a cell are added in a fixed order
+        // the two column halves of a row are added in a fixed order
         if (failed) epi_failed = 1;
         if (half == 1) half_sum[row] = sum;
         asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
-        if (half == 0 && live && !epi_failed) p.gain[(size_t)node * p.ld + cell] = sum + half_sum[row];
+        if (half == 0 && live && !epi_failed)
+            p.gain[(size_t)__ldg(p.nodes + 8 * rep + row / BC) * p.ld + cell] = sum + half_sum[row];
     }
     __syncthreads();
     if (PAIR) cluster_sync();  // no remote write or arrival can reach this CTA after it leaves
@@ -543,10 +552,10 @@ __global__ void assemble_b_kernel(Dims d, int ns_k, const uint32_t *__restrict__
 
 // F[c][a] (BF16 hi/lo, a contiguous, padded to ns_k) from f (FP32, [node][c])
 // in matrix order: column a holds node inv[a].  With fp set, also the FP32
-// rows in matrix order, fp[a][c] (leading dimension ldf), for the epilogue.
+// values, fp[cell tile][a][R][cell of the tile], for the epilogue.
 __global__ void convert_f_kernel(const float *__restrict__ f, int ns, int ns_k, int ncells, int ld,
                                  const int *__restrict__ inv, __nv_bfloat16 *__restrict__ fh,
-                                 __nv_bfloat16 *__restrict__ fl, float *__restrict__ fp, int ldf, int f_rows)
+                                 __nv_bfloat16 *__restrict__ fl, float *__restrict__ fp, int f_rows)
 {
     __shared__ float tile[32][33];
     const int a0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
@@ -556,12 +565,11 @@ __global__ void convert_f_kernel(const float *__restrict__ f, int ns, int ns_k, 
     inv += (size_t)R * ns;
     fh += (size_t)R * f_rows * ns_k;
     if (fl) fl += (size_t)R * f_rows * ns_k;
-    if (fp) fp += (size_t)R * ns_k * ldf;
     for (int r = threadIdx.y; r < 32; r += blockDim.y) {
         const int a = a0 + r, c = c0 + threadIdx.x;
         const float v = (a < ns && c < ncells) ? f[(size_t)__ldg(inv + a) * ld + c] : 0.f;
         tile[r][threadIdx.x] = v;
-        if (fp && a < ns_k && c < ncells) fp[(size_t)a * ldf + c] = v;
+        if (fp && a < ns_k && c < ncells) fp[((size_t)(c / BC) * ns_k + a) * BM + R * BC + c % BC] = v;
     }
     __syncthreads();
     for (int r = threadIdx.y; r < 32; r += blockDim.y) {
@@ -615,19 +623,18 @@ struct gd_cmatrix {
     int tiles = 0;       // BN x BK tiles of one node's block upper triangle
     int cluster = 2;     // CTAs per MMA: 2 (CTA-pair MMA, M = 256 cells; the default) or 1
     // matrices are stored for one representative per orbit of the nodes under
-    // the reflections of the lattice (x -> nx - 1 - x per symmetric axis)
-    int nreps = 0;       // orbit representatives (ns / 8 on a lattice symmetric in all three axes)
-    int nrefl = 1;       // reflections of f kept on the device: 8, or 1 without a symmetric axis
-    int *orbit = nullptr;  // [ns] rep slot << 3 | reflection bits (bit a: axis a mirrored)
-    int *order = nullptr;  // [ns] the gain kernel's launch order (reflection-major)
+    // the reflections of the lattice (x -> nx - 1 - x per axis)
+    int nreps = 0;       // orbit representatives (ns / 8)
+    int nrefl = 1;       // reflections of f kept on the device: 8, or 1 for the loss alone
+    int *nodes = nullptr;  // [nreps][8] the node R(representative), bit a of R: axis a mirrored
     int64_t slots = 0;   // stored (not all-zero) tiles over the representatives
-    int64_t slices = 0;  // 16-column slices with a nonzero entry issued per cell tile (all nodes)
-    int64_t node_tiles = 0;  // stored tiles issued per cell tile (all nodes)
+    int64_t slices = 0;  // 16-column slices with a nonzero entry issued per 128 cells (all nodes)
+    int64_t node_tiles = 0;  // stored tiles issued per 128 cells (all nodes)
     int *node_off = nullptr;    // [nreps + 1] into list
     uint32_t *list = nullptr;   // stored tiles per representative, mask << 28 | n << 16 | k
     __nv_bfloat16 *gh = nullptr, *gl = nullptr;
     // f per reflection R, stacked R-major: [R][cell][matrix index] BF16 hi / lo
-    // (f_cells rows per R) and [R][matrix index][cell] FP32 (epilogue)
+    // (f_cells rows per R) and [cell tile][matrix index][R][16 cells] FP32 (epilogue)
     __nv_bfloat16 *fh = nullptr, *fl = nullptr;
     float *fp = nullptr;
     int f_cells = 0;
@@ -648,30 +655,6 @@ struct gd_cmatrix {
 
 namespace gd {
 int ensure_f(gd_cmatrix *h, int ncells);
-
-// Axes along which the node set is symmetric (bit a: x_a -> n_a - 1 - x_a maps
-// every in-sphere node to an in-sphere node).  The weights depend on |g|,
-// |d| and whether s - i lies in the box, all invariant under these
-// reflections, so G_R(i)[R a][R b] = G_i[a][b] exactly.
-int lattice_reflections(const Context &c)
-{
-    const Dims &d = c.d;
-    std::vector<char> in(d.nxyz, 0);
-    for (int m = 0; m < d.n_pnt; m++) in[((size_t)c.ui[m] * d.ny + c.vi[m]) * d.nz + c.wi[m]] = 1;
-    int axes = 0;
-    const int n[3] = {d.nx, d.ny, d.nz};
-    for (int a = 0; a < 3; a++) {
-        if (n[a] & 1) continue;  // a middle plane would be its own mirror
-        bool sym = true;
-        for (int m = 0; sym && m < d.n_pnt; m++) {
-            int x[3] = {c.ui[m], c.vi[m], c.wi[m]};
-            x[a] = n[a] - 1 - x[a];
-            sym = in[((size_t)x[0] * d.ny + x[1]) * d.nz + x[2]] != 0;
-        }
-        if (sym) axes |= 1 << a;
-    }
-    return axes;
-}
 
 // Index of (x, y, z) along a 3-D Hilbert curve through the 2^bits cube
 // (Skilling's transpose algorithm: "Programming the Hilbert curve", AIP Conf.
@@ -808,47 +791,27 @@ extern "C" int gd_cmatrix_create(gd_ctx *ctx, int mode, gd_cmatrix **out)
     for (int n = 0; n < num_n; n++)
         for (int k = 0; k < k_end(n, num_k); k++) tile_nk.push_back(make_int2(n, k));
     h->tiles = (int)tile_nk.size();
-    // orbits of the nodes under the lattice's reflections: the representative
-    // of node x mirrors every symmetric axis with x_a >= n_a / 2 (n_a is even,
-    // so no node is its own mirror and every orbit has 2^axes nodes)
-    const int axes = lattice_reflections(c);
-    h->nrefl = axes ? 8 : 1;
+    // orbits of the nodes under the lattice's reflections: every n_a is even and
+    // the sphere is centred in the box, so each node of the low octant (the
+    // representative) has seven mirrors.  The weights depend on |g|, |d| and
+    // whether s - i lies in the box, all invariant under the reflections, so
+    // G_R(i)[R a][R b] = G_i[a][b] exactly.
+    h->nrefl = 8;
     const int nax[3] = {d.nx, d.ny, d.nz};
-    std::vector<int> box_map(d.nxyz, -1);
-    for (int m = 0; m < h->ns; m++) box_map[((size_t)c.ui[m] * d.ny + c.vi[m]) * d.nz + c.wi[m]] = m;
     auto reflect = [&](int m, int R) {
         int x[3] = {c.ui[m], c.vi[m], c.wi[m]};
         for (int a = 0; a < 3; a++)
             if ((R >> a) & 1) x[a] = nax[a] - 1 - x[a];
-        return box_map[((size_t)x[0] * d.ny + x[1]) * d.nz + x[2]];
+        return c.cmap[(x[0] * d.ny + x[1]) * d.nz + x[2]];
     };
-    std::vector<int> orbit(h->ns), rep_slot(h->ns, -1), order(h->ns);
+    std::vector<int> nodes;
     std::vector<uint32_t> rep_nodes;
-    std::vector<int> orbit_size;
     for (int m = 0; m < h->ns; m++) {
-        int R = 0;
-        for (int a = 0; a < 3; a++) {
-            const int xa = a == 0 ? c.ui[m] : a == 1 ? c.vi[m] : c.wi[m];
-            if (((axes >> a) & 1) && 2 * xa >= nax[a]) R |= 1 << a;
-        }
-        const int r = reflect(m, R);
-        if (rep_slot[r] < 0) {
-            rep_slot[r] = (int)rep_nodes.size();
-            rep_nodes.push_back((uint32_t)c.ui[r] | ((uint32_t)c.vi[r] << 10) | ((uint32_t)c.wi[r] << 20));
-            orbit_size.push_back(0);
-        }
-        orbit[m] = rep_slot[r] << 3 | R;
-        orbit_size[rep_slot[r]]++;
+        if (c.ui[m] >= d.hx || c.vi[m] >= d.hy || c.wi[m] >= d.hz) continue;
+        rep_nodes.push_back((uint32_t)c.ui[m] | ((uint32_t)c.vi[m] << 10) | ((uint32_t)c.wi[m] << 20));
+        for (int R = 0; R < 8; R++) nodes.push_back(reflect(m, R));
     }
     h->nreps = (int)rep_nodes.size();
-    // launch order: reflection-major, so that the CTAs in flight read one
-    // reflected copy of f (60 MB at 20^3 / 4096 cells, L2-resident) rather
-    // than all eight; each representative's tiles are then read once per
-    // reflection (orbit-major order ran 13 % slower: 233 against 207 ms)
-    for (int m = 0; m < h->ns; m++) order[m] = m;
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
-        return ((orbit[a] & 7) << 24 | orbit[a] >> 3) < ((orbit[b] & 7) << 24 | orbit[b] >> 3);
-    });
     const size_t ntri = (size_t)h->nreps * h->tiles;  // triangle tiles over the representatives
     float *w = nullptr;
     int2 *d_tiles = nullptr;
@@ -861,11 +824,9 @@ extern "C" int gd_cmatrix_create(gd_ctx *ctx, int mode, gd_cmatrix **out)
     int rc = GD_OK;
     cudaError_t e = cudaMalloc(&h->inv, sizeof(int) * h->ns * h->nrefl);
     if (e == cudaSuccess) e = cudaMalloc(&h->mnodes, sizeof(uint32_t) * h->ns);
-    if (e == cudaSuccess) e = cudaMalloc(&h->orbit, sizeof(int) * h->ns);
-    if (e == cudaSuccess) e = cudaMalloc(&h->order, sizeof(int) * h->ns);
+    if (e == cudaSuccess) e = cudaMalloc(&h->nodes, sizeof(int) * h->ns);
     if (e == cudaSuccess) e = cudaMalloc(&d_reps, sizeof(uint32_t) * h->nreps);
-    if (e == cudaSuccess) e = cudaMemcpy(h->orbit, orbit.data(), sizeof(int) * h->ns, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(h->order, order.data(), sizeof(int) * h->ns, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(h->nodes, nodes.data(), sizeof(int) * h->ns, cudaMemcpyHostToDevice);
     if (e == cudaSuccess)
         e = cudaMemcpy(d_reps, rep_nodes.data(), sizeof(uint32_t) * h->nreps, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMalloc(&h->err, sizeof(int));
@@ -923,7 +884,7 @@ extern "C" int gd_cmatrix_create(gd_ctx *ctx, int mode, gd_cmatrix **out)
         std::vector<int> inv_r((size_t)h->ns * h->nrefl);
         for (int R = 0; R < h->nrefl; R++)
             for (int m = 0; m < h->ns; m++)
-                inv_r[(size_t)R * h->ns + m] = (R & ~axes) ? inv[m] : reflect(inv[m], R);
+                inv_r[(size_t)R * h->ns + m] = reflect(inv[m], R);
         if (e == cudaSuccess)
             e = cudaMemcpy(h->inv, inv_r.data(), sizeof(int) * inv_r.size(), cudaMemcpyHostToDevice);
         if (e == cudaSuccess)
@@ -952,8 +913,8 @@ extern "C" int gd_cmatrix_create(gd_ctx *ctx, int mode, gd_cmatrix **out)
                 for (int q = 0; q < kSlices; q++)
                     if (nz[((size_t)i * h->tiles + t) * kSlices + q]) mask |= 1u << q;
                 if (mask) {
-                    h->slices += (int64_t)__builtin_popcount(mask) * orbit_size[i];
-                    h->node_tiles += orbit_size[i];
+                    h->slices += (int64_t)__builtin_popcount(mask) * 8;
+                    h->node_tiles += 8;
                     slot_of[(size_t)i * h->tiles + t] = (int)list.size();
                     list.push_back(mask << 28 | ((uint32_t)tile_nk[t].x << 16) | (uint32_t)tile_nk[t].y);
                 }
@@ -1024,8 +985,7 @@ extern "C" int gd_cmatrix_create(gd_ctx *ctx, int mode, gd_cmatrix **out)
         cudaFree(h->err);
         cudaFree(h->inv);
         cudaFree(h->mnodes);
-        cudaFree(h->orbit);
-        cudaFree(h->order);
+        cudaFree(h->nodes);
         delete h;
         return rc;
     }
@@ -1064,8 +1024,7 @@ extern "C" int gd_cmatrix_destroy(gd_cmatrix *h)
     cudaFree(h->err);
     cudaFree(h->inv);
     cudaFree(h->mnodes);
-    cudaFree(h->orbit);
-    cudaFree(h->order);
+    cudaFree(h->nodes);
     delete h;
     return GD_OK;
 }
@@ -1082,7 +1041,7 @@ int launch_cmatrix(const CmJob *jobs, int njobs, cudaStream_t st)
     if (njobs < 1 || njobs > kCmMaxGrids) return set_error(GD_ERR_UNSUPPORTED, "collision-matrix launch: 1-4 grids");
     if (!jobs[0].cm) return set_error(GD_ERR_INVALID_ARG, "NULL argument");
     const bool split = jobs[0].cm->mode == GD_CMATRIX_BF16X3;
-    // a CTA pair per MMA when every grid allows it (cluster 2, more than one cell tile)
+    // a CTA pair per MMA when every grid allows it (cluster 2, more than one 16-cell tile)
     int cl = 2;
     int64_t total_nodes = 0;
     for (int j = 0; j < njobs; j++) {
@@ -1094,7 +1053,7 @@ int launch_cmatrix(const CmJob *jobs, int njobs, cudaStream_t st)
             return set_error(GD_ERR_UNSUPPORTED, "collision-matrix launch: one mode for every grid");
         for (int k = 0; k < j; k++)
             if (jobs[k].cm == jb.cm) return set_error(GD_ERR_UNSUPPORTED, "one launch serves distinct matrices");
-        if (jb.cm->cluster != 2 || jb.ncells <= BM) cl = 1;
+        if (jb.cm->cluster != 2 || jb.ncells <= BC) cl = 1;
         total_nodes += jb.cm->ns;
     }
     if (total_nodes > 65535) return set_error(GD_ERR_UNSUPPORTED, "collision-matrix launch: too many nodes");
@@ -1105,19 +1064,20 @@ int launch_cmatrix(const CmJob *jobs, int njobs, cudaStream_t st)
     CmLaunch L{};
     L.ngrids = njobs;
     int mx = 0;
+    int64_t bytes = 0;  // of the largest grid's rows
     for (int j = 0; j < njobs; j++) {
         const CmJob &jb = jobs[j];
         gd_cmatrix *h = jb.cm;
         if ((rc = ensure_f(h, jb.ncells))) return rc;
         dim3 cb(32, 8), cg((h->ns_k + 31) / 32, (jb.ncells + 31) / 32, h->nrefl);
         convert_f_kernel<<<cg, cb, 0, st>>>(jb.f, h->ns, h->ns_k, jb.ncells, jb.ld, h->inv, h->fh,
-                                            split ? h->fl : nullptr, h->fp, h->f_cells, h->f_cells);
+                                            split ? h->fl : nullptr, h->fp, h->f_cells);
         GD_CUDA(cudaGetLastError());
         // f per reflection: [R][cell][matrix index], f_cells rows per R (cells
         // past ncells read as zeros)
         const cuuint64_t fdims[3] = {(cuuint64_t)h->ns_k, (cuuint64_t)jb.ncells, (cuuint64_t)h->nrefl};
         const cuuint64_t fstr[2] = {(cuuint64_t)h->ns_k * 2, (cuuint64_t)h->f_cells * h->ns_k * 2};
-        const cuuint32_t fbox[3] = {BK, BM, 1};
+        const cuuint32_t fbox[3] = {BK, BC, 8};
         const cuuint64_t gdims[3] = {(cuuint64_t)BK, (cuuint64_t)BN, (cuuint64_t)std::max<int64_t>(h->slots, 1)};
         const cuuint64_t gstr[2] = {(cuuint64_t)BK * 2, (cuuint64_t)BN * BK * 2};
         // with a CTA pair each CTA loads half of a G tile
@@ -1132,16 +1092,22 @@ int launch_cmatrix(const CmJob *jobs, int njobs, cudaStream_t st)
             maps.gl[j] = maps.gh[j];
         }
         // cell tiles padded to whole clusters: a tile past ncells reads zeros and stores nothing
-        const int m_tiles = ((jb.ncells + BM - 1) / BM + cl - 1) / cl * cl;
-        L.g[j] = CmParams{h->ns,     h->ns_k,     jb.ncells, jb.ld,    h->fp,    h->f_cells, jb.gain,
-                          h->err,    h->node_off, h->list,   h->orbit, h->order, m_tiles,    h->chain};
-        L.ystart[j + 1] = L.ystart[j] + h->ns;
+        const int m_tiles = ((jb.ncells + BC - 1) / BC + cl - 1) / cl * cl;
+        L.g[j] = CmParams{h->ns,  h->ns_k,     jb.ncells, jb.ld,    h->fp,   jb.gain,
+                          h->err, h->node_off, h->list,   h->nodes, m_tiles, h->chain};
+        L.ystart[j + 1] = L.ystart[j] + h->nreps;
         mx = std::max(mx, m_tiles);
+        // a tile's rows in the BF16 copies and in FP32
+        bytes = std::max(bytes, (int64_t)h->ns_k * BM * (split ? 8 : 6) * m_tiles);
     }
-    // one CTA per (cell tile, node), cell tiles fastest so that the CTAs in flight
-    // share a few nodes' matrix tiles in L2 (a persistent grid of one CTA per SM
-    // taking the tiles round-robin measured 3-4 % slower at 20^3 / 4096 cells)
-    dim3 grid((unsigned)mx, (unsigned)L.ystart[njobs]);
+    // one CTA per (cell tile, representative), cell tiles fastest so that the CTAs
+    // in flight share a few representatives' matrix tiles in L2 (a persistent grid
+    // of one CTA per SM taking the tiles round-robin measured 3-4 % slower at 20^3 /
+    // 4096 cells), in groups of cell tiles whose rows stay in L2 while all the
+    // matrices pass once
+    const int groups = (int)std::max<int64_t>(1, (bytes + kGroupBytes - 1) / kGroupBytes);
+    const int gx = ((mx + groups - 1) / groups + cl - 1) / cl * cl;
+    dim3 grid((unsigned)gx, (unsigned)L.ystart[njobs], (unsigned)((mx + gx - 1) / gx));
     const int npass = split ? 3 : 1;
     const size_t smem = (size_t)cm_stages(npass, cl) * cm_stage_bytes(npass, cl) + 1024;
     void (*kern)(const CmMaps, const CmLaunch) =
@@ -1230,6 +1196,7 @@ int ensure_f(gd_cmatrix *h, int ncells)
     h->fh = h->fl = nullptr;
     h->fp = nullptr;
     h->f_cells = 0;
+    ncells = (ncells + BC - 1) / BC * BC;
     const size_t per = (size_t)ncells * h->ns_k * h->nrefl;  // one copy of f per reflection
     GD_CUDA(cudaMalloc(&h->fh, per * 2));
     GD_CUDA(cudaMalloc(&h->fl, per * 2));
@@ -1246,7 +1213,7 @@ int cmatrix_loss(gd_cmatrix *h, const float *f, int ncells, int ld, float *nu, c
     int rc = ensure_f(h, ncells);
     if (rc) return rc;
     dim3 cb(32, 8), cg((h->ns_k + 31) / 32, (ncells + 31) / 32, 1);  // f itself (R = 0)
-    convert_f_kernel<<<cg, cb, 0, st>>>(f, h->ns, h->ns_k, ncells, ld, h->inv, h->fh, h->fl, nullptr, 0, h->f_cells);
+    convert_f_kernel<<<cg, cb, 0, st>>>(f, h->ns, h->ns_k, ncells, ld, h->inv, h->fh, h->fl, nullptr, h->f_cells);
     GD_CUDA(cudaGetLastError());
     const int stall = h->stall_next;  // a pending time-out injection fires here, once
     h->stall_next = 0;
@@ -1266,9 +1233,7 @@ double cmatrix_bytes_bound(const Context &c, int mode)
     const int num_n = (ns + BN - 1) / BN, num_k = ns_k / BK;
     int64_t tiles = 0;
     for (int n = 0; n < num_n; n++) tiles += k_end(n, num_k);
-    // matrices of one representative per orbit of the reflections
-    const int axes = lattice_reflections(c);
-    const double reps = (double)ns / (double)(1 << __builtin_popcount(axes));
+    const double reps = ns / 8.0;  // matrices of one representative per orbit of the reflections
     return (double)tiles * reps * BN * BK * 2.0 * (mode == GD_CMATRIX_BF16X3 ? 2.0 : 1.0);
 }
 

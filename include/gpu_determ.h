@@ -63,9 +63,9 @@ typedef struct {
     int64_t scatter_terms;     /* (s, g, sign) output updates per cell-eval */
     int64_t cmatrix_tiles;     /* stored 256 x 64 tiles of the collision matrices (0 without, see gd_ctx_set_gain_path) */
     int64_t cmatrix_slices;    /* 256 x 16 slices with a nonzero entry over every node's matrix: the MMA
-                                  K steps one cell tile issues in GD_CMATRIX_BF16X3 mode */
+                                  K steps 128 cells issue in GD_CMATRIX_BF16X3 mode */
     int64_t cmatrix_node_tiles; /* tiles over every node's matrix (a node uses the stored tiles of its
-                                   orbit's representative): what one BF16 pass issues per cell tile */
+                                   orbit's representative): what one BF16 pass issues per 128 cells */
 } gd_info;
 
 /* Library version (major*10000 + minor*100 + patch). */
@@ -193,11 +193,11 @@ enum { GD_CMATRIX_BF16 = 0, GD_CMATRIX_BF16X3 = 1 };
 int gd_cmatrix_create(gd_ctx *ctx, int mode, gd_cmatrix **out);
 int gd_cmatrix_gain(gd_cmatrix *cm, const float *f, int ncells, int ld, float *gain, gd_stream stream);
 int gd_cmatrix_destroy(gd_cmatrix *cm);
-/* CTAs per tensor-core MMA of the gain kernel: 2 (the default) or 1.  With
- * 2, the CTAs of a node's two adjacent 128-cell tiles form a cluster and run
- * each MMA as a CTA pair (M = 256 cells): each loads its own cells and half
- * of every collision-matrix tile; a call with at most 128 cells runs one CTA
- * per MMA.  Results are bitwise the same either way. */
+/* CTAs per tensor-core MMA of the gain kernel: 2 (the default) or 1.  A CTA
+ * takes 16 cells under all eight reflections (128 rows).  With 2, the CTAs of
+ * two adjacent 16-cell tiles form a cluster and run each MMA as a CTA pair (M =
+ * 256 rows): each loads its own rows and half of every collision-matrix tile; a
+ * call with at most 16 cells runs one CTA per MMA.  Results are bitwise the same either way. */
 int gd_cmatrix_set_cluster(gd_cmatrix *cm, int ctas);
 /* Longest run of stored tiles (an even count; 0 = unlimited) summed into
  * one tensor-memory accumulator before the epilogue folds it into the FP32
@@ -288,7 +288,7 @@ int gd_batch_step(gd_batch *b, int use_graph, gd_stream stream);
  * recorded on the first group's context.  GD_BATCH_FUSED_CMATRIX: the same
  * with the gains of all groups (at most 4, on distinct contexts whose gain
  * path is the same collision-matrix mode) in one launch of the
- * collision-matrix kernel over every grid's (cell tile, node) pairs; results
+ * collision-matrix kernel over every grid's (cell tile, representative) pairs; results
  * equal gd_step bit for bit, time-outs are recorded per context. */
 enum { GD_BATCH_STREAMS = 0, GD_BATCH_FUSED_PAIR_TC = 1, GD_BATCH_FUSED_CMATRIX = 2 };
 int gd_batch_set_mode(gd_batch *b, int mode);
