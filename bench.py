@@ -378,8 +378,7 @@ def run_ours(args):
              "bf16x3": "bf16x3 (hi/lo split, FP32 accumulate, at most 256 products per tensor-core accumulation)"
              }[args.gain]
     if fp32_gain(args.gain, ctx):
-        dtype = "f32 gain" + ("" if args.gain == "pair" else
-                              "; bf16x3 loss (hi/lo split, FP32 accumulate, at most 256 products per accumulation)")
+        dtype = "f32"
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None,
@@ -434,22 +433,20 @@ def run_ours(args):
 
 
 def fp32_gain(name, ctx):
-    """Whether the FP32 kernel that does all reflections of a pair sum at once
-    computes this path's gain: every lattice of this workload but, for BF16x3,
+    """Whether the FP32 kernels that do all reflections at once compute this
+    path's loss and gain: every lattice of this workload but, for BF16x3,
     those small enough that their matrices are faster (then they are built)."""
     return name in ("pair", "pair_tc") or (name == "bf16x3" and ctx._info()["cmatrix_tiles"] == 0)
 
 
 def path_launches(name, ctx):
     """Kernel launches of the loss and of the gain on a gain path: the FP32
-    loss kernel, or on the tensor-core paths the BF16 conversion of f and one
+    loss kernel, or with the collision matrices the BF16 conversion of f and one
     tensor-core GEMM; the packing of f, the FP32 gain kernel and its chunk
     reduction (on the tensor-core paths that it serves after the cells'
     scales), or the conversion of f and the collision-matrix kernel."""
-    if name == "pair":
-        return 1, 3
     if fp32_gain(name, ctx):
-        return 2, 4
+        return 1, 3 if name == "pair" else 4
     if name == "pair_tc":
         return 2, 3
     return 2, 2

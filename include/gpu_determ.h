@@ -125,8 +125,8 @@ int gd_correction_basis(gd_ctx *ctx, float *basis, gd_stream stream);
 /* Loss frequency nu[i][c] = sum_j b(|i-j|) f[j][c] and gain I[i][c] over the
  * in-sphere nodes (either output may be NULL), on the context's gain path:
  * GD_GAIN_PAIR computes both in FP32 (SIMT kernels); the other paths compute
- * the gain as gd_ctx_set_gain_path says and, when ld is a multiple of 4, the
- * loss as one BF16x3 GEMM on the tensor cores.  Replaces the
+ * the gain as gd_ctx_set_gain_path says and the loss, where the gain is not the
+ * FP32 kernel's and ld is a multiple of 4, as one BF16x3 GEMM on the tensor cores.  Replaces the
  * loss and gain stages of evolve_colisions (collision_integral.h:11-17,
  * collision_integral.cu:32-188, 587-648). */
 int gd_collision(gd_ctx *ctx, const float *f, int ncells, int ld, float *nu, float *gain,
@@ -183,9 +183,10 @@ int gd_ctx_check(gd_ctx *ctx, gd_stream stream);
  * than one matrix per node).  GD_CMATRIX_BF16 rounds f and G to BF16
  * (relative error ~3e-4 on I); GD_CMATRIX_BF16X3 splits both into BF16 hi +
  * lo parts and sums hi*hi + hi*lo + lo*hi (~4e-6).  With a context's gain
- * path set to either mode (or to GD_GAIN_PAIR_TC), its loss nu = B f also
- * runs on the tensor cores (B and f split into BF16 hi + lo, three products
- * per K step in one launch, ~5e-6) when ld is a multiple of 4.  No reference
+ * path set to either mode (or to GD_GAIN_PAIR_TC) and its gain on the tensor
+ * cores (see gd_ctx_set_gain_path), its loss nu = B f also runs there (B and f
+ * split into BF16 hi + lo, three products per K step in one launch, ~5e-6) when
+ * ld is a multiple of 4.  No reference
  * counterpart: the reference forms these matrices only implicitly in its
  * gain loop (collision_integral.cu:75-188). */
 typedef struct gd_cmatrix gd_cmatrix;
@@ -222,8 +223,8 @@ int gd_cmatrix_check(gd_cmatrix *cm, gd_stream stream);
  * cell's outputs summed in 64-bit fixed point scaled by a bound on its gain;
  * builds a per-class-box weight table of a few GB at 24^3 instead of n^3
  * matrices, so it serves the grids whose collision matrices do not fit).
- * Where the FP32 kernel is faster, and its error no larger, it computes the gain
- * of GD_GAIN_CMATRIX_BF16X3 (lattices of 512 nodes or more; the matrices are then
+ * Where the FP32 kernel is faster, and its error no larger, it computes the gain,
+ * and an FP32 kernel the loss, of GD_GAIN_CMATRIX_BF16X3 (lattices of 512 nodes or more; the matrices are then
  * not built) and of GD_GAIN_PAIR_TC too: every lattice whose half-box rows fit
  * its shared memory, up to 24^3 with R = 4.8.
  * The two pair paths need n_pnt * ld < 2^31 (GD_ERR_UNSUPPORTED otherwise). */
