@@ -30,16 +30,21 @@ namespace {
 using namespace tc;
 using bf16 = __nv_bfloat16;
 
-constexpr int GM = 128, GN = 256, GK = 64, GS = 4;
-constexpr uint32_t kA = GM * GK * 2, kB = GN * GK * 2, kStageBytes = kA + kB;
-constexpr uint32_t kGIdesc = umma_idesc_bf16(GM, GN);
+// GEMM tile of GM rows x GN columns (see gemm_nt), K steps of GK.
+constexpr int GM = 128, GK = 64;
+constexpr uint32_t kA = GM * GK * 2;
 constexpr int kGThreads = 192;
-constexpr size_t kGemmSmem = GS * kStageBytes + 1024;
+constexpr uint32_t gemm_stage(int gn) { return kA + (uint32_t)gn * GK * 2; }
+constexpr int kGMaxStages = 4;
+// the epilogue warps' 32 x 32 tiles (rows of 33), then the stages
+constexpr uint32_t kEpiTile = 32 * 33 * 4, kEpiBytes = (4 * kEpiTile + 1023) / 1024 * 1024;
+constexpr size_t gemm_smem(int gn, int stages) { return 1024 + kEpiBytes + (size_t)stages * gemm_stage(gn); }
 
-enum { EPI_NONE = 0, EPI_GELU = 1, EPI_DGELU = 2 };
+enum { EPI_NONE = 0, EPI_GELU = 1, EPI_DGELU = 2, EPI_NODE = 3 };
 
 struct GemmArgs {
     int M, N, K;
+    int stages, kps;    // stages of shared memory and K steps of each, set by gemm_nt
     const float *bias;  // [N] or null
     const float *add;   // [M][ld32] added after the bias, or null
     const float *aux;   // EPI_DGELU: pre-activation [M][ld32]
@@ -47,6 +52,12 @@ struct GemmArgs {
     float *c32;         // [M][ld32] or null
     bf16 *c16;          // [M][ld16] or null
     int ld32, ld16;
+    // EPI_NODE: c32 is [column][ld32], each row's values times its scale (the
+    // network's output in the library's layout): columns < n_out, times
+    // out_gain and, when scale2 is set, scale2[row]^2
+    const float *scale2;
+    float out_gain;
+    int n_out;
     int *err;
     // failure-detection test hook: > 0 makes every CTA wait this many polls on
     // a barrier that nothing arrives at (before any copy or MMA is issued),
@@ -60,35 +71,44 @@ __device__ __forceinline__ float gelu_grad(float x)
     return 0.5f * (1.f + erff(x * 0.70710678118654752f)) + x * 0.39894228040143268f * expf(-0.5f * x * x);
 }
 
+// extra: the row's value of p.add (or of p.aux)
 template <int EPI>
-__device__ __forceinline__ void epilogue_value(const GemmArgs &p, size_t o32, int n, float &x)
+__device__ __forceinline__ void epilogue_value(const GemmArgs &p, size_t o32, float bias, float extra, float &x)
 {
-    if (p.bias) x += __ldg(p.bias + n);
-    if (p.add) x += p.add[o32];
-    if (EPI == EPI_GELU) {
-        if (p.pre_out) p.pre_out[o32] = x;
-        x = gelu(x);
-    } else if (EPI == EPI_DGELU) {
-        x *= gelu_grad(p.aux[o32]);
+    if (p.bias) x += bias;
+    if (EPI == EPI_DGELU) {
+        x *= gelu_grad(extra);
+    } else {
+        if (p.add) x += extra;
+        if (EPI == EPI_GELU) {
+            if (p.pre_out) p.pre_out[o32] = x;
+            x = gelu(x);
+        }
     }
 }
 
-// C[M][N] = sum_k A[m][k] B[n][k] (A: M x K, B: N x K, both K-major BF16),
-// one 128 x 256 tile per CTA; warp 0 issues TMA, warp 1 the MMAs, warps 2..5
-// read the accumulator (row m = thread) and apply the epilogue.
-template <int EPI>
+// C[M][N] = sum_k A[m][k] B[n][k] (A: M x K, B: N x K, both K-major BF16), in
+// 128 x GN tiles, gridDim.x CTAs taking them in turn; warp 0 issues TMA, warp 1
+// the MMAs into one of two accumulators, warps 2..5 read the other (row m = thread)
+// and apply the epilogue.  A warp turns its 32 x 32 values in shared memory, so
+// that its lanes hold 32 columns of a row and every access of C and of the added or
+// multiplied arrays is one segment (a row per lane before: 32 segments of 16 bytes);
+// the added or multiplied values are requested before the accumulator is awaited.
+template <int EPI, int GN>
 __global__ void __launch_bounds__(kGThreads, 1)
     gemm_nt_kernel(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUtensorMap tB, GemmArgs p)
 {
+    constexpr uint32_t kStageBytes = gemm_stage(GN), kIdesc = umma_idesc_bf16(GM, GN);
     extern __shared__ __align__(1024) unsigned char dsmem[];
-    unsigned char *base = reinterpret_cast<unsigned char *>(
+    unsigned char *epi = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(dsmem) + 1023) & ~static_cast<uintptr_t>(1023));
-    __shared__ __align__(8) uint64_t full_bar[GS], empty_bar[GS], acc_bar, stall_bar;
+    unsigned char *base = epi + kEpiBytes;
+    __shared__ __align__(8) uint64_t full_bar[kGMaxStages], empty_bar[kGMaxStages], accf_bar[2], acce_bar[2], stall_bar;
     __shared__ uint32_t tmem_holder;
     __shared__ int abort_flag;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m0 = blockIdx.x * GM, n0 = blockIdx.y * GN;
-    const int num_k = p.K / GK;
+    const int num_k = p.K / GK, GS = p.stages, KPS = p.kps;
+    const int mt = (p.M + GM - 1) / GM, tiles = mt * ((p.N + GN - 1) / GN);
 
     if (threadIdx.x == 0) abort_flag = *(volatile int *)p.err;
     __syncthreads();
@@ -98,13 +118,16 @@ __global__ void __launch_bounds__(kGThreads, 1)
             mbar_init(smem_u32(&full_bar[s]), 1);
             mbar_init(smem_u32(&empty_bar[s]), 1);
         }
-        mbar_init(smem_u32(&acc_bar), 1);
+        for (int b = 0; b < 2; b++) {
+            mbar_init(smem_u32(&accf_bar[b]), 1);
+            mbar_init(smem_u32(&acce_bar[b]), 4);  // the four epilogue warps
+        }
         mbar_init(smem_u32(&stall_bar), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_holder)),
-                     "r"(GN)
+                     "r"(2 * GN)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -127,82 +150,125 @@ __global__ void __launch_bounds__(kGThreads, 1)
         // every thread skips the work alike and meets the barrier below
     } else if (warp == 0) {
         if (lane == 0) {
-            for (int k = 0; k < num_k; k++) {
-                const int s = k % GS;
-                const uint32_t ph = (uint32_t)(k / GS) & 1u;
-                if (!mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1u, p.err)) break;
-                unsigned char *st = base + (size_t)s * kStageBytes;
-                const uint32_t fb = smem_u32(&full_bar[s]);
-                mbar_expect_tx(fb, kStageBytes);
-                tma_load_2d(smem_u32(st), &tA, k * GK, m0, fb);
-                tma_load_2d(smem_u32(st + kA), &tB, k * GK, n0, fb);
+            bool ok = true;
+            int s = 0;
+            uint32_t ph = 0;
+            for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
+                const int m0 = t % mt * GM, n0 = t / mt * GN;
+                for (int k = 0; k < num_k; k += KPS) {
+                    if (!mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1u, p.err)) {
+                        ok = false;
+                        break;
+                    }
+                    uint32_t st = smem_u32(base) + (uint32_t)(s * KPS) * kStageBytes;
+                    const uint32_t fb = smem_u32(&full_bar[s]);
+                    const int kn = min(KPS, num_k - k);
+                    mbar_expect_tx(fb, (uint32_t)kn * kStageBytes);
+                    for (int q = 0; q < kn; q++, st += kStageBytes) {
+                        tma_load_2d(st, &tA, (k + q) * GK, m0, fb);
+                        tma_load_2d(st + kA, &tB, (k + q) * GK, n0, fb);
+                    }
+                    if (++s == GS) {
+                        s = 0;
+                        ph ^= 1u;
+                    }
+                }
             }
         }
     } else if (warp == 1) {
         if (lane == 0) {
             bool ok = true;
-            for (int k = 0; k < num_k; k++) {
-                const int s = k % GS;
-                const uint32_t ph = (uint32_t)(k / GS) & 1u;
-                if (!mbar_wait(smem_u32(&full_bar[s]), ph, p.err)) {
-                    ok = false;
-                    break;
-                }
+            int s = 0, i = 0;
+            uint32_t ph = 0;
+            for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x, i++) {
+                const int buf = i & 1;
+                if (!mbar_wait(smem_u32(&acce_bar[buf]), ((uint32_t)(i >> 1) & 1u) ^ 1u, p.err)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t st = smem_u32(base + (size_t)s * kStageBytes);
+                for (int k = 0; k < num_k; k += KPS) {
+                    if (!mbar_wait(smem_u32(&full_bar[s]), ph, p.err)) {
+                        ok = false;
+                        break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    uint32_t st = smem_u32(base) + (uint32_t)(s * KPS) * kStageBytes;
+                    const int kn = min(KPS, num_k - k);
+                    for (int q = 0; q < kn; q++, st += kStageBytes) {
 #pragma unroll
-                for (int kk = 0; kk < GK / 16; kk++) {
-                    const uint32_t off = (uint32_t)kk * 32u;
-                    umma_bf16(tmem, umma_desc(st + off), umma_desc(st + kA + off), kGIdesc, (k > 0 || kk > 0) ? 1u : 0u);
+                        for (int kk = 0; kk < GK / 16; kk++) {
+                            const uint32_t off = (uint32_t)kk * 32u;
+                            umma_bf16(tmem + (uint32_t)(buf * GN), umma_desc(st + off), umma_desc(st + kA + off),
+                                      kIdesc, (k + q > 0 || kk > 0) ? 1u : 0u);
+                        }
+                    }
+                    umma_commit(smem_u32(&empty_bar[s]));
+                    if (++s == GS) {
+                        s = 0;
+                        ph ^= 1u;
+                    }
                 }
-                umma_commit(smem_u32(&empty_bar[s]));
+                if (ok) umma_commit(smem_u32(&accf_bar[buf]));
             }
-            if (ok) umma_commit(smem_u32(&acc_bar));
         }
     } else {
         const int quad = warp & 3;
-        const int m = m0 + quad * 32 + lane;
-        bool ok = true;
-        if (lane == 0) ok = mbar_wait(smem_u32(&acc_bar), 0u, p.err);
-        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-        if (ok) {
+        float *tile = reinterpret_cast<float *>(epi + quad * kEpiTile);
+        const float *ex = EPI == EPI_DGELU ? p.aux : p.add;
+        int i = 0;
+        for (int t = blockIdx.x; t < tiles; t += gridDim.x, i++) {
+            const int mw = t % mt * GM + quad * 32, m = mw + lane;  // the warp's first row, the lane's
+            const int n0 = t / mt * GN, rows = min(32, p.M - mw);
+            float s = 0.f;
+            if (EPI == EPI_NODE && m < p.M)
+                s = (p.scale2 ? __ldg(p.scale2 + m) * __ldg(p.scale2 + m) : 1.f) * p.out_gain;
+            float extra[32];
+            auto load_extra = [&](int n) {
+                if (EPI == EPI_NODE || EPI == EPI_GELU || !ex) return;
+#pragma unroll
+                for (int r = 0; r < 32; r++) extra[r] = r < rows && n < p.N ? ex[(size_t)(mw + r) * p.ld32 + n] : 0.f;
+            };
+            load_extra(n0 + lane);
+            const int buf = i & 1;
+            bool ok = true;
+            if (lane == 0) ok = mbar_wait(smem_u32(&accf_bar[buf]), (uint32_t)(i >> 1) & 1u, p.err);
+            if (__shfl_sync(0xffffffffu, ok ? 1 : 0, 0) == 0) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16);
+            const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * GN);
+#pragma unroll 1
             for (int c0 = 0; c0 < GN; c0 += 32) {
+                const int n = n0 + c0 + lane;
+                const float bias = p.bias && n < p.N ? __ldg(p.bias + n) : 0.f;
                 float v[32];
                 tmem_ld32(taddr + (uint32_t)c0, v);
-                if (m >= p.M || n0 + c0 >= p.N) continue;
-                const size_t r32 = (size_t)m * p.ld32, r16 = (size_t)m * p.ld16;
-                if (n0 + c0 + 32 <= p.N) {
-                    // full 32-column chunk: 16-byte FP32 and 8-byte BF16 stores
-                    // (ld32, ld16 are multiples of 4 and n0 + c0 of 32)
-#pragma unroll
-                    for (int j = 0; j < 32; j += 4) {
-                        const int n = n0 + c0 + j;
-                        float x[4] = {v[j], v[j + 1], v[j + 2], v[j + 3]};
-#pragma unroll
-                        for (int q = 0; q < 4; q++) epilogue_value<EPI>(p, r32 + n + q, n + q, x[q]);
-                        if (p.c32) *reinterpret_cast<float4 *>(p.c32 + r32 + n) = make_float4(x[0], x[1], x[2], x[3]);
-                        if (p.c16) {
-                            __nv_bfloat162 lo = __floats2bfloat162_rn(x[0], x[1]);
-                            __nv_bfloat162 hi = __floats2bfloat162_rn(x[2], x[3]);
-                            uint2 pk;
-                            pk.x = *reinterpret_cast<uint32_t *>(&lo);
-                            pk.y = *reinterpret_cast<uint32_t *>(&hi);
-                            *reinterpret_cast<uint2 *>(p.c16 + r16 + n) = pk;
-                        }
-                    }
-                } else {
+                if (c0 + 32 == GN) {
+                    // the accumulator is read: the next tile but one may use it
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&acce_bar[buf]));
+                }
+                if (EPI == EPI_NODE) {
+                    // lanes hold 32 rows of a column: the output's layout
 #pragma unroll
                     for (int j = 0; j < 32; j++) {
-                        const int n = n0 + c0 + j;
-                        if (n < p.N) {
-                            float x = v[j];
-                            epilogue_value<EPI>(p, r32 + n, n, x);
-                            if (p.c32) p.c32[r32 + n] = x;
-                            if (p.c16) p.c16[r16 + n] = __float2bfloat16_rn(x);
+                        float x = v[j];
+                        epilogue_value<EPI>(p, 0, __shfl_sync(0xffffffffu, bias, j), 0.f, x);
+                        if (m < p.M && n0 + c0 + j < p.n_out) p.c32[(size_t)(n0 + c0 + j) * p.ld32 + m] = x * s;
+                    }
+                } else {
+                    if (c0 > 0) load_extra(n);
+#pragma unroll
+                    for (int j = 0; j < 32; j++) tile[lane * 33 + j] = v[j];
+                    __syncwarp();
+                    if (n < p.N) {
+#pragma unroll
+                        for (int r = 0; r < 32; r++) {
+                            if (r >= rows) continue;
+                            float x = tile[r * 33 + lane];
+                            epilogue_value<EPI>(p, (size_t)(mw + r) * p.ld32 + n, bias, extra[r], x);
+                            if (p.c32) p.c32[(size_t)(mw + r) * p.ld32 + n] = x;
+                            if (p.c16) p.c16[(size_t)(mw + r) * p.ld16 + n] = __float2bfloat16_rn(x);
                         }
                     }
+                    __syncwarp();
                 }
             }
         }
@@ -210,7 +276,7 @@ __global__ void __launch_bounds__(kGThreads, 1)
     __syncthreads();
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(GN) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * GN) : "memory");
     }
 }
 
@@ -523,20 +589,30 @@ __global__ void __launch_bounds__(1024) cell_scale_kernel(const float *__restric
 
 __device__ __forceinline__ float inv_or_zero(float s) { return s != 0.f ? 1.f / s : 0.f; }
 
-// node-major FP32 x[i][r] (ld) -> cell-major BF16 xb[r][i] * gain / scale[r] (pad to n_p)
+// node-major FP32 x[i][r] (ld) -> cell-major BF16 xb[r][i] * gain / scale[r] (pad to
+// n_p).  Block = 64 nodes x 32 cells: eight loads in flight per thread and whole
+// 128-byte rows on both sides (4096 cells, 3648 nodes: 39 -> 15 us).
 __global__ void gather_in_kernel(const float *__restrict__ x, int n, int ld, int B, const float *__restrict__ scale,
                                  float gain, bf16 *__restrict__ xb, int n_p)
 {
-    __shared__ float tile[32][33];
-    const int i0 = blockIdx.y * 32, r0 = blockIdx.x * 32;
-    for (int y = threadIdx.y; y < 32; y += blockDim.y) {
-        const int i = i0 + y, r = r0 + threadIdx.x;
-        tile[y][threadIdx.x] = (i < n && r < B) ? x[(size_t)i * ld + r] : 0.f;
+    __shared__ float tile[64][33];
+    const int i0 = blockIdx.y * 64, r0 = blockIdx.x * 32, r = r0 + threadIdx.x;
+    const float s = r < B ? inv_or_zero(scale[r]) * gain : 0.f;
+    float v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const int i = i0 + threadIdx.y + 8 * k;
+        v[k] = i < n && r < B ? __ldg(x + (size_t)i * ld + r) : 0.f;
     }
+#pragma unroll
+    for (int k = 0; k < 8; k++) tile[threadIdx.y + 8 * k][threadIdx.x] = v[k] * s;
     __syncthreads();
-    for (int y = threadIdx.y; y < 32; y += blockDim.y) {
-        const int r = r0 + y, i = i0 + threadIdx.x;
-        if (r < B && i < n_p) xb[(size_t)r * n_p + i] = __float2bfloat16_rn(tile[threadIdx.x][y] * (inv_or_zero(scale[r]) * gain));
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int y = threadIdx.y + 8 * k, c = 2 * threadIdx.x;
+        if (r0 + y < B)
+            *reinterpret_cast<__nv_bfloat162 *>(xb + (size_t)(r0 + y) * n_p + i0 + c) =
+                __floats2bfloat162_rn(tile[c][y], tile[c + 1][y]);
     }
 }
 
@@ -557,27 +633,6 @@ __global__ void gather_target_kernel(const float *__restrict__ t, int n, int ld,
         if (r < B && i < n_p) {
             const float s = (pw ? inv_or_zero(scale[r] * scale[r]) : 1.f) * inv_gain;
             tt[(size_t)r * n_p + i] = tile[threadIdx.x][y] * s;
-        }
-    }
-}
-
-// cell-major FP32 y[r][i] (ld n_p) -> node-major out[i][r] * gain * scale[r]^2 (the scale
-// only when pw)
-__global__ void scatter_out_kernel(const float *__restrict__ y, int n_p, int n, int B, const float *__restrict__ scale,
-                                   int pw, float gain, float *__restrict__ out, int ld)
-{
-    __shared__ float tile[32][33];
-    const int i0 = blockIdx.y * 32, r0 = blockIdx.x * 32;
-    for (int yy = threadIdx.y; yy < 32; yy += blockDim.y) {
-        const int r = r0 + yy, i = i0 + threadIdx.x;
-        tile[yy][threadIdx.x] = (r < B && i < n) ? y[(size_t)r * n_p + i] : 0.f;
-    }
-    __syncthreads();
-    for (int yy = threadIdx.y; yy < 32; yy += blockDim.y) {
-        const int i = i0 + yy, r = r0 + threadIdx.x;
-        if (i < n && r < B) {
-            const float s = (pw ? scale[r] * scale[r] : 1.f) * gain;
-            out[(size_t)i * ld + r] = tile[threadIdx.x][yy] * s;
         }
     }
 }
@@ -720,26 +775,47 @@ int make_map(CUtensorMap *m, const bf16 *ptr, int rows, int K, int box_rows)
 // output strides ld32, ld16 multiples of 4.
 int gemm_nt(int epi, const bf16 *A, const bf16 *B, const GemmArgs &a, cudaStream_t st)
 {
-    if (a.K % GK || a.K <= 0 || a.M <= 0 || a.N <= 0 || (a.ld32 & 3) || (a.ld16 & 3))
+    if (a.K % GK || a.K <= 0 || a.M <= 0 || a.N <= 0 || (epi != EPI_NODE && ((a.ld32 & 3) || (a.ld16 & 3))))
         return set_error(GD_ERR_INVALID_ARG, "GEMM shape: K a multiple of 64, strides multiples of 4");
+    int dev = 0, sms = 0;
+    GD_CUDA(cudaGetDevice(&dev));
+    GD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    // Tile width, K steps per stage and stages.  A K of up to 8 steps (every layer
+    // but the first and the weights' gradients): 32 columns and two CTAs per SM,
+    // since a CTA's fixed costs and its epilogue bound it (1024 x 512, K = 512: 10 us;
+    // 13 with 64 columns, 20 with 128, 34 with 256; 4096 x 3648, K = 256: 26 us, 36
+    // with 64, 33 with 128).  A longer K is bound by the handshakes and copies of its
+    // stages: four steps in each, in the narrowest tiles that one wave holds (1024 x
+    // 256, K = 3648: 17 us with 32 columns, 18 with 64, 27 with 128, one step per
+    // stage 24; 4096 x 256: 22 us with 64 columns, 32 with 32).
+    const int mt = (a.M + GM - 1) / GM, num_k = a.K / GK;
+    const bool longk = num_k > 8;
+    int gn = 32;
+    while (longk && gn < 256 && mt * ((a.N + gn - 1) / gn) > sms) gn *= 2;
     CUtensorMap tA, tB;
     int rc = make_map(&tA, A, a.M, a.K, GM);
-    if (!rc) rc = make_map(&tB, B, a.N, a.K, GN);
+    if (!rc) rc = make_map(&tB, B, a.N, a.K, gn);
     if (rc) return rc;
-    dim3 grid((a.M + GM - 1) / GM, (a.N + GN - 1) / GN);
-    switch (epi) {
-#define GD_GEMM_CASE(E)                                                                                          \
-    case E:                                                                                                      \
-        GD_CUDA(cudaFuncSetAttribute(gemm_nt_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem)); \
-        gemm_nt_kernel<E><<<grid, kGThreads, kGemmSmem, st>>>(tA, tB, a);                                        \
-        break;
-        GD_GEMM_CASE(EPI_NONE)
-        GD_GEMM_CASE(EPI_GELU)
-        GD_GEMM_CASE(EPI_DGELU)
-#undef GD_GEMM_CASE
-    default:
-        return set_error(GD_ERR_INVALID_ARG, "unknown GEMM epilogue");
+    GemmArgs b = a;
+    b.kps = longk ? 4 : 2;
+    b.stages = longk ? std::min((num_k + b.kps - 1) / b.kps, (int)((200u << 10) / (b.kps * gemm_stage(gn)))) : 2;
+    if (b.stages < 2) {  // 256 columns
+        b.kps = 2;
+        b.stages = 2;
     }
+    const size_t smem = gemm_smem(gn, b.stages * b.kps);
+    const int grid = std::min(mt * ((a.N + gn - 1) / gn), sms * (longk ? 1 : 2));
+    using Kernel = void (*)(const CUtensorMap, const CUtensorMap, GemmArgs);
+    Kernel kern = nullptr;
+    if (longk && epi == EPI_NONE)
+        kern = gn == 32 ? gemm_nt_kernel<EPI_NONE, 32> : gn == 64 ? gemm_nt_kernel<EPI_NONE, 64>
+             : gn == 128 ? gemm_nt_kernel<EPI_NONE, 128> : gemm_nt_kernel<EPI_NONE, 256>;
+    else if (!longk)
+        kern = epi == EPI_NONE ? gemm_nt_kernel<EPI_NONE, 32> : epi == EPI_GELU ? gemm_nt_kernel<EPI_GELU, 32>
+             : epi == EPI_DGELU ? gemm_nt_kernel<EPI_DGELU, 32> : epi == EPI_NODE ? gemm_nt_kernel<EPI_NODE, 32> : nullptr;
+    if (!kern) return set_error(GD_ERR_INVALID_ARG, "unknown GEMM epilogue for this K");
+    GD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<grid, kGThreads, smem, st>>>(tA, tB, b);
     GD_CUDA(cudaGetLastError());
     return GD_OK;
 }
@@ -863,14 +939,15 @@ int load_input(gd_mlp *h, const float *x, int ldx, int B, cudaStream_t st)
     int rc = gd::launch_ordered(gd::cell_scale_kernel, B, st, x, h->n_in, ldx, B,
                                 (int)(h->flags & GD_MLP_SCALE_INPUT), h->scale);
     if (rc) return rc;
-    dim3 blk(32, 8), grd((B + 31) / 32, h->n_in_p / 32);
+    dim3 blk(32, 8), grd((B + 31) / 32, h->n_in_p / 64);
     gd::gather_in_kernel<<<grd, blk, 0, st>>>(x, h->n_in, ldx, B, h->scale, h->in_gain, h->xb, h->n_in_p);
     GD_CUDA(cudaGetLastError());
     return GD_OK;
 }
 
-// forward on rows [0, B) of h->xb; y (FP32, [B][n_out_p]) into h->y
-int forward(gd_mlp *h, int B, cudaStream_t st)
+// forward on rows [0, B) of h->xb; the output times its scales into out
+// [n_out][ld_out], or, when out is null, unscaled into h->y ([B][n_out_p])
+int forward(gd_mlp *h, int B, float *out, int ld_out, cudaStream_t st)
 {
     using namespace gd;
     int rc;
@@ -906,6 +983,14 @@ int forward(gd_mlp *h, int B, cudaStream_t st)
     if ((rc = gemm_nt(EPI_NONE, h->h2b, h->L[3].wb, a, st))) return rc;
     a = args(B, h->n_out_p, 256, h->err);
     a.bias = h->L[4].b;
+    if (out) {
+        a.c32 = out;
+        a.ld32 = ld_out;
+        a.n_out = h->n_out;
+        a.scale2 = (h->flags & GD_MLP_SCALE_OUTPUT) ? h->scale : nullptr;
+        a.out_gain = h->out_gain;
+        return gemm_nt(EPI_NODE, h->zb, h->L[4].wb, a, st);
+    }
     a.c32 = h->y;
     a.ld32 = h->n_out_p;
     return gemm_nt(EPI_NONE, h->zb, h->L[4].wb, a, st);
@@ -1159,13 +1244,8 @@ extern "C" int gd_mlp_forward(gd_mlp *h, const float *x, int ldx, int batch, flo
     gd::DeviceGuard ds(h->device);
     cudaStream_t st = (cudaStream_t)stream;
     int rc = load_input(h, x, ldx, batch, st);
-    if (!rc) rc = forward(h, batch, st);
-    if (rc) return rc;
-    dim3 blk(32, 8), grd((batch + 31) / 32, h->n_out_p / 32);
-    scatter_out_kernel<<<grd, blk, 0, st>>>(h->y, h->n_out_p, h->n_out, batch, h->scale,
-                                            (h->flags & GD_MLP_SCALE_OUTPUT) ? 1 : 0, h->out_gain, y, ldy);
-    GD_CUDA(cudaGetLastError());
-    return GD_OK;
+    if (!rc) rc = forward(h, batch, y, ldy, st);
+    return rc;
 }
 
 extern "C" int gd_mlp_train_step(gd_mlp *h, const float *x, int ldx, const float *t, int ldt, const float *tden,
@@ -1178,7 +1258,7 @@ extern "C" int gd_mlp_train_step(gd_mlp *h, const float *x, int ldx, const float
     gd::DeviceGuard ds(h->device);
     cudaStream_t st = (cudaStream_t)stream;
     int rc = load_input(h, x, ldx, batch, st);
-    if (!rc) rc = forward(h, batch, st);
+    if (!rc) rc = forward(h, batch, nullptr, 0, st);
     if (!rc) rc = loss_grad(h, t, ldt, tden, ldd, batch, st);
     if (rc) return rc;
     if (loss) {
@@ -1212,7 +1292,7 @@ extern "C" int gd_mlp_loss(gd_mlp *h, const float *x, int ldx, const float *t, i
     gd::DeviceGuard ds(h->device);
     cudaStream_t st = (cudaStream_t)stream;
     int rc = load_input(h, x, ldx, batch, st);
-    if (!rc) rc = forward(h, batch, st);
+    if (!rc) rc = forward(h, batch, nullptr, 0, st);
     if (!rc) rc = loss_grad(h, t, ldt, tden, ldd, batch, st);
     if (rc) return rc;
     GD_CUDA(cudaMemcpyAsync(row_loss, h->row_err, (size_t)batch * sizeof(float), cudaMemcpyDeviceToDevice, st));
