@@ -51,7 +51,8 @@ struct GemmArgs {
     float *pre_out;     // EPI_GELU: pre-activation out [M][ld32], or null
     float *c32;         // [M][ld32] or null
     bf16 *c16;          // [M][ld16] or null
-    int ld32, ld16;
+    bf16 *c16t;         // the transpose, [N][ldt], or null
+    int ld32, ld16, ldt;
     // EPI_NODE: c32 is [column][ld32], each row's values times its scale (the
     // network's output in the library's layout): columns < n_out, times
     // out_gain and, when scale2 is set, scale2[row]^2
@@ -70,6 +71,14 @@ __device__ __forceinline__ float gelu_grad(float x)
 {
     return 0.5f * (1.f + erff(x * 0.70710678118654752f)) + x * 0.39894228040143268f * expf(-0.5f * x * x);
 }
+
+// The products of one launch: G of one K, their tiles one after another.
+template <int G>
+struct GemmSet {
+    CUtensorMap a[G], b[G];
+    GemmArgs g[G];
+    int end[G];  // of each product's tiles
+};
 
 // extra: the row's value of p.add (or of p.aux)
 template <int EPI>
@@ -94,10 +103,11 @@ __device__ __forceinline__ void epilogue_value(const GemmArgs &p, size_t o32, fl
 // that its lanes hold 32 columns of a row and every access of C and of the added or
 // multiplied arrays is one segment (a row per lane before: 32 segments of 16 bytes);
 // the added or multiplied values are requested before the accumulator is awaited.
-template <int EPI, int GN>
-__global__ void __launch_bounds__(kGThreads, 1)
-    gemm_nt_kernel(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUtensorMap tB, GemmArgs p)
+template <int EPI, int GN, int G>
+__global__ void __launch_bounds__(kGThreads, 1) gemm_nt_kernel(const __grid_constant__ GemmSet<G> set)
 {
+    // K, the stages, err and the test hook are the first product's
+    const GemmArgs p = set.g[0];
     constexpr uint32_t kStageBytes = gemm_stage(GN), kIdesc = umma_idesc_bf16(GM, GN);
     extern __shared__ __align__(1024) unsigned char dsmem[];
     unsigned char *epi = reinterpret_cast<unsigned char *>(
@@ -108,7 +118,18 @@ __global__ void __launch_bounds__(kGThreads, 1)
     __shared__ int abort_flag;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int num_k = p.K / GK, GS = p.stages, KPS = p.kps;
-    const int mt = (p.M + GM - 1) / GM, tiles = mt * ((p.N + GN - 1) / GN);
+    const int tiles = set.end[G - 1];
+    // product, first row and first column of a tile
+    auto locate = [&](int t, int *g, int *m0, int *n0) {
+        *g = 0;
+        if (G > 1) {
+            while (t >= set.end[*g]) (*g)++;
+            if (*g > 0) t -= set.end[*g - 1];
+        }
+        const int mt = (set.g[*g].M + GM - 1) / GM;
+        *m0 = t % mt * GM;
+        *n0 = t / mt * GN;
+    };
 
     if (threadIdx.x == 0) abort_flag = *(volatile int *)p.err;
     __syncthreads();
@@ -154,7 +175,8 @@ __global__ void __launch_bounds__(kGThreads, 1)
             int s = 0;
             uint32_t ph = 0;
             for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
-                const int m0 = t % mt * GM, n0 = t / mt * GN;
+                int g, m0, n0;
+                locate(t, &g, &m0, &n0);
                 for (int k = 0; k < num_k; k += KPS) {
                     if (!mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1u, p.err)) {
                         ok = false;
@@ -165,8 +187,8 @@ __global__ void __launch_bounds__(kGThreads, 1)
                     const int kn = min(KPS, num_k - k);
                     mbar_expect_tx(fb, (uint32_t)kn * kStageBytes);
                     for (int q = 0; q < kn; q++, st += kStageBytes) {
-                        tma_load_2d(st, &tA, (k + q) * GK, m0, fb);
-                        tma_load_2d(st + kA, &tB, (k + q) * GK, n0, fb);
+                        tma_load_2d(st, &set.a[g], (k + q) * GK, m0, fb);
+                        tma_load_2d(st + kA, &set.b[g], (k + q) * GK, n0, fb);
                     }
                     if (++s == GS) {
                         s = 0;
@@ -212,19 +234,24 @@ __global__ void __launch_bounds__(kGThreads, 1)
     } else {
         const int quad = warp & 3;
         float *tile = reinterpret_cast<float *>(epi + quad * kEpiTile);
-        const float *ex = EPI == EPI_DGELU ? p.aux : p.add;
         int i = 0;
         for (int t = blockIdx.x; t < tiles; t += gridDim.x, i++) {
-            const int mw = t % mt * GM + quad * 32, m = mw + lane;  // the warp's first row, the lane's
-            const int n0 = t / mt * GN, rows = min(32, p.M - mw);
+            int g, m0, n0;
+            locate(t, &g, &m0, &n0);
+            const GemmArgs p = set.g[g];  // a copy: stores to C cannot change it
+            const float *ex = EPI == EPI_DGELU ? p.aux : p.add;
+            const int mw = m0 + quad * 32, m = mw + lane, rows = min(32, p.M - mw);  // the warp's first row, the lane's
             float s = 0.f;
             if (EPI == EPI_NODE && m < p.M)
                 s = (p.scale2 ? __ldg(p.scale2 + m) * __ldg(p.scale2 + m) : 1.f) * p.out_gain;
             float extra[32];
             auto load_extra = [&](int n) {
-                if (EPI == EPI_NODE || EPI == EPI_GELU || !ex) return;
+                if constexpr (EPI == EPI_NONE || EPI == EPI_DGELU) {
+                    if (!ex) return;
 #pragma unroll
-                for (int r = 0; r < 32; r++) extra[r] = r < rows && n < p.N ? ex[(size_t)(mw + r) * p.ld32 + n] : 0.f;
+                    for (int r = 0; r < 32; r++)
+                        extra[r] = r < rows && n < p.N ? ex[(size_t)(mw + r) * p.ld32 + n] : 0.f;
+                }
             };
             load_extra(n0 + lane);
             const int buf = i & 1;
@@ -266,9 +293,17 @@ __global__ void __launch_bounds__(kGThreads, 1)
                             epilogue_value<EPI>(p, (size_t)(mw + r) * p.ld32 + n, bias, extra[r], x);
                             if (p.c32) p.c32[(size_t)(mw + r) * p.ld32 + n] = x;
                             if (p.c16) p.c16[(size_t)(mw + r) * p.ld16 + n] = __float2bfloat16_rn(x);
+                            if (p.c16t) tile[r * 33 + lane] = x;
                         }
                     }
                     __syncwarp();
+                    if (p.c16t) {
+#pragma unroll
+                        for (int j = 0; j < 32; j++)
+                            if (n0 + c0 + j < p.N && m < p.M)
+                                p.c16t[(size_t)(n0 + c0 + j) * p.ldt + m] = __float2bfloat16_rn(tile[lane * 33 + j]);
+                        __syncwarp();
+                    }
                 }
             }
         }
@@ -487,7 +522,7 @@ __global__ void to_bf16_kernel(const float *__restrict__ in, int R, int Cc, int 
 // cycles each); a thread per column that loads as it adds waits for memory
 // instead (3648 rows: 240 -> 17 us; 1024 rows: 60 -> 6.5 us).  Four-byte copies
 // alone: 22 and 8.4 us.
-constexpr int kOrdPer = 4, kOrdRows = 32 * kOrdPer, kOrdStages = 8;  // rows per thread and per stage
+constexpr int kOrdPer = 4, kOrdRows = 32 * kOrdPer, kOrdStages = 6;  // rows per thread and per stage
 constexpr size_t kOrdSmem = (size_t)kOrdStages * kOrdRows * 32 * sizeof(float);
 template <bool SQUARE>
 __device__ __forceinline__ float ordered_sum(const float *__restrict__ src, int rows, size_t ld, int col, bool live)
@@ -568,32 +603,39 @@ __device__ __forceinline__ float ordered_sum(const float *__restrict__ src, int 
 }
 
 template <typename... P, typename... A>
-int launch_ordered(void (*kern)(P...), int cols, cudaStream_t st, A... a)
+int launch_ordered(void (*kern)(P...), dim3 grid, cudaStream_t st, A... a)
 {
     GD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOrdSmem));
-    kern<<<(cols + 31) / 32, dim3(32, 32), kOrdSmem, st>>>(a...);
+    kern<<<grid, dim3(32, 32), kOrdSmem, st>>>(a...);
     GD_CUDA(cudaGetLastError());
     return GD_OK;
 }
 
-// Per-cell scale: mean of x over the n nodes (fixed order), or 1.  Block = 32
-// cells x 32 warps.
-__global__ void __launch_bounds__(1024) cell_scale_kernel(const float *__restrict__ x, int n, int ld, int B,
-                                                          int use_mean, float *__restrict__ scale)
+// Per-cell scale: mean of x over the n nodes (fixed order), or 1; in the blocks of
+// a second row, the sum of squares of d over m nodes.  Block = 32 cells x 32 warps.
+__global__ void __launch_bounds__(1024) cell_sums_kernel(const float *__restrict__ x, int n, int ldx, int use_mean,
+                                                         float *__restrict__ scale, const float *__restrict__ d, int m,
+                                                         int ldd, float *__restrict__ squares, int B)
 {
     const int r = blockIdx.x * 32 + threadIdx.x;
     const bool live = r < B;
-    const float s = use_mean ? ordered_sum<false>(x, n, ld, r, live) / (float)n : 1.f;
-    if (live && threadIdx.y == 0) scale[r] = s;
+    if (blockIdx.y == 0) {
+        const float s = use_mean ? ordered_sum<false>(x, n, ldx, r, live) / (float)n : 1.f;
+        if (live && threadIdx.y == 0) scale[r] = s;
+    } else {
+        const float s = ordered_sum<true>(d, m, ldd, r, live);
+        if (live && threadIdx.y == 0) squares[r] = s;
+    }
 }
 
 __device__ __forceinline__ float inv_or_zero(float s) { return s != 0.f ? 1.f / s : 0.f; }
 
 // node-major FP32 x[i][r] (ld) -> cell-major BF16 xb[r][i] * gain / scale[r] (pad to
-// n_p).  Block = 64 nodes x 32 cells: eight loads in flight per thread and whole
+// n_p), for training also its transpose xt[i][r].  Block = 64 nodes x 32 cells: eight loads in flight per thread and whole
 // 128-byte rows on both sides (4096 cells, 3648 nodes: 39 -> 15 us).
+template <bool TRANSPOSE>
 __global__ void gather_in_kernel(const float *__restrict__ x, int n, int ld, int B, const float *__restrict__ scale,
-                                 float gain, bf16 *__restrict__ xb, int n_p)
+                                 float gain, bf16 *__restrict__ xb, bf16 *__restrict__ xt, int n_p)
 {
     __shared__ float tile[64][33];
     const int i0 = blockIdx.y * 64, r0 = blockIdx.x * 32, r = r0 + threadIdx.x;
@@ -605,7 +647,11 @@ __global__ void gather_in_kernel(const float *__restrict__ x, int n, int ld, int
         v[k] = i < n && r < B ? __ldg(x + (size_t)i * ld + r) : 0.f;
     }
 #pragma unroll
-    for (int k = 0; k < 8; k++) tile[threadIdx.y + 8 * k][threadIdx.x] = v[k] * s;
+    for (int k = 0; k < 8; k++) {
+        v[k] *= s;
+        tile[threadIdx.y + 8 * k][threadIdx.x] = v[k];
+        if (TRANSPOSE && r < B) xt[(size_t)(i0 + threadIdx.y + 8 * k) * B + r] = __float2bfloat16_rn(v[k]);
+    }
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < 4; k++) {
@@ -616,47 +662,21 @@ __global__ void gather_in_kernel(const float *__restrict__ x, int n, int ld, int
     }
 }
 
-// node-major FP32 t[i][r] -> cell-major FP32 tt[r][i] * inv_gain / scale[r]^2 (the
-// scale only when pw; pad to n_p)
-__global__ void gather_target_kernel(const float *__restrict__ t, int n, int ld, int B, const float *__restrict__ scale,
-                                     int pw, float inv_gain, float *__restrict__ tt, int n_p)
-{
-    __shared__ float tile[32][33];
-    const int i0 = blockIdx.y * 32, r0 = blockIdx.x * 32;
-    for (int y = threadIdx.y; y < 32; y += blockDim.y) {
-        const int i = i0 + y, r = r0 + threadIdx.x;
-        tile[y][threadIdx.x] = (i < n && r < B) ? t[(size_t)i * ld + r] : 0.f;
-    }
-    __syncthreads();
-    for (int y = threadIdx.y; y < 32; y += blockDim.y) {
-        const int r = r0 + y, i = i0 + threadIdx.x;
-        if (r < B && i < n_p) {
-            const float s = (pw ? inv_or_zero(scale[r] * scale[r]) : 1.f) * inv_gain;
-            tt[(size_t)r * n_p + i] = tile[threadIdx.x][y] * s;
-        }
-    }
-}
-
-// Loss denominators per cell: sum_i d[i][r]^2 (scaled like the targets) for the
-// relative losses, or n for the mean squared error.  Block = 32 cells x 32 warps.
-__global__ void __launch_bounds__(1024) row_den_kernel(const float *__restrict__ d, int n, int ld, int B,
-                                                       const float *__restrict__ scale, int pw, float inv_gain, int mse,
-                                                       float *__restrict__ den)
-{
-    const int r = blockIdx.x * 32 + threadIdx.x;
-    const bool live = r < B;
-    const float s = mse ? 0.f : ordered_sum<true>(d, n, ld, r, live);
-    if (!live || threadIdx.y != 0) return;
-    const float sc = (pw ? inv_or_zero(scale[r] * scale[r]) : 1.f) * inv_gain;
-    den[r] = mse ? (float)n : s * sc * sc;
-}
-
-// den[r] <- mean over the batch of den (fixed order), for the batch-relative loss
-__global__ void batch_mean_den_kernel(float *__restrict__ den, int B)
+// Loss denominators per cell from the sums of squares in den: scaled like the
+// targets for the relative losses, or n for the mean squared error; with mean set
+// their mean over the batch (fixed order).  One block.
+__global__ void den_kernel(float *__restrict__ den, int B, const float *__restrict__ scale, int pw, float inv_gain,
+                           int mse, int n, int mean)
 {
     __shared__ double s[256];
     double a = 0.0;
-    for (int i = threadIdx.x; i < B; i += blockDim.x) a += den[i];
+    for (int i = threadIdx.x; i < B; i += blockDim.x) {
+        const float sc = (pw ? inv_or_zero(scale[i] * scale[i]) : 1.f) * inv_gain;
+        const float v = mse ? (float)n : den[i] * sc * sc;
+        den[i] = v;
+        a += v;
+    }
+    if (!mean) return;
     s[threadIdx.x] = a;
     __syncthreads();
     for (int k = blockDim.x / 2; k > 0; k >>= 1) {
@@ -668,73 +688,155 @@ __global__ void batch_mean_den_kernel(float *__restrict__ den, int B)
     for (int i = threadIdx.x; i < B; i += blockDim.x) den[i] = m;
 }
 
-// column sums out[n] = sum_r d[r][n], r < R (fixed order).  Block = 32 columns x 32 warps.
-__global__ void __launch_bounds__(1024) colsum_kernel(const float *__restrict__ d, int R, int N, int ld,
-                                                      float *__restrict__ out)
+// The layers' bias gradients: column sums gb[n] = sum_r d[r][n], r < R (fixed
+// order).  Block = 32 columns x 32 warps, layer by layer.
+struct ColSums {
+    const float *d[5];
+    float *out[5];
+    int n[5], end[5];  // columns; end of the layer's blocks
+};
+__global__ void __launch_bounds__(1024) colsum_kernel(const __grid_constant__ ColSums c, int R)
 {
-    const int n = blockIdx.x * 32 + threadIdx.x;
-    const bool live = n < N;
-    const float s = ordered_sum<false>(d, R, ld, n, live);
-    if (live && threadIdx.y == 0) out[n] = s;
+    int g = 0;
+    while ((int)blockIdx.x >= c.end[g]) g++;
+    const int n = ((int)blockIdx.x - (g > 0 ? c.end[g - 1] : 0)) * 32 + threadIdx.x;
+    const bool live = n < c.n[g];
+    const float s = ordered_sum<false>(c.d[g], R, c.n[g], n, live);
+    if (live && threadIdx.y == 0) c.out[g][n] = s;
 }
 
-// e_r = sum_n (y - t)^2 / den_r; dy = 2 (y - t) / den_r / B.  One block per row.
-__global__ void loss_grad_kernel(const float *__restrict__ y, const float *__restrict__ t, int ld, int N, int B,
+// Output gradient dy = 2 (y - t') / den / B with t'[r][i] = t[i][r] inv_gain /
+// scale[r]^2 (the scale only when pw): FP32 dy and BF16 dyb [r][n_p], its transpose
+// dyt [n_p][B] when set, and per 64 nodes the sum of (y - t')^2 in
+// err_part[node tile][r].  Block = 64 nodes x 32 cells.
+__global__ void loss_grad_kernel(const float *__restrict__ y, const float *__restrict__ t, int ldt, int n, int n_p,
+                                 int B, const float *__restrict__ scale, int pw, float inv_gain,
                                  const float *__restrict__ den, float *__restrict__ dy, bf16 *__restrict__ dyb,
-                                 float *__restrict__ row_err)
+                                 bf16 *__restrict__ dyt, float *__restrict__ err_part)
 {
-    __shared__ float s_e[256];
-    const int r = blockIdx.x;
-    const float dr = fmaxf(den[r], 1e-30f);
-    float e = 0.f;
-    for (int n = threadIdx.x; n < ld; n += blockDim.x) {
-        float g = 0.f;
-        if (n < N) {
-            const float d = y[(size_t)r * ld + n] - t[(size_t)r * ld + n];
-            e += d * d;
-            g = 2.f * d / dr / (float)B;
+    __shared__ float tile[64][33];
+    const int i0 = blockIdx.y * 64, r0 = blockIdx.x * 32, tx = threadIdx.x, ty = threadIdx.y;
+    {
+        const int r = r0 + tx;
+        const float s = r < B ? (pw ? inv_or_zero(scale[r] * scale[r]) : 1.f) * inv_gain : 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const int i = i0 + ty + 8 * k;
+            tile[ty + 8 * k][tx] = i < n && r < B ? __ldg(t + (size_t)i * ldt + r) * s : 0.f;
         }
-        dy[(size_t)r * ld + n] = g;
-        dyb[(size_t)r * ld + n] = __float2bfloat16_rn(g);
     }
-    s_e[threadIdx.x] = e;
     __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) s_e[threadIdx.x] += s_e[threadIdx.x + s];
-        __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int yy = ty + 8 * k, r = r0 + yy, i = i0 + 2 * tx;
+        if (r >= B) continue;  // the whole warp
+        const float dr = fmaxf(den[r], 1e-30f);
+        const float2 v = *reinterpret_cast<const float2 *>(y + (size_t)r * n_p + i);
+        float2 g = make_float2(0.f, 0.f);
+        float e = 0.f;
+        if (i < n) {
+            const float d = v.x - tile[2 * tx][yy];
+            e += d * d;
+            g.x = 2.f * d / dr / (float)B;
+        }
+        if (i + 1 < n) {
+            const float d = v.y - tile[2 * tx + 1][yy];
+            e += d * d;
+            g.y = 2.f * d / dr / (float)B;
+        }
+        *reinterpret_cast<float2 *>(dy + (size_t)r * n_p + i) = g;
+        *reinterpret_cast<__nv_bfloat162 *>(dyb + (size_t)r * n_p + i) = __floats2bfloat162_rn(g.x, g.y);
+        tile[2 * tx][yy] = g.x;
+        tile[2 * tx + 1][yy] = g.y;
+        for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+        if (tx == 0) err_part[(size_t)blockIdx.y * B + r] = e;
     }
-    if (threadIdx.x == 0) row_err[r] = s_e[0] / dr;
+    if (!dyt) return;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+        if (r0 + tx < B) dyt[(size_t)(i0 + ty + 8 * k) * B + r0 + tx] = __float2bfloat16_rn(tile[ty + 8 * k][tx]);
 }
 
-__global__ void mean_kernel(const float *__restrict__ v, int n, float *__restrict__ out)
+// row_err[r] = sum of the node tiles' errors / den[r]; with out set also their
+// mean over the batch (fixed order, one block).
+__global__ void __launch_bounds__(1024) row_err_kernel(const float *__restrict__ err_part, int tiles, int B, const float *__restrict__ den,
+                               float *__restrict__ row_err, float *__restrict__ out)
 {
-    __shared__ double s[256];
+    __shared__ double s[1024];
     double a = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) a += v[i];
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < B; r += gridDim.x * blockDim.x) {
+        float e = 0.f;
+#pragma unroll 8
+        for (int k = 0; k < tiles; k++) e += __ldg(err_part + (size_t)k * B + r);
+        e /= fmaxf(den[r], 1e-30f);
+        row_err[r] = e;
+        a += e;
+    }
+    if (!out) return;
     s[threadIdx.x] = a;
     __syncthreads();
     for (int k = blockDim.x / 2; k > 0; k >>= 1) {
         if (threadIdx.x < k) s[threadIdx.x] += s[threadIdx.x + k];
         __syncthreads();
     }
-    if (threadIdx.x == 0) *out = (float)(s[0] / n);
+    if (threadIdx.x == 0) *out = (float)(s[0] / B);
 }
 
-// Adam (decoupled weight decay) on an FP32 master tensor; writes the BF16 copy.
-__global__ void adam_kernel(float *__restrict__ w, const float *__restrict__ g, float *__restrict__ m,
-                            float *__restrict__ v, bf16 *__restrict__ wb, int64_t n, float lr, float b1, float b2,
-                            float c1, float c2, float eps, float wd)
+// Adam (decoupled weight decay) on the FP32 masters of all layers; writes the BF16
+// copies and their transposes (bound by its bytes, 32 per weight, from L2: one
+// launch instead of fourteen, 55 -> 20 us).  Block = 32 x 32 of a weight matrix, or
+// 1024 of a bias; threads 32 x 8.
+struct AdamSet {
+    struct {
+        float *w, *b, *mw, *vw, *mb, *vb;
+        const float *gw, *gb;
+        bf16 *wb, *wt;
+        int out, in, wend, bend;  // ends of the weight's and of the bias's blocks
+    } l[5];
+    float lr, b1, b2, c1, c2, eps, wd;
+};
+__device__ __forceinline__ float adam(const AdamSet &a, float *w, const float *g, float *m, float *v, size_t i, float wd)
 {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const float gi = g[i];
-        const float mi = b1 * m[i] + (1.f - b1) * gi;
-        const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        const float upd = (mi / c1) / (sqrtf(vi / c2) + eps) + wd * w[i];
-        const float wn = w[i] - lr * upd;
-        w[i] = wn;
-        if (wb) wb[i] = __float2bfloat16_rn(wn);
+    const float gi = g[i];
+    const float mi = __fmaf_rn(1.f - a.b1, gi, __fmul_rn(a.b1, m[i]));
+    const float vi = __fmaf_rn(__fmul_rn(1.f - a.b2, gi), gi, __fmul_rn(a.b2, v[i]));
+    m[i] = mi;
+    v[i] = vi;
+    const float upd = __fmaf_rn(wd, w[i], (mi / a.c1) / (sqrtf(vi / a.c2) + a.eps));
+    const float wn = __fmaf_rn(-a.lr, upd, w[i]);
+    w[i] = wn;
+    return wn;
+}
+__global__ void adam_kernel(const __grid_constant__ AdamSet a)
+{
+    __shared__ float tile[32][33];
+    int k = 0;
+    while ((int)blockIdx.x >= a.l[k].bend) k++;
+    const auto &l = a.l[k];
+    const int blk = (int)blockIdx.x - (k > 0 ? a.l[k - 1].bend : 0), nw = l.wend - (k > 0 ? a.l[k - 1].bend : 0);
+    if (blk >= nw) {
+        const int i0 = (blk - nw) * 1024;
+        for (int i = i0 + threadIdx.y * 32 + threadIdx.x; i < min(i0 + 1024, l.out); i += 256)
+            adam(a, l.b, l.gb, l.mb, l.vb, i, 0.f);
+        return;
+    }
+    // out and in are multiples of 32
+    const int cols = l.in / 32, o0 = blk / cols * 32, i0 = blk % cols * 32;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const int y = threadIdx.y + 8 * q;
+        const size_t i = (size_t)(o0 + y) * l.in + i0 + threadIdx.x;
+        const float wn = adam(a, l.w, l.gw, l.mw, l.vw, i, a.wd);
+        l.wb[i] = __float2bfloat16_rn(wn);
+        tile[y][threadIdx.x] = wn;
+    }
+    if (!l.wt) return;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const int y = threadIdx.y + 8 * q;
+        l.wt[(size_t)(i0 + y) * l.out + o0 + threadIdx.x] = __float2bfloat16_rn(tile[threadIdx.x][y]);
     }
 }
 
@@ -771,53 +873,81 @@ int make_map(CUtensorMap *m, const bf16 *ptr, int rows, int K, int box_rows)
     return GD_OK;
 }
 
-// C = A B^T with A [M][K], B [N][K] (BF16, row stride K), K % 64 == 0;
-// output strides ld32, ld16 multiples of 4.
-int gemm_nt(int epi, const bf16 *A, const bf16 *B, const GemmArgs &a, cudaStream_t st)
+// One of the products of a launch.
+struct Product {
+    const bf16 *A, *B;
+    GemmArgs a;
+};
+
+template <int EPI, int GN, int G>
+int launch_gemm(const Product *pr, int kps, int stages, int ctas, cudaStream_t st)
 {
-    if (a.K % GK || a.K <= 0 || a.M <= 0 || a.N <= 0 || (epi != EPI_NODE && ((a.ld32 & 3) || (a.ld16 & 3))))
-        return set_error(GD_ERR_INVALID_ARG, "GEMM shape: K a multiple of 64, strides multiples of 4");
+    GemmSet<G> set;
+    int end = 0;
+    for (int g = 0; g < G; g++) {
+        int rc = make_map(&set.a[g], pr[g].A, pr[g].a.M, pr[g].a.K, GM);
+        if (!rc) rc = make_map(&set.b[g], pr[g].B, pr[g].a.N, pr[g].a.K, GN);
+        if (rc) return rc;
+        set.g[g] = pr[g].a;
+        set.g[g].kps = kps;
+        set.g[g].stages = stages;
+        set.end[g] = end += (pr[g].a.M + GM - 1) / GM * ((pr[g].a.N + GN - 1) / GN);
+    }
+    const size_t smem = gemm_smem(GN, stages * kps);
+    GD_CUDA(cudaFuncSetAttribute(gemm_nt_kernel<EPI, GN, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    gemm_nt_kernel<EPI, GN, G><<<std::min(end, ctas), kGThreads, smem, st>>>(set);
+    GD_CUDA(cudaGetLastError());
+    return GD_OK;
+}
+
+// C = A B^T with A [M][K], B [N][K] (BF16, row stride K), K % 64 == 0, for G
+// products of one K in one launch; output strides ld32, ld16 multiples of 4.
+//
+// Tile width, K steps per stage and stages.  A K of up to 8 steps (every layer
+// but the first and the weights' gradients): 32 columns and two CTAs per SM,
+// since a CTA's fixed costs and its epilogue bound it (1024 x 512, K = 512: 10 us;
+// 13 with 64 columns, 20 with 128, 34 with 256; 4096 x 3648, K = 256: 26 us, 36
+// with 64, 33 with 128).  A longer K is bound by the handshakes and copies of its
+// stages: four steps in each, in the narrowest tiles that one wave holds (1024 x
+// 256, K = 3648: 17 us with 32 columns, 18 with 64, 27 with 128, one step per
+// stage 24; 4096 x 256: 22 us with 64 columns, 32 with 32).
+template <int G>
+int gemm_nt(int epi, const Product *pr, cudaStream_t st)
+{
     int dev = 0, sms = 0;
     GD_CUDA(cudaGetDevice(&dev));
     GD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    // Tile width, K steps per stage and stages.  A K of up to 8 steps (every layer
-    // but the first and the weights' gradients): 32 columns and two CTAs per SM,
-    // since a CTA's fixed costs and its epilogue bound it (1024 x 512, K = 512: 10 us;
-    // 13 with 64 columns, 20 with 128, 34 with 256; 4096 x 3648, K = 256: 26 us, 36
-    // with 64, 33 with 128).  A longer K is bound by the handshakes and copies of its
-    // stages: four steps in each, in the narrowest tiles that one wave holds (1024 x
-    // 256, K = 3648: 17 us with 32 columns, 18 with 64, 27 with 128, one step per
-    // stage 24; 4096 x 256: 22 us with 64 columns, 32 with 32).
-    const int mt = (a.M + GM - 1) / GM, num_k = a.K / GK;
-    const bool longk = num_k > 8;
-    int gn = 32;
-    while (longk && gn < 256 && mt * ((a.N + gn - 1) / gn) > sms) gn *= 2;
-    CUtensorMap tA, tB;
-    int rc = make_map(&tA, A, a.M, a.K, GM);
-    if (!rc) rc = make_map(&tB, B, a.N, a.K, gn);
-    if (rc) return rc;
-    GemmArgs b = a;
-    b.kps = longk ? 4 : 2;
-    b.stages = longk ? std::min((num_k + b.kps - 1) / b.kps, (int)((200u << 10) / (b.kps * gemm_stage(gn)))) : 2;
-    if (b.stages < 2) {  // 256 columns
-        b.kps = 2;
-        b.stages = 2;
+    const int K = pr[0].a.K;
+    for (int g = 0; g < G; g++) {
+        const GemmArgs &a = pr[g].a;
+        if (a.K != K || K % GK || K <= 0 || a.M <= 0 || a.N <= 0 || (epi != EPI_NODE && ((a.ld32 & 3) || (a.ld16 & 3))))
+            return set_error(GD_ERR_INVALID_ARG, "GEMM shape: K a multiple of 64, strides multiples of 4");
     }
-    const size_t smem = gemm_smem(gn, b.stages * b.kps);
-    const int grid = std::min(mt * ((a.N + gn - 1) / gn), sms * (longk ? 1 : 2));
-    using Kernel = void (*)(const CUtensorMap, const CUtensorMap, GemmArgs);
-    Kernel kern = nullptr;
-    if (longk && epi == EPI_NONE)
-        kern = gn == 32 ? gemm_nt_kernel<EPI_NONE, 32> : gn == 64 ? gemm_nt_kernel<EPI_NONE, 64>
-             : gn == 128 ? gemm_nt_kernel<EPI_NONE, 128> : gemm_nt_kernel<EPI_NONE, 256>;
-    else if (!longk)
-        kern = epi == EPI_NONE ? gemm_nt_kernel<EPI_NONE, 32> : epi == EPI_GELU ? gemm_nt_kernel<EPI_GELU, 32>
-             : epi == EPI_DGELU ? gemm_nt_kernel<EPI_DGELU, 32> : epi == EPI_NODE ? gemm_nt_kernel<EPI_NODE, 32> : nullptr;
-    if (!kern) return set_error(GD_ERR_INVALID_ARG, "unknown GEMM epilogue for this K");
-    GD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<grid, kGThreads, smem, st>>>(tA, tB, b);
-    GD_CUDA(cudaGetLastError());
-    return GD_OK;
+    const int num_k = K / GK;
+    auto tiles = [&](int gn) {
+        int n = 0;
+        for (int g = 0; g < G; g++) n += (pr[g].a.M + GM - 1) / GM * ((pr[g].a.N + gn - 1) / gn);
+        return n;
+    };
+    if (num_k <= 8) {
+        if (epi == EPI_NONE) return launch_gemm<EPI_NONE, 32, G>(pr, 2, 2, 2 * sms, st);
+        if (G == 1 && epi == EPI_GELU) return launch_gemm<EPI_GELU, 32, 1>(pr, 2, 2, 2 * sms, st);
+        if (G == 1 && epi == EPI_DGELU) return launch_gemm<EPI_DGELU, 32, 1>(pr, 2, 2, 2 * sms, st);
+        if (G == 1 && epi == EPI_NODE) return launch_gemm<EPI_NODE, 32, 1>(pr, 2, 2, 2 * sms, st);
+    } else if (epi == EPI_NONE) {
+        const int steps = (num_k + 3) / 4;  // stages of four
+        if (tiles(32) <= sms) return launch_gemm<EPI_NONE, 32, G>(pr, 4, std::min(steps, 2), sms, st);
+        if (tiles(64) <= sms) return launch_gemm<EPI_NONE, 64, G>(pr, 4, std::min(steps, 2), sms, st);
+        if (tiles(128) <= sms) return launch_gemm<EPI_NONE, 128, G>(pr, 2, 3, sms, st);
+        return launch_gemm<EPI_NONE, 256, G>(pr, 2, 2, sms, st);
+    }
+    return set_error(GD_ERR_INVALID_ARG, "unknown GEMM epilogue for this K");
+}
+
+int gemm_nt(int epi, const bf16 *A, const bf16 *B, const GemmArgs &a, cudaStream_t st)
+{
+    const Product p{A, B, a};
+    return gemm_nt<1>(epi, &p, st);
 }
 
 int transpose(const bf16 *in, int R, int Cc, int ldi, bf16 *out, int ldo, cudaStream_t st)
@@ -875,11 +1005,13 @@ struct gd_mlp {
     int stall_next = 0;  // gd_mlp_inject_timeout: polls for the next forward's first GEMM
     // activations, [cap][features]
     bf16 *xb = nullptr, *h0b = nullptr, *h1b = nullptr, *h2b = nullptr, *zb = nullptr;
-    float *h0 = nullptr, *a1 = nullptr, *a2 = nullptr, *y = nullptr, *tt = nullptr;
+    float *h0 = nullptr, *a1 = nullptr, *a2 = nullptr, *y = nullptr;
     float *dy = nullptr, *dz = nullptr, *da2 = nullptr, *da1 = nullptr, *dh0 = nullptr;
-    bf16 *dyb = nullptr, *dzb = nullptr, *da2b = nullptr, *da1b = nullptr, *dh0b = nullptr;
-    bf16 *tmp1 = nullptr, *tmp2 = nullptr;  // transposes [features][cap]
-    float *scale = nullptr, *den = nullptr, *row_err = nullptr;
+    bf16 *dyb = nullptr, *dzb = nullptr, *da2b = nullptr, *da1b = nullptr;
+    // transposes [features][batch]: the operands of the weights' gradients
+    bf16 *xt = nullptr, *h0t = nullptr, *h1t = nullptr, *h2t = nullptr, *zt = nullptr;
+    bf16 *dyt = nullptr, *dzt = nullptr, *da2t = nullptr, *da1t = nullptr, *dh0t = nullptr;
+    float *scale = nullptr, *den = nullptr, *row_err = nullptr, *err_part = nullptr;
     int *err = nullptr;
     std::vector<void *> allocs;
 };
@@ -933,24 +1065,32 @@ gd::GemmArgs args(int M, int N, int K, int *err)
     return a;
 }
 
-// network input: per-cell scales and the BF16 cell-major copy of x
-int load_input(gd_mlp *h, const float *x, int ldx, int B, cudaStream_t st)
+// network input: per-cell scales and the BF16 cell-major copy of x (with train its
+// transpose too), and the sums of squares of d [n_out][ldd] into h->den when set
+int load_input(gd_mlp *h, const float *x, int ldx, int B, bool train, const float *d, int ldd, cudaStream_t st)
 {
-    int rc = gd::launch_ordered(gd::cell_scale_kernel, B, st, x, h->n_in, ldx, B,
-                                (int)(h->flags & GD_MLP_SCALE_INPUT), h->scale);
+    if (h->flags & GD_MLP_LOSS_MSE) d = nullptr;
+    int rc = gd::launch_ordered(gd::cell_sums_kernel, dim3((B + 31) / 32, d ? 2 : 1), st, x, h->n_in, ldx,
+                                (int)(h->flags & GD_MLP_SCALE_INPUT), h->scale, d, h->n_out, ldd, h->den, B);
     if (rc) return rc;
     dim3 blk(32, 8), grd((B + 31) / 32, h->n_in_p / 64);
-    gd::gather_in_kernel<<<grd, blk, 0, st>>>(x, h->n_in, ldx, B, h->scale, h->in_gain, h->xb, h->n_in_p);
+    auto gather = train ? gd::gather_in_kernel<true> : gd::gather_in_kernel<false>;
+    gather<<<grd, blk, 0, st>>>(x, h->n_in, ldx, B, h->scale, h->in_gain, h->xb, h->xt, h->n_in_p);
     GD_CUDA(cudaGetLastError());
     return GD_OK;
 }
 
 // forward on rows [0, B) of h->xb; the output times its scales into out
-// [n_out][ld_out], or, when out is null, unscaled into h->y ([B][n_out_p])
-int forward(gd_mlp *h, int B, float *out, int ld_out, cudaStream_t st)
+// [n_out][ld_out], or, when out is null, unscaled into h->y ([B][n_out_p]); with
+// train also the layers' transposes
+int forward(gd_mlp *h, int B, float *out, int ld_out, bool train, cudaStream_t st)
 {
     using namespace gd;
     int rc;
+    auto transposed = [&](GemmArgs &a, bf16 *t) {
+        if (train) a.c16t = t;
+        a.ldt = B;
+    };
     GemmArgs a = args(B, 256, h->n_in_p, h->err);
     a.stall_polls = h->stall_next;  // a pending time-out injection fires here, once
     h->stall_next = 0;
@@ -959,6 +1099,7 @@ int forward(gd_mlp *h, int B, float *out, int ld_out, cudaStream_t st)
     a.ld32 = 256;
     a.c16 = h->h0b;
     a.ld16 = 256;
+    transposed(a, h->h0t);
     if ((rc = gemm_nt(EPI_NONE, h->xb, h->L[0].wb, a, st))) return rc;
     a = args(B, 512, 256, h->err);
     a.bias = h->L[1].b;
@@ -966,6 +1107,7 @@ int forward(gd_mlp *h, int B, float *out, int ld_out, cudaStream_t st)
     a.ld32 = 512;
     a.c16 = h->h1b;
     a.ld16 = 512;
+    transposed(a, h->h1t);
     if ((rc = gemm_nt(EPI_GELU, h->h0b, h->L[1].wb, a, st))) return rc;
     a = args(B, 512, 512, h->err);
     a.bias = h->L[2].b;
@@ -973,6 +1115,7 @@ int forward(gd_mlp *h, int B, float *out, int ld_out, cudaStream_t st)
     a.ld32 = 512;
     a.c16 = h->h2b;
     a.ld16 = 512;
+    transposed(a, h->h2t);
     if ((rc = gemm_nt(EPI_GELU, h->h1b, h->L[2].wb, a, st))) return rc;
     a = args(B, 256, 512, h->err);
     a.bias = h->L[3].b;
@@ -980,6 +1123,7 @@ int forward(gd_mlp *h, int B, float *out, int ld_out, cudaStream_t st)
     a.ld32 = 256;
     a.c16 = h->zb;
     a.ld16 = 256;
+    transposed(a, h->zt);
     if ((rc = gemm_nt(EPI_NONE, h->h2b, h->L[3].wb, a, st))) return rc;
     a = args(B, h->n_out_p, 256, h->err);
     a.bias = h->L[4].b;
@@ -1000,73 +1144,79 @@ int backward(gd_mlp *h, int B, cudaStream_t st)
 {
     using namespace gd;
     int rc;
-    auto grad_w = [&](int k, const bf16 *dY, int nout, const bf16 *X, int nin) -> int {
-        // dW[o][i] = sum_b dY[b][o] X[b][i]: A = dY^T [nout][B], B = X^T [nin][B]
-        int r = transpose(dY, B, nout, nout, h->tmp1, B, st);
-        if (!r) r = transpose(X, B, nin, nin, h->tmp2, B, st);
-        if (r) return r;
-        GemmArgs a = args(nout, nin, B, h->err);
-        a.c32 = h->L[k].gw;
-        a.ld32 = nin;
-        return gemm_nt(EPI_NONE, h->tmp1, h->tmp2, a, st);
-    };
-    auto grad_b = [&](int k, const float *dY, int n) -> int {
-        return launch_ordered(colsum_kernel, n, st, dY, B, n, n, h->L[k].gb);
+    auto transposed = [&](GemmArgs &a, bf16 *t) {
+        a.c16t = t;
+        a.ldt = B;
     };
     // y = W4 z + b4
-    if ((rc = grad_w(4, h->dyb, h->n_out_p, h->zb, 256)) || (rc = grad_b(4, h->dy, h->n_out_p))) return rc;
     GemmArgs a = args(B, 256, h->n_out_p, h->err);
     a.c32 = h->dz;
     a.ld32 = 256;
     a.c16 = h->dzb;
     a.ld16 = 256;
+    transposed(a, h->dzt);
     if ((rc = gemm_nt(EPI_NONE, h->dyb, h->L[4].wt, a, st))) return rc;
     // z = W3 h2 + b3 + h0
-    if ((rc = grad_w(3, h->dzb, 256, h->h2b, 512)) || (rc = grad_b(3, h->dz, 256))) return rc;
     a = args(B, 512, 256, h->err);
     a.aux = h->a2;
     a.c32 = h->da2;
     a.ld32 = 512;
     a.c16 = h->da2b;
     a.ld16 = 512;
+    transposed(a, h->da2t);
     if ((rc = gemm_nt(EPI_DGELU, h->dzb, h->L[3].wt, a, st))) return rc;
     // h2 = GELU(W2 h1 + b2)
-    if ((rc = grad_w(2, h->da2b, 512, h->h1b, 512)) || (rc = grad_b(2, h->da2, 512))) return rc;
     a = args(B, 512, 512, h->err);
     a.aux = h->a1;
     a.c32 = h->da1;
     a.ld32 = 512;
     a.c16 = h->da1b;
     a.ld16 = 512;
+    transposed(a, h->da1t);
     if ((rc = gemm_nt(EPI_DGELU, h->da2b, h->L[2].wt, a, st))) return rc;
     // h1 = GELU(W1 h0 + b1); dh0 also receives dz through the residual
-    if ((rc = grad_w(1, h->da1b, 512, h->h0b, 256)) || (rc = grad_b(1, h->da1, 512))) return rc;
     a = args(B, 256, 512, h->err);
     a.add = h->dz;
     a.c32 = h->dh0;
     a.ld32 = 256;
-    a.c16 = h->dh0b;
-    a.ld16 = 256;
+    transposed(a, h->dh0t);
     if ((rc = gemm_nt(EPI_NONE, h->da1b, h->L[1].wt, a, st))) return rc;
-    // h0 = W0 x + b0
-    if ((rc = grad_w(0, h->dh0b, 256, h->xb, h->n_in_p)) || (rc = grad_b(0, h->dh0, 256))) return rc;
-    return GD_OK;
+    // all weights' gradients in one launch: dW[o][i] = sum_b dY[b][o] X[b][i], A =
+    // dY^T [out][B], B = X^T [in][B]
+    const bf16 *dYt[5] = {h->dh0t, h->da1t, h->da2t, h->dzt, h->dyt};
+    const bf16 *Xt[5] = {h->xt, h->h0t, h->h1t, h->h2t, h->zt};
+    const float *dY[5] = {h->dh0, h->da1, h->da2, h->dz, h->dy};
+    Product pr[5];
+    ColSums cs;
+    for (int k = 0; k < 5; k++) {
+        const gd_mlp::Layer &l = h->L[k];
+        pr[k] = Product{dYt[k], Xt[k], args(l.out, l.in, B, h->err)};
+        pr[k].a.c32 = l.gw;
+        pr[k].a.ld32 = l.in;
+        cs.d[k] = dY[k];
+        cs.out[k] = l.gb;
+        cs.n[k] = l.out;
+        cs.end[k] = (k > 0 ? cs.end[k - 1] : 0) + (l.out + 31) / 32;
+    }
+    if ((rc = gemm_nt<5>(EPI_NONE, pr, st))) return rc;
+    return launch_ordered(colsum_kernel, dim3(cs.end[4]), st, cs, B);
 }
 
-// loss and output gradient for targets t (loss denominators from tden, or t)
-int loss_grad(gd_mlp *h, const float *t, int ldt, const float *tden, int ldd, int B, cudaStream_t st)
+// loss and output gradient for targets t (the sums of squares for the
+// denominators in h->den); the batch's mean loss into loss when set
+int loss_grad(gd_mlp *h, const float *t, int ldt, int B, bool train, float *loss, cudaStream_t st)
 {
     const int pw = (h->flags & GD_MLP_SCALE_OUTPUT) ? 1 : 0;
     const int mse = (h->flags & GD_MLP_LOSS_MSE) ? 1 : 0;
-    dim3 blk(32, 8), grd((B + 31) / 32, h->n_out_p / 32);
     const float inv_gain = 1.f / h->out_gain;
-    gd::gather_target_kernel<<<grd, blk, 0, st>>>(t, h->n_out, ldt, B, h->scale, pw, inv_gain, h->tt, h->n_out_p);
-    GD_CUDA(cudaGetLastError());
-    int rc = gd::launch_ordered(gd::row_den_kernel, B, st, tden ? tden : t, h->n_out, tden ? ldd : ldt, B,
-                                (const float *)h->scale, pw, inv_gain, mse, h->den);
-    if (rc) return rc;
-    if (!mse && (h->flags & GD_MLP_LOSS_BATCH)) gd::batch_mean_den_kernel<<<1, 256, 0, st>>>(h->den, B);
-    gd::loss_grad_kernel<<<B, 256, 0, st>>>(h->y, h->tt, h->n_out_p, h->n_out, B, h->den, h->dy, h->dyb, h->row_err);
+    gd::den_kernel<<<1, 256, 0, st>>>(h->den, B, h->scale, pw, inv_gain, mse, h->n_out,
+                                      !mse && (h->flags & GD_MLP_LOSS_BATCH));
+    dim3 blk(32, 8), grd((B + 31) / 32, h->n_out_p / 64);
+    gd::loss_grad_kernel<<<grd, blk, 0, st>>>(h->y, t, ldt, h->n_out, h->n_out_p, B, h->scale, pw, inv_gain, h->den,
+                                              h->dy, h->dyb, train ? h->dyt : nullptr, h->err_part);
+    if (loss || !train)
+        gd::row_err_kernel<<<loss ? 1 : (B + 1023) / 1024, 1024, 0, st>>>(h->err_part, h->n_out_p / 64, B, h->den,
+                                                                       h->row_err, loss);
     GD_CUDA(cudaGetLastError());
     return GD_OK;
 }
@@ -1164,7 +1314,6 @@ extern "C" int gd_mlp_create(int n_in, int n_out, int batch_cap, int flags, uint
     if (!rc) rc = alloc_n(h, &h->a1, c * 512);
     if (!rc) rc = alloc_n(h, &h->a2, c * 512);
     if (!rc) rc = alloc_n(h, &h->y, c * h->n_out_p);
-    if (!rc) rc = alloc_n(h, &h->tt, c * h->n_out_p);
     if (!rc) rc = alloc_n(h, &h->dy, c * h->n_out_p);
     if (!rc) rc = alloc_n(h, &h->dyb, c * h->n_out_p);
     if (!rc) rc = alloc_n(h, &h->dz, c * 256);
@@ -1174,10 +1323,17 @@ extern "C" int gd_mlp_create(int n_in, int n_out, int batch_cap, int flags, uint
     if (!rc) rc = alloc_n(h, &h->da1, c * 512);
     if (!rc) rc = alloc_n(h, &h->da1b, c * 512);
     if (!rc) rc = alloc_n(h, &h->dh0, c * 256);
-    if (!rc) rc = alloc_n(h, &h->dh0b, c * 256);
-    const size_t widest = (size_t)std::max(h->n_in_p, std::max(h->n_out_p, 512));
-    if (!rc) rc = alloc_n(h, &h->tmp1, c * widest);
-    if (!rc) rc = alloc_n(h, &h->tmp2, c * widest);
+    if (!rc) rc = alloc_n(h, &h->xt, c * h->n_in_p);
+    if (!rc) rc = alloc_n(h, &h->h0t, c * 256);
+    if (!rc) rc = alloc_n(h, &h->h1t, c * 512);
+    if (!rc) rc = alloc_n(h, &h->h2t, c * 512);
+    if (!rc) rc = alloc_n(h, &h->zt, c * 256);
+    if (!rc) rc = alloc_n(h, &h->dyt, c * h->n_out_p);
+    if (!rc) rc = alloc_n(h, &h->dzt, c * 256);
+    if (!rc) rc = alloc_n(h, &h->da2t, c * 512);
+    if (!rc) rc = alloc_n(h, &h->da1t, c * 512);
+    if (!rc) rc = alloc_n(h, &h->dh0t, c * 256);
+    if (!rc) rc = alloc_n(h, &h->err_part, c * (h->n_out_p / 64));
     if (!rc) rc = alloc_n(h, &h->scale, c);
     if (!rc) rc = alloc_n(h, &h->den, c);
     if (!rc) rc = alloc_n(h, &h->row_err, c);
@@ -1243,8 +1399,8 @@ extern "C" int gd_mlp_forward(gd_mlp *h, const float *x, int ldx, int batch, flo
         return set_error(GD_ERR_INVALID_ARG, "bad surrogate forward arguments (1 <= batch <= cap, ld >= batch)");
     gd::DeviceGuard ds(h->device);
     cudaStream_t st = (cudaStream_t)stream;
-    int rc = load_input(h, x, ldx, batch, st);
-    if (!rc) rc = forward(h, batch, y, ldy, st);
+    int rc = load_input(h, x, ldx, batch, false, nullptr, 0, st);
+    if (!rc) rc = forward(h, batch, y, ldy, false, st);
     return rc;
 }
 
@@ -1257,28 +1413,31 @@ extern "C" int gd_mlp_train_step(gd_mlp *h, const float *x, int ldx, const float
         return set_error(GD_ERR_INVALID_ARG, "bad surrogate training arguments (batch a multiple of 64, <= cap)");
     gd::DeviceGuard ds(h->device);
     cudaStream_t st = (cudaStream_t)stream;
-    int rc = load_input(h, x, ldx, batch, st);
-    if (!rc) rc = forward(h, batch, nullptr, 0, st);
-    if (!rc) rc = loss_grad(h, t, ldt, tden, ldd, batch, st);
+    int rc = load_input(h, x, ldx, batch, true, tden ? tden : t, tden ? ldd : ldt, st);
+    if (!rc) rc = forward(h, batch, nullptr, 0, true, st);
+    if (!rc) rc = loss_grad(h, t, ldt, batch, true, loss, st);
     if (rc) return rc;
-    if (loss) {
-        mean_kernel<<<1, 256, 0, st>>>(h->row_err, batch, loss);
-        GD_CUDA(cudaGetLastError());
-    }
     if ((rc = backward(h, batch, st))) return rc;
     h->step++;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     const float c1 = 1.f - (float)std::pow(0.9, (double)h->step), c2 = 1.f - (float)std::pow(0.999, (double)h->step);
+    AdamSet ad;
+    ad.lr = lr;
+    ad.b1 = b1;
+    ad.b2 = b2;
+    ad.c1 = c1;
+    ad.c2 = c2;
+    ad.eps = eps;
+    ad.wd = weight_decay;
+    int blocks = 0;
     for (int k = 0; k < 5; k++) {
         gd_mlp::Layer &l = h->L[k];
-        const int64_t nw = (int64_t)l.out * l.in;
-        adam_kernel<<<(int)std::min<int64_t>((nw + 255) / 256, 4096), 256, 0, st>>>(l.w, l.gw, l.mw, l.vw, l.wb, nw, lr, b1,
-                                                                                     b2, c1, c2, eps, weight_decay);
-        adam_kernel<<<(l.out + 255) / 256, 256, 0, st>>>(l.b, l.gb, l.mb, l.vb, nullptr, l.out, lr, b1, b2, c1, c2, eps,
-                                                         0.f);
-        GD_CUDA(cudaGetLastError());
-        if (k > 0 && (rc = transpose(l.wb, l.out, l.in, l.in, l.wt, l.out, st))) return rc;
+        const int wend = blocks + l.out / 32 * (l.in / 32);
+        blocks = wend + (l.out + 1023) / 1024;
+        ad.l[k] = {l.w, l.b, l.mw, l.vw, l.mb, l.vb, l.gw, l.gb, l.wb, k > 0 ? l.wt : nullptr, l.out, l.in, wend, blocks};
     }
+    adam_kernel<<<blocks, dim3(32, 8), 0, st>>>(ad);
+    GD_CUDA(cudaGetLastError());
     return GD_OK;
 }
 
@@ -1291,9 +1450,9 @@ extern "C" int gd_mlp_loss(gd_mlp *h, const float *x, int ldx, const float *t, i
         return set_error(GD_ERR_INVALID_ARG, "bad surrogate loss arguments");
     gd::DeviceGuard ds(h->device);
     cudaStream_t st = (cudaStream_t)stream;
-    int rc = load_input(h, x, ldx, batch, st);
-    if (!rc) rc = forward(h, batch, nullptr, 0, st);
-    if (!rc) rc = loss_grad(h, t, ldt, tden, ldd, batch, st);
+    int rc = load_input(h, x, ldx, batch, false, tden ? tden : t, tden ? ldd : ldt, st);
+    if (!rc) rc = forward(h, batch, nullptr, 0, false, st);
+    if (!rc) rc = loss_grad(h, t, ldt, batch, false, nullptr, st);
     if (rc) return rc;
     GD_CUDA(cudaMemcpyAsync(row_loss, h->row_err, (size_t)batch * sizeof(float), cudaMemcpyDeviceToDevice, st));
     return GD_OK;
