@@ -400,25 +400,11 @@ static int create_context(Context &c, const gd_grid_spec &spec, int device)
     if (rc) return rc;
     if ((rc = build_row_groups(c))) return rc;
     if ((rc = orbit_build(c))) return rc;
-    // scatter updates: distinct sign patterns of g whose target lies in the sphere
-    int64_t sc = 0;
-    for (int sx = 0; sx < d.sx; sx++)
-        for (int sy = 0; sy < d.sy; sy++)
-            for (int sz = 0; sz < d.sz; sz++) {
-                const int Dx = std::min(sx, 2 * d.nx - 2 - sx), Dy = std::min(sy, 2 * d.ny - 2 - sy),
-                          Dz = std::min(sz, 2 * d.nz - 2 - sz);
-                for (int gx = sx & 1; gx <= Dx; gx += 2)
-                    for (int gy = sy & 1; gy <= Dy; gy += 2)
-                        for (int gz = sz & 1; gz <= Dz; gz += 2)
-                            for (int sg = 0; sg < 8; sg++) {
-                                if (((sg & 1) && gx == 0) || ((sg & 2) && gy == 0) || ((sg & 4) && gz == 0)) continue;
-                                const int ix = (sx + ((sg & 1) ? -gx : gx)) >> 1;
-                                const int iy = (sy + ((sg & 2) ? -gy : gy)) >> 1;
-                                const int iz = (sz + ((sg & 4) ? -gz : gz)) >> 1;
-                                sc += c.cmap[(ix * d.ny + iy) * d.nz + iz] >= 0;
-                            }
-            }
-    c.scatter_terms = sc;
+    // scatter updates: for every pair sum s the distinct sign patterns of g whose
+    // target i = (s +- g) / 2 lies in the sphere.  A node i and s determine g = |2 i - s|,
+    // which is one of s's when the partner s - i lies in the box: one update for every
+    // pair of an in-sphere node and a node of the box.
+    c.scatter_terms = (int64_t)d.n_pnt * d.nxyz;
     GD_CUDA(cudaDeviceSynchronize());
     return GD_OK;
 }
