@@ -16,8 +16,8 @@
 // warp by warp, then CTA by CTA, in fixed order, so the sums are reproducible.
 // Bound: the FP64 pipe (its rate is 1/64 of the FP32 rate and a hardware float to
 // double conversion takes a slot of it, so to_double does that in integers).
-// 20^3: 4096 cells 1.54 -> 0.88 ms (the FP64 pipe 76 % busy where SMs have work; a
-// cluster of eight leaves some without), 256 cells 1.6 -> 0.105, one cell 1.6 -> 0.06.
+// 20^3: 4096 cells 1.54 -> 0.84 ms (the FP64 pipe three quarters busy), 256 cells 1.6 ->
+// 0.092, one cell 1.6 -> 0.057.
 #include "gd_internal.h"
 #include "gd_tc.cuh"
 
@@ -118,6 +118,7 @@ __global__ void __launch_bounds__(kWarps * 32) project_kernel(const __grid_const
     extern __shared__ __align__(16) double red[];  // [kWarps][kSums][32], then the CTA's sums [kSums][32]
     __shared__ double xs[5][32];
     double *mine = red + kWarps * kSums * 32;
+    constexpr int NS = M5 ? kSums : kSums - 5;  // without the moments
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int rank = (int)blockIdx.x % cs;
     constexpr int G = 32 / LC;  // lines side by side in a warp
@@ -127,7 +128,7 @@ __global__ void __launch_bounds__(kWarps * 32) project_kernel(const __grid_const
     const int first = (rank * kWarps + warp) * G + lane / LC, step = cs * kWarps * G;
     double s[kSums];
 #pragma unroll
-    for (int k = 0; k < kSums; k++) s[k] = 0.;
+    for (int k = 0; k < NS; k++) s[k] = 0.;
     if (live) {
         for (int l = first; l < a.nlines; l += step) {
             const int4 ln = __ldg(a.lines + l);
@@ -147,8 +148,8 @@ __global__ void __launch_bounds__(kWarps * 32) project_kernel(const __grid_const
                 S2 += fn * z2;
                 S3 += fn * zp[1].x;
                 S4 += fn * zp[1].y;
-                M0 += fv;
                 if (M5) {
+                    M0 += fv;
                     M1 += fv * z;
                     M2 += fv * z2;
                 }
@@ -176,8 +177,8 @@ __global__ void __launch_bounds__(kWarps * 32) project_kernel(const __grid_const
             s[17] += S2;
             s[18] += E1;
             s[19] += E2;
-            s[20] += M0;
             if (M5) {
+                s[20] += M0;
                 s[21] += x * M0;
                 s[22] += y * M0;
                 s[23] += M1;
@@ -188,13 +189,13 @@ __global__ void __launch_bounds__(kWarps * 32) project_kernel(const __grid_const
     // combine the lane groups' partial sums, the warps' in warp order, then the
     // CTAs' in rank order
 #pragma unroll
-    for (int k = 0; k < kSums; k++) {
+    for (int k = 0; k < NS; k++) {
 #pragma unroll
         for (int w = LC; w < 32; w *= 2) s[k] += __shfl_xor_sync(0xffffffffu, s[k], w);
         red[((size_t)warp * kSums + k) * 32 + lane] = s[k];
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < kSums * 32; t += kWarps * 32) {
+    for (int t = threadIdx.x; t < NS * 32; t += kWarps * 32) {
         double v = red[t];
         for (int w = 1; w < kWarps; w++) v += red[(size_t)w * kSums * 32 + t];
         mine[t] = v;
@@ -203,7 +204,7 @@ __global__ void __launch_bounds__(kWarps * 32) project_kernel(const __grid_const
     else __syncthreads();
     if (rank == 0) {
         if (cs > 1) {
-            for (int t = threadIdx.x; t < kSums * 32; t += kWarps * 32) {
+            for (int t = threadIdx.x; t < NS * 32; t += kWarps * 32) {
                 double v = mine[t];
                 for (int k = 1; k < cs; k++) v += peer_load(mine + t, (uint32_t)k);
                 red[t] = v;
@@ -212,9 +213,9 @@ __global__ void __launch_bounds__(kWarps * 32) project_kernel(const __grid_const
         }
         if (warp == 0) {
             const double *all = cs > 1 ? red : mine;
-            double tot[kSums];
+            double tot[kSums] = {};
 #pragma unroll
-            for (int k = 0; k < kSums; k++) tot[k] = all[k * 32 + lane];
+            for (int k = 0; k < NS; k++) tot[k] = all[k * 32 + lane];
             double A[5][5], B[5], X[5];
             int t = 5;
 #pragma unroll
@@ -229,14 +230,22 @@ __global__ void __launch_bounds__(kWarps * 32) project_kernel(const __grid_const
                 }
             bool finite = true;
 #pragma unroll
-            for (int k = 0; k < kSums; k++) finite = finite && isfinite(tot[k]);
+            for (int k = 0; k < NS; k++) finite = finite && isfinite(tot[k]);
             const bool solved = finite && solve5(A, B, X);
             if (!solved) {
 #pragma unroll
                 for (int k = 0; k < 5; k++) X[k] = 0.;
                 // recorded for gd_ctx_check: the flags OR together, the smallest
                 // failing cell wins, so the record does not depend on scheduling
-                if (live && lane < LC && a.status && (!finite || tot[20] != 0.0)) {  // an empty cell has nothing to correct
+                bool record = live && lane < LC && a.status;
+                if (record && finite) {
+                    // an empty cell has nothing to correct (its mass is not among the
+                    // sums: it would cost every cell a sixteenth of the pipe's time)
+                    double mass = 0.;
+                    for (int i = 0; i < a.d.n_pnt; i++) mass += to_double(a.f[(size_t)i * a.ld + cell]);
+                    record = mass != 0.;
+                }
+                if (record) {
                     atomicOr(a.status, finite ? 2u : 1u);
                     atomicMin(a.status + 1, (unsigned int)cell);
                 }
@@ -412,14 +421,19 @@ int run_project(Context &c, const float *f, const float *nu, const float *gain, 
 {
     const ProjArgs a{c.d,   f, nu, gain, ld,                     ncells, c.nlines, c.d_lines, c.d_line_xy, c.d_zpow, nu_corr,
                      q,     x, fixed_dt_mode ? 1 : 0, dt, f_out, m5,     c.d_status};
-    // cells per warp: 32, or eight or one when a cluster per 32 cells leaves
-    // SMs idle (20^3: 600 cells 0.230 ms with 32, 0.256 with 8; 256 cells 0.132
-    // and 0.105; one cell 0.132, 0.062 and 0.060 with 1)
-    const int lc = ncells > 512 ? 32 : ncells > 8 ? 8 : 1;
-    // CTAs per lc cells: about six CTAs per SM, so that the last wave costs little
-    const int blocks = (ncells + lc - 1) / lc;
+    // Cells per warp (32, 8 or 1) and CTAs per group of cells: about one CTA per SM,
+    // as long as each of its threads has a line, since what a CTA adds to the lines'
+    // own sums (25 sums combined over lanes, warps and CTAs, the solution) takes the
+    // FP64 pipe for as long as a line or two; two per SM from eight cells per SM on,
+    // which hide the loads from HBM.  (cells per warp, CTAs) at 20^3, us: one cell
+    // (1, 2) 58, (8, 8) 62; 128 cells (1, 1) 73, (8, 8) 105; 256 (8, 4) 96, (8, 8) 106;
+    // 500 (8, 2) 149, (8, 8) 195, (32, 8) 231; 1024 (32, 4) 243, (32, 8) 253; 2048 (32,
+    // 4) 460, (32, 2) 524, (32, 8) 480.  8^3, 500 cells: (8, 2) 36, (8, 8) 97.
+    const int sms = std::max(1, c.sm_count);
+    const int lc = ncells <= sms ? 1 : ncells <= 4 * sms ? 8 : 32;
+    const int blocks = (ncells + lc - 1) / lc, most = ncells > 8 * sms ? 2 * sms : sms;
     int cs = 1;
-    while (cs < 8 && blocks * cs < 6 * c.sm_count) cs *= 2;
+    while (cs < 8 && 2 * cs * blocks <= most && cs * kWarps * (32 / lc) < c.nlines) cs *= 2;
     auto kern = lc == 32 ? (m5 ? project_kernel<true, 32> : project_kernel<false, 32>)
                 : lc == 8 ? (m5 ? project_kernel<true, 8> : project_kernel<false, 8>)
                           : (m5 ? project_kernel<true, 1> : project_kernel<false, 1>);
