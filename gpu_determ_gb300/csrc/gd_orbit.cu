@@ -483,6 +483,35 @@ __global__ void orbit_reduce_kernel(const float *__restrict__ part, int nchunks,
     }
 }
 
+// The same for at most kOFewChunks chunks: a thread per row and four cells adds
+// them in order, all its loads in flight (16^3, 500 cells, 12 chunks: 45 -> 14 us).
+constexpr int kOFewChunks = 16;
+__global__ void __launch_bounds__(256) orbit_reduce_few_kernel(const float *__restrict__ part, int nchunks, int ns,
+                                                               int cells_pad, int ncells, int ld,
+                                                               const int *__restrict__ row_node,
+                                                               const float2 *__restrict__ scale,
+                                                               float *__restrict__ gain)
+{
+    const int cell = 4 * (blockIdx.x * 32 + threadIdx.x), row = blockIdx.y * 8 + threadIdx.y;
+    if (cell >= ncells || row >= ns) return;  // ns is a multiple of 8, cells_pad of 4
+    const float4 *p = reinterpret_cast<const float4 *>(part + (size_t)row * cells_pad + cell);
+    const size_t step = (size_t)ns * cells_pad / 4;
+    float4 s = __ldg(p);
+#pragma unroll 8
+    for (int k = 1; k < nchunks; k++) {
+        const float4 v = __ldg(p + (size_t)k * step);
+        s.x += v.x;
+        s.y += v.y;
+        s.z += v.z;
+        s.w += v.w;
+    }
+    float *g = gain + (size_t)__ldg(row_node + row) * ld + cell;
+    const float o[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        if (cell + q < ncells) g[q] = scale ? unscale(o[q], scale[cell + q].y) : o[q];
+}
+
 // One D of the low octant with anything to do.
 struct DItem {
     int K = 0, nblk = 0;
@@ -1045,7 +1074,11 @@ int launch_orbit(Context &c, const float *f, int ncells, int ld, float *gain, vo
     GD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
     kern<<<dim3(tiles, nchunks), kOThreads, g.smem, st>>>(a);
     GD_CUDA(cudaGetLastError());
-    if (part) {
+    if (part && nchunks <= kOFewChunks) {
+        orbit_reduce_few_kernel<<<dim3((cells_pad + 127) / 128, d.n_pnt / 8), dim3(32, 8), 0, st>>>(
+            part, nchunks, d.n_pnt, cells_pad, ncells, ld, g.row_node, scale, gain);
+        GD_CUDA(cudaGetLastError());
+    } else if (part) {
         const int64_t outs = (int64_t)d.n_pnt * ncells;
         orbit_reduce_kernel<<<(unsigned)((outs + 31) / 32), dim3(32, 8), 0, st>>>(part, nchunks, d.n_pnt, cells_pad, ncells,
                                                                                  ld, g.row_node, scale, gain);
