@@ -708,7 +708,8 @@ def run_kernels(args):
         ctx.set_gain_path(GAIN_PATHS[args.gain])
         torch.cuda.synchronize()
         build_s["gain_path"] = time.perf_counter() - t0
-        run("loss_tc", lambda: ctx.collision(f, nc, nc, nu, None))
+        if not fp32_gain(args.gain, ctx):
+            run("loss_tc", lambda: ctx.collision(f, nc, nc, nu, None))
     ctx.collision(f, nc, nc, nu, gain)
     run("project", lambda: ctx.project(f, nu, gain, nc, nc, nuc, q, None))
     run("relax_fixed", lambda: ctx.relax(fr, nuc, gain, nc, nc, gd.DT_FIXED, 1e-4, tm, dt))
@@ -737,8 +738,9 @@ def run_kernels(args):
         return e
 
     k = {}
-    k["loss_kernel (FP32)"] = entry(ms["loss_fp32"], flop=2.0 * n * n * nc, fpeak=pk["fp32"],
-                                    work="2 n^2 FLOP per cell (one FMA per partner), vs the FP32 FMA peak")
+    k["folded_loss_kernel (FP32)"] = entry(ms["loss_fp32"], flop=2.0 * n * n / 8 * nc, fpeak=pk["fp32"],
+                                           work="n^2 / 4 FLOP per cell (one FMA per pair of orbits and character of "
+                                                "the reflections), vs the FP32 FMA peak")
     if "loss_tc" in ms:
         rows, cols, kk = -(-n // 128) * 128, -(-nc // 128) * 128, -(-n // 64) * 64
         k["convert + gemm3_nt_kernel (loss on tensor cores)"] = entry(
@@ -746,9 +748,10 @@ def run_kernels(args):
             nbytes=4.0 * n * kk + 4.0 * kk * nc + 4.0 * cells + 4.0 * cells,
             work="3 BF16 MMA products per K step over the padded tiles, vs the BF16 peak; bytes: B and f "
                  "as BF16 hi/lo, f read and nu written in FP32")
-    k["project_kernel (FP64)"] = entry(ms["project"], flop=65.0 * cells, fpeak=pk["fp64"], nbytes=24.0 * cells,
-                                       work="65 FP64 FLOP per node and cell (53 for the 25 sums, 12 for nu' and "
-                                            "Q) and 7 conversions; bytes: f, nu, I read, nu' and FP64 Q written")
+    k["project_kernel (FP64)"] = entry(ms["project"], flop=23.0 * cells, fpeak=pk["fp64"], nbytes=24.0 * cells,
+                                       work="23 FP64 FLOP in 15 instructions per node and cell (16 for the sums over "
+                                            "a line, 7 for nu' and Q) and one conversion; bytes: f, nu, I read, nu' "
+                                            "and FP64 Q written")
     k["relax_kernel (FP64, fixed dt)"] = entry(ms["relax_fixed"], flop=4.0 * cells, fpeak=pk["fp64"],
                                                nbytes=16.0 * cells,
                                                work="f + dt (I - f nu') in FP64: 4 FLOP and 4 conversions; bytes: f, nu', "

@@ -415,25 +415,52 @@ __global__ void basis_kernel(Dims d, const float *__restrict__ u, const float *_
 
 }  // namespace
 
+// Cells per warp (32, 8 or 1) and CTAs per group of cells, by the FP64 pipe's time
+// in instructions of a warp: a CTA's threads take so many lines each (15 per node
+// and 40 per line), then combine 20 sums over lanes, warps and CTAs (about 125).  An
+// SM works off its CTAs one after the other; clusters of four and eight find room
+// in fewer SMs (their GPC's); one CTA per SM waits for its loads when they come from
+// HBM.  Measured at 20^3, us (cells per warp, CTAs): one cell (1, 2) 57, (8, 8) 62;
+// 152 cells (1, 1) 67, (8, 4) 92; 240 (8, 4) 92, (1, 1) 106; 420 (32, 8) 128, (8, 2)
+// 143; 600 (8, 2) 143, (32, 8) 221; 1064 (32, 4) 239; 1300 (32, 8) 340, (32, 4) 421;
+// 2100 (32, 4) 435, (32, 2) 500; 4096 (32, 2) 844, (32, 1) 909.
+struct ProjSplit {
+    int lc, cs;
+};
+ProjSplit project_split(const Context &c, int ncells)
+{
+    const int sms = std::max(1, c.sm_count);
+    const double nodes = (double)c.d.n_pnt / c.nlines;
+    const bool hbm = (int64_t)c.d.n_pnt * ncells > ((int64_t)100 << 20) / 24;
+    ProjSplit best{32, 1};
+    double least = 0.0;
+    for (int lc : {1, 8, 32})
+        for (int cs = 1; cs <= 8; cs *= 2) {
+            const int64_t ctas = ((int64_t)ncells + lc - 1) / lc * cs;
+            const int threads = cs * kWarps * (32 / lc);  // of a cell
+            const double lines = (c.nlines + threads - 1) / threads;
+            const int room = cs == 8 ? sms * 3 / 4 : cs == 4 ? sms * 11 / 12 : sms;
+            const int many = cs >= 4 ? std::max(1, sms * 14 / 15) : sms;
+            const int64_t turns = ctas <= room ? 1 : std::max<int64_t>(2, (ctas + many - 1) / many);
+            double cost = (double)turns * (lines * (15.0 * nodes + 40.0) + 125.0);
+            if (turns == 1 && hbm) cost *= 1.15;
+            if (lc == 8) cost *= 1.1;  // 32-byte rows
+            if (least == 0.0 || cost < least * (1.0 - 1e-9)) {
+                least = cost;
+                best = ProjSplit{lc, cs};
+            }
+        }
+    return best;
+}
+
 int run_project(Context &c, const float *f, const float *nu, const float *gain, int ncells, int ld,
                 float *nu_corr, double *q, double *x, int fixed_dt_mode, float dt, float *f_out,
                 double *m5, cudaStream_t st)
 {
     const ProjArgs a{c.d,   f, nu, gain, ld,                     ncells, c.nlines, c.d_lines, c.d_line_xy, c.d_zpow, nu_corr,
                      q,     x, fixed_dt_mode ? 1 : 0, dt, f_out, m5,     c.d_status};
-    // Cells per warp (32, 8 or 1) and CTAs per group of cells: about one CTA per SM,
-    // as long as each of its threads has a line, since what a CTA adds to the lines'
-    // own sums (25 sums combined over lanes, warps and CTAs, the solution) takes the
-    // FP64 pipe for as long as a line or two; two per SM from eight cells per SM on,
-    // which hide the loads from HBM.  (cells per warp, CTAs) at 20^3, us: one cell
-    // (1, 2) 58, (8, 8) 62; 128 cells (1, 1) 73, (8, 8) 105; 256 (8, 4) 96, (8, 8) 106;
-    // 500 (8, 2) 149, (8, 8) 195, (32, 8) 231; 1024 (32, 4) 243, (32, 8) 253; 2048 (32,
-    // 4) 460, (32, 2) 524, (32, 8) 480.  8^3, 500 cells: (8, 2) 36, (8, 8) 97.
-    const int sms = std::max(1, c.sm_count);
-    const int lc = ncells <= sms ? 1 : ncells <= 4 * sms ? 8 : 32;
-    const int blocks = (ncells + lc - 1) / lc, most = ncells > 8 * sms ? 2 * sms : sms;
-    int cs = 1;
-    while (cs < 8 && 2 * cs * blocks <= most && cs * kWarps * (32 / lc) < c.nlines) cs *= 2;
+    const ProjSplit split = project_split(c, ncells);
+    const int lc = split.lc, cs = split.cs, blocks = (ncells + lc - 1) / lc;
     auto kern = lc == 32 ? (m5 ? project_kernel<true, 32> : project_kernel<false, 32>)
                 : lc == 8 ? (m5 ? project_kernel<true, 8> : project_kernel<false, 8>)
                           : (m5 ? project_kernel<true, 1> : project_kernel<false, 1>);

@@ -1,7 +1,6 @@
-"""The projection's split of lines and cells over the chip at the cell counts
-where it changes (one cell per warp up to the number of SMs, eight up to four
-times, 32 beyond, two CTAs per SM from eight times): every split sums the same
-FP64 terms in another order, so a cell's Q agrees between batches to n_pnt
+"""The projection's split of lines and cells over the chip (one, eight or 32
+cells per warp, one to eight CTAs per group of cells, by the number of SMs and the
+lattice) over cell counts where it changes: every split sums the same FP64 terms in another order, so a cell's Q agrees between batches to n_pnt
 roundings, 1e-12 of its largest I.  An empty cell is left alone without a
 record, a cell whose system is singular is recorded."""
 import numpy as np
