@@ -630,14 +630,49 @@ __global__ void __launch_bounds__(1024) cell_sums_kernel(const float *__restrict
 
 __device__ __forceinline__ float inv_or_zero(float s) { return s != 0.f ? 1.f / s : 0.f; }
 
+// Loss denominators per cell from the sums of squares in den: scaled like the
+// targets for the relative losses, or n for the mean squared error; with mean set
+// their mean over the batch (fixed order).  One block of 256 threads, beside those
+// that copy the input.
+struct DenArgs {
+    float *den;  // null: nothing to do
+    int pw;
+    float inv_gain;
+    int mse, n, mean;
+};
+__device__ __forceinline__ void denominators(const DenArgs &a, int B, const float *__restrict__ scale, double *s)
+{
+    const int t = threadIdx.y * 32 + threadIdx.x;
+    double sum = 0.0;
+    for (int i = t; i < B; i += 256) {
+        const float sc = (a.pw ? inv_or_zero(scale[i] * scale[i]) : 1.f) * a.inv_gain;
+        const float v = a.mse ? (float)a.n : a.den[i] * sc * sc;
+        a.den[i] = v;
+        sum += v;
+    }
+    if (!a.mean) return;
+    s[t] = sum;
+    __syncthreads();
+    for (int k = 128; k > 0; k >>= 1) {
+        if (t < k) s[t] += s[t + k];
+        __syncthreads();
+    }
+    const float m = (float)(s[0] / B);
+    for (int i = t; i < B; i += 256) a.den[i] = m;
+}
+
 // node-major FP32 x[i][r] (ld) -> cell-major BF16 xb[r][i] * gain / scale[r] (pad to
 // n_p), for training also its transpose xt[i][r].  Block = 64 nodes x 32 cells: eight loads in flight per thread and whole
 // 128-byte rows on both sides (4096 cells, 3648 nodes: 39 -> 15 us).
 template <bool TRANSPOSE>
 __global__ void gather_in_kernel(const float *__restrict__ x, int n, int ld, int B, const float *__restrict__ scale,
-                                 float gain, bf16 *__restrict__ xb, bf16 *__restrict__ xt, int n_p)
+                                 float gain, bf16 *__restrict__ xb, bf16 *__restrict__ xt, int n_p, DenArgs den)
 {
-    __shared__ float tile[64][33];
+    __shared__ __align__(8) float tile[64][33];
+    if ((int)blockIdx.y == n_p / 64) {  // the row past the nodes: the denominators
+        if (blockIdx.x == 0) denominators(den, B, scale, reinterpret_cast<double *>(&tile[0][0]));
+        return;
+    }
     const int i0 = blockIdx.y * 64, r0 = blockIdx.x * 32, r = r0 + threadIdx.x;
     const float s = r < B ? inv_or_zero(scale[r]) * gain : 0.f;
     float v[8];
@@ -662,41 +697,62 @@ __global__ void gather_in_kernel(const float *__restrict__ x, int n, int ld, int
     }
 }
 
-// Loss denominators per cell from the sums of squares in den: scaled like the
-// targets for the relative losses, or n for the mean squared error; with mean set
-// their mean over the batch (fixed order).  One block.
-__global__ void den_kernel(float *__restrict__ den, int B, const float *__restrict__ scale, int pw, float inv_gain,
-                           int mse, int n, int mean)
+// Loss of cell r: the sum of the node tiles' errors / den[r].
+__device__ __forceinline__ float cell_loss(const float *__restrict__ err_part, int tiles, int B,
+                                           const float *__restrict__ den, int r)
 {
-    __shared__ double s[256];
+    float e = 0.f;
+#pragma unroll 8
+    for (int k = 0; k < tiles; k++) e += __ldg(err_part + (size_t)k * B + r);
+    return e / fmaxf(den[r], 1e-30f);
+}
+__global__ void row_err_kernel(const float *__restrict__ err_part, int tiles, int B, const float *__restrict__ den,
+                               float *__restrict__ row_err)
+{
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r < B) row_err[r] = cell_loss(err_part, tiles, B, den, r);
+}
+
+// The cells' losses and their mean over the batch (fixed order), by one block of 1024.
+struct MeanLoss {
+    const float *err_part;
+    int tiles;
+    const float *den;
+    float *row_err, *out;
+};
+__device__ __forceinline__ void mean_loss(const MeanLoss &m, int B, double *s)
+{
+    const int t = threadIdx.y * 32 + threadIdx.x;
     double a = 0.0;
-    for (int i = threadIdx.x; i < B; i += blockDim.x) {
-        const float sc = (pw ? inv_or_zero(scale[i] * scale[i]) : 1.f) * inv_gain;
-        const float v = mse ? (float)n : den[i] * sc * sc;
-        den[i] = v;
-        a += v;
+    for (int r = t; r < B; r += 1024) {
+        const float e = cell_loss(m.err_part, m.tiles, B, m.den, r);
+        m.row_err[r] = e;
+        a += e;
     }
-    if (!mean) return;
-    s[threadIdx.x] = a;
+    s[t] = a;
     __syncthreads();
-    for (int k = blockDim.x / 2; k > 0; k >>= 1) {
-        if (threadIdx.x < k) s[threadIdx.x] += s[threadIdx.x + k];
+    for (int k = 512; k > 0; k >>= 1) {
+        if (t < k) s[t] += s[t + k];
         __syncthreads();
     }
-    const float m = (float)(s[0] / B);
-    __syncthreads();
-    for (int i = threadIdx.x; i < B; i += blockDim.x) den[i] = m;
+    if (t == 0) *m.out = (float)(s[0] / B);
 }
 
 // The layers' bias gradients: column sums gb[n] = sum_r d[r][n], r < R (fixed
-// order).  Block = 32 columns x 32 warps, layer by layer.
+// order).  Block = 32 columns x 32 warps, layer by layer; one block past them the
+// batch's loss.
 struct ColSums {
     const float *d[5];
     float *out[5];
     int n[5], end[5];  // columns; end of the layer's blocks
 };
-__global__ void __launch_bounds__(1024) colsum_kernel(const __grid_constant__ ColSums c, int R)
+__global__ void __launch_bounds__(1024) colsum_kernel(const __grid_constant__ ColSums c, int R, MeanLoss loss)
 {
+    if ((int)blockIdx.x == c.end[4]) {
+        extern __shared__ __align__(16) float ord_ring[];
+        mean_loss(loss, R, reinterpret_cast<double *>(ord_ring));
+        return;
+    }
     int g = 0;
     while ((int)blockIdx.x >= c.end[g]) g++;
     const int n = ((int)blockIdx.x - (g > 0 ? c.end[g - 1] : 0)) * 32 + threadIdx.x;
@@ -756,31 +812,6 @@ __global__ void loss_grad_kernel(const float *__restrict__ y, const float *__res
 #pragma unroll
     for (int k = 0; k < 8; k++)
         if (r0 + tx < B) dyt[(size_t)(i0 + ty + 8 * k) * B + r0 + tx] = __float2bfloat16_rn(tile[ty + 8 * k][tx]);
-}
-
-// row_err[r] = sum of the node tiles' errors / den[r]; with out set also their
-// mean over the batch (fixed order, one block).
-__global__ void __launch_bounds__(1024) row_err_kernel(const float *__restrict__ err_part, int tiles, int B, const float *__restrict__ den,
-                               float *__restrict__ row_err, float *__restrict__ out)
-{
-    __shared__ double s[1024];
-    double a = 0.0;
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < B; r += gridDim.x * blockDim.x) {
-        float e = 0.f;
-#pragma unroll 8
-        for (int k = 0; k < tiles; k++) e += __ldg(err_part + (size_t)k * B + r);
-        e /= fmaxf(den[r], 1e-30f);
-        row_err[r] = e;
-        a += e;
-    }
-    if (!out) return;
-    s[threadIdx.x] = a;
-    __syncthreads();
-    for (int k = blockDim.x / 2; k > 0; k >>= 1) {
-        if (threadIdx.x < k) s[threadIdx.x] += s[threadIdx.x + k];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *out = (float)(s[0] / B);
 }
 
 // Adam (decoupled weight decay) on the FP32 masters of all layers; writes the BF16
@@ -1066,16 +1097,21 @@ gd::GemmArgs args(int M, int N, int K, int *err)
 }
 
 // network input: per-cell scales and the BF16 cell-major copy of x (with train its
-// transpose too), and the sums of squares of d [n_out][ldd] into h->den when set
+// transpose too), and, when d [n_out][ldd] is set, the loss denominators of its
+// sums of squares in h->den
 int load_input(gd_mlp *h, const float *x, int ldx, int B, bool train, const float *d, int ldd, cudaStream_t st)
 {
+    const bool loss = d != nullptr;
     if (h->flags & GD_MLP_LOSS_MSE) d = nullptr;
     int rc = gd::launch_ordered(gd::cell_sums_kernel, dim3((B + 31) / 32, d ? 2 : 1), st, x, h->n_in, ldx,
                                 (int)(h->flags & GD_MLP_SCALE_INPUT), h->scale, d, h->n_out, ldd, h->den, B);
     if (rc) return rc;
-    dim3 blk(32, 8), grd((B + 31) / 32, h->n_in_p / 64);
+    const int mse = (h->flags & GD_MLP_LOSS_MSE) ? 1 : 0;
+    const gd::DenArgs den{loss ? h->den : nullptr, (h->flags & GD_MLP_SCALE_OUTPUT) ? 1 : 0, 1.f / h->out_gain, mse,
+                          h->n_out, !mse && (h->flags & GD_MLP_LOSS_BATCH)};
+    dim3 blk(32, 8), grd((B + 31) / 32, h->n_in_p / 64 + (loss ? 1 : 0));
     auto gather = train ? gd::gather_in_kernel<true> : gd::gather_in_kernel<false>;
-    gather<<<grd, blk, 0, st>>>(x, h->n_in, ldx, B, h->scale, h->in_gain, h->xb, h->xt, h->n_in_p);
+    gather<<<grd, blk, 0, st>>>(x, h->n_in, ldx, B, h->scale, h->in_gain, h->xb, h->xt, h->n_in_p, den);
     GD_CUDA(cudaGetLastError());
     return GD_OK;
 }
@@ -1103,7 +1139,7 @@ int forward(gd_mlp *h, int B, float *out, int ld_out, bool train, cudaStream_t s
     if ((rc = gemm_nt(EPI_NONE, h->xb, h->L[0].wb, a, st))) return rc;
     a = args(B, 512, 256, h->err);
     a.bias = h->L[1].b;
-    a.pre_out = h->a1;
+    a.pre_out = train ? h->a1 : nullptr;
     a.ld32 = 512;
     a.c16 = h->h1b;
     a.ld16 = 512;
@@ -1111,7 +1147,7 @@ int forward(gd_mlp *h, int B, float *out, int ld_out, bool train, cudaStream_t s
     if ((rc = gemm_nt(EPI_GELU, h->h0b, h->L[1].wb, a, st))) return rc;
     a = args(B, 512, 512, h->err);
     a.bias = h->L[2].b;
-    a.pre_out = h->a2;
+    a.pre_out = train ? h->a2 : nullptr;
     a.ld32 = 512;
     a.c16 = h->h2b;
     a.ld16 = 512;
@@ -1140,7 +1176,8 @@ int forward(gd_mlp *h, int B, float *out, int ld_out, bool train, cudaStream_t s
     return gemm_nt(EPI_NONE, h->zb, h->L[4].wb, a, st);
 }
 
-int backward(gd_mlp *h, int B, cudaStream_t st)
+// all gradients; the batch's mean loss into loss when set
+int backward(gd_mlp *h, int B, float *loss, cudaStream_t st)
 {
     using namespace gd;
     int rc;
@@ -1199,24 +1236,21 @@ int backward(gd_mlp *h, int B, cudaStream_t st)
         cs.end[k] = (k > 0 ? cs.end[k - 1] : 0) + (l.out + 31) / 32;
     }
     if ((rc = gemm_nt<5>(EPI_NONE, pr, st))) return rc;
-    return launch_ordered(colsum_kernel, dim3(cs.end[4]), st, cs, B);
+    const MeanLoss ml{h->err_part, h->n_out_p / 64, h->den, h->row_err, loss};
+    return launch_ordered(colsum_kernel, dim3(cs.end[4] + (loss ? 1 : 0)), st, cs, B, ml);
 }
 
-// loss and output gradient for targets t (the sums of squares for the
-// denominators in h->den); the batch's mean loss into loss when set
-int loss_grad(gd_mlp *h, const float *t, int ldt, int B, bool train, float *loss, cudaStream_t st)
+// output gradient for targets t (the denominators in h->den) and the loss's parts;
+// without train the cells' losses
+int loss_grad(gd_mlp *h, const float *t, int ldt, int B, bool train, cudaStream_t st)
 {
     const int pw = (h->flags & GD_MLP_SCALE_OUTPUT) ? 1 : 0;
-    const int mse = (h->flags & GD_MLP_LOSS_MSE) ? 1 : 0;
     const float inv_gain = 1.f / h->out_gain;
-    gd::den_kernel<<<1, 256, 0, st>>>(h->den, B, h->scale, pw, inv_gain, mse, h->n_out,
-                                      !mse && (h->flags & GD_MLP_LOSS_BATCH));
     dim3 blk(32, 8), grd((B + 31) / 32, h->n_out_p / 64);
     gd::loss_grad_kernel<<<grd, blk, 0, st>>>(h->y, t, ldt, h->n_out, h->n_out_p, B, h->scale, pw, inv_gain, h->den,
                                               h->dy, h->dyb, train ? h->dyt : nullptr, h->err_part);
-    if (loss || !train)
-        gd::row_err_kernel<<<loss ? 1 : (B + 1023) / 1024, 1024, 0, st>>>(h->err_part, h->n_out_p / 64, B, h->den,
-                                                                       h->row_err, loss);
+    if (!train)
+        gd::row_err_kernel<<<(B + 1023) / 1024, 1024, 0, st>>>(h->err_part, h->n_out_p / 64, B, h->den, h->row_err);
     GD_CUDA(cudaGetLastError());
     return GD_OK;
 }
@@ -1415,9 +1449,9 @@ extern "C" int gd_mlp_train_step(gd_mlp *h, const float *x, int ldx, const float
     cudaStream_t st = (cudaStream_t)stream;
     int rc = load_input(h, x, ldx, batch, true, tden ? tden : t, tden ? ldd : ldt, st);
     if (!rc) rc = forward(h, batch, nullptr, 0, true, st);
-    if (!rc) rc = loss_grad(h, t, ldt, batch, true, loss, st);
+    if (!rc) rc = loss_grad(h, t, ldt, batch, true, st);
     if (rc) return rc;
-    if ((rc = backward(h, batch, st))) return rc;
+    if ((rc = backward(h, batch, loss, st))) return rc;
     h->step++;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     const float c1 = 1.f - (float)std::pow(0.9, (double)h->step), c2 = 1.f - (float)std::pow(0.999, (double)h->step);
@@ -1452,7 +1486,7 @@ extern "C" int gd_mlp_loss(gd_mlp *h, const float *x, int ldx, const float *t, i
     cudaStream_t st = (cudaStream_t)stream;
     int rc = load_input(h, x, ldx, batch, false, tden ? tden : t, tden ? ldd : ldt, st);
     if (!rc) rc = forward(h, batch, nullptr, 0, false, st);
-    if (!rc) rc = loss_grad(h, t, ldt, batch, false, nullptr, st);
+    if (!rc) rc = loss_grad(h, t, ldt, batch, false, st);
     if (rc) return rc;
     GD_CUDA(cudaMemcpyAsync(row_loss, h->row_err, (size_t)batch * sizeof(float), cudaMemcpyDeviceToDevice, st));
     return GD_OK;
