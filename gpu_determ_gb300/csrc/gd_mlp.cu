@@ -103,7 +103,8 @@ __device__ __forceinline__ void epilogue_value(const GemmArgs &p, size_t o32, fl
 // that its lanes hold 32 columns of a row and every access of C and of the added or
 // multiplied arrays is one segment (a row per lane before: 32 segments of 16 bytes);
 // the added or multiplied values are requested before the accumulator is awaited.
-template <int EPI, int GN, int G>
+// TR: c16t is written.
+template <int EPI, int GN, int G, bool TR>
 __global__ void __launch_bounds__(kGThreads, 1) gemm_nt_kernel(const __grid_constant__ GemmSet<G> set)
 {
     // K, the stages, err and the test hook are the first product's
@@ -293,11 +294,11 @@ __global__ void __launch_bounds__(kGThreads, 1) gemm_nt_kernel(const __grid_cons
                             epilogue_value<EPI>(p, (size_t)(mw + r) * p.ld32 + n, bias, extra[r], x);
                             if (p.c32) p.c32[(size_t)(mw + r) * p.ld32 + n] = x;
                             if (p.c16) p.c16[(size_t)(mw + r) * p.ld16 + n] = __float2bfloat16_rn(x);
-                            if (p.c16t) tile[r * 33 + lane] = x;
+                            if (TR) tile[r * 33 + lane] = x;
                         }
                     }
                     __syncwarp();
-                    if (p.c16t) {
+                    if (TR) {
 #pragma unroll
                         for (int j = 0; j < 32; j++)
                             if (n0 + c0 + j < p.N && m < p.M)
@@ -925,8 +926,12 @@ int launch_gemm(const Product *pr, int kps, int stages, int ctas, cudaStream_t s
         set.end[g] = end += (pr[g].a.M + GM - 1) / GM * ((pr[g].a.N + GN - 1) / GN);
     }
     const size_t smem = gemm_smem(GN, stages * kps);
-    GD_CUDA(cudaFuncSetAttribute(gemm_nt_kernel<EPI, GN, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    gemm_nt_kernel<EPI, GN, G><<<std::min(end, ctas), kGThreads, smem, st>>>(set);
+    // one product, not the output's layout: with or without the transpose
+    auto kern = gemm_nt_kernel<EPI, GN, G, false>;
+    if constexpr (G == 1 && EPI != EPI_NODE)
+        if (pr[0].a.c16t) kern = gemm_nt_kernel<EPI, GN, G, true>;
+    GD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<std::min(end, ctas), kGThreads, smem, st>>>(set);
     GD_CUDA(cudaGetLastError());
     return GD_OK;
 }
