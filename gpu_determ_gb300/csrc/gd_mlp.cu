@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(kGThreads, 1) gemm_nt_kernel(const __grid_cons
     } else if (warp == 0) {
         if (lane == 0) {
             bool ok = true;
-            int s = 0;
+            int s = 0, issued = 0;
             uint32_t ph = 0;
             for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
                 int g, m0, n0;
@@ -191,12 +191,18 @@ __global__ void __launch_bounds__(kGThreads, 1) gemm_nt_kernel(const __grid_cons
                         tma_load_2d(st, &set.a[g], (k + q) * GK, m0, fb);
                         tma_load_2d(st + kA, &set.b[g], (k + q) * GK, n0, fb);
                     }
+                    issued++;
                     if (++s == GS) {
                         s = 0;
                         ph ^= 1u;
                     }
                 }
             }
+            // after a time-out the copies in flight land (or this wait gives up too)
+            // before the CTA leaves; otherwise the accumulators were waited for
+            if (!ok || *(volatile int *)p.err)
+                for (int j = max(0, issued - GS); j < issued; j++)
+                    mbar_wait(smem_u32(&full_bar[j % GS]), (uint32_t)(j / GS) & 1u, p.err);
         }
     } else if (warp == 1) {
         if (lane == 0) {
