@@ -299,7 +299,7 @@ extern "C" int gd_batch_info(const gd_batch *b, int *groups, int *streams, int *
 // Autotuner: times the gain launch candidates of one context on the caller's
 // cells and keeps the fastest.  Candidates: the FP32 pair kernel with 1, 2 or
 // 4 CTAs per SM as the minimum s-chunk fill (trading partial-sum traffic for
-// parallelism), the pair formulation with its contraction on the tensor cores
+// parallelism; one and the same launch on lattices with orbit tables), the pair formulation with its contraction on the tensor cores
 // (when its per-class-box weight table fits the memory budget), and the
 // tensor-core collision matrices in BF16x3 and BF16 mode, each with 1 or 2
 // CTAs per MMA (2: CTA-pair MMA, M = 256 cells), when the caller's mask admits

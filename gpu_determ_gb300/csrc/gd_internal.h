@@ -63,15 +63,16 @@ struct OrbitGain {
     int cpt = 8, nslot = 0, norb = 0, pcap = 0, mcap = 0, nsteps = 0;
     uint32_t p_at = 0, zero_at = 0;  // shared-memory offsets of the P rows and of the zero C row
     size_t smem = 0, stream_bytes = 0;
+    int nparts = 0;                   // parts of the walk: each is summed by itself, in any batch
     std::vector<int> cuts;            // steps between which the walk may be cut (no D continues)
     std::vector<double> cost_prefix;  // work before each cut
     int *row_node = nullptr;          // [n_pnt]
     uint4 *stream = nullptr;
-    int *start = nullptr;  // [step][warp] position in the stream, in 16-byte units
+    int *start = nullptr;  // [part][warp] position in the stream, in 16-byte units
     int *err = nullptr;    // set by the kernel when a copy of the stream is not seen to land
     int opad = 0;               // orbits padded to the loss kernel's tile
     float *bx = nullptr;        // [8][o'][opad] loss matrices folded by the reflections' characters
-    std::map<int, int *> bounds_dev;
+    int *bounds = nullptr;      // [nparts + 1] their bounds in steps
 };
 
 // Floats of a context's reduction buffer (block maxima of nu', then dt).
@@ -219,17 +220,14 @@ int reduce_gain_partials(Context &c, const float *part, int nchunks, int cells_p
                          float *gain, cudaStream_t st);
 
 // FP32 gain with all eight reflections of a pair sum at once (gd_orbit.cu):
-// tables (built with the context), chunk count and bounds, buffer sizes, and
-// the launch into a caller-provided buffer (packed f, then chunk partials)
+// tables (built with the context), bytes of a batch's buffer, cells per launch in a
+// given room, and the launch into a caller-provided buffer
 int orbit_build(Context &c);
 int fold_loss_build(Context &c);  // its loss matrices (gd_loss.cu)
 void orbit_free(Context &c);
-int orbit_chunks(const Context &c, int ncells);
-void orbit_chunk_bounds(const Context &c, int nchunks, int *bounds);
-size_t orbit_pack_bytes(const Context &c, int ncells);
-size_t orbit_part_bytes(const Context &c, int ncells, int nchunks);
-int launch_orbit(Context &c, const float *f, int ncells, int ld, float *gain, void *buf, int nchunks,
-                 const int *d_bounds, float2 *scale, cudaStream_t st);
+size_t orbit_bytes(const Context &c, int ncells);
+int orbit_slice(const Context &c, int ncells, size_t room);
+int launch_orbit(Context &c, const float *f, int ncells, int ld, float *gain, void *buf, float2 *scale, cudaStream_t st);
 int run_orbit(Context &c, const float *f, int ncells, int ld, float *gain, bool guard, cudaStream_t st);
 bool orbit_serves(const Context &c, int path);  // whether run_orbit computes this path's gain
 // reads (synchronising st) and clears its pipeline time-out record

@@ -20,10 +20,11 @@
 // start-up.  Later calls only launch kernels and clear the partial sums with
 // cudaMemsetAsync.
 //
-// The chunking of the s walk is the one gd_collision picks when it fits the
-// array (at most kMaxChunks chunks); then the result is bitwise that of
-// gd_collision's FP32 pair gain.  When it does not fit, fewer chunks are
-// used, and the sums agree within FP32 rounding of the other order.
+// On lattices with orbit tables (gd_orbit.cu) the result is bitwise that of
+// gd_collision's FP32 gain, in slices of cells that fit the array.  On the others
+// the chunking of the s walk is the one gd_collision picks when it fits the
+// array (at most kMaxChunks chunks), and so are the bits; when it does not fit,
+// fewer chunks are used, and the sums agree within FP32 rounding of the other order.
 //
 // All calls share the one array and it keeps the last call's contents; the
 // partial sums are cleared at the start of every call.  Calls whose work
@@ -77,19 +78,6 @@ int scratch_address(int dev, void **out)
     return GD_OK;
 }
 
-// The array's address and, in its header, the chunk bounds of this call.
-int noalloc_bounds(Context &c, int nchunks, void (*fill)(const Context &, int, int *), cudaStream_t st, void **base)
-{
-    int rc = scratch_address(c.device, base);
-    if (rc) return rc;
-    ChunkBounds b{};
-    b.n = nchunks;
-    fill(c, nchunks, b.v);
-    write_bounds_kernel<<<1, kMaxChunks + 1, 0, st>>>(b, static_cast<int *>(*base));
-    GD_CUDA(cudaGetLastError());
-    return GD_OK;
-}
-
 }  // namespace
 }  // namespace gd
 
@@ -124,20 +112,28 @@ extern "C" int gd_gain_noalloc(gd_ctx *ctx, const float *f, int ncells, int ld, 
             break;
         }
         if (c.orbit) {
-            // the packed f and the partial sums of as many chunks as fit (one
-            // chunk writes the gain itself, and its packed f fits wherever one
-            // chunk's partial sums do)
-            int nchunks = std::min(orbit_chunks(c, ncells), kMaxChunks);
-            while (nchunks > 1 && orbit_pack_bytes(c, ncells) + orbit_part_bytes(c, ncells, nchunks) > room) nchunks--;
-            if ((rc = noalloc_bounds(c, nchunks, orbit_chunk_bounds, st, &base))) break;
-            rc = launch_orbit(c, f, ncells, ld, gain, static_cast<unsigned char *>(base) + kHeaderBytes, nchunks,
-                              static_cast<const int *>(base), nullptr, st);
+            // gd_collision's sums, in slices of cells that fit (a tile of cells
+            // does: its rows, for f and at most 152 parts of the walk, are 20 MB)
+            if ((rc = scratch_address(c.device, &base))) break;
+            const int slice = orbit_slice(c, ncells, room);
+            for (int at = 0; at < ncells && !rc; at += slice)
+                rc = launch_orbit(c, f + at, std::min(slice, ncells - at), ld, gain + at,
+                                  static_cast<unsigned char *>(base) + kHeaderBytes, nullptr, st);
             break;
         }
         const int nchunks = std::min(want, fit);
-        if ((rc = noalloc_bounds(c, nchunks, gain_chunk_bounds, st, &base))) break;
+        if ((rc = scratch_address(c.device, &base))) break;
+        int *d_bounds = static_cast<int *>(base);
         float *part = reinterpret_cast<float *>(static_cast<unsigned char *>(base) + kHeaderBytes);
-        const int *d_bounds = static_cast<const int *>(base);
+        ChunkBounds b{};
+        b.n = nchunks;
+        gain_chunk_bounds(c, nchunks, b.v);
+        write_bounds_kernel<<<1, kMaxChunks + 1, 0, st>>>(b, d_bounds);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) {
+            rc = cuda_error(e, "write_bounds_kernel");
+            break;
+        }
         rc = launch_gain_pair(c, f, ncells, ld, gain, part, nchunks, d_bounds, cb, smem, st);
     } while (0);
     if (prev >= 0 && prev != c.device) cudaSetDevice(prev);

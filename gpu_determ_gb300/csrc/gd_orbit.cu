@@ -16,13 +16,15 @@
 //    it and weights of absent products are not in the tables (20^3, R = 4.8:
 //    3.0e6 products, 2.4e6 group rows and 4.1e7 weight terms per cell; the class
 //    boxes hold 9.3e6, 3.9e6 and 1.4e8).
-//  - The outputs stay in registers for a whole chunk of the walk: a warp
+//  - The outputs stay in registers for a whole part of the walk: a warp
 //    owns groups of four neighbouring orbits and reads each C row once per
 //    target.  No output
 //    is read back or written in between, and no two warps share one, so every
 //    sum has a fixed order and results are bitwise reproducible.
 //
-// A CTA takes one tile of CPT cells and one chunk of the steps.  f of the tile,
+// The walk is cut into parts of about equal work, the same for every batch, and the
+// parts' sums are added in a fixed order: a cell's gain has the same bits alone and
+// in any batch.  A CTA takes one tile of CPT cells and one part.  f of the tile,
 // the P rows and the C rows of a step sit in shared memory.  A step is as many D
 // as fit these rows, or a part of one D's offsets (by shell |n|, its C rows then
 // accumulate over the parts).  Contraction works on blocks of four rows of
@@ -38,8 +40,10 @@
 // operation, the outputs' phase at the rate of the load unit) for 60 % of the
 // time, the rest the warps' own control flow, some 400 instructions per warp and
 // step.  It replaces gain_pair_kernel (gd_gain.cu) on every lattice whose rows
-// fit: 12^3 (R = 4.8), 1501 cells 20.3 -> 1.30 ms; 16^3 (whole box), 256 cells
-// 22.6 -> 3.82 ms; 20^3 (R = 4.8), one cell 10.5 -> 0.18 ms, 4096 cells 67.5 ms;
+// fit: 12^3 (R = 4.8), 1501 cells 20.3 -> 1.40 ms; 16^3 (whole box), 256 cells
+// 22.6 -> 3.83 ms; 20^3 (R = 4.8), one cell 10.5 -> 0.18 ms, 4096 cells 70.6 ms
+// (as many parts as the batch needs to fill the chip: 1.28, 3.79, 0.18 and 67.2 ms,
+// but other bits in other batches);
 // its error against FP64 is half as large (two-level sums: targets of a step,
 // then steps).  Measured and not better: 8, 12, 20 or 24 warps; groups of eight
 // slots with one target a round (73.4 ms at 20^3); chunk-free dense streams (78 ms:
@@ -65,21 +69,22 @@ constexpr uint32_t kOBars = kOWarps * kORing;    // offset of the rings' barrier
 constexpr uint32_t kOF = kOBars + 1024;          // offset of f
 constexpr uint32_t kOQuad = 80;                  // bytes of a contraction quad
 constexpr int kOMatrixNodes = 512;               // BF16x3 matrices stay below this (orbit_serves)
-constexpr int kOSlice = 65536;                   // cells of one launch of the guarded gain: n_pnt of them stay below 2^31
+constexpr size_t kOScratch = (size_t)2 << 30;    // scratch of a launch: larger batches run in slices of cells
 constexpr int kOSlots = 4;                       // output slots gathered side by side
+constexpr int kOParts = 152;                     // parts of the walk, each summed by itself (orbit_build)
 constexpr int kOGroup = 16;                      // rounds (two targets per slot, 32 bytes) of a group in a step: at most a chunk
 
 struct OrbitArgs {
     const float *ft;              // [tile][row][CPT]
     const unsigned char *stream;  // per warp: the chunks of every step
-    const int *start;             // [step][warp] first chunk
-    const int *bounds;            // [chunks + 1] step bounds
+    const int *start;             // [part][warp] position of its stream, in 16-byte units
+    const int *bounds;            // [parts + 1] step bounds
     const int *row_node;
-    float *part;                  // [chunk][row][cells_pad], or null: write gain
+    float *part;                  // [part][tile][row][CPT], or null (one part): write gain
     float *gain;
     const float2 *scale;          // [cells_pad] power-of-two factors of f and back, or null
     int *err;                     // set to 1 when a copy is not seen to land
-    int norb, ns, cells_pad, ncells, ld;
+    int norb, ns, ncells, ld;
     uint32_t p_at, zero_at;       // shared-memory offsets of the P rows and of the zero C row
 };
 
@@ -187,7 +192,16 @@ __global__ void __launch_bounds__(kOThreads, 1) orbit_gain_kernel(const __grid_c
     const int r = lane >> 2;
     const uint32_t sm = (uint32_t)__cvta_generic_to_shared(smem), slb = sm + lb;
 
+    // f of the tile, and eight zero rows, on their way before anything else
+    const float *ft = a.ft + (size_t)blockIdx.x * a.ns * CPT;
+    for (int i = threadIdx.x; i < (a.ns + 8) * CPT / 4; i += kOThreads) {
+        if (i < a.ns * CPT / 4)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sm + kOF + i * 16), "l"(ft + 4 * i) : "memory");
+        else
+            *reinterpret_cast<float4 *>(smem + kOF + i * 16) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
     const int s0 = a.bounds[blockIdx.y], s1 = a.bounds[blockIdx.y + 1];
+    const uint32_t first = (uint32_t)__ldg(a.start + blockIdx.y * kOWarps + warp) * 16u;
     if (s0 < s1) {
         const uint32_t ring = sm + warp * kORing, bar = sm + kOBars + warp * 32;
         if (lane == 0) {
@@ -196,7 +210,6 @@ __global__ void __launch_bounds__(kOThreads, 1) orbit_gain_kernel(const __grid_c
         }
         __syncwarp();
         // the ring: chunk c sits at (c % 4) chunks
-        const uint32_t first = (uint32_t)__ldg(a.start + s0 * kOWarps + warp) * 16u;
         const unsigned char *src = a.stream + (first & ~(kOChunk - 1));
         uint32_t issued = 0, taken = 0;
         uint32_t at = 0, room = 0;  // the stream's position, and the bytes to its chunk's end
@@ -232,15 +245,13 @@ __global__ void __launch_bounds__(kOThreads, 1) orbit_gain_kernel(const __grid_c
             room -= bytes;
         };
         for (int k = 0; k < 3; k++) fetch();
-        const float4 *ft = reinterpret_cast<const float4 *>(a.ft + (size_t)blockIdx.x * a.ns * CPT);
-        for (int i = threadIdx.x; i < (a.ns + 8) * CPT / 4; i += kOThreads)
-            *reinterpret_cast<float4 *>(smem + kOF + i * 16) = i < a.ns * CPT / 4 ? __ldg(ft + i) : make_float4(0.f, 0.f, 0.f, 0.f);
         if (warp == 0) sts(slb + a.zero_at, V::zero());  // padding targets read this row
         need(1);
         skip(first & (kOChunk - 1));
         T acc[NSLOT];
 #pragma unroll
         for (int j = 0; j < NSLOT; j++) acc[j] = V::zero();
+        asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
 
         // C rows of a step into this warp's outputs: a count of rounds per group of
@@ -400,12 +411,13 @@ __global__ void __launch_bounds__(kOThreads, 1) orbit_gain_kernel(const __grid_c
         if (!ok) return;  // recorded in err
         // lane (r, cells): output row 8 o + r
         const int cell = blockIdx.x * CPT + (lane & 3) * (CPT / 4);
+        float *part = a.part + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * (size_t)(a.ns * CPT) + (lane & 3) * (CPT / 4);
 #pragma unroll
         for (int j = 0; j < NSLOT; j++) {
             const int o = (j / kOSlots * kOWarps + warp) * kOSlots + j % kOSlots;
             if (o >= a.norb) continue;
             if (a.part) {
-                *reinterpret_cast<T *>(a.part + ((size_t)blockIdx.y * a.ns + 8 * o + r) * a.cells_pad + cell) = acc[j];
+                *reinterpret_cast<T *>(part + (8 * o + r) * CPT) = acc[j];
             } else {
                 float *g = a.gain + (size_t)__ldg(a.row_node + 8 * o + r) * a.ld + cell;
                 const float *v = reinterpret_cast<const float *>(&acc[j]);
@@ -414,9 +426,10 @@ __global__ void __launch_bounds__(kOThreads, 1) orbit_gain_kernel(const __grid_c
                     if (cell + q < a.ncells) g[q] = a.scale ? unscale(v[q], a.scale[cell + q].y) : v[q];
             }
         }
-    } else if (a.part) {  // an empty chunk (more chunks than work): zero partial sums
-        for (int t = threadIdx.x; t < a.ns * CPT; t += kOThreads)
-            a.part[((size_t)blockIdx.y * a.ns + t / CPT) * a.cells_pad + blockIdx.x * CPT + t % CPT] = 0.f;
+    } else {  // a part without steps (more parts than work): zero sums
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        float *part = a.part + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * (size_t)(a.ns * CPT);
+        for (int t = threadIdx.x; t < a.ns * CPT; t += kOThreads) part[t] = 0.f;
     }
 }
 
@@ -458,54 +471,40 @@ __global__ void orbit_pack_kernel(const float *__restrict__ f, int ld, int ncell
     ft[((size_t)(cell / cpt) * ns + row) * cpt + cell % cpt] = v;
 }
 
-// gain[node][cell] = sum over the chunks: each of the block's eight y rows adds
-// a contiguous eighth of the chunks in order, and the eight are added in order.
-__global__ void orbit_reduce_kernel(const float *__restrict__ part, int nchunks, int ns, int cells_pad, int ncells,
-                                    int ld, const int *__restrict__ row_node, const float2 *__restrict__ scale,
-                                    float *__restrict__ gain)
+// gain[node][cell] = sum over the parts of [part][tile][row][cpt]: each of the block's
+// eight y rows adds a contiguous eighth of the parts in order, four cells of a row
+// per thread, and the eight are added in order.
+__global__ void __launch_bounds__(256) orbit_reduce_kernel(const float4 *__restrict__ part, int nparts, int ns, int cpt,
+                                                           int ncells, int ld, const int *__restrict__ row_node,
+                                                           const float2 *__restrict__ scale, float *__restrict__ gain)
 {
-    __shared__ float red[8][32];
-    const int x = threadIdx.x, y = threadIdx.y;
-    const int o = blockIdx.x * 32 + x;
-    const int total = ns * ncells;
-    const int row = o < total ? o / ncells : 0, cell = o < total ? o - row * ncells : 0;
-    const int k0 = nchunks * y / 8, k1 = nchunks * (y + 1) / 8;
-    const float *p = part + (size_t)row * cells_pad + cell;
-    const size_t step = (size_t)ns * cells_pad;
-    float s = 0.f;
-#pragma unroll 4
-    for (int k = k0; k < k1; k++) s += __ldg(p + (size_t)k * step);
-    red[y][x] = s;
-    __syncthreads();
-    if (y == 0 && o < total) {
-        for (int k = 1; k < 8; k++) s += red[k][x];
-        gain[(size_t)__ldg(row_node + row) * ld + cell] = scale ? unscale(s, scale[cell].y) : s;
-    }
-}
-
-// The same for at most kOFewChunks chunks: a thread per row and four cells adds
-// them in order, all its loads in flight (16^3, 500 cells, 12 chunks: 45 -> 14 us).
-constexpr int kOFewChunks = 16;
-__global__ void __launch_bounds__(256) orbit_reduce_few_kernel(const float *__restrict__ part, int nchunks, int ns,
-                                                               int cells_pad, int ncells, int ld,
-                                                               const int *__restrict__ row_node,
-                                                               const float2 *__restrict__ scale,
-                                                               float *__restrict__ gain)
-{
-    const int cell = 4 * (blockIdx.x * 32 + threadIdx.x), row = blockIdx.y * 8 + threadIdx.y;
-    if (cell >= ncells || row >= ns) return;  // ns is a multiple of 8, cells_pad of 4
-    const float4 *p = reinterpret_cast<const float4 *>(part + (size_t)row * cells_pad + cell);
-    const size_t step = (size_t)ns * cells_pad / 4;
-    float4 s = __ldg(p);
+    __shared__ float4 red[8][32];
+    const int x = threadIdx.x, y = threadIdx.y, per = cpt / 4, n = ns * per;  // quads of a row, of a tile
+    const int i = blockIdx.y * 32 + x, tile = blockIdx.x;
+    const int k0 = nparts * y / 8, k1 = nparts * (y + 1) / 8;
+    const size_t step = (size_t)gridDim.x * n;
+    const float4 *p = part + (size_t)tile * n + min(i, n - 1);
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 8
-    for (int k = 1; k < nchunks; k++) {
+    for (int k = k0; k < k1; k++) {
         const float4 v = __ldg(p + (size_t)k * step);
         s.x += v.x;
         s.y += v.y;
         s.z += v.z;
         s.w += v.w;
     }
-    float *g = gain + (size_t)__ldg(row_node + row) * ld + cell;
+    red[y][x] = s;
+    __syncthreads();
+    if (y != 0 || i >= n) return;
+    for (int k = 1; k < 8; k++) {
+        const float4 v = red[k][x];
+        s.x += v.x;
+        s.y += v.y;
+        s.z += v.z;
+        s.w += v.w;
+    }
+    const int cell = tile * cpt + i % per * 4;
+    float *g = gain + (size_t)__ldg(row_node + i / per) * ld + cell;
     const float o[4] = {s.x, s.y, s.z, s.w};
 #pragma unroll
     for (int q = 0; q < 4; q++)
@@ -563,9 +562,32 @@ void orbit_free(Context &c)
     cudaFree(g->start);
     cudaFree(g->bx);
     cudaFree(g->err);
-    for (auto &kv : g->bounds_dev) cudaFree(kv.second);
+    cudaFree(g->bounds);
     delete g;
     c.orbit = nullptr;
+}
+
+// Bounds in steps of the walk's parts, of about equal work.  A part costs a large
+// batch some 5 us (start of its CTA, its sums stored and added) and a single cell
+// waits for the longest one, so their number goes with the root of the work, up to a
+// wave of CTAs.  Measured with 38, 76, 114 and 152 parts: 20^3, one cell 625, 325,
+// 225, 176 us, 4096 cells 68.3, 69.2, 70.5, 71.4 ms (152 now 70.6); 16^3, one cell
+// 148, 90, 70, 58 us, 1024 cells 4.11, 4.29, 4.45, 4.64 ms; 12^3, one cell 51, 38,
+// 36, 31 us, 1501 cells 1.44, 1.58, 1.73, 1.75 ms.
+static void orbit_parts(const OrbitGain &g, double cost, std::vector<int> &bounds)
+{
+    const std::vector<double> &pre = g.cost_prefix;
+    const int n = (int)g.cuts.size() - 1;
+    const int nparts = std::min(n, std::max(1, (int)(kOParts * std::min(1.0, std::sqrt(cost / 7e6)))));
+    bounds.assign(1, 0);
+    for (int k = 1, at = 0; k < nparts; k++) {
+        const double want = pre[n] * k / nparts;
+        int b = (int)(std::lower_bound(pre.begin(), pre.end(), want) - pre.begin());
+        if (b > 0 && want - pre[b - 1] < pre[b] - want) b--;
+        at = std::min(n, std::max(at, b));
+        bounds.push_back(g.cuts[at]);
+    }
+    bounds.push_back(g.nsteps);
 }
 
 // Tables of the orbit kernel; leaves c.orbit null (the pair kernel of
@@ -991,66 +1013,37 @@ int orbit_build(Context &c)
     c.orbit = og;
     int rc = upload(&og->row_node, row_node);
     if (!rc) rc = upload(&og->stream, stream);
-    if (!rc) rc = upload(&og->start, st);
+    std::vector<int> bounds, first;
+    orbit_parts(*og, cost, bounds);
+    for (int k = 0; k + 1 < (int)bounds.size(); k++)
+        for (int w = 0; w < kOWarps; w++) first.push_back(st[(size_t)std::min(bounds[k], og->nsteps - 1) * kOWarps + w]);
+    og->nparts = (int)bounds.size() - 1;
+    if (!rc) rc = upload(&og->bounds, bounds);
+    if (!rc) rc = upload(&og->start, first);
     if (!rc) rc = upload(&og->err, std::vector<int>(1, 0));
     if (!rc) rc = fold_loss_build(c);
     return rc;  // the caller destroys the context on failure
 }
 
-// Chunks of the steps for a batch: at least gain_waves CTAs per SM (a CTA
-// fills an SM), and of the next few counts the one whose last wave is fullest.
-int orbit_chunks(const Context &c, int ncells)
+// bytes of packed f and of the parts' sums (one part writes the gain itself)
+size_t orbit_bytes(const Context &c, int ncells)
 {
     const OrbitGain &g = *c.orbit;
-    const int tiles = (ncells + g.cpt - 1) / g.cpt, sms = std::max(1, c.sm_count);
-    const int most = (int)g.cuts.size() - 1;
-    const int lo = std::min(most, std::max(1, (std::max(1, c.gain_waves) * sms + tiles - 1) / tiles));
-    int best = lo;
-    double best_fill = 0.0;
-    for (int k = lo; k <= std::min(most, lo + 8); k++) {
-        const int64_t ctas = (int64_t)tiles * k;
-        const double fill = (double)ctas / (double)((ctas + sms - 1) / sms * sms) - 0.002 * (k - lo);
-        if (fill > best_fill + 1e-9) {
-            best_fill = fill;
-            best = k;
-        }
-    }
-    return best;
+    return (size_t)((ncells + g.cpt - 1) / g.cpt * g.cpt) * c.d.n_pnt * sizeof(float) * (g.nparts > 1 ? 1 + g.nparts : 1);
 }
 
-size_t orbit_pack_bytes(const Context &c, int ncells)
+// Cells of a launch for a batch of ncells in at most `room` bytes (a tile at
+// least): equal slices of whole tiles.
+int orbit_slice(const Context &c, int ncells, size_t room)
 {
-    const int cpt = c.orbit->cpt;
-    return (size_t)((ncells + cpt - 1) / cpt * cpt) * c.d.n_pnt * sizeof(float);
+    const int cpt = c.orbit->cpt, tiles = (ncells + cpt - 1) / cpt;
+    const int fit = (int)std::min<size_t>(std::max<size_t>(1, room / orbit_bytes(c, cpt)), tiles), slices = (tiles + fit - 1) / fit;
+    return (tiles + slices - 1) / slices * cpt;
 }
 
-// partial sums of nchunks chunks (one chunk writes the gain itself)
-size_t orbit_part_bytes(const Context &c, int ncells, int nchunks)
-{
-    return nchunks > 1 ? orbit_pack_bytes(c, ncells) * (size_t)nchunks : 0;
-}
-
-void orbit_chunk_bounds(const Context &c, int nchunks, int *bounds)
-{
-    const OrbitGain &g = *c.orbit;
-    const std::vector<double> &pre = g.cost_prefix;
-    const int n = (int)g.cuts.size() - 1;
-    int at = 0;
-    bounds[0] = 0;
-    for (int k = 1; k < nchunks; k++) {
-        const double want = pre[n] * k / nchunks;
-        int b = (int)(std::lower_bound(pre.begin(), pre.end(), want) - pre.begin());
-        if (b > 0 && want - pre[b - 1] < pre[b] - want) b--;
-        at = std::min(n, std::max(at, b));
-        bounds[k] = g.cuts[at];
-    }
-    bounds[nchunks] = g.nsteps;
-}
-
-// buf holds orbit_pack_bytes + orbit_part_bytes; scale is null or one entry per
+// buf holds orbit_bytes; scale is null or one entry per
 // cell of the padded tiles.
-int launch_orbit(Context &c, const float *f, int ncells, int ld, float *gain, void *buf, int nchunks,
-                 const int *d_bounds, float2 *scale, cudaStream_t st)
+int launch_orbit(Context &c, const float *f, int ncells, int ld, float *gain, void *buf, float2 *scale, cudaStream_t st)
 {
     OrbitGain &g = *c.orbit;
     const Dims &d = c.d;
@@ -1058,7 +1051,8 @@ int launch_orbit(Context &c, const float *f, int ncells, int ld, float *gain, vo
     if ((int64_t)d.n_pnt * (scale ? cells_pad : std::max(ld, cells_pad)) >= ((int64_t)1 << 31))
         return set_error(GD_ERR_UNSUPPORTED, "pair gain: n_pnt * ld must stay below 2^31");
     float *ft = static_cast<float *>(buf);
-    float *part = nchunks > 1 ? ft + (size_t)cells_pad * d.n_pnt : nullptr;
+    const int nparts = g.nparts;
+    float *part = nparts > 1 ? ft + (size_t)cells_pad * d.n_pnt : nullptr;
     if (scale) {
         orbit_scale_kernel<<<(cells_pad + 31) / 32, dim3(32, 32), 0, st>>>(f, ld, ncells, d.n_pnt, scale, cells_pad);
         GD_CUDA(cudaGetLastError());
@@ -1067,21 +1061,16 @@ int launch_orbit(Context &c, const float *f, int ncells, int ld, float *gain, vo
         f, ld, ncells, d.n_pnt, g.cpt, g.row_node, scale, ft, cells_pad);
     GD_CUDA(cudaGetLastError());
     const OrbitArgs a{ft,    reinterpret_cast<const unsigned char *>(g.stream),
-                      g.start, d_bounds, g.row_node, part, gain, scale, g.err, g.norb, d.n_pnt, cells_pad, ncells, ld,
+                      g.start, g.bounds, g.row_node, part, gain, scale, g.err, g.norb, d.n_pnt, ncells, ld,
                       g.p_at, g.zero_at};
     int nslot = 0;
     OrbitKernel kern = orbit_kernel(g.cpt, g.nslot, &nslot);
     GD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
-    kern<<<dim3(tiles, nchunks), kOThreads, g.smem, st>>>(a);
+    kern<<<dim3(tiles, nparts), kOThreads, g.smem, st>>>(a);
     GD_CUDA(cudaGetLastError());
-    if (part && nchunks <= kOFewChunks) {
-        orbit_reduce_few_kernel<<<dim3((cells_pad + 127) / 128, d.n_pnt / 8), dim3(32, 8), 0, st>>>(
-            part, nchunks, d.n_pnt, cells_pad, ncells, ld, g.row_node, scale, gain);
-        GD_CUDA(cudaGetLastError());
-    } else if (part) {
-        const int64_t outs = (int64_t)d.n_pnt * ncells;
-        orbit_reduce_kernel<<<(unsigned)((outs + 31) / 32), dim3(32, 8), 0, st>>>(part, nchunks, d.n_pnt, cells_pad, ncells,
-                                                                                 ld, g.row_node, scale, gain);
+    if (part) {
+        orbit_reduce_kernel<<<dim3(tiles, (d.n_pnt * (g.cpt / 4) + 31) / 32), dim3(32, 8), 0, st>>>(
+            reinterpret_cast<const float4 *>(part), nparts, d.n_pnt, g.cpt, ncells, ld, g.row_node, scale, gain);
         GD_CUDA(cudaGetLastError());
     }
     return GD_OK;
@@ -1105,37 +1094,17 @@ bool orbit_serves(const Context &c, int path)
 // non-finite f gets NaN for all its outputs; other cells' bits are the same.
 int run_orbit(Context &c, const float *f, int ncells, int ld, float *gain, bool guard, cudaStream_t st)
 {
-    OrbitGain &g = *c.orbit;
-    if (guard && ncells > kOSlice) {
-        // the BF16x3 path has no limit on n_pnt * ld: slices of cells
-        for (int at = 0; at < ncells; at += kOSlice) {
-            const int rc = run_orbit(c, f + at, std::min(kOSlice, ncells - at), ld, gain + at, guard, st);
-            if (rc) return rc;
-        }
-        return GD_OK;
-    }
-    int nchunks = orbit_chunks(c, ncells);
-    // the partial sums are bounded at 16 GiB
-    while (nchunks > 1 && orbit_part_bytes(c, ncells, nchunks) > ((size_t)16 << 30)) nchunks--;
-    auto it = g.bounds_dev.find(nchunks);
-    if (it == g.bounds_dev.end()) {
-        std::vector<int> b(nchunks + 1);
-        orbit_chunk_bounds(c, nchunks, b.data());
-        int *dev = nullptr;
-        GD_CUDA(cudaMalloc(&dev, sizeof(int) * (nchunks + 1)));
-        cudaError_t e = cudaMemcpy(dev, b.data(), sizeof(int) * (nchunks + 1), cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) {
-            cudaFree(dev);
-            return cuda_error(e, "gain chunk bounds");
-        }
-        it = g.bounds_dev.emplace(nchunks, dev).first;
-    }
-    const size_t bytes = orbit_pack_bytes(c, ncells) + orbit_part_bytes(c, ncells, nchunks);
-    const int cells_pad = (ncells + g.cpt - 1) / g.cpt * g.cpt;
-    int rc = ensure_scratch(c, bytes + (guard ? sizeof(float2) * cells_pad : 0));
+    if (!guard && (int64_t)c.d.n_pnt * ld >= ((int64_t)1 << 31))
+        return set_error(GD_ERR_UNSUPPORTED, "pair gain: n_pnt * ld must stay below 2^31");
+    // slices of cells: a cell's sums are the same in any batch
+    const int slice = orbit_slice(c, ncells, kOScratch);
+    const size_t bytes = orbit_bytes(c, slice);
+    int rc = ensure_scratch(c, bytes + (guard ? sizeof(float2) * slice : 0));
     if (rc) return rc;
     float2 *scale = guard ? reinterpret_cast<float2 *>(static_cast<char *>(c.scratch.ptr) + bytes) : nullptr;
-    return launch_orbit(c, f, ncells, ld, gain, c.scratch.ptr, nchunks, it->second, scale, st);
+    for (int at = 0; at < ncells && !rc; at += slice)
+        rc = launch_orbit(c, f + at, std::min(slice, ncells - at), ld, gain + at, c.scratch.ptr, scale, st);
+    return rc;
 }
 
 int orbit_take_timeout(Context &c, cudaStream_t st, bool *timed_out)

@@ -15,7 +15,9 @@
  *    the reference layout f[(i*ny + j)*nz + k][cell] with npx = ld.
  *  - Streams are cudaStream_t passed as gd_stream (NULL = legacy stream).
  *  - Results are bitwise reproducible run to run: floating-point sums run in
- *    a fixed order, and the one path that adds with atomics adds integers.
+ *    a fixed order, and the one path that adds with atomics adds integers.  A
+ *    cell's gain on lattices of at most 1024 orbits of nodes (or on any with the
+ *    collision matrices or the tensor-core pair path) is the same in any batch.
  *
  * Reference interfaces (savthe/gpu_determ) each entry point replaces are cited
  * as file:line.
@@ -249,8 +251,9 @@ int gd_compact_to_box(gd_ctx *ctx, const float *compact, int ncells, int ld, flo
  * library image, held on every GPU that loads the library until exit; a batch
  * needing more (about 4500 cells on a 20^3 grid cut to R=4.8) is rejected with
  * GD_ERR_UNSUPPORTED.  The result is bitwise equal to gd_collision's FP32
- * pair gain when the s-chunk count that call picks fits the array (at most
- * 64 chunks; then both sum in the same order); otherwise the array holds
+ * gain (in slices of cells that fit the array); on lattices of more than 1024
+ * orbits of nodes only when the s-chunk count that call picks fits the array (at
+ * most 64 chunks; then both sum in the same order): otherwise the array holds
  * fewer chunks and the sums, ordered differently, agree within FP32
  * rounding.  The first call on a device looks the array's address up, which
  * may also load the library's device code on that device and so reserve the
@@ -298,7 +301,8 @@ int gd_batch_info(const gd_batch *b, int *groups, int *streams, int *graph_nodes
 
 /* Times the gain candidates of a context on the given cells and keeps the
  * fastest (gain path, and for the pair kernel the minimum CTAs per SM of its
- * s-chunk split).  path_mask: bits (1 << GD_GAIN_*) that may be chosen; the
+ * s-chunk split, on lattices of more than 1024 orbits of nodes; on the others
+ * the split is fixed).  path_mask: bits (1 << GD_GAIN_*) that may be chosen; the
  * collision-matrix paths only when their stored tiles (at most every 256 x 64
  * tile of each G_i's block upper triangle, 2 bytes per entry in BF16, 4 in
  * BF16X3) fit mem_budget bytes, GD_GAIN_PAIR_TC only when its weight table
