@@ -6,18 +6,20 @@
 //   A_kl = sum_i f_i nu_i phi_k phi_l,  B_k = sum_i (I_i - f_i nu_i) phi_k,
 //   A X = B,  nu'_i = nu_i (1 + X.phi_i),  Q_i = I_i - f_i nu'_i,
 // after which sum_i Q_i phi_k = 0 (mass, momentum, energy) up to FP64 rounding.
-// A warp takes LC cells times 32 / LC lines.  The nodes of one (x, y) form a line along z, and the sums over a
-// line need only powers of z: 11 FP64 accumulators per node (z^0..z^4 of f nu,
-// z^0..z^2 of I - f nu and of f) that enter the 25 sums once per line, 18 FP64
-// operations per node and cell instead of 46; the second pass likewise takes
-// two fused operations for 1 + X.phi instead of five.  A cluster of CTAs shares
-// the lines of LC cells, and LC is smaller for few cells, so that they still
-// spread over the chip; partial sums are combined lane group by lane group,
-// warp by warp, then CTA by CTA, in fixed order, so the sums are reproducible.
+// The nodes of one (x, y) form a line along z, and the sums over a line need only
+// powers of z: 11 FP64 accumulators per node (z^0..z^4 of f nu, z^0..z^2 of I - f nu
+// and of f) that enter the 25 sums once per line, 18 FP64 operations per node and
+// cell instead of 46; the second pass likewise takes two fused operations for 1 +
+// X.phi instead of five.  The lines fall into 8 to 64 classes (project_classes): a
+// class is summed line after line, the classes' sums are added as a tree.  That order
+// is the lattice's alone, so a cell's results have the same bits in any batch,
+// whichever way the work is split: a warp takes LC cells times 32 / LC classes, or,
+// for few cells, lines of one cell (LC = 1), and a cluster of CTAs shares the lines
+// of its cells.
 // Bound: the FP64 pipe (its rate is 1/64 of the FP32 rate and a hardware float to
 // double conversion takes a slot of it, so to_double does that in integers).
-// 20^3: 4096 cells 1.54 -> 0.84 ms (the FP64 pipe three quarters busy), 256 cells 1.6 ->
-// 0.092, one cell 1.6 -> 0.057.
+// 20^3: 4096 cells 1.54 -> 0.84 ms, 256 cells 1.6 -> 0.095, one cell 1.6 -> 0.046
+// (with the splits free to change the order of the sums: 0.84, 0.092 and 0.057).
 #include "gd_internal.h"
 #include "gd_tc.cuh"
 
@@ -35,7 +37,7 @@ struct ProjArgs {
     Dims d;
     const float *f, *nu, *gain;
     int ld, ncells;
-    int nlines;
+    int nlines, classes;    // lines l, l + classes, ... are summed in order, the classes' sums as a tree
     const int4 *lines;      // {first node, end node, z index of the first, 0}
     const double2 *line_xy;
     const double2 *zpow;    // (z, z^2), (z^3, z^4) per z index
@@ -112,6 +114,92 @@ __device__ __forceinline__ double to_double(float v)
     return (double)v;
 }
 
+// What the 25 sums need of a line: powers of z.
+struct LineSums {
+    double S0, S1, S2, S3, S4, R0, R1, R2, M0, M1, M2;
+};
+constexpr int kLineSums = 11;
+
+template <bool M5>
+__device__ __forceinline__ LineSums sum_line(const ProjArgs &a, int4 ln, int cell)
+{
+    LineSums v = {};
+    const double2 *zp = a.zpow + 2 * ln.z;
+    size_t o = (size_t)ln.x * a.ld + cell;
+#pragma unroll 4
+    for (int i = ln.x; i < ln.y; i++, zp += 2, o += a.ld) {
+        const double fv = to_double(a.f[o]), nv = to_double(a.nu[o]), gv = to_double(a.gain[o]);
+        const double z = zp[0].x, z2 = zp[0].y;
+        const double fn = fv * nv, r = gv - fn;
+        v.R0 = __dadd_rn(v.R0, r);
+        v.R1 = __fma_rn(r, z, v.R1);
+        v.R2 = __fma_rn(r, z2, v.R2);
+        v.S0 = __dadd_rn(v.S0, fn);
+        v.S1 = __fma_rn(fn, z, v.S1);
+        v.S2 = __fma_rn(fn, z2, v.S2);
+        v.S3 = __fma_rn(fn, zp[1].x, v.S3);
+        v.S4 = __fma_rn(fn, zp[1].y, v.S4);
+        if (M5) {
+            v.M0 = __dadd_rn(v.M0, fv);
+            v.M1 = __fma_rn(fv, z, v.M1);
+            v.M2 = __fma_rn(fv, z2, v.M2);
+        }
+    }
+    return v;
+}
+
+// A line's part of the sums.  Every operation is spelled out: wherever a line is
+// added the bits are the same.
+template <bool M5>
+__device__ __forceinline__ void add_line(double *s, const LineSums &v, double2 xy)
+{
+    const double x = xy.x, y = xy.y, rho = __fma_rn(x, x, __dmul_rn(y, y));
+    const double E0 = __fma_rn(rho, v.S0, v.S2), E1 = __fma_rn(rho, v.S1, v.S3),
+                 E2 = __fma_rn(rho, __dadd_rn(E0, v.S2), v.S4), xS = __dmul_rn(x, v.S0), yS = __dmul_rn(y, v.S0);
+    s[0] = __dadd_rn(s[0], v.R0);
+    s[1] = __fma_rn(x, v.R0, s[1]);
+    s[2] = __fma_rn(y, v.R0, s[2]);
+    s[3] = __dadd_rn(s[3], v.R1);
+    s[4] = __dadd_rn(s[4], __fma_rn(rho, v.R0, v.R2));
+    s[5] = __dadd_rn(s[5], v.S0);
+    s[6] = __dadd_rn(s[6], xS);
+    s[7] = __dadd_rn(s[7], yS);
+    s[8] = __dadd_rn(s[8], v.S1);
+    s[9] = __dadd_rn(s[9], E0);
+    s[10] = __fma_rn(x, xS, s[10]);
+    s[11] = __fma_rn(x, yS, s[11]);
+    s[12] = __fma_rn(x, v.S1, s[12]);
+    s[13] = __fma_rn(x, E0, s[13]);
+    s[14] = __fma_rn(y, yS, s[14]);
+    s[15] = __fma_rn(y, v.S1, s[15]);
+    s[16] = __fma_rn(y, E0, s[16]);
+    s[17] = __dadd_rn(s[17], v.S2);
+    s[18] = __dadd_rn(s[18], E1);
+    s[19] = __dadd_rn(s[19], E2);
+    if (M5) {
+        s[20] = __dadd_rn(s[20], v.M0);
+        s[21] = __fma_rn(x, v.M0, s[21]);
+        s[22] = __fma_rn(y, v.M0, s[22]);
+        s[23] = __dadd_rn(s[23], v.M1);
+        s[24] = __dadd_rn(s[24], __fma_rn(rho, v.M0, v.M2));
+    }
+}
+
+// Sum of n = 1, 2, 4 or 8 values, neighbours first.
+template <typename F>
+__device__ __forceinline__ double tree8(int n, F value)
+{
+    double v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = k < n ? value(k) : 0.;
+#pragma unroll
+    for (int w = 1; w < 8; w *= 2)
+#pragma unroll
+        for (int k = 0; k < 8; k += 2 * w)
+            if (w < n) v[k] += v[k + w];
+    return v[0];
+}
+
 template <bool M5, int LC>
 __global__ void __launch_bounds__(kWarps * 32) project_kernel(const __grid_constant__ ProjArgs a, int cs)
 {
@@ -125,94 +213,72 @@ __global__ void __launch_bounds__(kWarps * 32) project_kernel(const __grid_const
     const int col = lane % LC;
     const int cell = (int)blockIdx.x / cs * LC + col;
     const bool live = cell < a.ncells;
-    const int first = (rank * kWarps + warp) * G + lane / LC, step = cs * kWarps * G;
+    // this thread's lines: a class of them, or where one cell has a CTA to itself
+    // (LC = 1) every line its own thread; CTA r then takes the classes c % cs == r
+    const int first = LC == 1 ? rank + (int)threadIdx.x * cs : (rank * kWarps + warp) * G + lane / LC;
+    const int step = LC == 1 ? (int)blockDim.x * cs : a.classes;
     double s[kSums];
 #pragma unroll
     for (int k = 0; k < NS; k++) s[k] = 0.;
-    if (live) {
-        for (int l = first; l < a.nlines; l += step) {
-            const int4 ln = __ldg(a.lines + l);
-            double S0 = 0., S1 = 0., S2 = 0., S3 = 0., S4 = 0., R0 = 0., R1 = 0., R2 = 0., M0 = 0., M1 = 0., M2 = 0.;
-            const double2 *zp = a.zpow + 2 * ln.z;
-            size_t o = (size_t)ln.x * a.ld + cell;
-#pragma unroll 4
-            for (int i = ln.x; i < ln.y; i++, zp += 2, o += a.ld) {
-                const double fv = to_double(a.f[o]), nv = to_double(a.nu[o]), gv = to_double(a.gain[o]);
-                const double z = zp[0].x, z2 = zp[0].y;
-                const double fn = fv * nv, r = gv - fn;
-                R0 += r;
-                R1 += r * z;
-                R2 += r * z2;
-                S0 += fn;
-                S1 += fn * z;
-                S2 += fn * z2;
-                S3 += fn * zp[1].x;
-                S4 += fn * zp[1].y;
-                if (M5) {
-                    M0 += fv;
-                    M1 += fv * z;
-                    M2 += fv * z2;
+    if (LC == 1) {
+        double *ls = red;  // [line of the CTA][kLineSums]
+        for (int l = first; l < a.nlines; l += step)
+            *reinterpret_cast<LineSums *>(ls + (size_t)(l / cs) * kLineSums) = sum_line<M5>(a, __ldg(a.lines + l), cell);
+        __syncthreads();
+        const int c = rank + (int)threadIdx.x * cs;
+        if (c < a.classes)
+            for (int l = c; l < a.nlines; l += a.classes)
+                add_line<M5>(s, *reinterpret_cast<const LineSums *>(ls + (size_t)(l / cs) * kLineSums), __ldg(a.line_xy + l));
+        __syncthreads();
+        double *cl = red;  // [class of the CTA][kSums]
+        if (c < a.classes)
+#pragma unroll
+            for (int k = 0; k < NS; k++) cl[(size_t)(c / cs) * kSums + k] = s[k];
+        if (cs > 1) tc::cluster_sync();
+        else __syncthreads();
+        // the classes' sums, neighbours first: a warp per sum
+        if (rank == 0)
+            for (int k = warp; k < NS; k += kWarps) {
+                double v[2];
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int q = lane + 32 * h;
+                    v[h] = q >= a.classes ? 0. : cs > 1 ? peer_load(cl + (size_t)(q / cs) * kSums + k, (uint32_t)(q % cs))
+                                                        : cl[(size_t)q * kSums + k];
+#pragma unroll
+                    for (int w = 1; w < 32; w *= 2) {
+                        const double u = __shfl_xor_sync(0xffffffffu, v[h], w);
+                        if (w < a.classes) v[h] += u;
+                    }
                 }
+                mine[k * 32 + lane] = __shfl_sync(0xffffffffu, a.classes > 32 ? v[0] + v[1] : v[0], 0);
             }
-            const double2 xy = __ldg(a.line_xy + l);
-            const double x = xy.x, y = xy.y, rho = x * x + y * y;
-            const double E0 = rho * S0 + S2, E1 = rho * S1 + S3, E2 = rho * (E0 + S2) + S4, xS = x * S0, yS = y * S0;
-            s[0] += R0;
-            s[1] += x * R0;
-            s[2] += y * R0;
-            s[3] += R1;
-            s[4] += rho * R0 + R2;
-            s[5] += S0;
-            s[6] += xS;
-            s[7] += yS;
-            s[8] += S1;
-            s[9] += E0;
-            s[10] += x * xS;
-            s[11] += x * yS;
-            s[12] += x * S1;
-            s[13] += x * E0;
-            s[14] += y * yS;
-            s[15] += y * S1;
-            s[16] += y * E0;
-            s[17] += S2;
-            s[18] += E1;
-            s[19] += E2;
-            if (M5) {
-                s[20] += M0;
-                s[21] += x * M0;
-                s[22] += y * M0;
-                s[23] += M1;
-                s[24] += rho * M0 + M2;
-            }
+        if (rank == 0) __syncthreads();
+    } else {
+        if (live)
+            for (int l = first; l < a.nlines; l += step)
+                add_line<M5>(s, sum_line<M5>(a, __ldg(a.lines + l), cell), __ldg(a.line_xy + l));
+        // the classes' sums, neighbours first: over the lane groups, the warps and the CTAs
+#pragma unroll
+        for (int k = 0; k < NS; k++) {
+#pragma unroll
+            for (int w = LC; w < 32; w *= 2) s[k] += __shfl_xor_sync(0xffffffffu, s[k], w);
+            red[((size_t)warp * kSums + k) * 32 + lane] = s[k];
         }
-    }
-    // combine the lane groups' partial sums, the warps' in warp order, then the
-    // CTAs' in rank order
-#pragma unroll
-    for (int k = 0; k < NS; k++) {
-#pragma unroll
-        for (int w = LC; w < 32; w *= 2) s[k] += __shfl_xor_sync(0xffffffffu, s[k], w);
-        red[((size_t)warp * kSums + k) * 32 + lane] = s[k];
-    }
-    __syncthreads();
-    for (int t = threadIdx.x; t < NS * 32; t += kWarps * 32) {
-        double v = red[t];
-        for (int w = 1; w < kWarps; w++) v += red[(size_t)w * kSums * 32 + t];
-        mine[t] = v;
-    }
-    if (cs > 1) tc::cluster_sync();
-    else __syncthreads();
-    if (rank == 0) {
-        if (cs > 1) {
-            for (int t = threadIdx.x; t < NS * 32; t += kWarps * 32) {
-                double v = mine[t];
-                for (int k = 1; k < cs; k++) v += peer_load(mine + t, (uint32_t)k);
-                red[t] = v;
-            }
+        __syncthreads();
+        for (int t = threadIdx.x; t < NS * 32; t += kWarps * 32)
+            mine[t] = tree8(kWarps, [&](int w) { return red[(size_t)w * kSums * 32 + t]; });
+        if (cs > 1) tc::cluster_sync();
+        else __syncthreads();
+        if (rank == 0 && cs > 1) {
+            for (int t = threadIdx.x; t < NS * 32; t += kWarps * 32)
+                red[t] = tree8(cs, [&](int k) { return k == 0 ? mine[t] : peer_load(mine + t, (uint32_t)k); });
             __syncthreads();
         }
+    }
+    if (rank == 0) {
         if (warp == 0) {
-            const double *all = cs > 1 ? red : mine;
+            const double *all = LC != 1 && cs > 1 ? red : mine;
             double tot[kSums] = {};
 #pragma unroll
             for (int k = 0; k < NS; k++) tot[k] = all[k * 32 + lane];
@@ -278,17 +344,18 @@ __global__ void __launch_bounds__(kWarps * 32) project_kernel(const __grid_const
         for (int l = first; l < a.nlines; l += step) {
             const int4 ln = __ldg(a.lines + l);
             const double2 xy = __ldg(a.line_xy + l);
-            const double c0 = 1. + X[0] + X[1] * xy.x + X[2] * xy.y + X[4] * (xy.x * xy.x + xy.y * xy.y);
+            const double rho = __fma_rn(xy.x, xy.x, __dmul_rn(xy.y, xy.y));
+            const double c0 = __fma_rn(X[4], rho, __fma_rn(X[2], xy.y, __fma_rn(X[1], xy.x, __dadd_rn(1., X[0]))));
             const double2 *zp = a.zpow + 2 * ln.z;
             size_t o = (size_t)ln.x * a.ld + cell;
 #pragma unroll 4
             for (int i = ln.x; i < ln.y; i++, zp += 2, o += a.ld) {
                 const double fv = to_double(a.f[o]), nv = to_double(a.nu[o]), gv = to_double(a.gain[o]);
-                const double nc = nv * (c0 + X[3] * zp->x + X[4] * zp->y);
-                const double qv = gv - fv * nc;
+                const double nc = __dmul_rn(nv, __fma_rn(X[4], zp->y, __fma_rn(X[3], zp->x, c0)));
+                const double qv = __fma_rn(-fv, nc, gv);
                 if (a.nu_corr) a.nu_corr[o] = (float)nc;
                 if (a.q) a.q[o] = qv;
-                if (a.update) a.f_out[o] = (float)(fv + (double)a.dt * qv);
+                if (a.update) a.f_out[o] = (float)__fma_rn((double)a.dt, qv, fv);
             }
         }
     }
@@ -415,36 +482,54 @@ __global__ void basis_kernel(Dims d, const float *__restrict__ u, const float *_
 
 }  // namespace
 
-// Cells per warp (32, 8 or 1) and CTAs per group of cells, by the FP64 pipe's time
-// in instructions of a warp: a CTA's threads take so many lines each (15 per node
-// and 40 per line), then combine 20 sums over lanes, warps and CTAs (about 125).  An
-// SM works off its CTAs one after the other; clusters of four and eight find room
-// in fewer SMs (their GPC's); one CTA per SM waits for its loads when they come from
-// HBM.  Measured at 20^3, us (cells per warp, CTAs): one cell (1, 2) 57, (8, 8) 62;
-// 152 cells (1, 1) 67, (8, 4) 92; 240 (8, 4) 92, (1, 1) 106; 420 (32, 8) 128, (8, 2)
-// 143; 600 (8, 2) 143, (32, 8) 221; 1064 (32, 4) 239; 1300 (32, 8) 340, (32, 4) 421;
-// 2100 (32, 4) 435, (32, 2) 500; 4096 (32, 2) 844, (32, 1) 909.
+// Classes of lines (8 to 64): about four lines in each.
+int project_classes(const Context &c)
+{
+    int n = 8;
+    while (n < 64 && n * 4 < c.nlines) n *= 2;
+    return n;
+}
+
+// Cells per warp (32, 16 or 8: a class of lines per thread; 1: a line per thread) and
+// CTAs per group of cells, by the FP64 pipe's time in instructions of a warp (about
+// ten in a us).  A class per thread: so many lines each (15 per node and 40 per
+// line), then 20 sums over lanes, warps and CTAs (about 125); an SM works off its
+// CTAs one after the other; clusters of four and eight find room in fewer SMs (their
+// GPC's); one CTA per SM waits for its loads when they come from HBM.  A line per
+// thread: three CTAs wait for their loads side by side.  Measured, us (cells per
+// warp, CTAs), 20^3: one cell (1, 2) 46, (1, 1) 59, (32, 8) 125; 256 cells (1, 1) 95,
+// (32, 8) 127; 512 (16, 4) 132, (1, 1) 182, (32, 8) 220; 1024 (32, 8) 237, (16, 4)
+// 241; 4096 (32, 8) 841, (16, 4) 881, (8, 2) 911; 8^3: 400 cells (1, 1) 35, (32, 2)
+// 46; 512 (1, 1) 61, (32, 2) 46.
 struct ProjSplit {
     int lc, cs;
 };
 ProjSplit project_split(const Context &c, int ncells)
 {
-    const int sms = std::max(1, c.sm_count);
-    const double nodes = (double)c.d.n_pnt / c.nlines;
+    const int sms = std::max(1, c.sm_count), classes = project_classes(c);
+    const double line = 15.0 * c.d.n_pnt / c.nlines + 40.0;
     const bool hbm = (int64_t)c.d.n_pnt * ncells > ((int64_t)100 << 20) / 24;
-    ProjSplit best{32, 1};
+    ProjSplit best{0, 0};
     double least = 0.0;
-    for (int lc : {1, 8, 32})
+    for (int lc : {32, 16, 8, 1})
         for (int cs = 1; cs <= 8; cs *= 2) {
             const int64_t ctas = ((int64_t)ncells + lc - 1) / lc * cs;
-            const int threads = cs * kWarps * (32 / lc);  // of a cell
-            const double lines = (c.nlines + threads - 1) / threads;
-            const int room = cs == 8 ? sms * 3 / 4 : cs == 4 ? sms * 11 / 12 : sms;
-            const int many = cs >= 4 ? std::max(1, sms * 14 / 15) : sms;
-            const int64_t turns = ctas <= room ? 1 : std::max<int64_t>(2, (ctas + many - 1) / many);
-            double cost = (double)turns * (lines * (15.0 * nodes + 40.0) + 125.0);
-            if (turns == 1 && hbm) cost *= 1.15;
-            if (lc == 8) cost *= 1.1;  // 32-byte rows
+            double cost = 0.0;
+            if (lc == 1) {
+                // the sums of a CTA's lines in shared memory
+                if (cs > 2 || (c.nlines + cs - 1) / cs * kLineSums > kWarps * kSums * 32) continue;
+                cost = 240.0 * (double)((ctas + 3 * sms - 1) / (3 * sms)) +
+                       (double)((ctas + sms - 1) / sms) * (c.nlines * line / (cs * kWarps * 32) + 50.0);
+                if (hbm) cost *= 1.2;  // a sector for each value
+            } else {
+                if (cs * kWarps * (32 / lc) != classes) continue;
+                const int room = cs == 8 ? sms * 3 / 4 : cs == 4 ? sms * 11 / 12 : sms;
+                const int many = cs >= 4 ? std::max(1, sms * 14 / 15) : sms;
+                const int64_t turns = ctas <= room ? 1 : std::max<int64_t>(2, (ctas + many - 1) / many);
+                cost = (double)turns * ((c.nlines + classes - 1) / classes * line + 125.0);
+                if (turns == 1 && hbm) cost *= 1.15;
+                cost *= lc == 8 ? 1.15 : lc == 16 ? 1.04 : 1.0;  // rows of 32 and 64 bytes
+            }
             if (least == 0.0 || cost < least * (1.0 - 1e-9)) {
                 least = cost;
                 best = ProjSplit{lc, cs};
@@ -457,11 +542,12 @@ int run_project(Context &c, const float *f, const float *nu, const float *gain, 
                 float *nu_corr, double *q, double *x, int fixed_dt_mode, float dt, float *f_out,
                 double *m5, cudaStream_t st)
 {
-    const ProjArgs a{c.d,   f, nu, gain, ld,                     ncells, c.nlines, c.d_lines, c.d_line_xy, c.d_zpow, nu_corr,
+    const ProjArgs a{c.d,   f, nu, gain, ld, ncells, c.nlines, project_classes(c), c.d_lines, c.d_line_xy, c.d_zpow, nu_corr,
                      q,     x, fixed_dt_mode ? 1 : 0, dt, f_out, m5,     c.d_status};
     const ProjSplit split = project_split(c, ncells);
     const int lc = split.lc, cs = split.cs, blocks = (ncells + lc - 1) / lc;
     auto kern = lc == 32 ? (m5 ? project_kernel<true, 32> : project_kernel<false, 32>)
+                : lc == 16 ? (m5 ? project_kernel<true, 16> : project_kernel<false, 16>)
                 : lc == 8 ? (m5 ? project_kernel<true, 8> : project_kernel<false, 8>)
                           : (m5 ? project_kernel<true, 1> : project_kernel<false, 1>);
     GD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProjSmem));

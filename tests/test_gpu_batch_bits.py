@@ -34,3 +34,38 @@ def test_gain_bits_do_not_depend_on_the_batch(cuda, gdlib, n, nc):
             ctx.collision(part, count, count, None, out)
             assert torch.equal(out, whole[:, first:first + count]), (path, first, count)
         ctx.check()
+
+
+@pytest.mark.parametrize("n,nc", [(2, 700), (6, 2500), (8, 2500), (12, 1300), (20, 1100), (24, 600)])
+def test_projection_bits_do_not_depend_on_the_batch(cuda, gdlib, n, nc):
+    """nu', Q, X and the step's moments over cell counts on both sides of every
+    split of the work (a line per thread; 8, 16 or 32 cells per warp)."""
+    torch = cuda
+    spec = gdlib.GridSpec(n, R=4.8 if n > 2 else 16.5)
+    ctx = gdlib.Context(spec)
+    rng = np.random.default_rng(n)
+    f = _batch(torch, spec, nc)
+    nu = torch.from_numpy(rng.uniform(1.0, 3.0, f.shape).astype(np.float32)).cuda()
+    gain = f * nu * torch.from_numpy(rng.uniform(0.7, 1.4, f.shape).astype(np.float32)).cuda()
+
+    def project(first, count):
+        part = [a[:, first:first + count].contiguous() for a in (f, nu, gain)]
+        out = (torch.empty_like(part[0]), torch.empty(part[0].shape, dtype=torch.float64, device="cuda"),
+               torch.empty((count, 5), dtype=torch.float64, device="cuda"))
+        ctx.project(*part, count, count, *out)
+        return out
+
+    def moments(first, count):
+        g = f[:, first:first + count].clone(memory_format=torch.contiguous_format)
+        m5 = torch.empty((count, 5), dtype=torch.float64, device="cuda")
+        ctx.step(g, count, count, gdlib.DT_FIXED, 1e-3, m5=m5)
+        return g, m5
+
+    whole, stepped = project(0, nc), moments(0, nc)
+    for first, count in ((0, 1), (7, 2), (1, 40), (2, 200), (3, 350), (0, nc // 2), (nc // 2, nc - nc // 2)):
+        cols = slice(first, first + count)
+        got = project(first, count)
+        assert torch.equal(got[0], whole[0][:, cols]) and torch.equal(got[1], whole[1][:, cols]), (first, count)
+        assert torch.equal(got[2], whole[2][cols]), (first, count)
+        got = moments(first, count)
+        assert torch.equal(got[0], stepped[0][:, cols]) and torch.equal(got[1], stepped[1][cols]), (first, count)
