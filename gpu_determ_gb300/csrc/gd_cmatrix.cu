@@ -1257,7 +1257,7 @@ int run_loss_path(Context &c, const float *f, int ncells, int ld, float *nu, cud
 {
     // With the FP32 kernel's gain the loss is FP32 too: the tensor cores' sums are
     // about 1e-6 low, which only a gain from the same sums balances in the
-    // projection (20^3, 4096 cells: 0.64 ms against 0.34, of 68; one cell 0.03
+    // projection (20^3, 4096 cells: 2.5 ms against 0.34, of 75; one cell 0.016
     // against 0.05).  A pending time-out injection is for the tensor cores' GEMM.
     if (c.gain_path != GD_GAIN_PAIR && c.cmatrix && (!orbit_serves(c, c.gain_path) || c.cmatrix->stall_next > 0)) {
         const int rc = cmatrix_loss(c.cmatrix, f, ncells, ld, nu, st);

@@ -71,7 +71,7 @@ struct OrbitGain {
     int *start = nullptr;  // [part][warp] position in the stream, in 16-byte units
     int *err = nullptr;    // set by the kernel when a copy of the stream is not seen to land
     int opad = 0;               // orbits padded to the loss kernel's tile
-    float *bx = nullptr;        // [8][o'][opad] loss matrices folded by the reflections' characters
+    float4 *bx = nullptr;       // [o'][2][opad] b of two orbits by reflection
     int *bounds = nullptr;      // [nparts + 1] their bounds in steps
 };
 
@@ -223,7 +223,7 @@ int reduce_gain_partials(Context &c, const float *part, int nchunks, int cells_p
 // tables (built with the context), bytes of a batch's buffer, cells per launch in a
 // given room, and the launch into a caller-provided buffer
 int orbit_build(Context &c);
-int fold_loss_build(Context &c);  // its loss matrices (gd_loss.cu)
+int orbit_loss_build(Context &c);  // its loss table (gd_loss.cu)
 void orbit_free(Context &c);
 size_t orbit_bytes(const Context &c, int ncells);
 int orbit_slice(const Context &c, int ncells, size_t room);

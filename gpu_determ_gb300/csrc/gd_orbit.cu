@@ -1021,7 +1021,7 @@ int orbit_build(Context &c)
     if (!rc) rc = upload(&og->bounds, bounds);
     if (!rc) rc = upload(&og->start, first);
     if (!rc) rc = upload(&og->err, std::vector<int>(1, 0));
-    if (!rc) rc = fold_loss_build(c);
+    if (!rc) rc = orbit_loss_build(c);
     return rc;  // the caller destroys the context on failure
 }
 

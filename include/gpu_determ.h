@@ -16,9 +16,10 @@
  *  - Streams are cudaStream_t passed as gd_stream (NULL = legacy stream).
  *  - Results are bitwise reproducible run to run: floating-point sums run in
  *    a fixed order, and the one path that adds with atomics adds integers.  A
- *    cell's loss and projection, and its gain on lattices of at most 1024 orbits
- *    of nodes (on any with the collision matrices or the tensor-core pair path),
- *    have the same bits in any batch.
+ *    cell's projection, its loss (on one of the tensor cores and the FP32 kernel,
+ *    see gd_collision) and its gain on lattices of at most 1024 orbits of nodes (on
+ *    any with the collision matrices or the tensor-core pair path) have the same
+ *    bits in any batch.
  *
  * Reference interfaces (savthe/gpu_determ) each entry point replaces are cited
  * as file:line.

@@ -69,3 +69,19 @@ def test_projection_bits_do_not_depend_on_the_batch(cuda, gdlib, n, nc):
         assert torch.equal(got[2], whole[2][cols]), (first, count)
         got = moments(first, count)
         assert torch.equal(got[0], stepped[0][:, cols]) and torch.equal(got[1], stepped[1][cols]), (first, count)
+
+
+# one orbit; tiles of 4 and of 16 orbits on both sides of the change
+@pytest.mark.parametrize("n,nc", [(2, 50), (12, 1300), (20, 300)])
+def test_loss_bits_do_not_depend_on_the_batch(cuda, gdlib, n, nc):
+    torch = cuda
+    spec = gdlib.GridSpec(n, R=4.8 if n > 2 else 16.5)
+    ctx = gdlib.Context(spec)
+    f = _batch(torch, spec, nc)
+    whole = torch.empty_like(f)
+    ctx.collision(f, nc, nc, whole, None)
+    for first, count in ((0, 1), (5, 9), (3, nc // 2), (nc // 2, nc - nc // 2)):
+        part = f[:, first:first + count].contiguous()
+        out = torch.empty_like(part)
+        ctx.collision(part, count, count, out, None)
+        assert torch.equal(out, whole[:, first:first + count]), (first, count)
