@@ -52,9 +52,16 @@ struct ProjArgs {
 };
 
 // Gaussian elimination with partial pivoting on a symmetric 5x5 system, all
-// indices static (rows swapped by selection).
+// indices static (rows swapped by selection).  Singular (false): what is left of a
+// column is nowhere above the rounding of the sums it came from, 2^-50 of the root of
+// the row's and the column's diagonal entries.  A cell with all its mass on one node
+// leaves at most 2.7e-16 there (all nodes of 8^3 to 20^3; an exact zero for two thirds
+// of them), a Maxwellian of half the lattice's step in width 1e-6.
 __device__ __forceinline__ bool solve5(double A[5][5], double b[5], double x[5])
 {
+    double rs[5], cs[5];  // the rows' and the columns' scales
+#pragma unroll
+    for (int k = 0; k < 5; k++) rs[k] = cs[k] = fabs(A[k][k]);
 #pragma unroll
     for (int k = 0; k < 5; k++) {
         int piv = k;
@@ -65,10 +72,16 @@ __device__ __forceinline__ bool solve5(double A[5][5], double b[5], double x[5])
                 best = fabs(A[r][k]);
                 piv = r;
             }
-        if (!(best > 0.0)) return false;
+        bool any = false;
+#pragma unroll
+        for (int r = k; r < 5; r++) any = any || A[r][k] * A[r][k] > 0x1p-100 * rs[r] * cs[k];
+        if (!(best > 0.0) || !any) return false;
 #pragma unroll
         for (int r = k + 1; r < 5; r++) {
             const bool p = piv == r;
+            const double su = rs[k], sv = rs[r];
+            rs[k] = p ? sv : su;
+            rs[r] = p ? su : sv;
 #pragma unroll
             for (int t = k; t < 5; t++) {
                 const double u = A[k][t], v = A[r][t];
@@ -201,7 +214,7 @@ __device__ __forceinline__ double tree8(int n, F value)
 }
 
 template <bool M5, int LC>
-__global__ void __launch_bounds__(kWarps * 32) project_kernel(const __grid_constant__ ProjArgs a, int cs)
+__global__ void __launch_bounds__(kWarps * 32, LC == 1 ? 3 : 2) project_kernel(const __grid_constant__ ProjArgs a, int cs)
 {
     extern __shared__ __align__(16) double red[];  // [kWarps][kSums][32], then the CTA's sums [kSums][32]
     __shared__ double xs[5][32];
