@@ -448,7 +448,11 @@ int gd_ctx_create(const gd_grid_spec *spec, int device, gd_ctx **out)
     if (rc) return rc;
     gd_ctx *ctx = new (std::nothrow) gd_ctx();
     if (!ctx) return set_error(GD_ERR_OUT_OF_MEMORY, "host allocation failed");
-    rc = gd::create_context(ctx->c, *spec, device);
+    try {
+        rc = gd::create_context(ctx->c, *spec, device);
+    } catch (const std::exception &) {  // host memory
+        rc = set_error(GD_ERR_OUT_OF_MEMORY, "host allocation failed while building the context's tables");
+    }
     if (rc) {
         gd::DeviceGuard g(device);
         gd::destroy_context(ctx->c);

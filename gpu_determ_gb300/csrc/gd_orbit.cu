@@ -50,12 +50,13 @@
 // a check per record costs more than the padding).
 #include "gd_internal.h"
 #include "gd_tc.cuh"
+#include "gd_workers.h"
 
 #include <algorithm>
 #include <array>
 #include <cmath>
 #include <cstring>
-#include <thread>
+#include <memory>
 
 namespace gd {
 namespace {
@@ -623,6 +624,18 @@ int orbit_build(Context &c)
     }
     if (8 * norb != d.n_pnt) return GD_OK;
 
+    // tile width: eight cells where their outputs, f and some rows fit, else four;
+    // seen before any table is built (they grow with the seventh power of n)
+    int max_smem = 0;
+    GD_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c.device));
+    const int slots = (norb + kOWarps * kOSlots - 1) / (kOWarps * kOSlots) * kOSlots;
+    auto rows_of = [&](int w) { return (max_smem - (int)kOF - (d.n_pnt + 8) * w * 4) / (32 * w) - 1; };  // P and C rows
+    auto c_rows = [](int rows) { return rows * 2 / 5 / kORows * kORows; };
+    int nslot = 0;
+    bool fits = false;
+    for (int w : {8, 4}) fits = fits || (orbit_kernel(w, slots, &nslot) && rows_of(w) - c_rows(rows_of(w)) >= 64);
+    if (!fits) return GD_OK;
+
     // group of every g and the groups' |g|^2
     std::vector<int> gid(d.nxyz, -1);
     std::vector<double> g2(c.n_groups, 0.0);
@@ -741,13 +754,9 @@ int orbit_build(Context &c)
             if (!it.nblk) it = DItem();
         }
     };
-    {
-        const int nt = std::max(1, std::min(8, (int)std::thread::hardware_concurrency()));
-        std::vector<std::thread> th;
-        for (int t = 1; t < nt; t++) th.emplace_back(build_items, t, nt);
-        build_items(0, nt);
-        for (auto &t : th) t.join();
-    }
+    const int nt = std::max(1, std::min(8, (int)std::thread::hardware_concurrency()));
+    if (!run_workers(nt, [&](int t) { build_items(t, nt); }))
+        return set_error(GD_ERR_OUT_OF_MEMORY, "host memory for the gain tables");
     int mmax = 0;
     int64_t ktotal = 0;
     for (const DItem &it : items) {
@@ -756,16 +765,12 @@ int orbit_build(Context &c)
     }
     if (!ktotal || !mmax) return GD_OK;
 
-    // tile width: eight cells where their outputs and rows fit, else four
-    int max_smem = 0;
-    GD_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c.device));
-    const int slots = (norb + kOWarps * kOSlots - 1) / (kOWarps * kOSlots) * kOSlots;
     auto orbit_of = [](int w, int j) { return (j / kOSlots * kOWarps + w) * kOSlots + j % kOSlots; };
-    int cpt = 0, nslot = 0, pcap = 0, mcap = 0;
+    int cpt = 0, pcap = 0, mcap = 0;
     for (int w : {8, 4}) {
         if (!orbit_kernel(w, slots, &nslot)) continue;
-        const int rows = (max_smem - (int)kOF - (d.n_pnt + 8) * w * 4) / (32 * w) - 1;  // P and C rows
-        mcap = std::max(mmax, rows * 2 / 5 / kORows * kORows);
+        const int rows = rows_of(w);
+        mcap = std::max(mmax, c_rows(rows));
         pcap = rows - mcap;
         if (pcap >= 64) {
             cpt = w;
@@ -777,7 +782,7 @@ int orbit_build(Context &c)
     const int kstep = std::min(pcap, std::max(32, (int)(ktotal / 96)));
     const uint32_t row_bytes = 32u * (uint32_t)cpt;
 
-    OrbitGain *og = new OrbitGain;
+    std::unique_ptr<OrbitGain> og(new OrbitGain);
     og->cuts.push_back(0);
     og->cost_prefix.push_back(0.0);
     double cost = 0.0;
@@ -956,7 +961,6 @@ int orbit_build(Context &c)
         const int parts = (it.K + kstep - 1) / kstep;
         for (int p = 0; p < parts; p++) {
             if (p == parts - 1 && !add_targets(it)) {
-                delete og;
                 return GD_OK;
             }
             emit({Part{Did, (int)((int64_t)it.K * p / parts), (int)((int64_t)it.K * (p + 1) / parts)}}, p == parts - 1);
@@ -976,7 +980,6 @@ int orbit_build(Context &c)
             }
         }
         if (cur.empty()) {  // a single D that does not fit
-            delete og;
             return GD_OK;
         }
         close();
@@ -997,7 +1000,6 @@ int orbit_build(Context &c)
     size_t total = 0;
     for (const auto &v : ws) total += v.size() + 5 * (kOChunk / 16);
     if (total * 16 >= (size_t)1 << 32) {  // positions are 32-bit
-        delete og;
         return GD_OK;
     }
     stream.reserve(total);
@@ -1010,17 +1012,17 @@ int orbit_build(Context &c)
         std::vector<uint4>().swap(ws[w]);
     }
     og->stream_bytes = stream.size() * 16;
-    c.orbit = og;
-    int rc = upload(&og->row_node, row_node);
-    if (!rc) rc = upload(&og->stream, stream);
+    OrbitGain *built = c.orbit = og.release();  // freed with the context from here on
+    int rc = upload(&built->row_node, row_node);
+    if (!rc) rc = upload(&built->stream, stream);
     std::vector<int> bounds, first;
-    orbit_parts(*og, cost, bounds);
+    orbit_parts(*built, cost, bounds);
     for (int k = 0; k + 1 < (int)bounds.size(); k++)
-        for (int w = 0; w < kOWarps; w++) first.push_back(st[(size_t)std::min(bounds[k], og->nsteps - 1) * kOWarps + w]);
-    og->nparts = (int)bounds.size() - 1;
-    if (!rc) rc = upload(&og->bounds, bounds);
-    if (!rc) rc = upload(&og->start, first);
-    if (!rc) rc = upload(&og->err, std::vector<int>(1, 0));
+        for (int w = 0; w < kOWarps; w++) first.push_back(st[(size_t)std::min(bounds[k], built->nsteps - 1) * kOWarps + w]);
+    built->nparts = (int)bounds.size() - 1;
+    if (!rc) rc = upload(&built->bounds, bounds);
+    if (!rc) rc = upload(&built->start, first);
+    if (!rc) rc = upload(&built->err, std::vector<int>(1, 0));
     if (!rc) rc = orbit_loss_build(c);
     return rc;  // the caller destroys the context on failure
 }
