@@ -153,6 +153,7 @@ def lib():
     L.gd_pair_tables.argtypes = [vp, P(_PairSizes), vp, vp, vp, vp, vp, vp]
     L.gd_pair_tc_table.argtypes = [vp, P(C.c_int64), vp, vp, vp]
     L.gd_ctx_inject_timeout.argtypes = [vp, i]
+    L.gd_mlp_inject_late_timeout.argtypes = L.gd_ctx_inject_late_timeout.argtypes = [vp, i]
     for name in ("gd_grid_count", "gd_grid_fill", "gd_ctx_create", "gd_ctx_destroy", "gd_ctx_info",
                  "gd_export_tables", "gd_correction_basis", "gd_collision", "gd_project",
                  "gd_relax", "gd_step", "gd_moments", "gd_ctx_check", "gd_set_memory_limit", "gd_gain_noalloc",
@@ -163,7 +164,8 @@ def lib():
                  "gd_surrogate_create", "gd_surrogate_destroy", "gd_surrogate_gain", "gd_cell_rel_l2",
                  "gd_cmatrix_check", "gd_batch_create", "gd_batch_destroy", "gd_batch_add", "gd_batch_step",
                  "gd_batch_check", "gd_batch_info", "gd_batch_set_mode", "gd_ctx_autotune", "gd_fma_peak",
-                 "gd_mlp_inject_timeout", "gd_ctx_inject_timeout", "gd_pair_tables", "gd_pair_tc_table"):
+                 "gd_mlp_inject_timeout", "gd_ctx_inject_timeout", "gd_mlp_inject_late_timeout",
+                 "gd_ctx_inject_late_timeout", "gd_pair_tables", "gd_pair_tc_table"):
         getattr(L, name).restype = i
     _lib = L
     return L
@@ -350,10 +352,12 @@ class Context:
                                       out["wl"].ctypes.data))
         return out
 
-    def inject_timeout(self, polls: int):
+    def inject_timeout(self, polls: int, late: bool = False):
         """Failure-detection test hook: the next tensor-core loss GEMM's bounded
-        wait runs out after `polls` polls; check() then reports it."""
-        _check(lib().gd_ctx_inject_timeout(self._h, int(polls)))
+        wait runs out after `polls` polls (late: its epilogue's, with copies and
+        MMAs in flight); check() then reports it."""
+        L = lib()
+        _check((L.gd_ctx_inject_late_timeout if late else L.gd_ctx_inject_timeout)(self._h, int(polls)))
 
 
 class CollisionMatrix:
@@ -428,10 +432,12 @@ class Mlp:
     def check(self, stream=None):
         _check(lib().gd_mlp_check(self._h, _stream(stream)))
 
-    def inject_timeout(self, polls: int):
+    def inject_timeout(self, polls: int, late: bool = False):
         """Failure-detection test hook: the next forward pass's first GEMM has
-        its bounded wait run out after `polls` polls; check() then reports it."""
-        _check(lib().gd_mlp_inject_timeout(self._h, int(polls)))
+        its bounded wait run out after `polls` polls (late: its epilogue's, with
+        copies and MMAs in flight); check() then reports it."""
+        L = lib()
+        _check((L.gd_mlp_inject_late_timeout if late else L.gd_mlp_inject_timeout)(self._h, int(polls)))
 
     def get_params(self):
         import numpy as np

@@ -263,16 +263,13 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
                 j += len;
             }
-            if (PAIR) {
-                // tail, bounded like every wait: the copies of the last stages have
-                // landed, and the pair MMAs that read them have completed (their
-                // commits have arrived here), before this CTA may leave the pair;
-                // after a time-out the waits give up at once
-                const int j0 = it > S ? it - S : 0;
-                for (int j = j0; j < it; j++)
-                    if (!mbar_wait(smem_u32(&full_bar[j % S]), (uint32_t)(j / S) & 1u, p.err)) break;
-                for (int j = j0; j < it; j++)
-                    if (!mbar_wait(smem_u32(&empty_bar[j % S]), (uint32_t)(j / S) & 1u, p.err)) break;
+            // tail, bounded like every wait: the copies of the last stages have
+            // landed, and the MMAs that read them have completed (their commits
+            // have arrived here), before this CTA may leave (the pair); after a
+            // time-out the waits run out by themselves
+            for (int j = it > S ? it - S : 0; j < it; j++) {
+                mbar_wait(smem_u32(&full_bar[j % S]), (uint32_t)(j / S) & 1u, p.err);
+                mbar_wait(smem_u32(&empty_bar[j % S]), (uint32_t)(j / S) & 1u, p.err);
             }
         }
     } else if (warp == 1 && PAIR && !leader) {
@@ -363,6 +360,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                 grp++;
             }
             if (!ok) abort_flag = 1;
+            // no arrival is on its way when the CTA (or the pair) leaves
+            for (int b = max(0, grp - 2); b < grp; b++)
+                mbar_wait(smem_u32(&accf_bar[b & 1]), (uint32_t)(b >> 1) & 1u, p.err);
         }
     } else if (warp >= 2) {
         // ---- epilogue: warps 2..9; warp % 4 is the TMEM lane quadrant it may
@@ -647,7 +647,7 @@ struct gd_cmatrix {
     uint32_t *mnodes = nullptr;
     __nv_bfloat16 *bh = nullptr, *bl = nullptr;  // loss matrix [node][ns_k] BF16 hi / lo
     int *err = nullptr;
-    int stall_next = 0;  // gd_ctx_inject_timeout: polls for the next tensor-core loss GEMM
+    int stall_next = 0;  // gd_ctx_inject_timeout: polls for the next tensor-core loss GEMM (late: negative)
     // stored tiles per tensor-memory accumulation of the gain (gd_cmatrix_set_chain)
     int chain = gd::kChainUnlimited;
     bool loss_only = false;  // the loss matrix alone (cmatrix_create_loss_only)
@@ -1157,6 +1157,13 @@ extern "C" int gd_ctx_inject_timeout(gd_ctx *ctx, int polls)
     return GD_OK;
 }
 
+extern "C" int gd_ctx_inject_late_timeout(gd_ctx *ctx, int polls)
+{
+    const int rc = gd_ctx_inject_timeout(ctx, polls);
+    if (!rc) ctx->c.cmatrix->stall_next = -polls;
+    return rc;
+}
+
 namespace gd {
 // Reads the collision-matrix time-out record on st (synchronising) and clears
 // it; *timed_out receives whether it was set.
@@ -1259,7 +1266,7 @@ int run_loss_path(Context &c, const float *f, int ncells, int ld, float *nu, cud
     // about 1e-6 low, which only a gain from the same sums balances in the
     // projection (20^3, 4096 cells: 2.5 ms against 0.34, of 75; one cell 0.016
     // against 0.05).  A pending time-out injection is for the tensor cores' GEMM.
-    if (c.gain_path != GD_GAIN_PAIR && c.cmatrix && (!orbit_serves(c, c.gain_path) || c.cmatrix->stall_next > 0)) {
+    if (c.gain_path != GD_GAIN_PAIR && c.cmatrix && (!orbit_serves(c, c.gain_path) || c.cmatrix->stall_next != 0)) {
         const int rc = cmatrix_loss(c.cmatrix, f, ncells, ld, nu, st);
         if (rc != GD_ERR_UNSUPPORTED) return rc;
     }

@@ -62,7 +62,8 @@ struct GemmArgs {
     int *err;
     // failure-detection test hook: > 0 makes every CTA wait this many polls on
     // a barrier that nothing arrives at (before any copy or MMA is issued),
-    // record the time-out, free its tensor memory and return
+    // record the time-out, free its tensor memory and return; < 0 makes its
+    // epilogue do so, with copies and MMAs in flight
     int stall_polls;
 };
 
@@ -70,6 +71,21 @@ __device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.f + erff(x
 __device__ __forceinline__ float gelu_grad(float x)
 {
     return 0.5f * (1.f + erff(x * 0.70710678118654752f)) + x * 0.39894228040143268f * expf(-0.5f * x * x);
+}
+
+// After a time-out: the producer (thread 0, which has begun that many stages of the
+// ring) waits for its last copies and for the MMAs that read them, the MMA thread (32)
+// for the arrivals of its last accumulators.
+__device__ __noinline__ void drain(int thread, int begun, int stages, uint64_t *full, uint64_t *empty, uint64_t *accf, int *err)
+{
+    if (thread == 0)
+        for (int j = max(0, begun - stages); j < begun; j++) {
+            mbar_wait(smem_u32(full + j % stages), (uint32_t)(j / stages) & 1u, err);
+            mbar_wait(smem_u32(empty + j % stages), (uint32_t)(j / stages) & 1u, err);
+        }
+    if (thread == 32)
+        for (int j = max(0, begun - 2); j < begun; j++)
+            mbar_wait(smem_u32(accf + (j & 1)), (uint32_t)(j >> 1) & 1u, err);
 }
 
 // The products of one launch: G of one K, their tiles one after another.
@@ -116,9 +132,10 @@ __global__ void __launch_bounds__(kGThreads, 1) gemm_nt_kernel(const __grid_cons
     unsigned char *base = epi + kEpiBytes;
     __shared__ __align__(8) uint64_t full_bar[kGMaxStages], empty_bar[kGMaxStages], accf_bar[2], acce_bar[2], stall_bar;
     __shared__ uint32_t tmem_holder;
-    __shared__ int abort_flag;
+    __shared__ int abort_flag, gave_up;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int num_k = p.K / GK, GS = p.stages, KPS = p.kps;
+    int begun = 0;  // the producer's stages, the MMA thread's accumulators
+    const int num_k = p.K / GK, GS = p.stages, KPS = p.kps, late = max(0, -p.stall_polls);
     const int tiles = set.end[G - 1];
     // product, first row and first column of a tile
     auto locate = [&](int t, int *g, int *m0, int *n0) {
@@ -136,6 +153,7 @@ __global__ void __launch_bounds__(kGThreads, 1) gemm_nt_kernel(const __grid_cons
     __syncthreads();
     if (abort_flag) return;
     if (threadIdx.x == 0) {
+        gave_up = 0;
         for (int s = 0; s < GS; s++) {
             mbar_init(smem_u32(&full_bar[s]), 1);
             mbar_init(smem_u32(&empty_bar[s]), 1);
@@ -173,7 +191,7 @@ __global__ void __launch_bounds__(kGThreads, 1) gemm_nt_kernel(const __grid_cons
     } else if (warp == 0) {
         if (lane == 0) {
             bool ok = true;
-            int s = 0, issued = 0;
+            int s = 0;
             uint32_t ph = 0;
             for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
                 int g, m0, n0;
@@ -191,18 +209,14 @@ __global__ void __launch_bounds__(kGThreads, 1) gemm_nt_kernel(const __grid_cons
                         tma_load_2d(st, &set.a[g], (k + q) * GK, m0, fb);
                         tma_load_2d(st + kA, &set.b[g], (k + q) * GK, n0, fb);
                     }
-                    issued++;
+                    begun++;
                     if (++s == GS) {
                         s = 0;
                         ph ^= 1u;
                     }
                 }
             }
-            // after a time-out the copies in flight land (or this wait gives up too)
-            // before the CTA leaves; otherwise the accumulators were waited for
-            if (!ok || *(volatile int *)p.err)
-                for (int j = max(0, issued - GS); j < issued; j++)
-                    mbar_wait(smem_u32(&full_bar[j % GS]), (uint32_t)(j / GS) & 1u, p.err);
+            if (!ok) gave_up = 1;
         }
     } else if (warp == 1) {
         if (lane == 0) {
@@ -211,7 +225,10 @@ __global__ void __launch_bounds__(kGThreads, 1) gemm_nt_kernel(const __grid_cons
             uint32_t ph = 0;
             for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x, i++) {
                 const int buf = i & 1;
-                if (!mbar_wait(smem_u32(&acce_bar[buf]), ((uint32_t)(i >> 1) & 1u) ^ 1u, p.err)) break;
+                if (!mbar_wait(smem_u32(&acce_bar[buf]), ((uint32_t)(i >> 1) & 1u) ^ 1u, p.err)) {
+                    ok = false;
+                    break;
+                }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 for (int k = 0; k < num_k; k += KPS) {
                     if (!mbar_wait(smem_u32(&full_bar[s]), ph, p.err)) {
@@ -235,8 +252,12 @@ __global__ void __launch_bounds__(kGThreads, 1) gemm_nt_kernel(const __grid_cons
                         ph ^= 1u;
                     }
                 }
-                if (ok) umma_commit(smem_u32(&accf_bar[buf]));
+                if (ok) {
+                    umma_commit(smem_u32(&accf_bar[buf]));
+                    begun++;
+                }
             }
+            if (!ok) gave_up = 1;
         }
     } else {
         const int quad = warp & 3;
@@ -263,8 +284,13 @@ __global__ void __launch_bounds__(kGThreads, 1) gemm_nt_kernel(const __grid_cons
             load_extra(n0 + lane);
             const int buf = i & 1;
             bool ok = true;
-            if (lane == 0) ok = mbar_wait(smem_u32(&accf_bar[buf]), (uint32_t)(i >> 1) & 1u, p.err);
-            if (__shfl_sync(0xffffffffu, ok ? 1 : 0, 0) == 0) break;
+            if (lane == 0)
+                ok = mbar_wait_limit(late ? smem_u32(&stall_bar) : smem_u32(&accf_bar[buf]), (uint32_t)(i >> 1) & 1u, p.err,
+                                     late ? (uint32_t)late : kWaitPolls);
+            if (__shfl_sync(0xffffffffu, ok ? 1 : 0, 0) == 0) {
+                gave_up = 1;
+                break;
+            }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * GN);
 #pragma unroll 1
@@ -316,6 +342,13 @@ __global__ void __launch_bounds__(kGThreads, 1) gemm_nt_kernel(const __grid_cons
         }
     }
     __syncthreads();
+    if (gave_up) {
+        // a wait of this CTA timed out: the copies in flight land, the MMAs that
+        // read them and the arrivals on their way are done before it leaves (waits
+        // that run out by themselves too)
+        drain(threadIdx.x, begun, GS, full_bar, empty_bar, accf_bar, p.err);
+        __syncthreads();
+    }
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * GN) : "memory");
@@ -353,16 +386,18 @@ __global__ void __launch_bounds__(kGThreads, 1)
         (reinterpret_cast<uintptr_t>(dsmem) + 1023) & ~static_cast<uintptr_t>(1023));
     __shared__ __align__(8) uint64_t full_bar[XS], empty_bar[XS], accf_bar[2], acce_bar[2], stall_bar;
     __shared__ uint32_t tmem_holder;
-    __shared__ int abort_flag;
+    __shared__ int abort_flag, gave_up;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int begun = 0;  // as in gemm_nt_kernel
     const int m0 = blockIdx.x * XM, n0 = blockIdx.y * XN;
-    const int num_k = p.K / GK, kcs = p.kchunk / GK;
+    const int num_k = p.K / GK, kcs = p.kchunk / GK, late = max(0, -p.stall_polls);
     const int nchunks = (num_k + kcs - 1) / kcs;
 
     if (threadIdx.x == 0) abort_flag = *(volatile int *)p.err;
     __syncthreads();
     if (abort_flag) return;
     if (threadIdx.x == 0) {
+        gave_up = 0;
         for (int s = 0; s < XS; s++) {
             mbar_init(smem_u32(&full_bar[s]), 1);
             mbar_init(smem_u32(&empty_bar[s]), 1);
@@ -400,7 +435,10 @@ __global__ void __launch_bounds__(kGThreads, 1)
             for (int k = 0; k < num_k; k++) {
                 const int s = k % XS;
                 const uint32_t ph = (uint32_t)(k / XS) & 1u;
-                if (!mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1u, p.err)) break;
+                if (!mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1u, p.err)) {
+                    gave_up = 1;
+                    break;
+                }
                 unsigned char *st = base + (size_t)s * kXStage;
                 const uint32_t fb = smem_u32(&full_bar[s]);
                 mbar_expect_tx(fb, kXStage);
@@ -408,6 +446,7 @@ __global__ void __launch_bounds__(kGThreads, 1)
                 tma_load_2d(smem_u32(st + kXA), &tAl, k * GK, m0, fb);
                 tma_load_2d(smem_u32(st + 2 * kXA), &tBh, k * GK, n0, fb);
                 tma_load_2d(smem_u32(st + 2 * kXA + kXB), &tBl, k * GK, n0, fb);
+                begun++;
             }
         }
     } else if (warp == 1) {
@@ -442,8 +481,12 @@ __global__ void __launch_bounds__(kGThreads, 1)
                     }
                     umma_commit(smem_u32(&empty_bar[s]));
                 }
-                if (ok) umma_commit(smem_u32(&accf_bar[buf]));
+                if (ok) {
+                    umma_commit(smem_u32(&accf_bar[buf]));
+                    begun++;
+                }
             }
+            if (!ok) gave_up = 1;
         }
     } else {
         const int quad = warp & 3;
@@ -455,9 +498,12 @@ __global__ void __launch_bounds__(kGThreads, 1)
         for (int c = 0; ok && c < nchunks; c++) {
             const int buf = c & 1;
             bool w = true;
-            if (lane == 0) w = mbar_wait(smem_u32(&accf_bar[buf]), (uint32_t)(c >> 1) & 1u, p.err);
+            if (lane == 0)
+                w = mbar_wait_limit(late ? smem_u32(&stall_bar) : smem_u32(&accf_bar[buf]), (uint32_t)(c >> 1) & 1u, p.err,
+                                    late ? (uint32_t)late : kWaitPolls);
             if (__shfl_sync(0xffffffffu, w ? 1 : 0, 0) == 0) {
                 ok = false;
+                gave_up = 1;
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -489,6 +535,10 @@ __global__ void __launch_bounds__(kGThreads, 1)
         }
     }
     __syncthreads();
+    if (gave_up) {
+        drain(threadIdx.x, begun, XS, full_bar, empty_bar, accf_bar, p.err);
+        __syncthreads();
+    }
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * XN) : "memory");
@@ -1044,7 +1094,7 @@ struct gd_mlp {
     float in_gain = 1.f, out_gain = 1.f;  // global input / output normalisation
     Layer L[5];
     int64_t step = 0;
-    int stall_next = 0;  // gd_mlp_inject_timeout: polls for the next forward's first GEMM
+    int stall_next = 0;  // gd_mlp_inject_timeout: polls for the next forward's first GEMM (late: negative)
     // activations, [cap][features]
     bf16 *xb = nullptr, *h0b = nullptr, *h1b = nullptr, *h2b = nullptr, *zb = nullptr;
     float *h0 = nullptr, *a1 = nullptr, *a2 = nullptr, *y = nullptr;
@@ -1562,4 +1612,11 @@ extern "C" int gd_mlp_inject_timeout(gd_mlp *h, int polls)
         return set_error(GD_ERR_INVALID_ARG, "gd_mlp_inject_timeout: need a network and 1 <= polls <= 2^20");
     h->stall_next = polls;
     return GD_OK;
+}
+
+extern "C" int gd_mlp_inject_late_timeout(gd_mlp *h, int polls)
+{
+    const int rc = gd_mlp_inject_timeout(h, polls);
+    if (!rc) h->stall_next = -polls;
+    return rc;
 }

@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(kPtThreads, 1)
     unsigned char *base = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(dsmem) + 1023) & ~static_cast<uintptr_t>(1023));
     int16_t *cmap_s = reinterpret_cast<int16_t *>(base + kPtStages * kPtStage);
-    __shared__ __align__(8) uint64_t full_bar[kPtStages], empty_bar[kPtStages], accf_bar[2], acce_bar[2];
+    __shared__ __align__(8) uint64_t full_bar[kPtStages], w_bar[kPtStages], empty_bar[kPtStages], accf_bar[2], acce_bar[2];
     __shared__ uint32_t tmem_base_holder;
     __shared__ int epi_fail;
     __shared__ int unit_slot, stop_flag;
@@ -179,7 +179,8 @@ __global__ void __launch_bounds__(kPtThreads, 1)
         epi_fail = 0;
         stop_flag = 0;
         for (int s = 0; s < kPtStages; s++) {
-            mbar_init(smem_u32(&full_bar[s]), 4 + 1);  // four producer warps + the TMA arrival
+            mbar_init(smem_u32(&full_bar[s]), 4);   // the products: four producer warps
+            mbar_init(smem_u32(&w_bar[s]), 1);      // the weight rows: the TMA arrival
             mbar_init(smem_u32(&empty_bar[s]), 1);      // the MMA commit
         }
         for (int b = 0; b < 2; b++) {
@@ -237,7 +238,7 @@ __global__ void __launch_bounds__(kPtThreads, 1)
                             break;
                         }
                         unsigned char *sb = base + (size_t)st * kPtStage;
-                        const uint32_t fb = smem_u32(&full_bar[st]);
+                        const uint32_t fb = smem_u32(&w_bar[st]);
                         mbar_expect_tx(fb, 2u * (uint32_t)u.npad * (PT_KC * 2));
                         const int row0 = u.wrow + ch * u.mpad + q * PT_NMAX;
                         for (int r = 0; r < u.npad; r += 16) {
@@ -269,7 +270,8 @@ __global__ void __launch_bounds__(kPtThreads, 1)
                     const uint32_t idesc = umma_idesc_bf16(PT_BM, u.npad);
                     for (int ch = 0; ch < u.nch; ch++, ck++) {
                         const int st = ck & 1;
-                        if (!mbar_wait(smem_u32(&full_bar[st]), (uint32_t)(ck >> 1) & 1u, L.err)) {
+                        if (!mbar_wait(smem_u32(&w_bar[st]), (uint32_t)(ck >> 1) & 1u, L.err) ||
+                            !mbar_wait(smem_u32(&full_bar[st]), (uint32_t)(ck >> 1) & 1u, L.err)) {
                             ok = false;
                             break;
                         }
@@ -470,6 +472,15 @@ __global__ void __launch_bounds__(kPtThreads, 1)
     // the unit is done in every role before unit_slot is written again
     __syncthreads();
     }  // units
+    // the copies have landed and the MMAs that read them are done before the CTA
+    // leaves; after a time-out these waits run out by themselves
+    if (threadIdx.x == 32)
+        for (int j = max(0, uc - 2); j < uc; j++) mbar_wait(smem_u32(&accf_bar[j & 1]), (uint32_t)(j >> 1) & 1u, L.err);
+    if (threadIdx.x == 0)
+        for (int j = max(0, ck - kPtStages); j < ck; j++) {
+            mbar_wait(smem_u32(&w_bar[j & 1]), (uint32_t)(j >> 1) & 1u, L.err);
+            mbar_wait(smem_u32(&empty_bar[j & 1]), (uint32_t)(j >> 1) & 1u, L.err);
+        }
     __syncthreads();
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

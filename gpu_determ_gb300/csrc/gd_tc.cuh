@@ -64,9 +64,10 @@ __device__ __forceinline__ bool mbar_wait_limit(uint32_t bar, uint32_t parity, i
 }
 
 // The pipeline waits of every kernel: 2^20 polls.
+constexpr uint32_t kWaitPolls = 1u << 20;
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int *err)
 {
-    return mbar_wait_limit(bar, parity, err, 1u << 20);
+    return mbar_wait_limit(bar, parity, err, kWaitPolls);
 }
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int c0, int c1, uint32_t bar)

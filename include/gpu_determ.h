@@ -432,10 +432,14 @@ int gd_pair_tc_table(gd_ctx *ctx, int64_t *rows, int *wrow, uint16_t *wh, uint16
  * next forward pass or training step) or gd_ctx_check (for
  * gd_ctx_inject_timeout: the first GEMM of the next tensor-core loss of a
  * context on a collision-matrix gain path, else GD_ERR_UNSUPPORTED).  The
- * call after that computes normally.  No reference counterpart: the
+ * call after that computes normally.  The late forms make each CTA's epilogue
+ * wait so instead, with copies and MMAs in flight; the CTA leaves when these are
+ * done.  No reference counterpart: the
  * reference has no failure handling (collision_integral.cu:601,622). */
 int gd_mlp_inject_timeout(gd_mlp *net, int polls);
 int gd_ctx_inject_timeout(gd_ctx *ctx, int polls);
+int gd_mlp_inject_late_timeout(gd_mlp *net, int polls);
+int gd_ctx_inject_late_timeout(gd_ctx *ctx, int polls);
 
 /* Measured fused multiply-add throughput of `device` in FLOP/s (2 per FMA),
  * precision 32 (FP32 FFMA) or 64 (FP64 DFMA): the roofline denominator of the
