@@ -1278,7 +1278,7 @@ int run_gain_path(Context &c, const float *f, int ncells, int ld, float *gain, c
     if (orbit_serves(c, c.gain_path)) {
         if (c.gain_path == GD_GAIN_PAIR_TC && (int64_t)c.d.n_pnt * ld >= ((int64_t)1 << 31))
             return set_error(GD_ERR_UNSUPPORTED, "pair gain: n_pnt * ld must stay below 2^31");
-        return run_orbit(c, f, ncells, ld, gain, true, st);
+        return run_orbit(c, f, ncells, ld, gain, st);
     }
     if (c.gain_path == GD_GAIN_PAIR_TC && c.pair_tc) return run_pair_tc(c, f, ncells, ld, gain, st);
     if (c.gain_path == GD_GAIN_PAIR || !c.cmatrix) return run_gain(c, f, ncells, ld, gain, st);

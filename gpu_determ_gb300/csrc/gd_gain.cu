@@ -313,7 +313,11 @@ int gain_bounds_device(Context &c, int nchunks, const int **out)
 
 int run_gain(Context &c, const float *f, int ncells, int ld, float *gain, cudaStream_t st)
 {
-    if (c.orbit) return run_orbit(c, f, ncells, ld, gain, false, st);
+    if (c.orbit) {
+        if ((int64_t)c.d.n_pnt * ld >= ((int64_t)1 << 31))
+            return set_error(GD_ERR_UNSUPPORTED, "pair gain: n_pnt * ld must stay below 2^31");
+        return run_orbit(c, f, ncells, ld, gain, st);
+    }
     const Dims &d = c.d;
     int cb = 0, nblk = 0, nchunks = 0;
     size_t smem = 0;

@@ -227,8 +227,8 @@ int orbit_loss_build(Context &c);  // its loss table (gd_loss.cu)
 void orbit_free(Context &c);
 size_t orbit_bytes(const Context &c, int ncells);
 int orbit_slice(const Context &c, int ncells, size_t room);
-int launch_orbit(Context &c, const float *f, int ncells, int ld, float *gain, void *buf, float2 *scale, cudaStream_t st);
-int run_orbit(Context &c, const float *f, int ncells, int ld, float *gain, bool guard, cudaStream_t st);
+int launch_orbit(Context &c, const float *f, int ncells, int ld, float *gain, void *buf, cudaStream_t st);
+int run_orbit(Context &c, const float *f, int ncells, int ld, float *gain, cudaStream_t st);
 bool orbit_serves(const Context &c, int path);  // whether run_orbit computes this path's gain
 // reads (synchronising st) and clears its pipeline time-out record
 int orbit_take_timeout(Context &c, cudaStream_t st, bool *timed_out);

@@ -114,11 +114,15 @@ extern "C" int gd_gain_noalloc(gd_ctx *ctx, const float *f, int ncells, int ld, 
         if (c.orbit) {
             // gd_collision's sums, in slices of cells that fit (a tile of cells
             // does: its rows, for f and at most 152 parts of the walk, are 20 MB)
+            if ((int64_t)c.d.n_pnt * ld >= ((int64_t)1 << 31)) {
+                rc = set_error(GD_ERR_UNSUPPORTED, "pair gain: n_pnt * ld must stay below 2^31");
+                break;
+            }
             if ((rc = scratch_address(c.device, &base))) break;
             const int slice = orbit_slice(c, ncells, room);
             for (int at = 0; at < ncells && !rc; at += slice)
                 rc = launch_orbit(c, f + at, std::min(slice, ncells - at), ld, gain + at,
-                                  static_cast<unsigned char *>(base) + kHeaderBytes, nullptr, st);
+                                  static_cast<unsigned char *>(base) + kHeaderBytes, st);
             break;
         }
         const int nchunks = std::min(want, fit);

@@ -83,7 +83,7 @@ struct OrbitArgs {
     const int *row_node;
     float *part;                  // [part][tile][row][CPT], or null (one part): write gain
     float *gain;
-    const float2 *scale;          // [cells_pad] power-of-two factors of f and back, or null
+    const float2 *scale;          // [cells_pad] power-of-two factors of f and back
     int *err;                     // set to 1 when a copy is not seen to land
     int norb, ns, ncells, ld;
     uint32_t p_at, zero_at;       // shared-memory offsets of the P rows and of the zero C row
@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(kOThreads, 1) orbit_gain_kernel(const __grid_c
                 const float *v = reinterpret_cast<const float *>(&acc[j]);
 #pragma unroll
                 for (int q = 0; q < CPT / 4; q++)
-                    if (cell + q < a.ncells) g[q] = a.scale ? unscale(v[q], a.scale[cell + q].y) : v[q];
+                    if (cell + q < a.ncells) g[q] = unscale(v[q], a.scale[cell + q].y);
             }
         }
     } else {  // a part without steps (more parts than work): zero sums
@@ -436,21 +436,23 @@ __global__ void __launch_bounds__(kOThreads, 1) orbit_gain_kernel(const __grid_c
 
 // scale[cell] = {2^-k, 2^k} for max|f| of the cell in [2^k, 2^(k+1)) where that
 // is beyond 2^+-40 (products could leave FP32's range), {1, 1} for the others,
-// {1, NaN} for a cell with a non-finite f.  Block = 32 cells x 32 node strides: 16 MB of
-// loads in flight at 4096 cells.
+// {1, NaN} for a cell with a non-finite f.  Block = 32 cells x 32 node strides (16 MB
+// of loads in flight at 4096 cells), for few cells 4 x 256 (one cell: 10 -> 6 us).
 __global__ void __launch_bounds__(1024) orbit_scale_kernel(const float *__restrict__ f, int ld, int ncells, int ns,
                                                            float2 *__restrict__ scale, int cells_pad)
 {
-    __shared__ unsigned red[32][32];
-    const int x = threadIdx.x, y = threadIdx.y, cell = blockIdx.x * 32 + x;
+    __shared__ unsigned red[1024];
+    const int w = blockDim.x, x = threadIdx.x, y = threadIdx.y, cell = blockIdx.x * w + x;
     unsigned m = 0;  // bit patterns of |f| order like the values, infinity and NaN above all
     if (cell < ncells)
 #pragma unroll 8
-        for (int p = y; p < ns; p += 32) m = max(m, __float_as_uint(__ldg(f + (size_t)p * ld + cell)) & 0x7fffffffu);
-    red[y][x] = m;
-    __syncthreads();
+        for (int p = y; p < ns; p += blockDim.y) m = max(m, __float_as_uint(__ldg(f + (size_t)p * ld + cell)) & 0x7fffffffu);
+    red[y * w + x] = m;
+    for (int h = blockDim.y / 2; h > 0; h /= 2) {
+        __syncthreads();
+        if (y < h) red[y * w + x] = m = max(m, red[(y + h) * w + x]);
+    }
     if (y == 0 && cell < cells_pad) {
-        for (int k = 1; k < 32; k++) m = max(m, red[k][x]);
         const int e = (int)(m >> 23);  // 0: zero or subnormal, 255: not finite
         int k = e == 0 ? -126 : min(126, e - 127);
         if (m == 0 || abs(k) <= 40) k = 0;
@@ -468,7 +470,7 @@ __global__ void orbit_pack_kernel(const float *__restrict__ f, int ld, int ncell
     const int cell = blockIdx.x * 32 + threadIdx.x, row = blockIdx.y * 8 + threadIdx.y;
     if (row >= ns || cell >= cells_pad) return;
     float v = cell < ncells ? f[(size_t)__ldg(row_node + row) * ld + cell] : 0.f;
-    if (scale) v = __fmul_rn(v, scale[cell].x);
+    v = __fmul_rn(v, scale[cell].x);
     ft[((size_t)(cell / cpt) * ns + row) * cpt + cell % cpt] = v;
 }
 
@@ -509,7 +511,7 @@ __global__ void __launch_bounds__(256) orbit_reduce_kernel(const float4 *__restr
     const float o[4] = {s.x, s.y, s.z, s.w};
 #pragma unroll
     for (int q = 0; q < 4; q++)
-        if (cell + q < ncells) g[q] = scale ? unscale(o[q], scale[cell + q].y) : o[q];
+        if (cell + q < ncells) g[q] = unscale(o[q], scale[cell + q].y);
 }
 
 // One D of the low octant with anything to do.
@@ -1027,11 +1029,13 @@ int orbit_build(Context &c)
     return rc;  // the caller destroys the context on failure
 }
 
-// bytes of packed f and of the parts' sums (one part writes the gain itself)
+// bytes of packed f, of the parts' sums (one part writes the gain itself) and of the
+// cells' scales
 size_t orbit_bytes(const Context &c, int ncells)
 {
     const OrbitGain &g = *c.orbit;
-    return (size_t)((ncells + g.cpt - 1) / g.cpt * g.cpt) * c.d.n_pnt * sizeof(float) * (g.nparts > 1 ? 1 + g.nparts : 1);
+    return (size_t)((ncells + g.cpt - 1) / g.cpt * g.cpt) *
+           (c.d.n_pnt * sizeof(float) * (g.nparts > 1 ? 1 + g.nparts : 1) + sizeof(float2));
 }
 
 // Cells of a launch for a batch of ncells in at most `room` bytes (a tile at
@@ -1043,22 +1047,25 @@ int orbit_slice(const Context &c, int ncells, size_t room)
     return (tiles + slices - 1) / slices * cpt;
 }
 
-// buf holds orbit_bytes; scale is null or one entry per
-// cell of the padded tiles.
-int launch_orbit(Context &c, const float *f, int ncells, int ld, float *gain, void *buf, float2 *scale, cudaStream_t st)
+// buf holds orbit_bytes.  A cell whose f is so large or small that products would
+// leave FP32's range is scaled by a power of two (orbit_scale_kernel), and a cell with
+// a non-finite f gets NaN for all its outputs; other cells' bits are as without.
+// (The contraction multiplies products by the zero weights of its blocks' other rows:
+// an infinite one would spread.)
+int launch_orbit(Context &c, const float *f, int ncells, int ld, float *gain, void *buf, cudaStream_t st)
 {
     OrbitGain &g = *c.orbit;
     const Dims &d = c.d;
     const int tiles = (ncells + g.cpt - 1) / g.cpt, cells_pad = tiles * g.cpt;
-    if ((int64_t)d.n_pnt * (scale ? cells_pad : std::max(ld, cells_pad)) >= ((int64_t)1 << 31))
-        return set_error(GD_ERR_UNSUPPORTED, "pair gain: n_pnt * ld must stay below 2^31");
+    if ((int64_t)d.n_pnt * cells_pad >= ((int64_t)1 << 31))
+        return set_error(GD_ERR_UNSUPPORTED, "FP32 gain: n_pnt * cells must stay below 2^31");
     float *ft = static_cast<float *>(buf);
     const int nparts = g.nparts;
     float *part = nparts > 1 ? ft + (size_t)cells_pad * d.n_pnt : nullptr;
-    if (scale) {
-        orbit_scale_kernel<<<(cells_pad + 31) / 32, dim3(32, 32), 0, st>>>(f, ld, ncells, d.n_pnt, scale, cells_pad);
-        GD_CUDA(cudaGetLastError());
-    }
+    float2 *scale = reinterpret_cast<float2 *>(ft + (size_t)cells_pad * d.n_pnt * (nparts > 1 ? 1 + nparts : 1));
+    const int sx = cells_pad <= 4 * c.sm_count ? 4 : 32;
+    orbit_scale_kernel<<<(cells_pad + sx - 1) / sx, dim3(sx, 1024 / sx), 0, st>>>(f, ld, ncells, d.n_pnt, scale, cells_pad);
+    GD_CUDA(cudaGetLastError());
     orbit_pack_kernel<<<dim3((cells_pad + 31) / 32, d.n_pnt / 8), dim3(32, 8), 0, st>>>(
         f, ld, ncells, d.n_pnt, g.cpt, g.row_node, scale, ft, cells_pad);
     GD_CUDA(cudaGetLastError());
@@ -1091,21 +1098,13 @@ bool orbit_serves(const Context &c, int path)
     return c.orbit && (path == GD_GAIN_PAIR_TC || (path == GD_GAIN_CMATRIX_BF16X3 && c.d.n_pnt >= kOMatrixNodes));
 }
 
-// With guard a cell whose f is so large or small that products would leave FP32's
-// range is scaled by a power of two (orbit_scale_kernel), and a cell with a
-// non-finite f gets NaN for all its outputs; other cells' bits are the same.
-int run_orbit(Context &c, const float *f, int ncells, int ld, float *gain, bool guard, cudaStream_t st)
+int run_orbit(Context &c, const float *f, int ncells, int ld, float *gain, cudaStream_t st)
 {
-    if (!guard && (int64_t)c.d.n_pnt * ld >= ((int64_t)1 << 31))
-        return set_error(GD_ERR_UNSUPPORTED, "pair gain: n_pnt * ld must stay below 2^31");
     // slices of cells: a cell's sums are the same in any batch
     const int slice = orbit_slice(c, ncells, kOScratch);
-    const size_t bytes = orbit_bytes(c, slice);
-    int rc = ensure_scratch(c, bytes + (guard ? sizeof(float2) * slice : 0));
-    if (rc) return rc;
-    float2 *scale = guard ? reinterpret_cast<float2 *>(static_cast<char *>(c.scratch.ptr) + bytes) : nullptr;
+    int rc = ensure_scratch(c, orbit_bytes(c, slice));
     for (int at = 0; at < ncells && !rc; at += slice)
-        rc = launch_orbit(c, f + at, std::min(slice, ncells - at), ld, gain + at, c.scratch.ptr, scale, st);
+        rc = launch_orbit(c, f + at, std::min(slice, ncells - at), ld, gain + at, c.scratch.ptr, st);
     return rc;
 }
 

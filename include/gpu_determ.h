@@ -231,6 +231,9 @@ int gd_cmatrix_check(gd_cmatrix *cm, gd_stream stream);
  * and an FP32 kernel the loss, of GD_GAIN_CMATRIX_BF16X3 (lattices of 512 nodes or more; the matrices are then
  * not built) and of GD_GAIN_PAIR_TC too: every lattice whose half-box rows fit
  * its shared memory, up to 24^3 with R = 4.8.
+ * That kernel scales a cell whose products would leave FP32's range by a power of
+ * two (its gain is infinite only where it exceeds FP32 itself), and a cell with a
+ * non-finite f gets NaN for all its outputs.
  * The two pair paths need n_pnt * ld < 2^31 (GD_ERR_UNSUPPORTED otherwise). */
 enum { GD_GAIN_PAIR = 0, GD_GAIN_CMATRIX_BF16 = 1, GD_GAIN_CMATRIX_BF16X3 = 2, GD_GAIN_PAIR_TC = 3 };
 int gd_ctx_set_gain_path(gd_ctx *ctx, int path);
