@@ -126,10 +126,10 @@ int check_fused(const gd_batch *b, int mode)
     if (b->groups.size() > 4) return set_error(GD_ERR_UNSUPPORTED, "fused batch: at most 4 groups");
     for (size_t k = 0; k < b->groups.size(); k++) {
         const Context &c = b->groups[k].ctx->c;
-        if (mode == GD_BATCH_FUSED_PAIR_TC && (c.gain_path != GD_GAIN_PAIR_TC || !c.pair_tc))
+        if (mode == GD_BATCH_FUSED_PAIR_TC && (c.gain_path != GD_GAIN_PAIR_TC || (!c.pair_tc && !orbit_serves(c, c.gain_path))))
             return set_error(GD_ERR_UNSUPPORTED, "fused batch: every group's context needs gain path GD_GAIN_PAIR_TC");
         if (mode == GD_BATCH_FUSED_CMATRIX &&
-            (c.gain_path != b->groups[0].ctx->c.gain_path || !c.cmatrix ||
+            (c.gain_path != b->groups[0].ctx->c.gain_path || (!c.cmatrix && !orbit_serves(c, c.gain_path)) ||
              (c.gain_path != GD_GAIN_CMATRIX_BF16 && c.gain_path != GD_GAIN_CMATRIX_BF16X3)))
             return set_error(GD_ERR_UNSUPPORTED,
                              "fused batch: every group's context needs the same collision-matrix gain path");

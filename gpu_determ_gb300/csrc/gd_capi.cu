@@ -487,16 +487,20 @@ int gd_ctx_set_gain_path(gd_ctx *ctx, int path)
     c.cmatrix = nullptr;
     gd::pair_tc_free(c);
     c.gain_path = GD_GAIN_PAIR;
-    if (path == GD_GAIN_PAIR_TC) {
+    if (gd::orbit_serves(c, path)) {
+        // no tables: the FP32 kernels' are the context's.  The weight table, which
+        // gd_pair_tc_table builds when it is asked for, still has to fit the limit
+        const size_t limit = gd::memory_limit();
+        if (path == GD_GAIN_PAIR_TC && limit && gd::pair_tc_bytes(c) > (double)limit)
+            return set_error(GD_ERR_OUT_OF_MEMORY, "pair weight table exceeds the memory limit");
+    } else if (path == GD_GAIN_PAIR_TC) {
         int rc = gd::pair_tc_build(c);
-        // the loss on the tensor cores too (the loss matrix alone), unless both are in FP32
-        if (!rc && !gd::orbit_serves(c, path) && (rc = gd::cmatrix_create_loss_only(ctx, &c.cmatrix)))
-            gd::pair_tc_free(c);
+        // the loss on the tensor cores too (the loss matrix alone)
+        if (!rc && (rc = gd::cmatrix_create_loss_only(ctx, &c.cmatrix))) gd::pair_tc_free(c);
         if (rc) return rc;
     } else if (path != GD_GAIN_PAIR) {
         const int mode = path == GD_GAIN_CMATRIX_BF16 ? GD_CMATRIX_BF16 : GD_CMATRIX_BF16X3;
-        int rc = gd::orbit_serves(c, path) ? gd::cmatrix_create_loss_only(ctx, &c.cmatrix)
-                                           : gd_cmatrix_create(ctx, mode, &c.cmatrix);
+        const int rc = gd_cmatrix_create(ctx, mode, &c.cmatrix);
         if (rc) return rc;
     }
     c.gain_path = path;

@@ -723,8 +723,8 @@ namespace gd {
 
 // The tensor-core loss alone (the loss matrix B in BF16 hi/lo, no collision
 // matrices), for contexts whose gain runs on the pair kernel with its
-// contraction on the tensor cores: nu = B f in one GEMM launch instead of the
-// FP32 loss kernel (20^3, 4096 cells: ~0.3 against 22 ms).  The handle serves
+// contraction on the tensor cores (lattices without orbit rows): nu = B f in one GEMM
+// launch instead of loss_kernel (20^3, 4096 cells: ~0.3 against 22 ms).  The handle serves
 // cmatrix_loss and the time-out records; it has no gain matrices.
 int cmatrix_create_loss_only(gd_ctx *ctx, gd_cmatrix **out)
 {
@@ -1151,16 +1151,18 @@ extern "C" int gd_ctx_inject_timeout(gd_ctx *ctx, int polls)
     using namespace gd;
     if (!ctx || polls < 1 || polls > (1 << 20))
         return set_error(GD_ERR_INVALID_ARG, "gd_ctx_inject_timeout: need a context and 1 <= polls <= 2^20");
-    if (!ctx->c.cmatrix || ctx->c.gain_path == GD_GAIN_PAIR || ctx->c.gain_path == GD_GAIN_PAIR_TC)
-        return set_error(GD_ERR_UNSUPPORTED, "gd_ctx_inject_timeout: the context's gain path has no tensor-core loss");
-    ctx->c.cmatrix->stall_next = polls;
+    Context &c = ctx->c;
+    if (c.gain_path == GD_GAIN_PAIR || c.gain_path == GD_GAIN_PAIR_TC)
+        return set_error(GD_ERR_UNSUPPORTED, "gd_ctx_inject_timeout: the context's gain path is not a collision-matrix one");
+    if (orbit_serves(c, c.gain_path)) c.orbit->stall_next = polls;
+    else c.cmatrix->stall_next = polls;
     return GD_OK;
 }
 
 extern "C" int gd_ctx_inject_late_timeout(gd_ctx *ctx, int polls)
 {
     const int rc = gd_ctx_inject_timeout(ctx, polls);
-    if (!rc) ctx->c.cmatrix->stall_next = -polls;
+    if (!rc && ctx->c.cmatrix) ctx->c.cmatrix->stall_next = -polls;
     return rc;
 }
 
@@ -1265,8 +1267,8 @@ int run_loss_path(Context &c, const float *f, int ncells, int ld, float *nu, cud
     // With the FP32 kernel's gain the loss is FP32 too: the tensor cores' sums are
     // about 1e-6 low, which only a gain from the same sums balances in the
     // projection (20^3, 4096 cells: 2.5 ms against 0.34, of 75; one cell 0.016
-    // against 0.05).  A pending time-out injection is for the tensor cores' GEMM.
-    if (c.gain_path != GD_GAIN_PAIR && c.cmatrix && (!orbit_serves(c, c.gain_path) || c.cmatrix->stall_next != 0)) {
+    // against 0.05): such a context has no loss matrix.
+    if (c.gain_path != GD_GAIN_PAIR && c.cmatrix) {
         const int rc = cmatrix_loss(c.cmatrix, f, ncells, ld, nu, st);
         if (rc != GD_ERR_UNSUPPORTED) return rc;
     }

@@ -70,6 +70,7 @@ struct OrbitGain {
     uint4 *stream = nullptr;
     int *start = nullptr;  // [part][warp] position in the stream, in 16-byte units
     int *err = nullptr;    // set by the kernel when a copy of the stream is not seen to land
+    int stall_next = 0;    // gd_ctx_inject_timeout: polls for the next launch
     int opad = 0;               // orbits padded to the loss kernel's tile
     float4 *bx = nullptr;       // [o'][2][opad] b of two orbits by reflection
     int *bounds = nullptr;      // [nparts + 1] their bounds in steps

@@ -87,6 +87,9 @@ struct OrbitArgs {
     int *err;                     // set to 1 when a copy is not seen to land
     int norb, ns, ncells, ld;
     uint32_t p_at, zero_at;       // shared-memory offsets of the P rows and of the zero C row
+    // failure-detection test hook: > 0 makes every warp wait this many polls, its
+    // first copies in flight, on a barrier that nothing arrives at
+    int stall_polls;
 };
 
 // Two FP32 operations per instruction where a lane holds two cells.
@@ -246,6 +249,14 @@ __global__ void __launch_bounds__(kOThreads, 1) orbit_gain_kernel(const __grid_c
             room -= bytes;
         };
         for (int k = 0; k < 3; k++) fetch();
+        if (a.stall_polls > 0) {
+            const uint32_t never = sm + kOBars + 32 * kOWarps + 8 * warp;
+            if (lane == 0) {
+                tc::mbar_init(never, 1);
+                tc::mbar_wait_limit(never, 0u, a.err, (uint32_t)a.stall_polls);
+            }
+            ok = false;
+        }
         if (warp == 0) sts(slb + a.zero_at, V::zero());  // padding targets read this row
         need(1);
         skip(first & (kOChunk - 1));
@@ -1071,7 +1082,8 @@ int launch_orbit(Context &c, const float *f, int ncells, int ld, float *gain, vo
     GD_CUDA(cudaGetLastError());
     const OrbitArgs a{ft,    reinterpret_cast<const unsigned char *>(g.stream),
                       g.start, g.bounds, g.row_node, part, gain, scale, g.err, g.norb, d.n_pnt, ncells, ld,
-                      g.p_at, g.zero_at};
+                      g.p_at, g.zero_at, g.stall_next};
+    g.stall_next = 0;  // fires once
     int nslot = 0;
     OrbitKernel kern = orbit_kernel(g.cpt, g.nslot, &nslot);
     GD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));

@@ -955,8 +955,13 @@ extern "C" int gd_pair_tc_table(gd_ctx *ctx, int64_t *rows, int *wrow, uint16_t 
     using namespace gd;
     if (!ctx || !rows) return set_error(GD_ERR_INVALID_ARG, "NULL argument");
     Context &c = ctx->c;
-    if (!c.pair_tc) return set_error(GD_ERR_UNSUPPORTED, "the pair tensor-core weight table is not built");
     DeviceGuard g(c.device);
+    // where the FP32 kernel computes the path's gain the table is built for this call
+    if (!c.pair_tc && c.gain_path == GD_GAIN_PAIR_TC) {
+        const int rc = pair_tc_build(c);
+        if (rc) return rc;
+    }
+    if (!c.pair_tc) return set_error(GD_ERR_UNSUPPORTED, "the pair tensor-core weight table is not built");
     *rows = c.pair_tc->rows;
     if (wrow) GD_CUDA(cudaMemcpy(wrow, c.pair_tc->wrow, sizeof(int) * c.d.nxyz, cudaMemcpyDeviceToHost));
     const size_t bytes = (size_t)c.pair_tc->rows * PT_KC * sizeof(__nv_bfloat16);

@@ -229,7 +229,8 @@ int gd_cmatrix_check(gd_cmatrix *cm, gd_stream stream);
  * matrices, so it serves the grids whose collision matrices do not fit).
  * Where the FP32 kernel is faster, and its error no larger, it computes the gain,
  * and an FP32 kernel the loss, of GD_GAIN_CMATRIX_BF16X3 (lattices of 512 nodes or more; the matrices are then
- * not built) and of GD_GAIN_PAIR_TC too: every lattice whose half-box rows fit
+ * not built) and of GD_GAIN_PAIR_TC (whose weight table only gd_pair_tc_table then
+ * builds; a memory limit below its size still refuses the path) too: every lattice whose half-box rows fit
  * its shared memory, up to 24^3 with R = 4.8.
  * That kernel scales a cell whose products would leave FP32's range by a power of
  * two (its gain is infinite only where it exceeds FP32 itself), and a cell with a
@@ -434,10 +435,11 @@ int gd_pair_tc_table(gd_ctx *ctx, int64_t *rows, int *wrow, uint16_t *wh, uint16
  * cleared by gd_mlp_check (for gd_mlp_inject_timeout: the first GEMM of the
  * next forward pass or training step) or gd_ctx_check (for
  * gd_ctx_inject_timeout: the first GEMM of the next tensor-core loss of a
- * context on a collision-matrix gain path, else GD_ERR_UNSUPPORTED).  The
+ * context on a collision-matrix gain path or, where the FP32 kernel computes that
+ * path's gain, its next launch; else GD_ERR_UNSUPPORTED).  The
  * call after that computes normally.  The late forms make each CTA's epilogue
  * wait so instead, with copies and MMAs in flight; the CTA leaves when these are
- * done.  No reference counterpart: the
+ * done (the FP32 kernel waits so in both forms).  No reference counterpart: the
  * reference has no failure handling (collision_integral.cu:601,622). */
 int gd_mlp_inject_timeout(gd_mlp *net, int polls);
 int gd_ctx_inject_timeout(gd_ctx *ctx, int polls);
