@@ -153,6 +153,7 @@ def lib():
     L.gd_pair_tables.argtypes = [vp, P(_PairSizes), vp, vp, vp, vp, vp, vp]
     L.gd_pair_tc_table.argtypes = [vp, P(C.c_int64), vp, vp, vp]
     L.gd_ctx_inject_timeout.argtypes = [vp, i]
+    L.gd_ctx_use_general_kernels.argtypes = [vp]
     L.gd_mlp_inject_late_timeout.argtypes = L.gd_ctx_inject_late_timeout.argtypes = [vp, i]
     for name in ("gd_grid_count", "gd_grid_fill", "gd_ctx_create", "gd_ctx_destroy", "gd_ctx_info",
                  "gd_export_tables", "gd_correction_basis", "gd_collision", "gd_project",
@@ -165,7 +166,7 @@ def lib():
                  "gd_cmatrix_check", "gd_batch_create", "gd_batch_destroy", "gd_batch_add", "gd_batch_step",
                  "gd_batch_check", "gd_batch_info", "gd_batch_set_mode", "gd_ctx_autotune", "gd_fma_peak",
                  "gd_mlp_inject_timeout", "gd_ctx_inject_timeout", "gd_mlp_inject_late_timeout",
-                 "gd_ctx_inject_late_timeout", "gd_pair_tables", "gd_pair_tc_table"):
+                 "gd_ctx_inject_late_timeout", "gd_ctx_use_general_kernels", "gd_pair_tables", "gd_pair_tc_table"):
         getattr(L, name).restype = i
     _lib = L
     return L
@@ -351,6 +352,11 @@ class Context:
         _check(lib().gd_pair_tc_table(self._h, C.byref(rows), out["wrow"].ctypes.data, out["wh"].ctypes.data,
                                       out["wl"].ctypes.data))
         return out
+
+    def use_general_kernels(self):
+        """Test hook: loss and gain by the kernels that serve lattices of more than 1024
+        orbits, on this context from now on; the gain path is GAIN_PAIR again."""
+        _check(lib().gd_ctx_use_general_kernels(self._h))
 
     def inject_timeout(self, polls: int, late: bool = False):
         """Failure-detection test hook: the next tensor-core loss GEMM's bounded

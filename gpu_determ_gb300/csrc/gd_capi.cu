@@ -507,6 +507,15 @@ int gd_ctx_set_gain_path(gd_ctx *ctx, int path)
     return GD_OK;
 }
 
+int gd_ctx_use_general_kernels(gd_ctx *ctx)
+{
+    const int rc = gd_ctx_set_gain_path(ctx, GD_GAIN_PAIR);
+    if (rc) return rc;
+    gd::DeviceGuard g(ctx->c.device);
+    gd::orbit_free(ctx->c);
+    return GD_OK;
+}
+
 int gd_ctx_info(const gd_ctx *ctx, gd_info *out)
 {
     if (!ctx || !out) return set_error(GD_ERR_INVALID_ARG, "NULL argument");

@@ -426,6 +426,12 @@ int gd_pair_tables(gd_ctx *ctx, gd_pair_table_sizes *sizes, int *grp_row_off, in
                    int *item_off, int *items, uint32_t *members);
 int gd_pair_tc_table(gd_ctx *ctx, int64_t *rows, int *wrow, uint16_t *wh, uint16_t *wl);
 
+/* Test hook: drops the context's tables by orbits of the lattice's reflections.  From
+ * then on its loss and gain come from the kernels that serve the lattices of more than
+ * 1024 orbits (and from the collision matrices), whatever its size; the gain path is
+ * GD_GAIN_PAIR again. */
+int gd_ctx_use_general_kernels(gd_ctx *ctx);
+
 /* Failure-detection test hooks (host-side injection; nothing faults).  The
  * next launch of the named tensor-core GEMM makes every CTA wait `polls`
  * polls (1..2^20) on an mbarrier that nothing arrives at, before it has
