@@ -18,7 +18,8 @@ f resident in HBM (CUDA events on the launching stream, L2 flushed between
 steps), `plain` the same for the plain step; `e2e` times the surrogate steps
 through the C ABI with the distribution copied host->device before and
 device->host after every step; `accuracy` compares the step's projected Q with
-the FP32 pair kernel's on the same cells, per cell, and (from the CPU-baseline
+that of the general FP32 kernels (no code in common with the timed ones) on the same
+cells, per cell, and (from the CPU-baseline
 leg, where the oracle runs) with the oracle's FP64 path on the first cells;
 `roofline` covers the plain gain kernel (tensor pipe for the collision
 matrices, measured FP32 FMA peak for the pair-product kernels); `cpu_baseline`
@@ -365,10 +366,11 @@ def run_ours(args):
     peak = peaks(gd, local)
     roof = gain_roofline(args.gain, ctx, f0, nc, stream, flush, peak, max(2, args.steps))
 
-    # accuracy: projected Q of one evaluation on the timed cells against the
-    # FP32 pair kernel's (the reference's arithmetic) on the same cells, per
-    # cell; and, in the CPU-baseline leg, against the oracle's FP64 path
+    # accuracy: projected Q of one evaluation on the timed cells against that of the
+    # general FP32 pair and loss kernels (the reference's arithmetic) on the same cells,
+    # per cell; and, in the CPU-baseline leg, against the oracle's FP64 path
     ref_ctx = gd.Context(spec, device=local)
+    ref_ctx.use_general_kernels()
     q_ref, _ = projected_q(gd, ref_ctx, f0, nc)
     ref_ctx.close()
     q_plain, _ = projected_q(gd, ctx, f0, nc)
@@ -393,7 +395,7 @@ def run_ours(args):
             "plain": {"value": plain_value, "unit": UNIT, "ms_per_step": ms_plain / args.steps,
                       "gain": args.gain, "clocks": clk_plain.summary(),
                       "accuracy": cell_stats(gd, ctx, q_plain, q_ref, nc)}}
-    n_loss, n_gain = path_launches(args.gain, ctx)
+    n_loss, n_gain = path_launches(args.gain, ctx, nc)
     if model is None:
         # per plain step: loss, gain, projection, max, dt, relaxation
         line["gpu_launches"] = (n_loss + n_gain + 4) * args.steps
@@ -403,13 +405,13 @@ def run_ours(args):
         # loss, error network 8, selection 1, projection 1, relaxation 3; then
         # either the plain gain in place when every cell falls back, or the
         # network 8 and nu f 1, plus gather 1, plain gain and scatter 1 when some do
-        line["gpu_launches"] = sum(n_loss + 13 + (n_gain if k == nc else 9 + (n_gain + 2 if k > 0 else 0))
+        line["gpu_launches"] = sum(n_loss + 13 + (n_gain if k == nc else 9 + (path_launches(args.gain, ctx, k)[1] + 2 if k > 0 else 0))
                                    for k in fb_timed)
         rep, q_main = surrogate_report(args, gd, ctx, model, f0, nc, stream, fit_s, fb_timed, plain_value, q_ref)
         rep["speedup_vs_plain"] = value / plain_value
         line["accuracy"] = next(c for c in rep["tolerance_curve"] if c["tol"] == args.tol)
         line["surrogate"] = rep
-    line["accuracy"]["reference"] = "FP32 pair kernel + FP64 projection on the same cells"
+    line["accuracy"]["reference"] = "general FP32 pair and loss kernels + FP64 projection on the same cells"
     alts = {}
     if rank == 0 and world == 1:
         alts = alternatives(args, ctx, f0, nc, stream, flush, peak, q_ref)
@@ -439,14 +441,14 @@ def fp32_gain(name, ctx):
     return name in ("pair", "pair_tc") or (name == "bf16x3" and ctx._info()["cmatrix_tiles"] == 0)
 
 
-def path_launches(name, ctx):
-    """Kernel launches of the loss and of the gain on a gain path: the FP32
-    loss kernel, or with the collision matrices the BF16 conversion of f and one
-    tensor-core GEMM; the packing of f, the FP32 gain kernel and its chunk
-    reduction (on the tensor-core paths that it serves after the cells'
-    scales), or the conversion of f and the collision-matrix kernel."""
+def path_launches(name, ctx, cells):
+    """Kernel launches of the loss and of the gain of that many cells on a gain
+    path: the FP32 loss kernel, or with the collision matrices the BF16 conversion of f
+    and one tensor-core GEMM; per slice of cells their scales, the packing of f, the
+    FP32 gain kernel and the sum of its parts, or the conversion of f and the
+    collision-matrix kernel."""
     if fp32_gain(name, ctx):
-        return 1, 3 if name == "pair" else 4
+        return 1, ctx.gain_work(cells)[1]
     if name == "pair_tc":
         return 2, 3
     return 2, 2
@@ -575,16 +577,15 @@ def time_gain(ctx, f0, nc, stream, flush, reps):
 def gain_roofline(name, ctx, f0, nc, stream, flush, peak, reps):
     """Throughput of the gain launch against its bounding pipe: the BF16
     tensor peak for the collision-matrix kernel (FLOP of the tiles issued),
-    the measured FP32 FMA peak for the pair-product kernel (algorithmic
-    FLOP of the pair-product formulation)."""
+    the measured FP32 FMA peak for the pair-product kernel (the FLOP that it
+    executes)."""
     g_avg = time_gain(ctx, f0, nc, stream, flush, reps)
     traffic, traffic_src = None, None
     if fp32_gain(name, ctx):
-        inf = ctx.info
-        flop = nc * (7 * inf["pair_products"] + 2 * inf["contraction_terms"] + inf["scatter_terms"])
-        kernel = "orbit_gain_kernel (+ packing of f, chunk reduction)"
-        work = "7 FLOP per pair product + 2 per nonzero-weight term + 1 per scatter update, over the class boxes " \
-            "(the kernel leaves out what lies outside the sphere: at 20^3 two thirds of them)"
+        flop = nc * ctx.gain_work(nc)[0]
+        kernel = "orbit_gain_kernel (+ scales and packing of f, sums of the parts)"
+        work = "FP32 FLOP executed, padding not counted: products in the sphere, 2 per nonzero-weight term of " \
+            "a present product, 1 per output update"
         bound, pk, src = "fp32", peak["fp32"], peak["fma_source"]
     else:
         # stored tiles: the nonzero 256 x 64 tiles of each G_i's block upper
@@ -738,9 +739,8 @@ def run_kernels(args):
         return e
 
     k = {}
-    k["folded_loss_kernel (FP32)"] = entry(ms["loss_fp32"], flop=2.0 * n * n / 8 * nc, fpeak=pk["fp32"],
-                                           work="n^2 / 4 FLOP per cell (one FMA per pair of orbits and character of "
-                                                "the reflections), vs the FP32 FMA peak")
+    k["orbit_loss_kernel (FP32)"] = entry(ms["loss_fp32"], flop=2.0 * n * n * nc, fpeak=pk["fp32"],
+                                          work="2 n^2 FLOP per cell (one FMA per partner), vs the FP32 FMA peak")
     if "loss_tc" in ms:
         rows, cols, kk = -(-n // 128) * 128, -(-nc // 128) * 128, -(-n // 64) * 64
         k["convert + gemm3_nt_kernel (loss on tensor cores)"] = entry(

@@ -154,6 +154,7 @@ def lib():
     L.gd_pair_tc_table.argtypes = [vp, P(C.c_int64), vp, vp, vp]
     L.gd_ctx_inject_timeout.argtypes = [vp, i]
     L.gd_ctx_use_general_kernels.argtypes = [vp]
+    L.gd_gain_work.argtypes = [vp, i, P(C.c_double), P(i)]
     L.gd_mlp_inject_late_timeout.argtypes = L.gd_ctx_inject_late_timeout.argtypes = [vp, i]
     for name in ("gd_grid_count", "gd_grid_fill", "gd_ctx_create", "gd_ctx_destroy", "gd_ctx_info",
                  "gd_export_tables", "gd_correction_basis", "gd_collision", "gd_project",
@@ -166,7 +167,8 @@ def lib():
                  "gd_cmatrix_check", "gd_batch_create", "gd_batch_destroy", "gd_batch_add", "gd_batch_step",
                  "gd_batch_check", "gd_batch_info", "gd_batch_set_mode", "gd_ctx_autotune", "gd_fma_peak",
                  "gd_mlp_inject_timeout", "gd_ctx_inject_timeout", "gd_mlp_inject_late_timeout",
-                 "gd_ctx_inject_late_timeout", "gd_ctx_use_general_kernels", "gd_pair_tables", "gd_pair_tc_table"):
+                 "gd_ctx_inject_late_timeout", "gd_ctx_use_general_kernels", "gd_gain_work",
+                 "gd_pair_tables", "gd_pair_tc_table"):
         getattr(L, name).restype = i
     _lib = L
     return L
@@ -352,6 +354,12 @@ class Context:
         _check(lib().gd_pair_tc_table(self._h, C.byref(rows), out["wrow"].ctypes.data, out["wh"].ctypes.data,
                                       out["wl"].ctypes.data))
         return out
+
+    def gain_work(self, ncells: int):
+        """The FP32 gain kernel's operations per cell and its launches for ncells."""
+        flop, launches = C.c_double(), C.c_int()
+        _check(lib().gd_gain_work(self._h, int(ncells), C.byref(flop), C.byref(launches)))
+        return flop.value, launches.value
 
     def use_general_kernels(self):
         """Test hook: loss and gain by the kernels that serve lattices of more than 1024

@@ -507,6 +507,17 @@ int gd_ctx_set_gain_path(gd_ctx *ctx, int path)
     return GD_OK;
 }
 
+int gd_gain_work(gd_ctx *ctx, int ncells, double *flop_per_cell, int *launches)
+{
+    if (!ctx || !flop_per_cell || !launches) return set_error(GD_ERR_INVALID_ARG, "NULL argument");
+    if (ncells < 1) return set_error(GD_ERR_INVALID_ARG, "ncells must be >= 1");
+    const gd::Context &c = ctx->c;
+    *flop_per_cell = c.orbit ? c.orbit->flop
+                             : 7.0 * c.pair_products + 2.0 * c.contraction_terms + (double)c.scatter_terms;
+    *launches = c.orbit ? gd::orbit_launches(c, ncells) : 2;
+    return GD_OK;
+}
+
 int gd_ctx_use_general_kernels(gd_ctx *ctx)
 {
     const int rc = gd_ctx_set_gain_path(ctx, GD_GAIN_PAIR);

@@ -63,6 +63,7 @@ struct OrbitGain {
     int cpt = 8, nslot = 0, norb = 0, pcap = 0, mcap = 0, nsteps = 0;
     uint32_t p_at = 0, zero_at = 0;  // shared-memory offsets of the P rows and of the zero C row
     size_t smem = 0, stream_bytes = 0;
+    double flop = 0.0;                // executed per cell, padding not counted
     int nparts = 0;                   // parts of the walk: each is summed by itself, in any batch
     std::vector<int> cuts;            // steps between which the walk may be cut (no D continues)
     std::vector<double> cost_prefix;  // work before each cut
@@ -230,6 +231,7 @@ size_t orbit_bytes(const Context &c, int ncells);
 int orbit_slice(const Context &c, int ncells, size_t room);
 int launch_orbit(Context &c, const float *f, int ncells, int ld, float *gain, void *buf, cudaStream_t st);
 int run_orbit(Context &c, const float *f, int ncells, int ld, float *gain, cudaStream_t st);
+int orbit_launches(const Context &c, int ncells);
 bool orbit_serves(const Context &c, int path);  // whether run_orbit computes this path's gain
 // reads (synchronising st) and clears its pipeline time-out record
 int orbit_take_timeout(Context &c, cudaStream_t st, bool *timed_out);

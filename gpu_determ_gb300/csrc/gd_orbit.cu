@@ -772,7 +772,12 @@ int orbit_build(Context &c)
         return set_error(GD_ERR_OUT_OF_MEMORY, "host memory for the gain tables");
     int mmax = 0;
     int64_t ktotal = 0;
+    double flop = 0.0;  // of a cell: a D stands for its distinct reflections
     for (const DItem &it : items) {
+        int64_t ops = (int64_t)it.targets.size();
+        for (const auto &pw : it.prod) ops += 2 * pw[8] - 1;
+        for (const float4 &v : it.w) ops += 2 * ((v.x != 0.f) + (v.y != 0.f) + (v.z != 0.f) + (v.w != 0.f));
+        if (it.nblk) flop += (double)ops * (8 >> __builtin_popcount(it.self));
         ktotal += it.K;
         mmax = std::max(mmax, it.nblk * kORows);
     }
@@ -999,6 +1004,7 @@ int orbit_build(Context &c)
         rest.swap(left);
     }
     og->cpt = cpt;
+    og->flop = flop;
     og->nslot = nslot;
     og->norb = norb;
     og->pcap = pcap;
@@ -1118,6 +1124,13 @@ int run_orbit(Context &c, const float *f, int ncells, int ld, float *gain, cudaS
     for (int at = 0; at < ncells && !rc; at += slice)
         rc = launch_orbit(c, f + at, std::min(slice, ncells - at), ld, gain + at, c.scratch.ptr, st);
     return rc;
+}
+
+// Launches of run_orbit for a batch.
+int orbit_launches(const Context &c, int ncells)
+{
+    const int slice = orbit_slice(c, ncells, kOScratch);
+    return (c.orbit->nparts > 1 ? 4 : 3) * ((ncells + slice - 1) / slice);
 }
 
 int orbit_take_timeout(Context &c, cudaStream_t st, bool *timed_out)

@@ -426,6 +426,11 @@ int gd_pair_tables(gd_ctx *ctx, gd_pair_table_sizes *sizes, int *grp_row_off, in
                    int *item_off, int *items, uint32_t *members);
 int gd_pair_tc_table(gd_ctx *ctx, int64_t *rows, int *wrow, uint16_t *wh, uint16_t *wl);
 
+/* FP32 operations per cell that the FP32 gain kernel of this context executes (padding
+ * not counted; gd_ctx_info counts the pair sums' whole class boxes) and its kernel
+ * launches for a batch of ncells. */
+int gd_gain_work(gd_ctx *ctx, int ncells, double *flop_per_cell, int *launches);
+
 /* Test hook: drops the context's tables by orbits of the lattice's reflections.  From
  * then on its loss and gain come from the kernels that serve the lattices of more than
  * 1024 orbits (and from the collision matrices), whatever its size; the gain path is

@@ -52,3 +52,18 @@ def test_timed_out_wait_of_the_fp32_gain_is_reported_once(cuda, gdlib, cells, la
     with pytest.raises(gdlib.GDError) as e:
         ctx.inject_timeout(256)
     assert e.value.code == 4
+
+
+@pytest.mark.parametrize("dims,R", [((2, 2, 2), 16.5), ((4, 2, 6), 16.5), ((12, 12, 12), 4.8)])
+def test_gain_work(cuda, gdlib, dims, R):
+    """The executed operations are at most those of the whole class boxes, and at
+    least one update for every pair of in-sphere nodes (its pair sum's shell holds the
+    pair itself); a batch beyond a launch's scratch takes more launches."""
+    ctx = gdlib.Context(gdlib.GridSpec(*dims, R=R))
+    flop, launches = ctx.gain_work(8)
+    i = ctx.info
+    assert ctx.n_pnt ** 2 <= flop <= 7 * i["pair_products"] + 2 * i["contraction_terms"] + i["scatter_terms"]
+    assert launches in (3, 4) and ctx.gain_work(1)[1] == launches
+    assert ctx.gain_work(1 << 28)[1] > launches
+    ctx.use_general_kernels()
+    assert ctx.gain_work(8)[0] >= flop
