@@ -44,8 +44,9 @@
 // 22.6 -> 3.83 ms; 20^3 (R = 4.8), one cell 10.5 -> 0.18 ms, 4096 cells 70.6 ms
 // (as many parts as the batch needs to fill the chip: 1.28, 3.79, 0.18 and 67.2 ms,
 // but other bits in other batches);
-// its error against FP64 is half as large (two-level sums: targets of a step,
-// then steps).  Measured and not better: 8, 12, 20 or 24 warps; groups of eight
+// its error against FP64 is a third to a half as large (relative L2 of the gain 6.0e-8
+// against 1.8e-7 at 20^3, 6.3e-8 against 1.27e-7 in the 16^3 box: sums of the targets
+// of a step, then of steps, then of parts).  Measured and not better: 8, 12, 20 or 24 warps; groups of eight
 // slots with one target a round (73.4 ms at 20^3); chunk-free dense streams (78 ms:
 // a check per record costs more than the padding).
 #include "gd_internal.h"
@@ -1105,12 +1106,12 @@ int launch_orbit(Context &c, const float *f, int ncells, int ld, float *gain, vo
 
 // The tensor-core gain paths whose gain this kernel computes: it is the faster
 // one, with a smaller error against FP64, on all but the smallest lattices.
-// Measured against the BF16x3 matrices (ms; R = 4.8, 4096 cells unless said): 12^3
-// 3.57 / 5.35 (one cell 0.03 / 0.28), 16^3 (1024 cells) 4.1 / 9.5, 20^3 67 / 208,
-// 24^3 (512 cells) 35 / 107, 8^3 whole box (512 nodes) 1.16 / 1.38; 10^3 (480 nodes)
-// 1.42 / 1.37 and 8^3 (208 nodes) 0.57 / 0.35, where the matrices stay.  Against
-// pair_tc_kernel it wins wherever it exists: 4^3 0.06 / 0.49, 8^3 0.57 / 5.5, 24^3
-// (512 cells) 35 / 168.
+// Measured against the BF16x3 matrices (ms of gain; R = 4.8, 4096 cells unless said):
+// 12^3 3.82 / 5.21 (one cell 0.060 / 0.057), 16^3 (1024 cells) 4.3 / 9.2, 20^3 (1024)
+// 17.8 / 50.7, 24^3 (512) 36 / 107, 10^3 (R = 5.2, 624 nodes) 2.13 / 2.58, 8^3 whole box
+// (512 nodes) 1.26 / 1.37; 10^3 (480 nodes) 1.53 / 1.35 and 8^3 (208 nodes) 0.61 / 0.34,
+// where the matrices stay.  Against pair_tc_kernel it wins wherever it exists: 4^3 0.06
+// / 0.50, 8^3 0.61 / 5.6, 24^3 (512 cells) 36 / 168.
 bool orbit_serves(const Context &c, int path)
 {
     return c.orbit && (path == GD_GAIN_PAIR_TC || (path == GD_GAIN_CMATRIX_BF16X3 && c.d.n_pnt >= kOMatrixNodes));
