@@ -434,7 +434,8 @@ int gd_gain_work(gd_ctx *ctx, int ncells, double *flop_per_cell, int *launches);
 /* Test hook: drops the context's tables by orbits of the lattice's reflections.  From
  * then on its loss and gain come from the kernels that serve the lattices of more than
  * 1024 orbits (and from the collision matrices), whatever its size; the gain path is
- * GD_GAIN_PAIR again. */
+ * GD_GAIN_PAIR again.  Call it on a new context: a captured step of a batch that the
+ * context is in still refers to the tables. */
 int gd_ctx_use_general_kernels(gd_ctx *ctx);
 
 /* Failure-detection test hooks (host-side injection; nothing faults).  The
